@@ -54,6 +54,22 @@ def test_unaligned_surfaces_take_narrower_words(torch, orientation):
 
 
 @pytest.mark.parametrize("orientation", range(8))
+@pytest.mark.parametrize("pixel_bytes,offsets", [(1, (0, 1, 3)), (2, (0, 2)), (3, (0, 1, 2, 3)), (4, (0, 4)), (6, (0, 2)),
+                                                 (8, (4,)), (12, (0,)), (16, (4,))])
+def test_pixel_kernels_at_tile_edges(torch, orientation, pixel_bytes, offsets):
+    """One row or column, one less and one more than a tile (64 or 32 pixels)
+    and several tiles, on surfaces that start at every byte of a word."""
+    rng = np.random.default_rng(pixel_bytes * 64 + orientation)
+    for width, height in [(1, 70), (67, 1), (31, 33), (63, 65), (64, 64), (129, 62), (200, 131)]:
+        src = rng.integers(0, 256, width * height * pixel_bytes, dtype=np.uint8)
+        rc, want = O.orient(src, width, height, pixel_bytes, orientation)
+        assert rc == 0
+        for offset in offsets:
+            got = gpu_orient(torch, src, width, height, pixel_bytes, orientation, offset)
+            assert np.array_equal(got, want), (width, height, offset)
+
+
+@pytest.mark.parametrize("orientation", range(8))
 def test_bit_packed_orientation_matches_the_oracle(torch, orientation):
     rng = np.random.default_rng(orientation)
     for width, height in [(3, 2), (9, 17), (70, 33)]:
