@@ -9,15 +9,19 @@
 // schedule for 4:2:0 / 4:2:2 chroma), the forward transform of each
 // macroblock's block DCs (halved first where the plane is scaled), and the
 // quantization of the DC, low-pass and high-pass bands (Quantizer::quantize,
-// crates/jxr-math/src/quantization.rs:28-50).  Here each stage is a kernel
-// over the plane: the overlap operators of one level are disjoint (the
-// subsampled corners aside, which run in three ordered phases as in the
-// decoder), so every operator, block and macroblock is its own work item.
-// The results equal the CPU analysis bit for bit.
+// crates/jxr-math/src/quantization.rs:28-50).  Here a plane takes two passes:
+// the second-level prefilter in place, then everything from the block
+// transforms to the quantized bands; overlap mode 2 takes the first-level
+// prefilter and the low-pass bands in kernels of their own after that.  The
+// overlap operators of one level are disjoint (the subsampled corners aside,
+// which run in three ordered phases as in the decoder), so every operator,
+// block and macroblock is its own work item.  The results equal the CPU
+// analysis bit for bit.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
+#include <cstring>
 #include <vector>
 
 #include "../../include/jxr_b200.h"
@@ -32,20 +36,65 @@ namespace {
 
 using namespace jxr::fwd;
 
+// Division by a step that does not change, as a multiplication and shifts
+// exact for every 32-bit dividend (Granlund and Montgomery, "Division by
+// invariant integers using multiplication", 1994, figure 4.1).
+struct Divider {
+    uint32_t mul, offset;      // multiplier; the rounding offset added before the division
+    uint32_t shift1, shift2;
+};
+
 // One plane on the device.  `starts` maps mark the macroblock columns / rows
-// where a hard tile begins (all zero with soft tiles).
+// where a hard tile begins (planes with soft tiles have none).  Maps and
+// region lists are at byte offsets of the set's blob.
 struct APlane {
     int32_t *samples;          // W x H, prefiltered in place
-    int32_t *low;              // block DCs, (W/4) x (H/4)
+    int32_t *low;              // block DCs, (W/4) x (H/4): overlap mode 2
     int32_t *low_q;            // 16 a macroblock
     int32_t *high_q;           // 256 a macroblock
-    const uint8_t *col_start, *row_start;
-    const uint32_t *cols;      // column region boundaries in macroblocks (0 .. mbs_x)
+    uint32_t col_at, row_at;   // tile-start maps
+    uint32_t cols_at;          // column region boundaries in macroblocks (0 .. mbs_x)
     uint32_t ncols;
     uint32_t W, H, mbs_x, mbs_y;
     int32_t bc, br, scale2, overlap, hard;
-    uint32_t q[3];
+    int32_t wide;              // outputs 16-byte aligned, block DCs 8-byte aligned
+    Divider q[3];              // DC, low-pass, high-pass
 };
+
+// The planes of a call.  A few planes (a picture's) travel in the kernels'
+// parameters; more of them, or longer tile lists, in device memory.
+constexpr uint32_t kInlinePlanes = 8, kInlineBlob = 2560;
+struct ASet {
+    const APlane *planes_mem;  // null: the planes and the blob below
+    const uint8_t *blob_mem;
+    APlane planes[kInlinePlanes];
+    uint32_t blob[kInlineBlob / 4];
+};
+static_assert(sizeof(ASet) <= 4096, "kernel parameters");
+
+__device__ __forceinline__ const APlane &plane_of(const ASet &s) {
+    return s.planes_mem ? s.planes_mem[blockIdx.y] : s.planes[blockIdx.y];
+}
+__device__ __forceinline__ const uint8_t *blob_of(const ASet &s) {
+    return s.planes_mem ? s.blob_mem : reinterpret_cast<const uint8_t *>(s.blob);
+}
+
+// quantize() of forward.h: (|c| + offset) / step.  The offset is at most half
+// the step, so the sum stays below 2^32.
+__device__ __forceinline__ int32_t quantized(int32_t c, const Divider &d) {
+    const uint32_t n = (c < 0 ? 0u - (uint32_t)c : (uint32_t)c) + d.offset;
+    const uint32_t t = __umulhi(d.mul, n);
+    const uint32_t q = (t + ((n - t) >> d.shift1)) >> d.shift2;
+    return c < 0 ? (int32_t)(0u - q) : (int32_t)q;
+}
+
+__device__ __forceinline__ void store4(int32_t *p, bool wide, int32_t a, int32_t b, int32_t c, int32_t d) {
+    if (wide) {
+        *reinterpret_cast<int4 *>(p) = make_int4(a, b, c, d);
+    } else {
+        p[0] = a; p[1] = b; p[2] = c; p[3] = d;
+    }
+}
 
 __device__ __forceinline__ bool boundary(int p, int extent, int lg, int hard, const uint8_t *starts) {
     if (p <= 0 || p >= extent) return true;
@@ -58,9 +107,11 @@ __device__ __forceinline__ int log2i(int v) { return 31 - __clz(v); }
 // macroblocks are 2^lx x 2^ly of them, run forward: one 4x4 cell a thread,
 // cells at origins 2 (mod 4); a cell a region boundary crosses takes the
 // edge strips or corner quarters (the decoder's window list, forward
-// operators; crates/jxr-native/src/reconstruct/overlap.rs:124-323).
+// operators; crates/jxr-native/src/reconstruct/overlap.rs:124-323).  A window
+// starts two values past a 16-byte boundary: with `pairs` (values 8-byte
+// aligned, W even) its rows move as two 8-byte pieces each.
 __device__ void prefilter_cells(int32_t *s, int W, int H, int lx, int ly, int hard, const uint8_t *col_start,
-                                const uint8_t *row_start) {
+                                const uint8_t *row_start, bool pairs) {
     const int ncx = W / 4 + 1, ncy = H / 4 + 1;
     auto at = [&](int x, int y) -> int32_t & { return s[(size_t)y * W + x]; };
     auto inside = [&](int x, int y) { return x >= 0 && x < W && y >= 0 && y < H; };
@@ -69,6 +120,23 @@ __device__ void prefilter_cells(int32_t *s, int W, int H, int lx, int ly, int ha
         const bool vs = boundary(cx + 2, W, lx, hard, col_start), hs = boundary(cy + 2, H, ly, hard, row_start);
         if (!vs && !hs) {
             int32_t v[16];
+            if (pairs) {
+#pragma unroll
+                for (int r = 0; r < 4; r++)
+#pragma unroll
+                    for (int c = 0; c < 4; c += 2) {
+                        const int2 q = *reinterpret_cast<const int2 *>(&at(cx + c, cy + r));
+                        v[r * 4 + c] = q.x;
+                        v[r * 4 + c + 1] = q.y;
+                    }
+                forward_pot4x4(v);
+#pragma unroll
+                for (int r = 0; r < 4; r++)
+#pragma unroll
+                    for (int c = 0; c < 4; c += 2)
+                        *reinterpret_cast<int2 *>(&at(cx + c, cy + r)) = make_int2(v[r * 4 + c], v[r * 4 + c + 1]);
+                continue;
+            }
 #pragma unroll
             for (int r = 0; r < 4; r++)
 #pragma unroll
@@ -93,41 +161,117 @@ __device__ void prefilter_cells(int32_t *s, int W, int H, int lx, int ly, int ha
     }
 }
 
-__global__ void __launch_bounds__(256) jxrb_analysis_prefilter(const APlane *__restrict__ planes) {
-    const APlane &p = planes[blockIdx.y];
+__global__ void __launch_bounds__(256) jxrb_analysis_prefilter(const __grid_constant__ ASet set) {
+    const APlane &p = plane_of(set);
     if (p.overlap < 1) return;
-    prefilter_cells(p.samples, (int)p.W, (int)p.H, log2i(p.bc * 4), log2i(p.br * 4), p.hard, p.col_start, p.row_start);
+    const uint8_t *blob = blob_of(set);
+    prefilter_cells(p.samples, (int)p.W, (int)p.H, log2i(p.bc * 4), log2i(p.br * 4), p.hard, blob + p.col_at,
+                    blob + p.row_at, true);
 }
 
-// Forward core transform of every block: its DC into the block-DC plane, its
-// other fifteen coefficients into the block's slot of the high-pass output
-// (quantized later).
-__global__ void __launch_bounds__(256) jxrb_analysis_blocks(const APlane *__restrict__ planes) {
-    const APlane &p = planes[blockIdx.y];
-    const uint32_t lw = p.W / 4, n = lw * (p.H / 4);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t bx = i % lw, by = i / lw;
-        int32_t v[16];
+// A macroblock's block DCs (raster in l; halved where the plane is scaled)
+// through the forward first-level transform, quantized, to its 16 low-pass
+// places (analyze.rs:88-131).
+__device__ __forceinline__ void analyze_low(const APlane &p, int32_t (&l)[16], uint32_t m) {
+    const int count = p.bc * p.br;
 #pragma unroll
-        for (int r = 0; r < 4; r++) {
-            const int4 q = *reinterpret_cast<const int4 *>(&p.samples[((size_t)by * 4 + r) * p.W + bx * 4]);
-            v[r * 4] = q.x; v[r * 4 + 1] = q.y; v[r * 4 + 2] = q.z; v[r * 4 + 3] = q.w;
+    for (int k = 0; k < 16; k++) l[k] = k < count ? (p.scale2 ? l[k] >> 1 : l[k]) : 0;
+    if (count == 16) {
+        forward_pct(l);
+    } else if (count == 4) {
+        int32_t w[4] = {l[0], l[1], l[2], l[3]};
+        forward_420(w);
+#pragma unroll
+        for (int k = 0; k < 4; k++) l[k] = w[k];
+    } else {
+        int32_t w[8] = {l[0], l[1], l[2], l[3], l[4], l[5], l[6], l[7]};
+        forward_422(w);
+#pragma unroll
+        for (int k = 0; k < 8; k++) l[k] = w[k];
+    }
+    l[0] = quantized(l[0], p.q[0]);
+#pragma unroll
+    for (int k = 1; k < 16; k++) l[k] = k < count ? quantized(l[k], p.q[1]) : 0;
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) store4(p.low_q + (size_t)m * 16 + k, p.wide, l[k], l[k + 1], l[k + 2], l[k + 3]);
+}
+
+// Forward core transform of every block, its fifteen coefficients quantized
+// (rounding offsets of half the step for DC and low-pass, a third for
+// high-pass), and, without a first-level prefilter, its macroblock's low-pass
+// band; overlap mode 2 writes the block DCs for the kernels below instead.
+//
+// One block a thread, the 256 blocks of 16 (full resolution), 32 or 64
+// macroblocks a CTA: threads take blocks along a block row, so that a warp
+// reads 512-byte row pieces, and the coefficients leave through shared memory
+// as the run of whole macroblocks they are in the output.  Memory traffic is
+// what bounds it: the separate transform and one-macroblock-a-thread
+// quantization kernels wrote 4-byte words 64 bytes and 1 KB apart (three
+// planes of a 2048 x 1536 4:2:0 picture, cold caches: 32 + 89 us, 18.7 us
+// here).
+constexpr int kBlocks = 256;
+__global__ void __launch_bounds__(kBlocks) jxrb_analysis_blocks(const __grid_constant__ ASet set) {
+    __shared__ __align__(16) int32_t coded[kBlocks * 16];
+    __shared__ int32_t dcs[kBlocks + 64];
+    const APlane &p = plane_of(set);
+    const int bc = p.bc, count = bc * p.br, lcount = log2i(count), n = kBlocks >> lcount;
+    const uint32_t mbs = p.mbs_x * p.mbs_y;
+    const int t = threadIdx.x;
+    const int across = n * bc, r = t / across, c = t % across;   // powers of two
+    const int i = c / bc, col = c % bc, s = i * count + r * bc + col;
+    // piece q of slot s sits at q ^ swizzle(s): the threads of a quarter-warp
+    // then write to distinct bank groups at every block shape
+    auto swizzle = [](int slot) { return ((slot >> 1) ^ (slot >> 3)) & 3; };
+    for (uint32_t first = blockIdx.x * n; first < mbs; first += gridDim.x * n) {
+        const uint32_t m = first + i;
+        if (m < mbs) {
+            const uint32_t my = m / p.mbs_x, mx = m - my * p.mbs_x;
+            const uint32_t by = my * p.br + r, bx = mx * bc + col;
+            const int32_t *from = p.samples + (size_t)by * 4 * p.W + bx * 4;
+            int32_t v[16];
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const int4 q = *reinterpret_cast<const int4 *>(from + (size_t)k * p.W);
+                v[k * 4] = q.x; v[k * 4 + 1] = q.y; v[k * 4 + 2] = q.z; v[k * 4 + 3] = q.w;
+            }
+            forward_pct(v);
+            if (p.overlap == 2) p.low[(size_t)by * (p.W / 4) + bx] = v[0];
+            else dcs[i * (count + 1) + r * bc + col] = v[0];
+            v[0] = 0;
+            const Divider d = p.q[2];
+#pragma unroll
+            for (int k = 1; k < 16; k++) v[k] = quantized(v[k], d);
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                *reinterpret_cast<int4 *>(&coded[s * 16 + ((k ^ swizzle(s)) << 2)]) =
+                    make_int4(v[k * 4], v[k * 4 + 1], v[k * 4 + 2], v[k * 4 + 3]);
         }
-        forward_pct(v);
-        p.low[i] = v[0];
-        const uint32_t m = (by / p.br) * p.mbs_x + bx / p.bc, b = (by % p.br) * p.bc + bx % p.bc;
-        int32_t *h = p.high_q + (size_t)m * 256 + b * 16;
-        h[0] = 0;
+        __syncthreads();
+        // past the macroblock's block count its places are zero
+        const uint32_t held = min((uint32_t)n, mbs - first);
+        int32_t *to = p.high_q + (size_t)first * 256;
+        for (uint32_t k = t; k < held * 64; k += kBlocks) {
+            const int b = (k & 63) >> 2, slot = (int)(k >> 6) * count + b;
+            const int4 q = b < count ? *reinterpret_cast<const int4 *>(&coded[slot * 16 + (((k & 3) ^ swizzle(slot)) << 2)])
+                                     : make_int4(0, 0, 0, 0);
+            store4(to + k * 4, p.wide, q.x, q.y, q.z, q.w);
+        }
+        if (p.overlap != 2 && t < (int)held) {
+            int32_t l[16];
 #pragma unroll
-        for (int k = 1; k < 16; k++) h[k] = v[k];
+            for (int k = 0; k < 16; k++) l[k] = k < count ? dcs[t * (count + 1) + k] : 0;
+            analyze_low(p, l, first + t);
+        }
+        __syncthreads();
     }
 }
 
 // First-level prefilter of full-resolution planes: the cells of the block-DC plane.
-__global__ void __launch_bounds__(256) jxrb_analysis_low_full(const APlane *__restrict__ planes) {
-    const APlane &p = planes[blockIdx.y];
+__global__ void __launch_bounds__(256) jxrb_analysis_low_full(const __grid_constant__ ASet set) {
+    const APlane &p = plane_of(set);
     if (p.overlap != 2 || p.bc != 4) return;
-    prefilter_cells(p.low, (int)(p.W / 4), (int)(p.H / 4), 2, 2, p.hard, p.col_start, p.row_start);
+    const uint8_t *blob = blob_of(set);
+    prefilter_cells(p.low, (int)(p.W / 4), (int)(p.H / 4), 2, 2, p.hard, blob + p.col_at, blob + p.row_at, p.wide);
 }
 
 // First-level prefilter of subsampled chroma, the decoder's ordered schedule
@@ -136,15 +280,16 @@ __global__ void __launch_bounds__(256) jxrb_analysis_low_full(const APlane *__re
 // first); phase 1, every two-sample pair and 2x2 square forward; phase 2, the
 // corners regain their (now filtered) neighbour.  A region two samples wide
 // runs its four corner steps in that order as well.
-__global__ void __launch_bounds__(256) jxrb_analysis_low_subsampled(const APlane *__restrict__ planes, int phase) {
-    const APlane &p = planes[blockIdx.y];
+__global__ void __launch_bounds__(256) jxrb_analysis_low_subsampled(const __grid_constant__ ASet set, int phase) {
+    const APlane &p = plane_of(set);
     if (p.overlap != 2 || p.bc != 2) return;
+    const uint8_t *blob = blob_of(set);
     const int W = (int)(p.W / 4), H = (int)(p.H / 4);
     const int lx = log2i(p.bc), ly = log2i(p.br);
     int32_t *s = p.low;
     auto at = [&](int x, int y) -> int32_t & { return s[(size_t)y * W + x]; };
-    auto vb = [&](int x) { return boundary(x, W, lx, p.hard, p.col_start); };
-    auto hb = [&](int y) { return boundary(y, H, ly, p.hard, p.row_start); };
+    auto vb = [&](int x) { return boundary(x, W, lx, p.hard, blob + p.col_at); };
+    auto hb = [&](int y) { return boundary(y, H, ly, p.hard, blob + p.row_at); };
     if (phase == 1) {
         auto inside = [&](int x, int y) { return x >= 0 && x < W && y >= 0 && y < H; };
         const int ncx = W / 2 + 1, ncy = H / 2 + 1;
@@ -166,11 +311,12 @@ __global__ void __launch_bounds__(256) jxrb_analysis_low_subsampled(const APlane
     }
     // phases 0 and 2: one (boundary row, column region) a thread
     const int nreg = (int)p.ncols - 1;
+    const uint32_t *cols = reinterpret_cast<const uint32_t *>(blob + p.cols_at);
     for (int item = blockIdx.x * blockDim.x + threadIdx.x; item < H * nreg; item += gridDim.x * blockDim.x) {
         const int y = item / nreg, k = item % nreg;
         const bool top = hb(y), bottom = hb(y + 1);
         if (!top && !bottom) continue;
-        const int l = (int)p.cols[k] * p.bc, r = (int)p.cols[k + 1] * p.bc;
+        const int l = (int)cols[k] * p.bc, r = (int)cols[k + 1] * p.bc;
         int32_t &c0 = at(l, y), &n0 = at(l + 1, y), &c1 = at(r - 1, y), &n1 = at(r - 2, y);
         if (phase == 0) {
             c1 -= n1;
@@ -182,45 +328,29 @@ __global__ void __launch_bounds__(256) jxrb_analysis_low_subsampled(const APlane
     }
 }
 
-// Each macroblock's block DCs (halved where the plane is scaled) through the
-// forward first-level transform, and every band quantized (analyze.rs:88-131;
-// rounding offsets of half the step for DC and low-pass, a third for
-// high-pass).
-__global__ void __launch_bounds__(256) jxrb_analysis_quantize(const APlane *__restrict__ planes) {
-    const APlane &p = planes[blockIdx.y];
+// The low-pass bands of two-level planes from their filtered block DCs, one
+// macroblock a thread.
+__global__ void __launch_bounds__(256) jxrb_analysis_low_bands(const __grid_constant__ ASet set) {
+    const APlane &p = plane_of(set);
+    if (p.overlap != 2) return;
     const uint32_t n = p.mbs_x * p.mbs_y, lw = p.W / 4;
-    const int count = p.bc * p.br;
+    const int lbc = log2i(p.bc), count = p.bc * p.br;
     for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += gridDim.x * blockDim.x) {
         const uint32_t mx = m % p.mbs_x, my = m / p.mbs_x;
+        const int32_t *from = p.low + (size_t)my * p.br * lw + mx * p.bc;
         int32_t l[16];
 #pragma unroll
-        for (int k = 0; k < 16; k++) l[k] = 0;
-        for (int r = 0; r < p.br; r++)
-            for (int c = 0; c < p.bc; c++) l[r * p.bc + c] = p.low[((size_t)my * p.br + r) * lw + mx * p.bc + c];
-        if (p.scale2)
-            for (int k = 0; k < count; k++) l[k] >>= 1;
-        if (count == 16) {
-            forward_pct(l);
-        } else if (count == 4) {
-            int32_t w[4] = {l[0], l[1], l[2], l[3]};
-            forward_420(w);
-            for (int k = 0; k < 4; k++) l[k] = w[k];
-        } else {
-            int32_t w[8] = {l[0], l[1], l[2], l[3], l[4], l[5], l[6], l[7]};
-            forward_422(w);
-            for (int k = 0; k < 8; k++) l[k] = w[k];
-        }
-        int32_t *lq = p.low_q + (size_t)m * 16;
-        lq[0] = quantize(l[0], p.q[0], p.q[0] / 2);
-        for (int k = 1; k < 16; k++) lq[k] = k < count ? quantize(l[k], p.q[1], p.q[1] / 2) : 0;
-        int32_t *h = p.high_q + (size_t)m * 256;
-        for (int b = 0; b < 16; b++) {
-            // element 0 of each block is the block DC's place: zero (past the
-            // block count the whole block is zero)
-            h[b * 16] = 0;
-            for (int k = 1; k < 16; k++) h[b * 16 + k] = b < count ? quantize(h[b * 16 + k], p.q[2], p.q[2] / 3) : 0;
-        }
+        for (int k = 0; k < 16; k++) l[k] = k < count ? from[(size_t)(k >> lbc) * lw + (k & (p.bc - 1))] : 0;
+        analyze_low(p, l, m);
     }
+}
+
+Divider divider(uint32_t step, uint32_t offset) {
+    if (offset >= step) offset = step - 1;
+    int l = 0;
+    while (l < 32 && (1ull << l) < step) l++;
+    return Divider{(uint32_t)((((1ull << l) - step) << 32) / step + 1), offset, (uint32_t)std::min(l, 1),
+                   (uint32_t)std::max(l - 1, 0)};
 }
 
 unsigned grid_for(uint64_t work) {
@@ -233,13 +363,11 @@ extern "C" jxrb_status jxrb_analyze_planes(const jxrb_analysis_plane *planes, ui
     if (!planes || count == 0) return jxr::report_error(JXRB_INVALID_PLAN, "no planes");
     if (count > 65535) return jxr::report_error(JXRB_RESOURCE_LIMIT, "too many planes in one call");
     cudaStream_t stream = static_cast<cudaStream_t>(cuda_stream);
-    // descriptors, tile-start maps and region lists in one allocation
+    // descriptors, and the blob of tile-start maps and region lists
     std::vector<APlane> dev(count);
-    std::vector<uint8_t> maps;
-    std::vector<uint32_t> cols;
-    std::vector<size_t> map_at(count), cols_at(count);
-    uint64_t max_samples = 0, max_mbs = 0, max_rows = 0;
-    bool two_level = false, subsampled = false;
+    std::vector<uint8_t> blob;
+    uint64_t max_samples = 0, max_mbs = 0, max_rows = 0, max_groups = 0;
+    bool filtered = false, two_level = false, subsampled = false;
     for (uint32_t i = 0; i < count; i++) {
         const jxrb_analysis_plane &a = planes[i];
         const bool full = a.block_columns == 4 && a.block_rows == 4;
@@ -262,15 +390,6 @@ extern "C" jxrb_status jxrb_analyze_planes(const jxrb_analysis_plane *planes, ui
             if (cb[k] <= cb[k - 1]) return jxr::report_error(JXRB_INVALID_PLAN, "tile column boundaries");
         for (uint32_t k = 1; k < a.row_count; k++)
             if (rb[k] <= rb[k - 1]) return jxr::report_error(JXRB_INVALID_PLAN, "tile row boundaries");
-        map_at[i] = maps.size();
-        maps.resize(maps.size() + mbs_x + mbs_y + 2, 0);
-        if (a.hard_tiles) {
-            for (uint32_t k = 1; k + 1 < a.column_count; k++) maps[map_at[i] + cb[k]] = 1;
-            for (uint32_t k = 1; k + 1 < a.row_count; k++) maps[map_at[i] + mbs_x + 1 + rb[k]] = 1;
-        }
-        cols_at[i] = cols.size();
-        if (a.hard_tiles) cols.insert(cols.end(), cb, cb + a.column_count);
-        else { cols.push_back(0); cols.push_back(mbs_x); }
         APlane &d = dev[i];
         d.samples = a.samples;
         d.low = a.low_scratch;
@@ -286,49 +405,74 @@ extern "C" jxrb_status jxrb_analyze_planes(const jxrb_analysis_plane *planes, ui
         d.overlap = a.overlap;
         d.hard = a.hard_tiles ? 1 : 0;
         d.ncols = a.hard_tiles ? a.column_count : 2;
-        for (int b = 0; b < 3; b++) d.q[b] = a.steps[b];
+        for (int b = 0; b < 3; b++) d.q[b] = divider(a.steps[b], a.steps[b] / (b < 2 ? 2 : 3));
+        d.wide = ((reinterpret_cast<uintptr_t>(a.low_q) | reinterpret_cast<uintptr_t>(a.high_q)) & 15) == 0 &&
+                 (reinterpret_cast<uintptr_t>(a.low_scratch) & 7) == 0;
+        if (a.hard_tiles) {
+            d.col_at = (uint32_t)blob.size();
+            d.row_at = d.col_at + mbs_x + 1;
+            blob.resize(blob.size() + mbs_x + mbs_y + 2, 0);
+            for (uint32_t k = 1; k + 1 < a.column_count; k++) blob[d.col_at + cb[k]] = 1;
+            for (uint32_t k = 1; k + 1 < a.row_count; k++) blob[d.row_at + rb[k]] = 1;
+        }
+        if (a.overlap == 2 && !full) {
+            const uint32_t whole[2] = {0, mbs_x};
+            const uint32_t *list = a.hard_tiles ? cb : whole;
+            blob.resize((blob.size() + 3) / 4 * 4, 0);
+            d.cols_at = (uint32_t)blob.size();
+            blob.insert(blob.end(), reinterpret_cast<const uint8_t *>(list),
+                        reinterpret_cast<const uint8_t *>(list + d.ncols));
+        }
         max_samples = std::max<uint64_t>(max_samples, (uint64_t)a.width * a.height);
         max_mbs = std::max<uint64_t>(max_mbs, (uint64_t)mbs_x * mbs_y);
+        max_groups = std::max<uint64_t>(max_groups, ((uint64_t)a.width * a.height / 16 + kBlocks - 1) / kBlocks);
         max_rows = std::max<uint64_t>(max_rows, (uint64_t)(a.height / 4) * (d.ncols - 1));
+        filtered |= a.overlap >= 1;
         two_level |= a.overlap == 2;
         subsampled |= a.overlap == 2 && !full;
     }
-    const size_t desc_bytes = sizeof(APlane) * count, maps_at = (desc_bytes + 255) / 256 * 256;
-    const size_t cols_at0 = (maps_at + maps.size() + 15) / 16 * 16, total = cols_at0 + cols.size() * 4;
+    // A call of a few planes needs no device memory for them: allocating,
+    // copying and freeing it cost about as long as a small picture's kernels.
+    ASet set;
+    std::memset(&set, 0, sizeof set);
     void *mem = nullptr;
-    cudaError_t e = cudaMallocAsync(&mem, total, stream);
-    if (e != cudaSuccess) return jxr::report_cuda(e, "cudaMallocAsync (analysis descriptors)");
-    uint8_t *base = static_cast<uint8_t *>(mem);
-    for (uint32_t i = 0; i < count; i++) {
-        dev[i].col_start = base + maps_at + map_at[i];
-        dev[i].row_start = base + maps_at + map_at[i] + dev[i].mbs_x + 1;
-        dev[i].cols = reinterpret_cast<const uint32_t *>(base + cols_at0) + cols_at[i];
+    std::vector<uint8_t> host;
+    cudaError_t e = cudaSuccess;
+    if (count <= kInlinePlanes && blob.size() <= kInlineBlob) {
+        std::copy(dev.begin(), dev.end(), set.planes);
+        if (!blob.empty()) std::memcpy(set.blob, blob.data(), blob.size());
+    } else {
+        const size_t blob_at = (sizeof(APlane) * count + 255) / 256 * 256;
+        e = cudaMallocAsync(&mem, blob_at + blob.size(), stream);
+        if (e != cudaSuccess) return jxr::report_cuda(e, "cudaMallocAsync (analysis descriptors)");
+        host.assign(blob_at + blob.size(), 0);
+        std::memcpy(host.data(), dev.data(), sizeof(APlane) * count);
+        if (!blob.empty()) std::memcpy(host.data() + blob_at, blob.data(), blob.size());
+        set.planes_mem = static_cast<const APlane *>(mem);
+        set.blob_mem = static_cast<const uint8_t *>(mem) + blob_at;
+        e = cudaMemcpyAsync(mem, host.data(), host.size(), cudaMemcpyHostToDevice, stream);
     }
-    std::vector<uint8_t> host(total, 0);
-    std::copy(reinterpret_cast<const uint8_t *>(dev.data()), reinterpret_cast<const uint8_t *>(dev.data()) + desc_bytes,
-              host.begin());
-    std::copy(maps.begin(), maps.end(), host.begin() + maps_at);
-    std::copy(reinterpret_cast<const uint8_t *>(cols.data()), reinterpret_cast<const uint8_t *>(cols.data()) + cols.size() * 4,
-              host.begin() + cols_at0);
-    e = cudaMemcpyAsync(mem, host.data(), total, cudaMemcpyHostToDevice, stream);
-    const APlane *d = static_cast<const APlane *>(mem);
-    const dim3 g_cells(grid_for(max_samples / 16 + 64), count), g_blocks(grid_for(max_samples / 16), count);
+    const dim3 g_cells(grid_for(max_samples / 16 + 64), count);
+    const dim3 g_blocks((unsigned)std::min<uint64_t>(max_groups, 4096), count);
     const dim3 g_mbs(grid_for(max_mbs), count), g_rows(grid_for(max_rows), count);
     if (e == cudaSuccess) {
-        jxrb_analysis_prefilter<<<g_cells, 256, 0, stream>>>(d);
-        jxrb_analysis_blocks<<<g_blocks, 256, 0, stream>>>(d);
-        if (two_level) jxrb_analysis_low_full<<<g_cells, 256, 0, stream>>>(d);
-        if (subsampled) {
-            jxrb_analysis_low_subsampled<<<g_rows, 256, 0, stream>>>(d, 0);
-            jxrb_analysis_low_subsampled<<<g_cells, 256, 0, stream>>>(d, 1);
-            jxrb_analysis_low_subsampled<<<g_rows, 256, 0, stream>>>(d, 2);
+        if (filtered) jxrb_analysis_prefilter<<<g_cells, 256, 0, stream>>>(set);
+        jxrb_analysis_blocks<<<g_blocks, kBlocks, 0, stream>>>(set);
+        if (two_level) {
+            jxrb_analysis_low_full<<<g_cells, 256, 0, stream>>>(set);
+            if (subsampled) {
+                jxrb_analysis_low_subsampled<<<g_rows, 256, 0, stream>>>(set, 0);
+                jxrb_analysis_low_subsampled<<<g_cells, 256, 0, stream>>>(set, 1);
+                jxrb_analysis_low_subsampled<<<g_rows, 256, 0, stream>>>(set, 2);
+            }
+            jxrb_analysis_low_bands<<<g_mbs, 256, 0, stream>>>(set);
         }
-        jxrb_analysis_quantize<<<g_mbs, 256, 0, stream>>>(d);
         e = cudaGetLastError();
     }
-    // the host image of the descriptors is read by the copy: wait for it
+    // the outputs are written, and the host image of the descriptors read,
+    // once the stream has come this far
     const cudaError_t s = cudaStreamSynchronize(stream);
-    cudaFreeAsync(mem, stream);
+    if (mem) cudaFreeAsync(mem, stream);
     if (e != cudaSuccess) return jxr::report_cuda(e, "analysis launch");
     if (s != cudaSuccess) return jxr::report_cuda(s, "analysis");
     return JXRB_OK;

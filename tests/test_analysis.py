@@ -83,3 +83,34 @@ def test_gpu_analysis_of_a_large_plane_round_trips():
                          column_boundaries=cols, row_boundaries=rows)
     rc, back = O.reconstruct_plane(plane, threads=8)
     assert rc == 0 and np.array_equal(back, s)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("bc,br", SHAPES)
+@pytest.mark.parametrize("mx,my", [(1, 1), (15, 1), (16, 1), (17, 3), (33, 2), (64, 1), (65, 2)])
+def test_gpu_analysis_around_a_group_of_macroblocks(bc, br, mx, my):
+    """Planes of one macroblock less and more than the 16, 32 or 64 a CTA
+    takes, hard tiles, the widest and narrowest steps, and outputs that start
+    at any word: every coefficient equals the CPU analysis's, and nothing is
+    written past the outputs."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.fail("no B200 visible: the GPU tests need the CUDA engine")
+    cols, rows = ([0, mx // 2, mx] if mx > 1 else [0, 1]), [0, my]
+    for overlap, steps, words in [(1, (1, 1, 1), 0), (0, (7, 2 ** 31 + 1, 3), 1), (2, (2 ** 32 - 1, 24, 641), 0),
+                                  (2, (3, 5, 2 ** 20), 3)]:
+        s = plane_samples(bc, br, (mx, my), seed=mx + words, lo=-2 ** 20, hi=2 ** 20)
+        want = api.analyze_plane_cpu(s, bc, br, 1, overlap, steps, cols, rows, 1)
+        d = torch.from_numpy(s).to("cuda:0")
+        low = torch.zeros(s.size // 16 + words, dtype=torch.int32, device="cuda:0")
+        lq = torch.full((mx * my * 16 + words + 4,), -77, dtype=torch.int32, device="cuda:0")
+        hq = torch.full((mx * my * 256 + words + 4,), -77, dtype=torch.int32, device="cuda:0")
+        cb, rb = np.array(cols, np.uint32), np.array(rows, np.uint32)
+        p = (api.AnalysisPlaneC * 1)(api.AnalysisPlaneC(
+            d.data_ptr(), s.shape[1], s.shape[0], bc, br, 1, overlap, (api.C.c_uint32 * 3)(*steps), cb.ctypes.data,
+            cb.size, rb.ctypes.data, rb.size, 1, low.data_ptr() + 4 * words, lq.data_ptr() + 4 * words,
+            hq.data_ptr() + 4 * words))
+        api._check(api.lib().jxrb_analyze_planes(p, 1, None))
+        for got, w in ((lq.cpu().numpy(), want[0]), (hq.cpu().numpy(), want[1])):
+            assert np.array_equal(got[words:words + w.size], w.reshape(-1)), (overlap, steps)
+            assert (got[:words] == -77).all() and (got[words + w.size:] == -77).all()
