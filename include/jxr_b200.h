@@ -247,7 +247,8 @@ typedef struct jxrb_surface_layout {
 jxrb_status jxrb_plan_output_layout(const jxrb_plan *plan, jxrb_surface_layout *out);
 /* How the plan's 4 x 4-macroblock tiles split between the tile kernels:
  * interior tiles (full-resolution planes, 4:2:0), tiles on the plane's edge
- * away from hard tile boundaries (likewise) and the general kernel's tiles.
+ * away from hard tile boundaries (likewise) and, as `general`, the tiles that
+ * meet a hard tile boundary and those only the general kernel takes.
  * No counterpart in the reference: a diagnostic of this engine's launches. */
 typedef struct jxrb_tile_kinds {
     uint32_t interior, interior_420, edge, edge_420, general;

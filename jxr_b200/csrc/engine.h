@@ -135,8 +135,10 @@ struct QuarterImage {
 // 1..4 full-resolution planes (segments 0..3), interior tiles of YUV 4:2:0
 // images (segment 4), tiles of images with 1..4 full-resolution planes that
 // touch the plane's edge but no hard tile boundary (segments 5..8), such tiles
-// of 4:2:0 images (segment 9), then every other tile (segment 10).  A work
-// item carries a tag in the top bits of its image index: its segment + 1, or
+// of 4:2:0 images (segment 9), then every other tile (segment 10).  Tiles that
+// meet a hard tile boundary sit in the edge segments of their plane count
+// too, 4:2:0 images with two overlap levels aside.  A work item carries a tag
+// in the top bits of its image index: its segment + 1, a hard tag (below), or
 // 0 for the last segment (edge tiles folded into their interior kernel, see
 // kFoldEdges, keep their edge tag but sit in the interior segment).
 constexpr int kSegments = 11;
@@ -144,6 +146,8 @@ constexpr int kSegmentOther = kSegments - 1;
 constexpr uint32_t kTag420 = 5;
 constexpr uint32_t kTagEdge = 5;               // + plane count: edge tiles
 constexpr uint32_t kTagEdge420 = 10;
+constexpr uint32_t kTagHard = 10;              // + plane count: tiles that meet hard tile boundaries
+constexpr uint32_t kTagHard420 = 15;
 constexpr int kTagShift = 28;
 constexpr uint32_t kImageMask = (1u << kTagShift) - 1;
 constexpr int kSideSegment0 = 5;               // segments run beside the interior ones

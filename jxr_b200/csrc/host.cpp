@@ -115,9 +115,9 @@ bool interior_tile_at(uint32_t tx, uint32_t ty, uint32_t T, uint32_t mbs_x, uint
     return true;
 }
 
-// Whether tile (tx, ty) of a full-resolution image may take the edge kernel:
-// no hard tile starts at its macroblock columns mx0 .. mx0+4 or rows
-// my0 .. my0+4 inside the window, the window's own edges aside.
+// Whether tile (tx, ty) meets no hard tile boundary: no hard tile starts at
+// its macroblock columns mx0 .. mx0+4 or rows my0 .. my0+4 inside the window,
+// the window's own edges aside.
 bool edge_tile_at(uint32_t tx, uint32_t ty, uint32_t T, uint32_t mbs_x, uint32_t mbs_y, const uint8_t *starts_x,
                   const uint8_t *starts_y) {
     if (!starts_x) return true;
@@ -131,15 +131,18 @@ bool edge_tile_at(uint32_t tx, uint32_t ty, uint32_t T, uint32_t mbs_x, uint32_t
 
 // The tag of tile (tx, ty) of an image whose interior tag is `kind`: the
 // interior kernels' where the tile qualifies, the edge kernels' for the other
-// tiles that qualify, else 0 (the general kernel).
+// tiles that qualify, else 0 (the general kernel).  `two_level`: the image has
+// a first-level overlap.
 uint32_t tile_tag(uint32_t kind, uint32_t tx, uint32_t ty, uint32_t T, uint32_t mbs_x, uint32_t mbs_y,
-                  const uint8_t *starts_x, const uint8_t *starts_y) {
+                  const uint8_t *starts_x, const uint8_t *starts_y, bool two_level) {
     if (!kind) return 0;
     if (interior_tile_at(tx, ty, T, mbs_x, mbs_y, starts_x, starts_y)) return kind;
-    if (!edge_tile_at(tx, ty, T, mbs_x, mbs_y, starts_x, starts_y)) return 0;
-    if (kind <= 4) return kTagEdge + kind;
-    // 4:2:0 edge tiles need two chroma DC samples between the plane's corners
-    return kind == kTag420 && mbs_x >= 2 && mbs_y >= 2 ? kTagEdge420 : 0;
+    const bool hard = !edge_tile_at(tx, ty, T, mbs_x, mbs_y, starts_x, starts_y);
+    if (kind <= 4) return (hard ? kTagHard : kTagEdge) + kind;
+    // 4:2:0 edge tiles need two chroma DC samples between the plane's corners;
+    // the ordered chroma corners of hard tiles' first level need the general kernel
+    if (kind != kTag420 || mbs_x < 2 || mbs_y < 2 || (hard && two_level)) return 0;
+    return hard ? kTagHard420 : kTagEdge420;
 }
 
 // Work-list segment of a tag (engine.h).  Folded edge tiles (kFoldEdges) go
@@ -151,6 +154,7 @@ bool folded_edge_tag(uint32_t tag) {
 }
 int segment_of_tag(uint32_t tag) {
     if (folded_edge_tag(tag)) return tag == kTagEdge420 ? 4 : (int)(tag - kTagEdge) - 1;
+    if (tag > kTagHard) return kSideSegment0 + (int)(tag - kTagHard) - 1;   // the edge segments, 4:2:0's last
     return tag ? (int)tag - 1 : kSegmentOther;
 }
 int rank_of_tag(uint32_t tag) { return folded_edge_tag(tag) ? 0 : 1; }
@@ -858,11 +862,12 @@ jxrb_status build_device_set(const jxrb_plan *const *plans, uint32_t count, cuda
         // interior tiles (interior_tile / interior_tile_420 in recon_kernel.cu)
         const uint32_t kind = interior_tag(p.planes, p.chroma, p.out);
         const PlaneHost &p0 = p.planes[0];
+        const bool two_level = p0.overlap == 2;
         const uint8_t *sx = p0.hard ? p0.col_start.data() : nullptr, *sy = p0.hard ? p0.row_start.data() : nullptr;
         uint32_t it = set.image_items[i];
         for (uint32_t ty = 0; ty < im.tiles_y; ty++)
             for (uint32_t tx = 0; tx < im.tiles_x; tx++) {
-                const uint32_t tag = tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy);
+                const uint32_t tag = tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level);
                 set.host_items[it++] = WorkItemHost{i | tag << kTagShift, (uint16_t)tx, (uint16_t)ty};
             }
     }
@@ -1285,12 +1290,13 @@ jxrb_status stage_plan(const jxrb_plan *plan, const int32_t *coefficients, const
     const int np = (int)p.planes.size();
     const uint32_t kind = interior_tag(p.planes, p.chroma, p.out);
     const PlaneHost &p0 = p.planes[0];
+    const bool two_level = p0.overlap == 2;
     const uint8_t *sx = p0.hard ? p0.col_start.data() : nullptr, *sy = p0.hard ? p0.row_start.data() : nullptr;
     // count the tiles of each segment, then place each at its segment's cursor
     uint32_t count[kSegments] = {};
     for (uint32_t ty = 0; ty < tiles_y; ty++)
         for (uint32_t tx = 0; tx < tiles_x; tx++)
-            count[segment_of_tag(tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy))]++;
+            count[segment_of_tag(tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level))]++;
     uint32_t cursor[kSegments];
     layout.bounds[0] = 0;
     for (int s = 0; s < kSegments; s++) {
@@ -1301,7 +1307,7 @@ jxrb_status stage_plan(const jxrb_plan *plan, const int32_t *coefficients, const
     WorkItemHost *list = reinterpret_cast<WorkItemHost *>(host + layout.items_at);
     for (uint32_t ty = 0; ty < tiles_y; ty++)
         for (uint32_t tx = 0; tx < tiles_x; tx++) {
-            const uint32_t tag = tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy);
+            const uint32_t tag = tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level);
             list[cursor[segment_of_tag(tag)]++] = WorkItemHost{tag << kTagShift, (uint16_t)tx, (uint16_t)ty};
         }
     return JXRB_OK;
@@ -1436,12 +1442,14 @@ jxrb_status jxrb_plan_tile_kinds(const jxrb_plan *plan, jxrb_tile_kinds *out) {
     const uint32_t T = (uint32_t)tile_mbs();
     const uint32_t kind = interior_tag(p.planes, p.chroma, p.out);
     const PlaneHost &p0 = p.planes[0];
+    const bool two_level = p0.overlap == 2;
     const uint8_t *sx = p0.hard ? p0.col_start.data() : nullptr, *sy = p0.hard ? p0.row_start.data() : nullptr;
     *out = jxrb_tile_kinds{};
     for (uint32_t ty = 0; ty < (p.mbs_y + T - 1) / T; ty++)
         for (uint32_t tx = 0; tx < (p.mbs_x + T - 1) / T; tx++) {
-            const uint32_t tag = tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy);
-            if (tag == 0) out->general++;
+            const uint32_t tag = tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level);
+            // tiles at hard boundaries count as general, whichever kernel takes them
+            if (tag == 0 || tag > kTagHard) out->general++;
             else if (tag == kTagEdge420) out->edge_420++;
             else if (tag > kTagEdge) out->edge++;
             else if (tag == kTag420) out->interior_420++;
@@ -2053,12 +2061,13 @@ jxrb_status build_request_set(jxrb_session *s, const jxrb_request *const *reqs, 
         // (interior tiles never touch its first macroblock row or column)
         const uint32_t kind = interior_tag(img.planes, img.chroma, r.out);
         const ImagePlane &p0 = img.planes[0];
+        const bool two_level = p0.overlap == 2;
         const uint8_t *sx = p0.hard ? p0.col_start.data() + r.ox : nullptr;
         const uint8_t *sy = p0.hard ? p0.row_start.data() + r.oy : nullptr;
         uint32_t it = set.image_items[i];
         for (uint32_t ty = 0; ty < im.tiles_y; ty++)
             for (uint32_t tx = 0; tx < im.tiles_x; tx++) {
-                const uint32_t tag = tile_tag(kind, tx, ty, T, r.wx, r.wy, sx, sy);
+                const uint32_t tag = tile_tag(kind, tx, ty, T, r.wx, r.wy, sx, sy, two_level);
                 set.host_items[it++] = WorkItemHost{i | tag << kTagShift, (uint16_t)tx, (uint16_t)ty};
             }
     }

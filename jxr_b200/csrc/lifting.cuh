@@ -233,17 +233,19 @@ JXR_HD bool inverse_pot4x4(int32_t (&v)[16]) {
     return bad;
 }
 
-// Four-sample edge / corner operator (overlap.rs:10-55); always checked:
-// edges are a small share of the work.
-JXR_HD bool inverse_pot4(int32_t &a, int32_t &b, int32_t &c, int32_t &d) {
-    using A = Ar<true>;
+// Four-sample edge / corner operator (overlap.rs:10-55).  Inputs below the
+// overlap bound of 2^23 keep every intermediate below 2^28.4 (interval
+// arithmetic over the steps), so the wrapping form is exact for them.
+template <bool CK>
+JXR_HD bool inverse_pot4_steps(int32_t &a, int32_t &b, int32_t &c, int32_t &d) {
+    using A = Ar<CK>;
     bool bad = false;
     a = A::add(a, d, bad);
     b = A::add(b, c, bad);
     d = A::sub(d, A::add(a, 1, bad) >> 1, bad);
     c = A::sub(c, A::add(b, 1, bad) >> 1, bad);
-    inverse_scale<true>(a, d, bad);
-    inverse_scale<true>(b, c, bad);
+    inverse_scale<CK>(a, d, bad);
+    inverse_scale<CK>(b, c, bad);
     a = A::add(a, A::add(A::mul3(d, bad), 4, bad) >> 3, bad);
     b = A::add(b, A::add(A::mul3(c, bad), 4, bad) >> 3, bad);
     d = A::sub(d, a >> 1, bad);
@@ -252,12 +254,17 @@ JXR_HD bool inverse_pot4(int32_t &a, int32_t &b, int32_t &c, int32_t &d) {
     b = A::add(b, c, bad);
     d = A::neg(d, bad);
     c = A::neg(c, bad);
-    inverse_rotate<true>(c, d, bad);
+    inverse_rotate<CK>(c, d, bad);
     d = A::add(d, A::add(a, 1, bad) >> 1, bad);
     c = A::add(c, A::add(b, 1, bad) >> 1, bad);
     a = A::sub(a, d, bad);
     b = A::sub(b, c, bad);
     return bad;
+}
+
+JXR_HD bool inverse_pot4(int32_t &a, int32_t &b, int32_t &c, int32_t &d) {
+    if ((mag(a) | mag(b) | mag(c) | mag(d)) < (uint32_t)kOverlapBound) return inverse_pot4_steps<false>(a, b, c, d);
+    return inverse_pot4_steps<true>(a, b, c, d);
 }
 
 // Subsampled first-level operators (overlap.rs:167-227); always checked.

@@ -775,6 +775,7 @@ struct WorkItem {
 };
 
 struct TileShared {
+    uint32_t hard;   // edge kernels: hard tile starts, columns mx0 + 0..4 in bits 0..4, rows my0 + 0..4 in bits 8..12
     PlaneGeom geo[JXRB_MAX_PLANES];
     int bad;
     uint32_t next;   // interior kernels: the work item claimed to follow the current one
@@ -1367,12 +1368,72 @@ __device__ __forceinline__ void edge_grid(const EdgeCells &ec, int mx0, int my0,
     in = t < ncx * ncy;
 }
 
+// The hard tile boundaries a tile meets, for sh.hard (engine.h's tile-start
+// maps; the plane's own edges are not among them).  Called by the first warp.
+__device__ __forceinline__ uint32_t hard_starts(const ImageDev &im, int mx0, int my0) {
+    const PlaneDev &p = im.plane[0];
+    const int lane = threadIdx.x & 31, k = lane & 7;
+    const bool row = lane >= 8;
+    const int m = (row ? my0 : mx0) + k;
+    bool v = false;
+    if (p.hard && lane < 16 && k < 5 && m > 0 && m < (int)(row ? p.mbs_y : p.mbs_x))
+        v = (row ? p.row_start : p.col_start)[m] != 0;
+    return __ballot_sync(0xffffffffu, v);
+}
+
+// Whether a hard boundary runs through the middle of grid cell column / row c
+// (cells 3, 7, 11 and 15, on macroblock boundaries 1..4); `starts`: five bits.
+__device__ __forceinline__ bool hard_cell(uint32_t starts, int c) {
+    return (c & 3) == 3 && ((starts >> ((c + 1) >> 2)) & 1);
+}
+
+// Stage D at hard tile boundaries, in place: the grid cells wholly inside the
+// plane that such a boundary runs through, one four-sample operator a thread
+// -- down a column of the cell, along a row, or on a quarter of it where two
+// boundaries cross (second_level_overlap,
+// crates/jxr-native/src/reconstruct/overlap.rs).  The grid's pass then takes
+// those cells' samples as they are.  Returns the overflow flag.
+template <int NP>
+__device__ __forceinline__ bool hard_overlap(const ImageDev &im, int32_t *tiles, int mx0, int my0, uint32_t hard) {
+    const uint32_t cols = hard & 0x1eu, rows = (hard >> 8) & 0x1eu;
+    const int nv = __popc(cols), n = nv + __popc(rows);
+    const int ncx = min(16, (16 * (int)im.plane[0].mbs_x - 16 * mx0) / 4 - 1);   // cells wholly inside the plane
+    const int ncy = min(16, (16 * (int)im.plane[0].mbs_y - 16 * my0) / 4 - 1);
+    bool bad = false;
+    for (int item = threadIdx.x; item < NP * n * 64; item += kThreads) {
+        const int pi = item / (n * 64), q = item - pi * (n * 64), line = q >> 6, at_line = (q >> 2) & 15, o = q & 3;
+        if (im.plane[pi].overlap < 1) continue;
+        // the line'th boundary: the vertical ones first
+        uint32_t left = line < nv ? cols : rows;
+        for (int k = line < nv ? line : line - nv; k > 0; k--) left &= left - 1;
+        const int on = 4 * (__ffs(left) - 1) - 1;
+        const int cx = line < nv ? on : at_line, cy = line < nv ? at_line : on;
+        const bool vs = hard_cell(cols, cx), hs = hard_cell(rows, cy);
+        if (cx >= ncx || cy >= ncy || (line >= nv && vs)) continue;   // a crossing belongs to its column
+        int32_t *t = tiles + pi * kPlaneInts;
+        auto at = [&](int c, int r) -> int32_t & {
+            const int sx = 4 * cx + 2 + c, sy = 4 * cy + 2 + r;
+            return t[elem((sy >> 2) * kIB + (sx >> 2), sy & 3, sx & 3)];
+        };
+        // sample k of the operator: down column o, along row o, or quarter o in raster order
+        const int c0 = vs && hs ? 2 * (o & 1) : vs ? o : 0, r0 = vs && hs ? (o & 2) : vs ? 0 : o;
+        const int c1 = vs && hs ? c0 + 1 : vs ? o : 1, r1 = vs && hs ? r0 : vs ? 1 : o;
+        const int c2 = vs && hs ? c0 : vs ? o : 2, r2 = vs && hs ? r0 + 1 : vs ? 2 : o;
+        const int c3 = vs && hs ? c0 + 1 : vs ? o : 3, r3 = vs && hs ? r0 + 1 : vs ? 3 : o;
+        bad |= inverse_pot4(at(c0, r0), at(c1, r1), at(c2, r2), at(c3, r3));
+    }
+    return bad;
+}
+
 // Stage D at the plane's edge, in place: in each cell the edge cuts, the
 // four-sample operator down each of its two columns in the plane, along each
-// of its two rows, or on its corner quarter (second_level_overlap,
-// crates/jxr-native/src/reconstruct/overlap.rs).  Returns the overflow flag.
+// of its two rows, or on its corner quarter, or, where a hard tile boundary
+// (`hard`) crosses the edge, on each of its two quarters in the plane
+// (second_level_overlap, crates/jxr-native/src/reconstruct/overlap.rs).
+// Returns the overflow flag.
 template <int NP>
-__device__ __forceinline__ bool edge_overlap(const ImageDev &im, int32_t *tiles, int mx0, int my0, const EdgeCells &ec) {
+__device__ __forceinline__ bool edge_overlap(const ImageDev &im, int32_t *tiles, int mx0, int my0, const EdgeCells &ec,
+                                             uint32_t hard) {
     const int cells = ec.n[0] + ec.n[1] + ec.n[2] + ec.n[3];
     bool bad = false;
     for (int item = threadIdx.x; item < cells * 2 * NP; item += kThreads) {
@@ -1386,6 +1447,15 @@ __device__ __forceinline__ bool edge_overlap(const ImageDev &im, int32_t *tiles,
             return t[elem((sy >> 2) * kIB + (sx >> 2), sy & 3, sx & 3)];
         };
         const bool vs = c1 - c0 < 4, hs = r1 - r0 < 4;
+        if (hard && vs != hs) {
+            // quarter o of the part inside the plane
+            const int m = vs ? Y + 2 - 16 * my0 : X + 2 - 16 * mx0;
+            if ((m & 15) == 0 && m >= 0 && ((hard >> ((vs ? 8 : 0) + (m >> 4))) & 1)) {
+                const int x = vs ? c0 : X + 2 * o, y = vs ? Y + 2 * o : r0;
+                bad |= inverse_pot4(at(x, y), at(x + 1, y), at(x, y + 1), at(x + 1, y + 1));
+                continue;
+            }
+        }
         if (vs && !hs) {
             const int x = c0 + o;
             bad |= inverse_pot4(at(x, Y), at(x, Y + 1), at(x, Y + 2), at(x, Y + 3));
@@ -1473,8 +1543,14 @@ __device__ __forceinline__ bool edge_pixels(const ImageDev &im, const int32_t *t
 // while the previous tile ran); while it runs, the entries of the next work
 // item go into `mbc_next`.  `claimed` is thread 0's claim of that next item.
 //
-// Tiles that touch the plane's edge (and no hard tile boundary) run here
-// too.  Macroblocks outside the plane carry zero entries, so every stage runs
+// Tiles that touch the plane's edge run here too, and, in the edge kernels
+// (MODE 1), tiles that meet hard tile boundaries: those change no geometry,
+// only the operators of the windows and cells they run through, which are
+// done before the grid (hard_overlap).  The general kernel takes 62.6 k warp
+// instructions for a three-plane tile, the interior form 22.8 k (2500 x 1900
+// RGB8, 256 x 256 hard tiles, 848 of 1200 tiles at a hard boundary: 151 us
+// through the general kernel, 67 us here).
+// Macroblocks outside the plane carry zero entries, so every stage runs
 // unchanged over them and leaves zeros; the overlap windows and cells whose
 // centre lies on the plane's edge take the reference's edge and corner
 // operators, cells outside the plane are skipped, and the cells the edge cuts
@@ -1493,6 +1569,10 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
     int32_t *dcs = smem + NP * kPlaneInts;       // NP DC tiles of kIDC x kIDC
     int32_t *lps = dcs + NP * kDcInts;           // NP x 36 macroblocks x 16 DC / low-pass coefficients (lp_stride<NP>() apart)
     if (tid == 0) sh.bad = 0;
+    if (MODE == 1 && tid < 32) {
+        const uint32_t starts = hard_starts(im, mx0, my0);
+        if (tid == 0) sh.hard = starts;
+    }
     int bad = 0;
     // phase 1: every coefficient the tile reads, in flight at once.  The DC /
     // low-pass coefficients of the ring of 20 macroblocks around the tile, 4
@@ -1628,7 +1708,11 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 const PlaneDev &p = im.plane[pi];
                 const int ca = mx0 + c % 5, cb = my0 + c / 5;
                 if (ca > (int)p.mbs_x || cb > (int)p.mbs_y) continue;   // beyond the plane
-                const bool vs = ca == 0 || ca == (int)p.mbs_x, hs = cb == 0 || cb == (int)p.mbs_y;
+                bool vs = ca == 0 || ca == (int)p.mbs_x, hs = cb == 0 || cb == (int)p.mbs_y;
+                if (MODE == 1) {
+                    vs |= (sh.hard >> (c % 5)) & 1;
+                    hs |= (sh.hard >> (8 + c / 5)) & 1;
+                }
                 if (vs || hs) {
                     if (dc_edge_window(dcs + pi * kDcInts, 2 + 4 * (c % 5), 2 + 4 * (c / 5), 4 * (mx0 - 1),
                                        4 * (my0 - 1), 4 * (int)p.mbs_x, 4 * (int)p.mbs_y, vs, hs))
@@ -1747,17 +1831,22 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             *reinterpret_cast<int4 *>(blk + ((r ^ sw) << 2)) = make_int4(v[r * 4], v[r * 4 + 1], v[r * 4 + 2], v[r * 4 + 3]);
     }
     const bool tile_small = __syncthreads_and(small) != 0;
-    bool grid_cell = true;
+    bool grid_cell = true, cut = false;
     int gcx = tid & 15, gcy = tid >> 4;   // the thread's cell of the 16 x 16 grid
     EdgeCells ec;
     if (edge) {
         ec = edge_cells(im, mx0, my0);
-        if (edge_overlap<NP>(im, tiles, mx0, my0, ec)) bad |= kFlagOverlap;
+        const uint32_t hard = MODE == 1 ? sh.hard : 0;
+        if (edge_overlap<NP>(im, tiles, mx0, my0, ec, hard)) bad |= kFlagOverlap;
+        if (hard && hard_overlap<NP>(im, tiles, mx0, my0, hard)) bad |= kFlagOverlap;
         __syncthreads();
         // cells past the plane's edge, or cut by it, leave the grid; the
         // rest are packed onto the first threads, so that whole warps idle
         edge_grid(ec, mx0, my0, gcx, gcy, grid_cell);
+        // cells that a hard boundary cuts have their operators behind them
+        cut = hard && (hard_cell(hard & 0x1fu, gcx) || hard_cell((hard >> 8) & 0x1fu, gcy));
     }
+    auto overlap_of = [&](int pi) { return MODE == 1 && cut ? 0 : im.plane[pi].overlap; };
     // stage D + E: the thread's sample cell, every plane, then its 16 pixels
     if (grid_cell) {
         const int cx = gcx, cy = gcy;
@@ -1771,9 +1860,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         bool obad = false, done = false;
         if (inside && kind == kOutRgb8 && NP >= 3 && !o.premultiply) {
             int32_t y[16], u[16], v[16];
-            bool ov = cell_samples(tiles, b00, im.plane[0].overlap, y, tile_small);
-            ov |= cell_samples(tiles + kPlaneInts, b00, im.plane[1].overlap, u, tile_small);
-            ov |= cell_samples(tiles + 2 * kPlaneInts, b00, im.plane[2].overlap, v, tile_small);
+            bool ov = cell_samples(tiles, b00, overlap_of(0), y, tile_small);
+            ov |= cell_samples(tiles + kPlaneInts, b00, overlap_of(1), u, tile_small);
+            ov |= cell_samples(tiles + 2 * kPlaneInts, b00, overlap_of(2), v, tile_small);
             if (ov) bad |= kFlagOverlap;
             uint32_t m = 0;
             if (!tile_small) {
@@ -1799,7 +1888,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 bool alpha_ok = true;
                 if (NP == 4 && has_alpha) {
                     int32_t a[16];
-                    if (cell_samples(tiles + 3 * kPlaneInts, b00, im.plane[3].overlap, a, tile_small))
+                    if (cell_samples(tiles + 3 * kPlaneInts, b00, overlap_of(3), a, tile_small))
                         bad |= kFlagOverlap;
                     const ChannelScale &sa = o.ch[3];
                     const int32_t aadd = sa.shifted_bias + sa.rounding;
@@ -1824,7 +1913,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             }
         } else if (inside && kind == kOutDirect && NP == 1) {
             int32_t y[16];
-            if (cell_samples(tiles, b00, im.plane[0].overlap, y, tile_small)) bad |= kFlagOverlap;
+            if (cell_samples(tiles, b00, overlap_of(0), y, tile_small)) bad |= kFlagOverlap;
             const ChannelScale &s = o.ch[0];
             const int eb = o.elem_bytes;
 #pragma unroll
@@ -1841,9 +1930,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         } else if (inside && kind == kOutF16Wide && o.nchw && NP == 4 && o.channels <= NP) {
             // colour channel planes first, then alpha
             int32_t y[16], u[16], v[16];
-            bool ov = cell_samples(tiles, b00, im.plane[0].overlap, y, tile_small);
-            ov |= cell_samples(tiles + kPlaneInts, b00, im.plane[1].overlap, u, tile_small);
-            ov |= cell_samples(tiles + 2 * kPlaneInts, b00, im.plane[2].overlap, v, tile_small);
+            bool ov = cell_samples(tiles, b00, overlap_of(0), y, tile_small);
+            ov |= cell_samples(tiles + kPlaneInts, b00, overlap_of(1), u, tile_small);
+            ov |= cell_samples(tiles + 2 * kPlaneInts, b00, overlap_of(2), v, tile_small);
             if (ov) bad |= kFlagOverlap;
             uint8_t *base = o.base + (uint64_t)(y0 - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * 4;
             const int primaries = has_alpha ? o.channels - 1 : o.channels;
@@ -1906,7 +1995,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             }
             if (has_alpha && NP == 4) {
                 int32_t a[16];
-                if (cell_samples(tiles + 3 * kPlaneInts, b00, im.plane[3].overlap, a, tile_small)) bad |= kFlagOverlap;
+                if (cell_samples(tiles + 3 * kPlaneInts, b00, overlap_of(3), a, tile_small)) bad |= kFlagOverlap;
                 const ChannelScale &s = o.ch[o.channels - 1];
                 bool alean = s.post_shift < 0 && mag(s.shifted_bias) < (1u << 28) && mag(s.rounding) < (1u << 28);
                 if (alean && !tile_small) {
@@ -1930,9 +2019,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         } else if (inside && kind == kOutF16Wide && o.nchw && NP == 3 && o.channels <= NP) {
             // colour channel planes first, then alpha
             int32_t y[16], u[16], v[16];
-            bool ov = cell_samples(tiles, b00, im.plane[0].overlap, y, tile_small);
-            ov |= cell_samples(tiles + kPlaneInts, b00, im.plane[1].overlap, u, tile_small);
-            ov |= cell_samples(tiles + 2 * kPlaneInts, b00, im.plane[2].overlap, v, tile_small);
+            bool ov = cell_samples(tiles, b00, overlap_of(0), y, tile_small);
+            ov |= cell_samples(tiles + kPlaneInts, b00, overlap_of(1), u, tile_small);
+            ov |= cell_samples(tiles + 2 * kPlaneInts, b00, overlap_of(2), v, tile_small);
             if (ov) bad |= kFlagOverlap;
             uint8_t *base = o.base + (uint64_t)(y0 - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * 4;
             const int primaries = has_alpha ? o.channels - 1 : o.channels;
@@ -1961,7 +2050,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             }
             if (has_alpha && NP == 4) {
                 int32_t a[16];
-                if (cell_samples(tiles + 3 * kPlaneInts, b00, im.plane[3].overlap, a, tile_small)) bad |= kFlagOverlap;
+                if (cell_samples(tiles + 3 * kPlaneInts, b00, overlap_of(3), a, tile_small)) bad |= kFlagOverlap;
                 const ChannelScale &s = o.ch[o.channels - 1];
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
@@ -1983,7 +2072,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             int32_t w[NP][16];
 #pragma unroll
             for (int pi = 0; pi < NP; pi++)
-                if (cell_samples(tiles + pi * kPlaneInts, b00, im.plane[pi].overlap, w[pi], tile_small))
+                if (cell_samples(tiles + pi * kPlaneInts, b00, overlap_of(pi), w[pi], tile_small))
                     bad |= kFlagOverlap;
             const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
             const uint64_t chs = o.nchw ? o.plane_stride : (uint64_t)o.elem_bytes;
@@ -2280,24 +2369,25 @@ __device__ bool chroma_edge_square(int32_t *cd, int wx, int wy, bool vs, bool hs
     return bad;
 }
 
-// A second-level chroma cell of a 4:2:0 edge tile that the plane's edge cuts,
-// at chroma position (X, Y), in place: the four-sample operator down each
-// column inside the plane, along each row, or on the corner quarter.  (ox, oy):
-// the chroma position of the tile's sample origin; (Wc, Hc): the chroma plane.
-__device__ bool chroma_cut_cell(int32_t *t, int X, int Y, int ox, int oy, int Wc, int Hc) {
+// A second-level chroma cell of a 4:2:0 edge tile that the plane's edge or a
+// hard tile boundary cuts (vs: from top to bottom, hs: from left to right), at
+// chroma position (X, Y), in place: the four-sample operator down each column
+// inside the plane, along each row, or on each quarter.  (ox, oy): the chroma
+// position of the tile's sample origin; (Wc, Hc): the chroma plane.
+__device__ bool chroma_cut_cell(int32_t *t, int X, int Y, int ox, int oy, int Wc, int Hc, bool vs, bool hs) {
     auto at = [&](int x, int y) -> int32_t & {
         const int sx = x - ox, sy = y - oy;
         return t[elem((sy >> 2) * kCB + (sx >> 2), sy & 3, sx & 3)];
     };
     const int c0 = max(X, 0), c1 = min(X + 4, Wc), r0 = max(Y, 0), r1 = min(Y + 4, Hc);
-    const bool vs = c1 - c0 < 4, hs = r1 - r0 < 4;
     bool bad = false;
     if (vs && !hs) {
         for (int x = c0; x < c1; x++) bad |= inverse_pot4(at(x, Y), at(x, Y + 1), at(x, Y + 2), at(x, Y + 3));
     } else if (!vs && hs) {
         for (int y = r0; y < r1; y++) bad |= inverse_pot4(at(X, y), at(X + 1, y), at(X + 2, y), at(X + 3, y));
     } else {
-        bad |= inverse_pot4(at(c0, r0), at(c0 + 1, r0), at(c0, r0 + 1), at(c0 + 1, r0 + 1));
+        for (int y = r0; y < r1; y += 2)
+            for (int x = c0; x < c1; x += 2) bad |= inverse_pot4(at(x, y), at(x + 1, y), at(x, y + 1), at(x + 1, y + 1));
     }
     return bad;
 }
@@ -2346,8 +2436,10 @@ __device__ bool edge_pixels_420(const ImageDev &im, const int32_t *ytile, const 
 }
 
 // Edge tiles (MODE 1, or MODE 2 by position): tiles of a 4:2:0 image (at
-// least 2 x 2 macroblocks) that touch the plane's edge and no hard tile
-// boundary, as the full-resolution edge tiles, with the chroma planes'
+// least 2 x 2 macroblocks) that touch the plane's edge, or, with at most one
+// overlap level, a hard tile boundary (the ordered first-level chroma corners
+// at hard boundaries stay with the general kernel), as the full-resolution
+// edge tiles, with the chroma planes'
 // first-level squares and second-level cells on the plane's edge taking the
 // edge operators (and corner residuals).
 template <int MODE>
@@ -2366,6 +2458,10 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
     int32_t *cdc = ctile + 2 * kCPlaneInts;             // 2 x 12 x 12
     int32_t *clp = cdc + 2 * kCDC * kCDC;               // 2 x 36 x 4
     if (tid == 0) sh.bad = 0;
+    if (MODE == 1 && tid < 32) {
+        const uint32_t starts = hard_starts(im, mx0, my0);
+        if (tid == 0) sh.hard = starts;
+    }
     int bad = 0;
     // phase 1: the DC / low-pass values (luma 16, chroma 4 a macroblock) of
     // the ring of luma macroblocks and of the 6 x 6 chroma macroblocks, then
@@ -2679,8 +2775,14 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
             const int Wc = 8 * (int)im.plane[1].mbs_x, Hc = 8 * (int)im.plane[1].mbs_y;
             const int X = 8 * mx0 - 2 + 4 * (c % 9), Y = 8 * my0 - 2 + 4 * (c / 9);
             if (X >= Wc || Y >= Hc) continue;
-            if (X + 2 == 0 || X + 2 == Wc || Y + 2 == 0 || Y + 2 == Hc) {
-                if (im.plane[1 + pc].overlap >= 1 && chroma_cut_cell(t, X, Y, 8 * mx0 - 8, 8 * my0 - 8, Wc, Hc))
+            bool vs = X + 2 == 0 || X + 2 == Wc, hs = Y + 2 == 0 || Y + 2 == Hc;
+            if (MODE == 1) {
+                // the cell's middle is on macroblock boundary (c % 9) / 2 (c / 9 / 2) where that is even
+                vs |= ((c % 9) & 1) == 0 && ((sh.hard >> ((c % 9) >> 1)) & 1);
+                hs |= ((c / 9) & 1) == 0 && ((sh.hard >> (8 + ((c / 9) >> 1))) & 1);
+            }
+            if (vs || hs) {
+                if (im.plane[1 + pc].overlap >= 1 && chroma_cut_cell(t, X, Y, 8 * mx0 - 8, 8 * my0 - 8, Wc, Hc, vs, hs))
                     bad |= kFlagOverlap;
                 continue;
             }
@@ -2690,13 +2792,16 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
             bad |= kFlagOverlap;
     }
     EdgeCells ec;
-    bool grid_cell = true;
+    bool grid_cell = true, cut = false;
     int gcx = tid & 15, gcy = tid >> 4;   // the thread's cell of the 16 x 16 grid
     if (edge) {
         // stage D for the luma cells the plane's edge cuts, in place
         ec = edge_cells(im, mx0, my0);
-        if (edge_overlap<1>(im, ytile, mx0, my0, ec)) bad |= kFlagOverlap;
+        const uint32_t hard = MODE == 1 ? sh.hard : 0;
+        if (edge_overlap<1>(im, ytile, mx0, my0, ec, hard)) bad |= kFlagOverlap;
+        if (hard && hard_overlap<1>(im, ytile, mx0, my0, hard)) bad |= kFlagOverlap;
         edge_grid(ec, mx0, my0, gcx, gcy, grid_cell);
+        cut = hard && (hard_cell(hard & 0x1fu, gcx) || hard_cell((hard >> 8) & 0x1fu, gcy));
     }
     __syncthreads();
     // stage E: each thread's luma cell, the chroma around it interpolated
@@ -2709,7 +2814,7 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
                             y0 + 4 <= (int)(o.crop_y + o.crop_h);
         bool obad = false, done = false;
         int32_t y[16];
-        if (cell_rw(ytile, cy * kIB + cx, kIB, im.plane[0].overlap, y, false, tile_small)) bad |= kFlagOverlap;
+        if (cell_rw(ytile, cy * kIB + cx, kIB, MODE == 1 && cut ? 0 : im.plane[0].overlap, y, false, tile_small)) bad |= kFlagOverlap;
         // chroma samples (tile coordinates) 8 + 2cx .. 11 + 2cx, 8 + 2cy .. 11 + 2cy
         if (tile_small && !edge && inside && o.kind == kOutRgb8 && !o.premultiply &&
             (o.channels == 3 || o.ch[3].padding)) {

@@ -307,6 +307,34 @@ def test_edge_tiles_with_hard_tiles(session, tiles):
     check(session, img, rgb8(336, 304))
 
 
+@pytest.mark.parametrize("tiles", [(1, 1), (2, 3), (4, 4), (5, 7), (8, 3), (16, 16)])
+@pytest.mark.parametrize("overlap", [0, 1, 2])
+@pytest.mark.parametrize("fmt", ["LUMA", "YUV444", "RGBA", "YUV420", "RANDOM"])
+def test_hard_tiles_in_the_edge_kernels(session, tiles, overlap, fmt):
+    """Hard boundaries at every macroblock of a tile, crossing each other and
+    the plane's edge, one to four planes and 4:2:0, on a plane that ends inside
+    a tile and one that ends on its boundary; random content reaches the
+    checked operators."""
+    tw, th = tiles
+    for w, h in [(336, 304), (192, 256)]:
+        kw = dict(overlap=overlap, tile_width=tw, tile_height=th, hard_tiles=1, seed=200 + tw * 3 + overlap)
+        if fmt == "LUMA":
+            img = J.synth(w, h, content=J.CONTENT["GRAY16"], color_format=C_["LUMA"], quality=100, scaled=0, **kw)
+            out = J.OutputFormat(C_["LUMA"], D["U16"], S["U16"], L["LUMA"], w - 3, h - 5, crop_x=1, crop_y=2)
+        elif fmt == "RGBA":
+            img = J.synth(w, h, alpha_mode=A["INTEGRATED"], quality=85, alpha_overlap=overlap, alpha_qp=(8, 8, 8), **kw)
+            out = J.OutputFormat(C_["RGB"], D["U8"], S["U8"], L["RGBA"], w, h, alpha_bit_depth=D["U8"])
+        elif fmt == "RANDOM":
+            img = J.synth(w, h, content=J.CONTENT["RANDOM"], **kw)
+            out = J.OutputFormat(C_["RGB"], D["I32"], S["I32"], L["RGB"], w, h)
+            check(session, img, out, expect_ok=False)
+            continue
+        else:
+            img = J.synth(w, h, color_format=C_[fmt], quality=80, **kw)
+            out = rgb8(w - 2, h - 1, crop_x=1)
+        check(session, img, out)
+
+
 def test_edge_tiles_overflow(session):
     img = J.synth(208, 176, quality=75, overlap=2, seed=140)
     img.arena.coefficients[:64] = 2**30
