@@ -132,34 +132,33 @@ struct QuarterImage {
 };
 
 // Work-list segments, one tile kernel each: interior tiles of images with
-// 1..4 full-resolution planes (segments 0..3), interior tiles of YUV 4:2:0
-// images (segment 4), tiles of images with 1..4 full-resolution planes that
-// touch the plane's edge but no hard tile boundary (segments 5..8), such tiles
-// of 4:2:0 images (segment 9), then every other tile (segment 10).  Tiles that
-// meet a hard tile boundary sit in the edge segments of their plane count
-// too, 4:2:0 images with two overlap levels aside.  A work item carries a tag
-// in the top bits of its image index: its segment + 1, a hard tag (below), or
-// 0 for the last segment (edge tiles folded into their interior kernel, see
-// kFoldEdges, keep their edge tag but sit in the interior segment).
-constexpr int kSegments = 11;
-constexpr int kSegmentOther = kSegments - 1;
-constexpr uint32_t kTag420 = 5;
-constexpr uint32_t kTagEdge = 5;               // + plane count: edge tiles
-constexpr uint32_t kTagEdge420 = 10;
-constexpr uint32_t kTagHard = 10;              // + plane count: tiles that meet hard tile boundaries
-constexpr uint32_t kTagHard420 = 15;
-constexpr int kTagShift = 28;
+// 1..4 full-resolution planes (segments 0..3), of YUV 4:2:0 images (4) and of
+// 4:2:2 images (5), then tiles that touch the plane's edge or meet a hard tile
+// boundary in the same order (6..11), then every other tile (12).  A work item
+// carries a tag in the top bits of its image index, by which the host sorts
+// the list: a kind -- 1..4 the plane count, then 4:2:0 and 4:2:2 -- plus
+// nothing for interior tiles, kTagEdge for tiles on the plane's edge alone and
+// kTagHard for tiles that meet a hard tile boundary; 0 is every other tile.
+// Subsampled images with two overlap levels keep their hard tiles in the last
+// segment.
+constexpr int kKinds = 6;
+constexpr uint32_t kTag420 = 5, kTag422 = 6;
+constexpr uint32_t kTagEdge = kKinds;
+constexpr uint32_t kTagHard = 2 * kKinds;
+constexpr int kTagShift = 27;
 constexpr uint32_t kImageMask = (1u << kTagShift) - 1;
-constexpr int kSideSegment0 = 5;               // segments run beside the interior ones
+constexpr int kSideSegment0 = kKinds;          // segments run beside the interior ones
+constexpr int kSegments = 2 * kKinds + 1;
+constexpr int kSegmentOther = kSegments - 1;
 // Edge tiles that the interior kernel of the same images takes instead of an
-// edge kernel (one launch, edge tiles first in it), by plane count 1..4, then
-// 4:2:0; their edge segment then stays empty.
-constexpr bool kFoldEdges[5] = {false, false, true, false, false};
+// edge kernel (one launch, edge tiles first in it), by kind; their edge
+// segment then holds their hard tiles alone.
+constexpr bool kFoldEdges[kKinds] = {false, false, true, false, false, false};
 constexpr int kCounterWords = 2 * kSegments;   // two scheduling words a segment
 
 // Launch shape of the tile kernels, chosen by the autotuner.  Entries 0..3
 // serve the full-resolution segments by plane count, entry 4 the other tiles;
-// the 4:2:0 interior segment, a three-plane interior kernel, takes entry 2.
+// the subsampled segments, three-plane kernels, take entry 2.
 struct LaunchTuning {
     uint32_t blocks_per_sm[5];   // resident CTAs per SM; 0 = as many as fit
     int32_t side_stream;         // other tiles' kernel on a second stream beside the interior ones

@@ -83,10 +83,11 @@ struct PlaneHost {
     int bc = 4, br = 4, scale2 = 0, overlap = 0, hard = 0;
 };
 
-// The interior tag an image's interior tiles carry (engine.h): its plane
-// count when every plane is at full resolution (at most four), kTag420 for a
-// YUV 4:2:0 image of three planes, 0 when every tile takes the general kernel.
-// 1-bit and planar outputs always take the general kernel.
+// The kind of an image's tiles (engine.h), the tag its interior tiles carry:
+// its plane count when every plane is at full resolution (at most four),
+// kTag420 or kTag422 for a YUV 4:2:0 or 4:2:2 image of three planes, 0 when
+// every tile takes the general kernel.  1-bit and planar outputs always take
+// the general kernel.
 template <class Planes>
 uint32_t interior_tag(const Planes &planes, int chroma, const OutputDev &out) {
     const size_t np = planes.size();
@@ -94,9 +95,9 @@ uint32_t interior_tag(const Planes &planes, int chroma, const OutputDev &out) {
     bool full = true;
     for (const auto &p : planes) full &= p.bc == 4 && p.br == 4;
     if (full) return (uint32_t)np;
-    if (np == 3 && chroma == 1 && planes[0].bc == 4 && planes[0].br == 4 && planes[1].bc == 2 && planes[1].br == 2 &&
-        planes[2].bc == 2 && planes[2].br == 2)
-        return kTag420;
+    if (np != 3 || planes[0].bc != 4 || planes[0].br != 4 || planes[1].bc != 2 || planes[2].bc != 2) return 0;
+    if (chroma == 1 && planes[1].br == 2 && planes[2].br == 2) return kTag420;
+    if (chroma == 2 && planes[1].br == 4 && planes[2].br == 4) return kTag422;
     return 0;
 }
 
@@ -138,24 +139,23 @@ uint32_t tile_tag(uint32_t kind, uint32_t tx, uint32_t ty, uint32_t T, uint32_t 
     if (!kind) return 0;
     if (interior_tile_at(tx, ty, T, mbs_x, mbs_y, starts_x, starts_y)) return kind;
     const bool hard = !edge_tile_at(tx, ty, T, mbs_x, mbs_y, starts_x, starts_y);
-    if (kind <= 4) return (hard ? kTagHard : kTagEdge) + kind;
-    // 4:2:0 edge tiles need two chroma DC samples between the plane's corners;
-    // the ordered chroma corners of hard tiles' first level need the general kernel
-    if (kind != kTag420 || mbs_x < 2 || mbs_y < 2 || (hard && two_level)) return 0;
-    return hard ? kTagHard420 : kTagEdge420;
+    // edge tiles of subsampled images need two chroma DC samples between the
+    // plane's corners, and the ordered chroma corners of hard tiles' first
+    // level the general kernel
+    if (kind >= kTag420 && (mbs_x < 2 || mbs_y < 2 || (hard && two_level))) return 0;
+    return (hard ? kTagHard : kTagEdge) + kind;
 }
 
 // Work-list segment of a tag (engine.h).  Folded edge tiles (kFoldEdges) go
 // to their interior kernel's segment -- one kernel, so that their latency
 // hides among the interior tiles -- ahead of its interior tiles.
 bool folded_edge_tag(uint32_t tag) {
-    if (tag > kTagEdge && tag <= kTagEdge + 4) return kFoldEdges[tag - kTagEdge - 1];
-    return tag == kTagEdge420 && kFoldEdges[4];
+    return tag > kTagEdge && tag <= kTagHard && kFoldEdges[tag - kTagEdge - 1];
 }
 int segment_of_tag(uint32_t tag) {
-    if (folded_edge_tag(tag)) return tag == kTagEdge420 ? 4 : (int)(tag - kTagEdge) - 1;
-    if (tag > kTagHard) return kSideSegment0 + (int)(tag - kTagHard) - 1;   // the edge segments, 4:2:0's last
-    return tag ? (int)tag - 1 : kSegmentOther;
+    if (tag == 0) return kSegmentOther;
+    if (tag > kTagHard) return kSideSegment0 + (int)(tag - kTagHard) - 1;
+    return folded_edge_tag(tag) ? (int)(tag - kTagEdge) - 1 : (int)tag - 1;
 }
 int rank_of_tag(uint32_t tag) { return folded_edge_tag(tag) ? 0 : 1; }
 
@@ -1448,12 +1448,12 @@ jxrb_status jxrb_plan_tile_kinds(const jxrb_plan *plan, jxrb_tile_kinds *out) {
     for (uint32_t ty = 0; ty < (p.mbs_y + T - 1) / T; ty++)
         for (uint32_t tx = 0; tx < (p.mbs_x + T - 1) / T; tx++) {
             const uint32_t tag = tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level);
-            // tiles at hard boundaries count as general, whichever kernel takes them
-            if (tag == 0 || tag > kTagHard) out->general++;
-            else if (tag == kTagEdge420) out->edge_420++;
-            else if (tag > kTagEdge) out->edge++;
-            else if (tag == kTag420) out->interior_420++;
-            else out->interior++;
+            // tiles at hard boundaries and 4:2:2's count as general,
+            // whichever kernel takes them
+            const bool edge = tag > kTagEdge;
+            if (tag == 0 || tag > kTagHard || kind == kTag422) out->general++;
+            else if (kind == kTag420) (edge ? out->edge_420 : out->interior_420)++;
+            else (edge ? out->edge : out->interior)++;
         }
     return JXRB_OK;
 }

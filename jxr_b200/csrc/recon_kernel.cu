@@ -2300,23 +2300,45 @@ jxrb_reconstruct_tiles(const ImageDev *__restrict__ images, const WorkItem *__re
 }
 
 // ---------------------------------------------------------------------------
-// Interior tiles of YUV 4:2:0 images (three planes, chroma 2 x 2 blocks a
-// macroblock).  Luma is the full-resolution interior tile above.  Each
-// chroma plane holds the 11 x 11 blocks of macroblocks mx0-1 .. mx0+4 (the
-// last one's first block column / row only): block column 2*mx0-2 is there
-// for high-pass prediction alone; columns 2*mx0-1 .. 2*mx0+8 are
+// Interior tiles of YUV 4:2:0 and 4:2:2 images (three planes, chroma 2 x 2 or
+// 2 x 4 blocks a macroblock).  Luma is the full-resolution interior tile
+// above.  Across, each chroma plane holds the 11 block columns of macroblocks
+// mx0-1 .. mx0+4 (the last one's first alone): block column 2*mx0-2 is there
+// for high-pass prediction only; columns 2*mx0-1 .. 2*mx0+8 are
 // reconstructed, and their samples, after the second-level overlap cells at
-// chroma origins 8*mx0-2 + 4k (k = 0..8), are the ones the luma pixels of the
-// tile interpolate from (4 chroma columns and rows around each luma cell).
-// In the interior every first-level chroma window is a plain 2 x 2 square
-// at odd DC origins and every overlap cell a plain 4 x 4 window.
+// chroma columns 8*mx0-2 + 4k (k = 0..8), are the ones the luma pixels of the
+// tile interpolate from (4 chroma columns around each luma cell).  Down, 4:2:0
+// is the same; 4:2:2 has the luma plane's 17 block rows and 16 cell rows, and
+// no interpolation.  In the interior every first-level chroma window is a
+// plain 2 x 2 square at odd DC origins and every overlap cell a plain 4 x 4
+// window.
 // ---------------------------------------------------------------------------
-constexpr int kCB = 11;                          // chroma blocks across / down
-constexpr int kCBlocks = kCB * kCB;
-constexpr int kCPlaneInts = kCBlocks * 16;
-constexpr int kCDC = 12;                         // chroma DC tile side
-constexpr int kCLpInts = 36 * 4;                 // DC / low-pass of 6 x 6 macroblocks
-constexpr int kSmem420Ints = kPlaneInts + kDcInts + kLpInts + 2 * (kCPlaneInts + kCDC * kCDC + kCLpInts) + 2 * 3 * kMbcInts;
+constexpr int kCB = 11;                          // chroma blocks across
+constexpr int kCDC = 12;                         // chroma DC tile columns
+
+// The chroma tile by block rows a macroblock (CV: 2 for 4:2:0, 4 for 4:2:2).
+template <int CV>
+struct ChromaTile {
+    static constexpr int kFirstMb = CV == 2 ? -1 : 0;        // first macroblock row held, from my0
+    static constexpr int kMbRows = CV == 2 ? 6 : 5;          // the last one's first block row alone
+    static constexpr int kRows = CV * (kMbRows - 1) + 1;     // blocks down: 11 or 17
+    static constexpr int kInts = kCB * kRows * 16;
+    static constexpr int kDcRows = 6 * CV;                   // macroblocks my0-1 .. my0+4
+    static constexpr int kDcInts = kCDC * kDcRows;
+    static constexpr int kDcRow0 = CV == 2 ? 0 : CV;         // DC row of block row 0
+    static constexpr int kLow = 2 * CV;                      // DC / low-pass values a macroblock
+    static constexpr int kLpInts = 36 * kLow;
+    static constexpr int kRow0 = CV == 2 ? 1 : 0;            // block rows reconstructed
+    static constexpr int kTransRows = CV == 2 ? 10 : 17;
+    static constexpr int kSquares = CV == 2 ? 5 : 9;         // first-level squares down
+    static constexpr int kSquare0 = CV == 2 ? 1 : 3;         // DC row of the first
+    static constexpr int kCells = CV == 2 ? 9 : 17;          // cells down; 4:2:2's first is the plane's top edge only
+    static constexpr int kSmemInts =
+        kPlaneInts + jxr::kDcInts + jxr::kLpInts + 2 * (kInts + kDcInts + kLpInts) + 2 * 3 * kMbcInts;
+    // plane row of the tile's first sample, and of cell row 0
+    __device__ static int sample0(int my0) { return CV == 2 ? 8 * my0 - 8 : 16 * my0; }
+    __device__ static int cell0(int my0) { return 4 * CV * my0 - 2; }
+};
 
 // The 16 samples of the 4 x 4 cell whose upper-left quarter is the lower-right
 // quarter of block b00 of a tile `stride` blocks wide; second-level overlap
@@ -2342,7 +2364,7 @@ __device__ __forceinline__ bool cell_rw(int32_t *t, int b00, int stride, int ove
     return bad;
 }
 
-// A first-level chroma square of a 4:2:0 edge tile whose centre lies on the
+// A first-level chroma square of a subsampled edge tile whose centre lies on the
 // plane's edge (subsampled_overlap.rs:244-296): the two-sample operator on
 // its column (vs) or row (hs) inside the plane; none on a plane corner.  On
 // the top and bottom rows the plane's corner samples take their residual
@@ -2369,7 +2391,7 @@ __device__ bool chroma_edge_square(int32_t *cd, int wx, int wy, bool vs, bool hs
     return bad;
 }
 
-// A second-level chroma cell of a 4:2:0 edge tile that the plane's edge or a
+// A second-level chroma cell of a subsampled edge tile that the plane's edge or a
 // hard tile boundary cuts (vs: from top to bottom, hs: from left to right), at
 // chroma position (X, Y), in place: the four-sample operator down each column
 // inside the plane, along each row, or on each quarter.  (ox, oy): the chroma
@@ -2392,15 +2414,17 @@ __device__ bool chroma_cut_cell(int32_t *t, int X, int Y, int ox, int oy, int Wc
     return bad;
 }
 
-// Stage E at the plane's edge of a 4:2:0 tile: the pixels of the cut luma
+// Stage E at the plane's edge of a 4:2:0 or 4:2:2 tile: the pixels of the cut luma
 // cells, one a thread; chroma interpolated with its reads clamped to the
 // plane, as the general path does.  Returns the output flag.
-__device__ bool edge_pixels_420(const ImageDev &im, const int32_t *ytile, const int32_t *ctile, int mx0, int my0,
+template <int CV>
+__device__ bool edge_pixels_chroma(const ImageDev &im, const int32_t *ytile, const int32_t *ctile, int mx0, int my0,
                                 const EdgeCells &ec) {
     const OutputDev &o = im.out;
     const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
     const uint64_t chs = o.nchw ? o.plane_stride : (uint64_t)o.elem_bytes;
-    const int Wc = ec.W >> 1, Hc = ec.H >> 1, ox = 8 * mx0 - 8, oy = 8 * my0 - 8;
+    using CT = ChromaTile<CV>;
+    const int Wc = ec.W >> 1, Hc = CV == 2 ? ec.H >> 1 : ec.H, ox = 8 * mx0 - 8, oy = CT::sample0(my0);
     const int cells = ec.n[0] + ec.n[1] + ec.n[2] + ec.n[3];
     bool bad = false;
     for (int item = threadIdx.x; item < cells * 8; item += kThreads) {
@@ -2414,10 +2438,10 @@ __device__ bool edge_pixels_420(const ImageDev &im, const int32_t *ytile, const 
             continue;
         const int sx = x - 16 * mx0, sy = y - 16 * my0;
         int32_t comp[4] = {ytile[elem((sy >> 2) * kIB + (sx >> 2), sy & 3, sx & 3)], 0, 0, 0};
-        const int cx = x >> 1, cy = y >> 1;
+        const int cx = x >> 1, cy = CV == 2 ? y >> 1 : y;
 #pragma unroll
         for (int pc = 0; pc < 2; pc++) {
-            const int32_t *t = ctile + pc * kCPlaneInts;
+            const int32_t *t = ctile + pc * CT::kInts;
             auto C = [&](int a, int b) {
                 const int ta = min(max(a, 0), Wc - 1) - ox, tb = min(max(b, 0), Hc - 1) - oy;
                 return t[elem((tb >> 2) * kCB + (ta >> 2), tb & 3, ta & 3)];
@@ -2425,7 +2449,8 @@ __device__ bool edge_pixels_420(const ImageDev &im, const int32_t *ytile, const 
             int32_t col[3];
 #pragma unroll
             for (int d = -1; d <= 1; d++)
-                col[d + 1] = (y & 1) ? up_odd(C(cx + d, cy), C(cx + d, cy + 1), im.centering_y)
+                col[d + 1] = CV == 4 ? C(cx + d, cy)
+                           : (y & 1) ? up_odd(C(cx + d, cy), C(cx + d, cy + 1), im.centering_y)
                                      : up_even(C(cx + d, cy - 1), C(cx + d, cy), im.centering_y);
             comp[1 + pc] = (x & 1) ? up_odd(col[1], col[2], im.centering_x) : up_even(col[0], col[1], im.centering_x);
         }
@@ -2435,43 +2460,46 @@ __device__ bool edge_pixels_420(const ImageDev &im, const int32_t *ytile, const 
     return bad;
 }
 
-// Edge tiles (MODE 1, or MODE 2 by position): tiles of a 4:2:0 image (at
-// least 2 x 2 macroblocks) that touch the plane's edge, or, with at most one
+// Edge tiles (MODE 1, or MODE 2 by position): tiles of a 4:2:0 or 4:2:2 image
+// (at least 2 x 2 macroblocks) that touch the plane's edge, or, with at most one
 // overlap level, a hard tile boundary (the ordered first-level chroma corners
 // at hard boundaries stay with the general kernel), as the full-resolution
 // edge tiles, with the chroma planes'
 // first-level squares and second-level cells on the plane's edge taking the
 // edge operators (and corner residuals).
-template <int MODE>
-__device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *smem, const uint4 *mbc, uint4 *mbc_next,
+// 4:2:2 tiles took the general kernel before, at 46 k warp instructions a
+// tile (1920 x 1080 RGB8 from 4:2:2: 47.5 us, 24.3 us here).
+template <int MODE, int CV>
+__device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t *smem, const uint4 *mbc, uint4 *mbc_next,
                                   uint32_t claimed, const ImageDev *__restrict__ images,
                                   const WorkItem *__restrict__ items, uint32_t item_count, TileShared &sh,
                                   uint32_t *status) {
     const int mx0 = tx * kTileMbs, my0 = ty * kTileMbs;
     const int tid = threadIdx.x;
+    using CT = ChromaTile<CV>;
     const bool edge = MODE == 1 || (MODE == 2 && (mx0 == 0 || my0 == 0 || mx0 + kTileMbs >= (int)im.plane[0].mbs_x ||
                                                   my0 + kTileMbs >= (int)im.plane[0].mbs_y));
     int32_t *ytile = smem;                              // luma: 17 x 17 blocks
     int32_t *ydc = ytile + kPlaneInts;                  // 24 x 24
     int32_t *ylp = ydc + kDcInts;                       // 36 x 16
-    int32_t *ctile = ylp + kLpInts;                     // chroma: 2 x 11 x 11 blocks
-    int32_t *cdc = ctile + 2 * kCPlaneInts;             // 2 x 12 x 12
-    int32_t *clp = cdc + 2 * kCDC * kCDC;               // 2 x 36 x 4
+    int32_t *ctile = ylp + kLpInts;                     // chroma: 2 x 11 x 11 or 17 blocks
+    int32_t *cdc = ctile + 2 * CT::kInts;               // 2 x 12 x 12 or 24
+    int32_t *clp = cdc + 2 * CT::kDcInts;               // 2 x 36 x 4 or 8
     if (tid == 0) sh.bad = 0;
     if (MODE == 1 && tid < 32) {
         const uint32_t starts = hard_starts(im, mx0, my0);
         if (tid == 0) sh.hard = starts;
     }
     int bad = 0;
-    // phase 1: the DC / low-pass values (luma 16, chroma 4 a macroblock) of
+    // phase 1: the DC / low-pass values (luma 16, chroma 4 or 8 a macroblock) of
     // the ring of luma macroblocks and of the 6 x 6 chroma macroblocks, then
     // the blocks.  Those of the tile's own luma macroblocks arrive with their
     // blocks (coefficient 0 of each) and are read from the slots.
-    for (int k = tid; k < 320 + 2 * kCLpInts; k += kThreads) {
+    for (int k = tid; k < 320 + 2 * CT::kLpInts; k += kThreads) {
         int pi, m, kk;
         int32_t *dst;
         if (k < 320) { pi = 0; m = ring_mb(k >> 4); kk = k & 15; dst = ylp + m * 16 + kk; }
-        else { const int q = k - 320; pi = 1 + q / kCLpInts; const int r = q - (pi - 1) * kCLpInts; m = r >> 2; kk = r & 3; dst = clp + q; }
+        else { const int q = k - 320; pi = 1 + q / CT::kLpInts; const int r = q - (pi - 1) * CT::kLpInts; m = r / CT::kLow; kk = r % CT::kLow; dst = clp + q; }
         const uint4 e = mbc[pi * 36 + m];
         const int bands = (e.x >> 28) & 3;
         if (kk == 0 || bands != 0)
@@ -2497,11 +2525,12 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
                        (((j & 3) << 2) + (i & 3)) * 16 + r * 4);
         }
     }
-    for (int k = tid; k < 2 * kCBlocks * 4; k += kThreads) {
-        const int pc = k / (kCBlocks * 4), q = k - pc * (kCBlocks * 4), sidx = q >> 2, r = q & 3;
+    for (int k = tid; k < 2 * CT::kInts / 4; k += kThreads) {
+        const int pc = k / (CT::kInts / 4), q = k - pc * (CT::kInts / 4), sidx = q >> 2, r = q & 3;
         const int i = sidx % kCB, j = sidx / kCB;
-        copy_chunk(ctile + pc * kCPlaneInts + sidx * 16 + ((r ^ swz(sidx)) << 2), im.plane[1 + pc].coeff,
-                   mbc[(1 + pc) * 36 + (j >> 1) * 6 + (i >> 1)], (((j & 1) << 1) + (i & 1)) * 16 + r * 4);
+        copy_chunk(ctile + pc * CT::kInts + sidx * 16 + ((r ^ swz(sidx)) << 2), im.plane[1 + pc].coeff,
+                   mbc[(1 + pc) * 36 + (j / CV + 1 + CT::kFirstMb) * 6 + (i >> 1)],
+                   (((j % CV) << 1) + (i & 1)) * 16 + r * 4);
     }
     cp_async_commit();
     cp_async_wait_all();
@@ -2554,13 +2583,23 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
             for (int r = 0; r < 4; r++)
                 *reinterpret_cast<int4 *>(out + r * kIDC) = make_int4(v[r * 4], v[r * 4 + 1], v[r * 4 + 2], v[r * 4 + 3]);
         } else {
-            const int4 q = *reinterpret_cast<const int4 *>(clp + (pi - 1) * kCLpInts + m * 4);
-            int32_t w[4] = {dequant(q.x, e.y, b), dequant(q.y, e.z, b), dequant(q.z, e.z, b), dequant(q.w, e.z, b)};
-            b |= inverse_chroma_420<true>(w);
+            const int32_t *l = clp + (pi - 1) * CT::kLpInts + m * CT::kLow;
+            int32_t w[CT::kLow];
 #pragma unroll
-            for (int k = 0; k < 4; k++) w[k] = p.scale2 ? dequant(w[k], 2, b) : w[k];
-            int32_t *out = cdc + (pi - 1) * kCDC * kCDC + (m / 6) * 2 * kCDC + (m % 6) * 2;
-            out[0] = w[0]; out[1] = w[1]; out[kCDC] = w[2]; out[kCDC + 1] = w[3];
+            for (int k = 0; k < CT::kLow; k += 4) {
+                const int4 q = *reinterpret_cast<const int4 *>(l + k);
+                w[k] = dequant(q.x, k == 0 ? e.y : e.z, b);
+                w[k + 1] = dequant(q.y, e.z, b);
+                w[k + 2] = dequant(q.z, e.z, b);
+                w[k + 3] = dequant(q.w, e.z, b);
+            }
+            if constexpr (CV == 2) b |= inverse_chroma_420<true>(w);
+            else b |= inverse_chroma_422<true>(w);
+#pragma unroll
+            for (int k = 0; k < CT::kLow; k++) w[k] = p.scale2 ? dequant(w[k], 2, b) : w[k];
+            int32_t *out = cdc + (pi - 1) * CT::kDcInts + (m / 6) * CV * kCDC + (m % 6) * 2;
+#pragma unroll
+            for (int k = 0; k < CV; k++) { out[k * kCDC] = w[2 * k]; out[k * kCDC + 1] = w[2 * k + 1]; }
         }
         if (b) bad |= kFlagFirst;
     }
@@ -2575,30 +2614,34 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
     // rows and columns of the high-pass blocks); the overlap items go to
     // threads that get no second item.
     //   B: first-level overlap -- luma 5 x 5 windows at DC (2 + 4a, 2 + 4b),
-    //      chroma 5 x 5 squares at DC (1 + 2a, 1 + 2b);
+    //      chroma 5 x 5 (4:2:2: 5 x 9) squares at DC (1 + 2a, 1 (3) + 2b);
     //   C1: high-pass prediction.  Luma as in the full-resolution tile;
-    //      chroma within each 2 x 2-block macroblock: from left, block column
-    //      1 from column 0 of a block row; from top, block row 1 from row 0.
-    constexpr int kItemsB = 3 * 25, kItemsC1 = 100 + 2 * 72;
+    //      chroma within each 2-block-wide macroblock: from left, block column
+    //      1 from column 0 of a block row; from top, each block row from the
+    //      one above.
+    constexpr int kSq = 5 * CT::kSquares, kPred = 6 * CT::kMbRows * CV;
+    constexpr int kItemsB = 25 + 2 * kSq, kItemsC1 = 100 + 2 * kPred;
     constexpr int kFirstB = (kItemsB + kItemsC1 < kThreads ? kItemsB + kItemsC1 : kThreads) - kItemsB;
     for (int k = tid; k < kItemsB + kItemsC1; k += kThreads) {
         if (k >= kFirstB && k < kFirstB + kItemsB) {
             const int item = k - kFirstB;
-            const int pi = item / 25, c = item - pi * 25;
+            const int pi = item < 25 ? 0 : 1 + (item - 25) / kSq, c = item < 25 ? item : (item - 25) % kSq;
             if (im.plane[pi].overlap != 2) continue;
             bool b;
             if (edge) {
-                // the window's or square's centre lies on macroblock boundary (mx0 + a, my0 + b)
+                // the window's or square's centre lies on macroblock boundary
+                // (mx0 + a, my0 + b); a 4:2:2 square's, half a macroblock apart down
                 const PlaneDev &p = im.plane[pi];
-                const int ca = mx0 + c % 5, cb = my0 + c / 5;
-                if (ca > (int)p.mbs_x || cb > (int)p.mbs_y) continue;   // beyond the plane
-                const bool vs = ca == 0 || ca == (int)p.mbs_x, hs = cb == 0 || cb == (int)p.mbs_y;
+                const int down = CV == 4 && pi > 0 ? 2 : 1;
+                const int ca = mx0 + c % 5, cb = down * my0 + c / 5, rows = down * (int)p.mbs_y;
+                if (ca > (int)p.mbs_x || cb > rows) continue;   // beyond the plane
+                const bool vs = ca == 0 || ca == (int)p.mbs_x, hs = cb == 0 || cb == rows;
                 if (vs || hs) {
                     if (pi == 0)
                         b = dc_edge_window(ydc, 2 + 4 * (c % 5), 2 + 4 * (c / 5), 4 * (mx0 - 1), 4 * (my0 - 1),
                                            4 * (int)p.mbs_x, 4 * (int)p.mbs_y, vs, hs);
                     else
-                        b = chroma_edge_square(cdc + (pi - 1) * kCDC * kCDC, 1 + 2 * (c % 5), 1 + 2 * (c / 5), vs, hs,
+                        b = chroma_edge_square(cdc + (pi - 1) * CT::kDcInts, 1 + 2 * (c % 5), CT::kSquare0 + 2 * (c / 5), vs, hs,
                                                ca == 0, cb == 0, 2 * (mx0 - 1), 2 * (int)p.mbs_x);
                     if (b) bad |= kFlagOverlap;
                     continue;
@@ -2620,7 +2663,7 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
                     *reinterpret_cast<int2 *>(base + r * kIDC + 2) = make_int2(v[r * 4 + 2], v[r * 4 + 3]);
                 }
             } else {
-                int32_t *base = cdc + (pi - 1) * kCDC * kCDC + (1 + 2 * (c / 5)) * kCDC + 1 + 2 * (c % 5);
+                int32_t *base = cdc + (pi - 1) * CT::kDcInts + (CT::kSquare0 + 2 * (c / 5)) * kCDC + 1 + 2 * (c % 5);
                 b = inverse_pot2x2(base[0], base[1], base[kCDC], base[kCDC + 1]);
             }
             if (b) bad |= kFlagOverlap;
@@ -2657,25 +2700,30 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
                     }
                 }
             } else {
-                const int q = item - 100, pc = q / 72, rem = q - pc * 72, line = rem & 1, m = rem >> 1;
+                const int q = item - 100, pc = q / kPred, rem = q - pc * kPred, line = rem % CV, m = rem / CV;
                 const int a = m % 6, b = m / 6;
-                const uint4 e = mbc[(1 + pc) * 36 + m];
+                constexpr int last = CT::kMbRows - 1;
+                const uint4 e = mbc[(1 + pc) * 36 + (1 + CT::kFirstMb) * 6 + m];
                 const int hp = (e.x >> 30) & 3, bands = (e.x >> 28) & 3;
                 if (hp == 0 || bands < 2) continue;
                 if (hp == 3) { bad |= kFlagInvalid; continue; }
-                int32_t *t = ctile + pc * kCPlaneInts;
+                int32_t *t = ctile + pc * CT::kInts;
                 if (hp == 1) {
-                    // block row 2b + line: column 2a + 1 from column 2a
-                    if (a == 5 || (b == 5 && line != 0)) continue;
-                    const int sidx = (2 * b + line) * kCB + 2 * a + 1;
+                    // block row CV b + line: column 2a + 1 from column 2a
+                    if (a == 5 || (b == last && line != 0)) continue;
+                    const int sidx = (CV * b + line) * kCB + 2 * a + 1;
 #pragma unroll
                     for (int r = 1; r < 4; r++) t[elem(sidx, r, 0)] = A::add(t[elem(sidx, r, 0)], t[elem(sidx - 1, r, 0)], ov);
                 } else {
-                    // block column 2a + line: row 2b + 1 from row 2b
-                    if (b == 5 || (a == 5 && line != 0)) continue;
-                    const int sidx = (2 * b + 1) * kCB + 2 * a + line;
+                    // block column 2a + line: rows CV b + 1 .. from the row above
+                    if (line > 1 || b == last || (a == 5 && line != 0)) continue;
 #pragma unroll
-                    for (int c = 1; c < 4; c++) t[elem(sidx, 0, c)] = A::add(t[elem(sidx, 0, c)], t[elem(sidx - kCB, 0, c)], ov);
+                    for (int r = 1; r < CV; r++) {
+                        const int sidx = (CV * b + r) * kCB + 2 * a + line;
+#pragma unroll
+                        for (int c = 1; c < 4; c++)
+                            t[elem(sidx, 0, c)] = A::add(t[elem(sidx, 0, c)], t[elem(sidx - kCB, 0, c)], ov);
+                    }
                 }
             }
             if (ov) bad |= kFlagPrediction;
@@ -2683,16 +2731,17 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
     }
     cp_async_wait_all();
     __syncthreads();
-    // stage C2: block transforms -- luma 17 x 17, chroma blocks 1..10 x 1..10;
+    // stage C2: block transforms -- luma 17 x 17, chroma columns 1..10 and
+    // rows 1..10 (4:2:2: 0..16);
     // an edge tile's items are only its blocks inside the plane (divisions
     // as multiplies by ceil(2^16 / n), exact for these small quotients)
-    int lcols = kIB, lrows = kIB, lmagic = 0, ccols = 10, crows = 10, cmagic = 0;
+    int lcols = kIB, lrows = kIB, lmagic = 0, ccols = 10, crows = CT::kTransRows, cmagic = 0;
     if (edge) {
         const int rx = (int)im.plane[0].mbs_x - mx0, ry = (int)im.plane[0].mbs_y - my0;
         lcols = min(kIB, 4 * rx);
         lrows = min(kIB, 4 * ry);
         ccols = min(10, 2 * rx + 1);
-        crows = min(10, 2 * ry + 1);
+        crows = CV == 2 ? min(10, 2 * ry + 1) : min(17, 4 * ry);
         lmagic = (65536 + lcols - 1) / lcols;
         cmagic = (65536 + ccols - 1) / ccols;
     }
@@ -2724,18 +2773,18 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
                 pc = q >= ccount ? 1 : 0;
                 const int rem = q - pc * ccount, r = (rem * cmagic) >> 16;
                 i = 1 + rem - r * ccols;
-                j = 1 + r;
+                j = CT::kRow0 + r;
             } else {
-                pc = q / 100;
-                const int rem = q - pc * 100;
+                pc = q / (10 * CT::kTransRows);
+                const int rem = q - pc * (10 * CT::kTransRows);
                 i = 1 + rem % 10;
-                j = 1 + rem / 10;
+                j = CT::kRow0 + rem / 10;
             }
             const int sidx = j * kCB + i;
-            step = mbc[(1 + pc) * 36 + (j >> 1) * 6 + (i >> 1)].w;
-            blk = ctile + pc * kCPlaneInts + sidx * 16;
+            step = mbc[(1 + pc) * 36 + (j / CV + 1 + CT::kFirstMb) * 6 + (i >> 1)].w;
+            blk = ctile + pc * CT::kInts + sidx * 16;
             sw = swz(sidx);
-            dcv = cdc[pc * kCDC * kCDC + j * kCDC + i];
+            dcv = cdc[pc * CT::kDcInts + (j + CT::kDcRow0) * kCDC + i];
         }
         int32_t v[16];
 #pragma unroll
@@ -2766,29 +2815,31 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
     // a small tile's overlap outputs stay below 2^27.8, and the chroma
     // interpolated from them below 2^28: no magnitude tests below
     const bool tile_small = __syncthreads_and(small) != 0;
-    // stage D (chroma): the 9 x 9 second-level cells of each chroma plane, in place
-    for (int item = tid; item < 2 * 81; item += kThreads) {
-        const int pc = item / 81, c = item - pc * 81;
-        int32_t *t = ctile + pc * kCPlaneInts;
+    // stage D (chroma): the 9 x 9 (4:2:2: 9 x 16) second-level cells of each
+    // chroma plane, in place; cell column k of the luma tile's macroblock
+    // boundary a is 2a, cell row likewise, 4:2:2's 4b
+    for (int item = tid; item < 2 * 9 * CT::kCells; item += kThreads) {
+        const int pc = item / (9 * CT::kCells), c = item - pc * (9 * CT::kCells);
+        if (CV == 4 && c < 9 && !(edge && my0 == 0)) continue;   // the row above is another tile's
+        int32_t *t = ctile + pc * CT::kInts;
         if (edge) {
             // cells past the chroma plane's edge, or cut by it
-            const int Wc = 8 * (int)im.plane[1].mbs_x, Hc = 8 * (int)im.plane[1].mbs_y;
-            const int X = 8 * mx0 - 2 + 4 * (c % 9), Y = 8 * my0 - 2 + 4 * (c / 9);
+            const int Wc = 8 * (int)im.plane[1].mbs_x, Hc = 4 * CV * (int)im.plane[1].mbs_y;
+            const int X = 8 * mx0 - 2 + 4 * (c % 9), Y = CT::cell0(my0) + 4 * (c / 9);
             if (X >= Wc || Y >= Hc) continue;
             bool vs = X + 2 == 0 || X + 2 == Wc, hs = Y + 2 == 0 || Y + 2 == Hc;
             if (MODE == 1) {
-                // the cell's middle is on macroblock boundary (c % 9) / 2 (c / 9 / 2) where that is even
-                vs |= ((c % 9) & 1) == 0 && ((sh.hard >> ((c % 9) >> 1)) & 1);
-                hs |= ((c / 9) & 1) == 0 && ((sh.hard >> (8 + ((c / 9) >> 1))) & 1);
+                vs |= (c % 9) % 2 == 0 && ((sh.hard >> ((c % 9) / 2)) & 1);
+                hs |= (c / 9) % CV == 0 && ((sh.hard >> (8 + (c / 9) / CV)) & 1);
             }
             if (vs || hs) {
-                if (im.plane[1 + pc].overlap >= 1 && chroma_cut_cell(t, X, Y, 8 * mx0 - 8, 8 * my0 - 8, Wc, Hc, vs, hs))
+                if (im.plane[1 + pc].overlap >= 1 && chroma_cut_cell(t, X, Y, 8 * mx0 - 8, CT::sample0(my0), Wc, Hc, vs, hs))
                     bad |= kFlagOverlap;
                 continue;
             }
         }
         int32_t w[16];
-        if (cell_rw(t, (1 + c / 9) * kCB + 1 + c % 9, kCB, im.plane[1 + pc].overlap, w, true, tile_small))
+        if (cell_rw(t, (CV == 2 ? 1 + c / 9 : c / 9 - 1) * kCB + 1 + c % 9, kCB, im.plane[1 + pc].overlap, w, true, tile_small))
             bad |= kFlagOverlap;
     }
     EdgeCells ec;
@@ -2815,7 +2866,7 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
         bool obad = false, done = false;
         int32_t y[16];
         if (cell_rw(ytile, cy * kIB + cx, kIB, MODE == 1 && cut ? 0 : im.plane[0].overlap, y, false, tile_small)) bad |= kFlagOverlap;
-        // chroma samples (tile coordinates) 8 + 2cx .. 11 + 2cx, 8 + 2cy .. 11 + 2cy
+        // chroma columns (tile coordinates) 8 + 2cx .. 11 + 2cx, rows 8 + 2cy .. 11 + 2cy (4:2:2: 2 + 4cy .. 5 + 4cy)
         if (tile_small && !edge && inside && o.kind == kOutRgb8 && !o.premultiply &&
             (o.channels == 3 || o.ch[3].padding)) {
             // RGB8 of an interior small tile, row by row: each luma row's
@@ -2835,7 +2886,16 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
                 int32_t ch[2][4];
 #pragma unroll
                 for (int pc = 0; pc < 2; pc++) {
-                    const int32_t *t = ctile + pc * kCPlaneInts;
+                    const int32_t *t = ctile + pc * CT::kInts;
+                    int32_t col[4];
+                    if (CV == 4) {
+#pragma unroll
+                        for (int h = 0; h < 2; h++) {
+                            const int sx = 8 + 2 * cx + 2 * h, sy = 2 + 4 * cy + r;
+                            const int2 p = *reinterpret_cast<const int2 *>(&t[elem((sy >> 2) * kCB + (sx >> 2), sy & 3, sx & 3)]);
+                            col[2 * h] = p.x; col[2 * h + 1] = p.y;
+                        }
+                    } else {
                     int32_t sa[4], sb[4];
 #pragma unroll
                     for (int h = 0; h < 2; h++) {
@@ -2845,10 +2905,10 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
                         sa[2 * h] = pa.x; sa[2 * h + 1] = pa.y;
                         sb[2 * h] = pb.x; sb[2 * h + 1] = pb.y;
                     }
-                    int32_t col[4];
 #pragma unroll
                     for (int k = 0; k < 4; k++)
                         col[k] = (r & 1) ? up_odd_small(sa[k], sb[k], cyc) : up_even_small(sa[k], sb[k], cyc);
+                    }
 #pragma unroll
                     for (int c = 0; c < 4; c++)
                         ch[pc][c] = (c & 1) ? up_odd_small(col[1 + (c >> 1)], col[2 + (c >> 1)], cxc)
@@ -2870,11 +2930,11 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
         int32_t u[16], v[16];
 #pragma unroll
         for (int pc = 0; pc < 2 && !done; pc++) {
-            const int32_t *t = ctile + pc * kCPlaneInts;
+            const int32_t *t = ctile + pc * CT::kInts;
             int32_t s[4][4];
 #pragma unroll
             for (int r = 0; r < 4; r++) {
-                const int sy = 8 + 2 * cy + r;
+                const int sy = CV == 2 ? 8 + 2 * cy + r : 2 + 4 * cy + r;
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const int sx = 8 + 2 * cx + 2 * h;
@@ -2902,7 +2962,8 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
                     int32_t col[4];
 #pragma unroll
                     for (int k = 0; k < 4; k++)
-                        col[k] = (r & 1) ? up_odd_small(s[1 + (r >> 1)][k], s[2 + (r >> 1)][k], im.centering_y)
+                        col[k] = CV == 4 ? s[r][k]
+                               : (r & 1) ? up_odd_small(s[1 + (r >> 1)][k], s[2 + (r >> 1)][k], im.centering_y)
                                          : up_even_small(s[(r >> 1)][k], s[1 + (r >> 1)][k], im.centering_y);
 #pragma unroll
                     for (int c = 0; c < 4; c++)
@@ -2916,7 +2977,8 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
                     int32_t col[4];
 #pragma unroll
                     for (int k = 0; k < 4; k++)
-                        col[k] = (r & 1) ? up_odd(s[1 + (r >> 1)][k], s[2 + (r >> 1)][k], im.centering_y)
+                        col[k] = CV == 4 ? s[r][k]
+                               : (r & 1) ? up_odd(s[1 + (r >> 1)][k], s[2 + (r >> 1)][k], im.centering_y)
                                          : up_even(s[(r >> 1)][k], s[1 + (r >> 1)][k], im.centering_y);
 #pragma unroll
                     for (int c = 0; c < 4; c++)
@@ -2974,7 +3036,7 @@ __device__ void interior_tile_420(const ImageDev &im, int tx, int ty, int32_t *s
         }
         if (obad) bad |= kFlagOutput;
     }
-    if (edge && edge_pixels_420(im, ytile, ctile, mx0, my0, ec)) bad |= kFlagOutput;
+    if (edge && edge_pixels_chroma<CV>(im, ytile, ctile, mx0, my0, ec)) bad |= kFlagOutput;
     if (bad) atomicOr(&sh.bad, bad);
     __syncthreads();
     if (tid == 0 && sh.bad) {
@@ -3004,15 +3066,16 @@ __device__ __forceinline__ void hold_image(const ImageDev *__restrict__ images, 
     __syncthreads();
 }
 
-// Tiles of YUV 4:2:0 images: interior (MODE 0), edge (MODE 1) or both (MODE 2).
-template <int MODE>
+// Tiles of YUV 4:2:0 (CV 2) and 4:2:2 (CV 4) images: interior (MODE 0), edge
+// (MODE 1) or both (MODE 2).
+template <int MODE, int CV>
 __global__ void __launch_bounds__(kThreads, 3)
-jxrb_interior420_tiles(const ImageDev *__restrict__ images, const WorkItem *__restrict__ items, uint32_t item_count,
+jxrb_interior_chroma_tiles(const ImageDev *__restrict__ images, const WorkItem *__restrict__ items, uint32_t item_count,
                        uint32_t *status, uint32_t *counters) {
-    extern __shared__ __align__(16) int32_t smem_420[];
+    extern __shared__ __align__(16) int32_t smem_chroma[];
     __shared__ TileShared sh;
     uint4 *mbc[2];
-    mbc[0] = reinterpret_cast<uint4 *>(smem_420 + kSmem420Ints - 2 * 3 * kMbcInts);
+    mbc[0] = reinterpret_cast<uint4 *>(smem_chroma + ChromaTile<CV>::kSmemInts - 2 * 3 * kMbcInts);
     mbc[1] = mbc[0] + 3 * 36;
     uint32_t i;
     if (claim(counters, item_count, i)) {
@@ -3028,7 +3091,7 @@ jxrb_interior420_tiles(const ImageDev *__restrict__ images, const WorkItem *__re
             const uint32_t claimed = threadIdx.x == 0 ? atomicAdd(&counters[0], 1u) : 0u;
             const WorkItem cur = items[i];
             hold_image(images, cur.image & kImageMask, simg, held);
-            interior_tile_420<MODE>(simg, cur.tx, cur.ty, smem_420, mbc[buf], mbc[buf ^ 1],
+            interior_tile_chroma<MODE, CV>(simg, cur.tx, cur.ty, smem_chroma, mbc[buf], mbc[buf ^ 1],
                                     claimed, images, items, item_count, sh, status);
             i = sh.next;
             __syncthreads();
@@ -3112,26 +3175,36 @@ static TileKernel segment_kernel(int segment) {
     case 1: return interior_kernel<2>();
     case 2: return interior_kernel<3>();
     case 3: return interior_kernel<4>();
-    case 4: return kFoldEdges[4] ? jxrb_interior420_tiles<2> : jxrb_interior420_tiles<0>;
-    case 5: return jxrb_interior_tiles<1, 1>;
-    case 6: return jxrb_interior_tiles<2, 1>;
-    case 7: return jxrb_interior_tiles<3, 1>;
-    case 8: return jxrb_interior_tiles<4, 1>;
-    case 9: return jxrb_interior420_tiles<1>;
+    case 4: return jxrb_interior_chroma_tiles<kFoldEdges[4] ? 2 : 0, 2>;
+    case 5: return jxrb_interior_chroma_tiles<0, 4>;
+    case 6: return jxrb_interior_tiles<1, 1>;
+    case 7: return jxrb_interior_tiles<2, 1>;
+    case 8: return jxrb_interior_tiles<3, 1>;
+    case 9: return jxrb_interior_tiles<4, 1>;
+    case 10: return jxrb_interior_chroma_tiles<1, 2>;
+    case 11: return jxrb_interior_chroma_tiles<1, 4>;
     default: return jxrb_reconstruct_tiles;
     }
+}
+
+// Segments of subsampled images: 4:2:0, 4:2:2, and their edge tiles.
+static bool chroma_segment(int segment) {
+    return segment == 4 || segment == 5 || segment == kSegmentOther - 2 || segment == kSegmentOther - 1;
 }
 
 // Planes of a segment's tiles (the general kernel: the set's most).
 static int segment_planes(int segment, int max_planes) {
     if (segment < 4) return segment + 1;
-    if (segment == 4 || segment == 9) return 3;
-    if (segment < kSegmentOther) return segment - 4;
+    if (chroma_segment(segment)) return 3;
+    if (segment < kSegmentOther) return segment - kSideSegment0 + 1;
     return max_planes;
 }
 
 static size_t segment_smem_bytes(int segment, int max_planes) {
-    if (segment == 4 || segment == 9) return (size_t)kSmem420Ints * sizeof(int32_t);
+    if (chroma_segment(segment)) {
+        const bool c422 = segment == 5 || segment == kSegmentOther - 1;
+        return (size_t)(c422 ? ChromaTile<4>::kSmemInts : ChromaTile<2>::kSmemInts) * sizeof(int32_t);
+    }
     if (segment < kSegmentOther) return interior_smem_bytes(segment_planes(segment, max_planes));
     return tile_smem_bytes(max_planes);
 }

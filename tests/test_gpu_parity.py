@@ -335,6 +335,28 @@ def test_hard_tiles_in_the_edge_kernels(session, tiles, overlap, fmt):
         check(session, img, out)
 
 
+@pytest.mark.parametrize("size", [(32, 32), (48, 32), (32, 80), (64, 64), (80, 144), (16, 48), (336, 304)])
+@pytest.mark.parametrize("overlap", [0, 1, 2])
+@pytest.mark.parametrize("tiles", [(0, 0, 0), (1, 2, 1), (3, 4, 1), (7, 5, 1)])
+def test_yuv422_tiles(session, size, overlap, tiles):
+    """4:2:2 interior and edge tiles, and their hard tiles: planes of part of a
+    tile, one tile exactly, one macroblock more, one macroblock wide; every
+    chroma centering, crops at odd pixels, other outputs than RGB8, random
+    coefficients up to the checked operators."""
+    w, h = size
+    tw, th, hard = tiles
+    kw = dict(color_format=C_["YUV422"], overlap=overlap, tile_width=tw, tile_height=th, hard_tiles=hard)
+    img = J.synth(w, h, quality=70, seed=300 + w + overlap, **kw)
+    check(session, img, rgb8(w, h))
+    for centering in [(0, 0), (1, 3), (4, 2)]:
+        img.geometry.chroma_centering_x, img.geometry.chroma_centering_y = centering
+        check(session, img, rgb8(w - 3, h - 2, crop_x=1, crop_y=1))
+    check(session, img, J.OutputFormat(C_["RGB"], D["U8"], S["U8"], L["BGRX"], w, h))
+    check(session, img, J.OutputFormat(C_["RGB"], D["U8"], S["U8"], L["RGB"], w, h, nchw=1))
+    rnd = J.synth(w, h, content=J.CONTENT["RANDOM"], seed=310 + h, **kw)
+    check(session, rnd, rgb8(w, h), expect_ok=False)
+
+
 def test_edge_tiles_overflow(session):
     img = J.synth(208, 176, quality=75, overlap=2, seed=140)
     img.arena.coefficients[:64] = 2**30
