@@ -1129,25 +1129,42 @@ template <int NP> __host__ __device__ constexpr int lp_stride() { return NP == 3
 template <int NP> __host__ __device__ constexpr int lp_ints() { return 36 * lp_stride<NP>(); }
 constexpr int kMbcInts = 36 * 4;    // their 16-byte entries
 
+// `n` little-endian words to any address: whole words where the destination
+// is aligned, the two ends in bytes and half-words.  The rows of images whose
+// width is no multiple of four start at every byte of a word; twelve single
+// bytes for such rows cost a 3999 x 2999 4:2:0 decode 13 us (107.5 us, 94.7 us here).
+template <int N>
+__device__ __forceinline__ void store_words(uint8_t *d, const uint32_t (&w)[N]) {
+    const uint32_t m = (uint32_t)reinterpret_cast<uintptr_t>(d) & 3;
+    uint32_t *q = reinterpret_cast<uint32_t *>(d + ((4 - m) & 3));
+    if (m == 0) {
+#pragma unroll
+        for (int k = 0; k < N; k++) q[k] = w[k];
+    } else if (m == 2) {
+        *reinterpret_cast<uint16_t *>(d) = (uint16_t)w[0];
+#pragma unroll
+        for (int k = 0; k + 1 < N; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 16);
+        *reinterpret_cast<uint16_t *>(d + 4 * N - 2) = (uint16_t)(w[N - 1] >> 16);
+    } else if (m == 1) {
+        d[0] = (uint8_t)w[0];
+        *reinterpret_cast<uint16_t *>(d + 1) = (uint16_t)(w[0] >> 8);
+#pragma unroll
+        for (int k = 0; k + 1 < N; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 24);
+        d[4 * N - 1] = (uint8_t)(w[N - 1] >> 24);
+    } else {
+        d[0] = (uint8_t)w[0];
+#pragma unroll
+        for (int k = 0; k + 1 < N; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 8);
+        *reinterpret_cast<uint16_t *>(d + 4 * N - 3) = (uint16_t)(w[N - 1] >> 8);
+        d[4 * N - 1] = (uint8_t)(w[N - 1] >> 24);
+    }
+}
+
 __device__ __forceinline__ void store12(uint8_t *d, const uint32_t px[4]) {
     // R0 G0 B0 R1 | G1 B1 R2 G2 | B2 R3 G3 B3
-    const uint32_t w0 = (px[0] & 0xffffffu) | (px[1] << 24);
-    const uint32_t w1 = ((px[1] >> 8) & 0xffffu) | (px[2] << 16);
-    const uint32_t w2 = ((px[2] >> 16) & 0xffu) | ((px[3] & 0xffffffu) << 8);
-    const uintptr_t a = reinterpret_cast<uintptr_t>(d);
-    if ((a & 3) == 0) {
-        uint32_t *q = reinterpret_cast<uint32_t *>(d);
-        q[0] = w0; q[1] = w1; q[2] = w2;
-    } else if ((a & 1) == 0) {
-        *reinterpret_cast<uint16_t *>(d) = (uint16_t)w0;
-        *reinterpret_cast<uint32_t *>(d + 2) = (w0 >> 16) | (w1 << 16);
-        *reinterpret_cast<uint32_t *>(d + 6) = (w1 >> 16) | (w2 << 16);
-        *reinterpret_cast<uint16_t *>(d + 10) = (uint16_t)(w2 >> 16);
-    } else {
-        const uint32_t w[3] = {w0, w1, w2};
-#pragma unroll
-        for (int k = 0; k < 12; k++) d[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
-    }
+    const uint32_t w[3] = {(px[0] & 0xffffffu) | (px[1] << 24), ((px[1] >> 8) & 0xffffu) | (px[2] << 16),
+                           ((px[2] >> 16) & 0xffu) | ((px[3] & 0xffffffu) << 8)};
+    store_words(d, w);
 }
 
 __device__ __forceinline__ void store16(uint8_t *d, uint32_t a, uint32_t b, uint32_t c, uint32_t e) {
@@ -1168,16 +1185,11 @@ __device__ __forceinline__ void store16(uint8_t *d, uint32_t a, uint32_t b, uint
 }
 
 __device__ __forceinline__ void store8(uint8_t *d, uint32_t a, uint32_t b) {
-    const uintptr_t p = reinterpret_cast<uintptr_t>(d);
-    if ((p & 7) == 0) {
+    if ((reinterpret_cast<uintptr_t>(d) & 7) == 0) {
         *reinterpret_cast<uint2 *>(d) = make_uint2(a, b);
-    } else if ((p & 3) == 0) {
-        reinterpret_cast<uint32_t *>(d)[0] = a;
-        reinterpret_cast<uint32_t *>(d)[1] = b;
     } else {
         const uint32_t w[2] = {a, b};
-#pragma unroll
-        for (int k = 0; k < 8; k++) d[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
+        store_words(d, w);
     }
 }
 
@@ -1924,7 +1936,10 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 uint8_t *dst = o.base + (uint64_t)(y0 + r - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * eb;
                 if (eb == 2) store8(dst, (q[0] & 0xffffu) | (q[1] << 16), (q[2] & 0xffffu) | (q[3] << 16));
                 else if (eb == 4) store16(dst, q[0], q[1], q[2], q[3]);
-                else for (int c = 0; c < 4; c++) dst[c] = (uint8_t)q[c];
+                else {
+                    const uint32_t w[1] = {(q[0] & 0xffu) | ((q[1] & 0xffu) << 8) | ((q[2] & 0xffu) << 16) | (q[3] << 24)};
+                    store_words(dst, w);
+                }
             }
             done = true;
         } else if (inside && kind == kOutF16Wide && o.nchw && NP == 4 && o.channels <= NP) {
