@@ -156,12 +156,16 @@ constexpr int kSegmentOther = kSegments - 1;
 constexpr bool kFoldEdges[kKinds] = {false, false, true, false, false, false};
 constexpr int kCounterWords = 2 * kSegments;   // two scheduling words a segment
 
+// Side streams a set's kernels may run on beside its own: with the set's
+// stream, one for each of the six kinds of tiles a mixed set holds.
+constexpr int kMaxSides = 5;
+
 // Launch shape of the tile kernels, chosen by the autotuner.  Entries 0..3
 // serve the full-resolution segments by plane count, entry 4 the other tiles;
 // the subsampled segments, three-plane kernels, take entry 2.
 struct LaunchTuning {
     uint32_t blocks_per_sm[5];   // resident CTAs per SM; 0 = as many as fit
-    int32_t side_stream;         // other tiles' kernel on a second stream beside the interior ones
+    int32_t side_stream;         // the segments' kernels on streams beside each other
 };
 
 // Where the descriptors of one plan sit inside a fixed device region (the

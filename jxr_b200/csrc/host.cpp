@@ -30,8 +30,8 @@
 namespace jxr {
 size_t tile_smem_bytes(int planes);
 cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32_t *bounds, int max_planes,
-                         uint32_t *status, uint32_t *counters, cudaStream_t stream, cudaStream_t side,
-                         cudaEvent_t fork, cudaEvent_t join, const LaunchTuning *tune);
+                         uint32_t *status, uint32_t *counters, const cudaStream_t *lanes, int lane_count,
+                         const LaunchTuning *tune);
 int tile_mbs();
 cudaError_t launch_quarter(const ImageDev *images, const QuarterImage *quarters, uint32_t count,
                            const QuarterPlane *planes, uint32_t plane_count, bool two_level, bool sixteenth_sums,
@@ -714,6 +714,37 @@ private:
 // ---------------------------------------------------------------------------
 // device buffers of one launch set (one or more images)
 // ---------------------------------------------------------------------------
+// Side streams forked from a stream and joined back to it by a launch.
+struct Sides {
+    std::vector<cudaStream_t> streams;
+    std::vector<cudaEvent_t> joins;   // one a stream
+    cudaEvent_t fork = nullptr;
+
+    jxrb_status grow(int n) {
+        if (n > 0 && !fork) CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "cudaEventCreate");
+        while ((int)streams.size() < n) {
+            cudaStream_t st = nullptr;
+            cudaEvent_t e = nullptr;
+            CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
+            streams.push_back(st);
+            CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+            joins.push_back(e);
+        }
+        return JXRB_OK;
+    }
+    void release() {
+        for (cudaStream_t st : streams) {
+            cudaStreamSynchronize(st);
+            cudaStreamDestroy(st);
+        }
+        for (cudaEvent_t e : joins) cudaEventDestroy(e);
+        if (fork) cudaEventDestroy(fork);
+        streams.clear();
+        joins.clear();
+        fork = nullptr;
+    }
+};
+
 struct DeviceSet {
     void *mem = nullptr;              // one allocation
     bool stream_ordered = false;      // allocated with cudaMallocAsync
@@ -724,9 +755,8 @@ struct DeviceSet {
     uint32_t *counters = nullptr;     // two words a kernel segment (dynamic tile scheduling)
     uint32_t item_count = 0;
     uint32_t bounds[kSegments + 1] = {};   // work-list segment boundaries (engine.h)
-    cudaStream_t side = nullptr;      // second stream for the other tiles' kernel
-    bool own_side = true;             // created for this set (else the session's)
-    cudaEvent_t fork = nullptr, join = nullptr;
+    Sides own_sides;                  // this set's own side streams,
+    Sides *sides = nullptr;           // or the session's for the stream it runs on
     LaunchTuning tune{{0, 0, 0, 0, 0}, 1};
     int max_planes = 1;
     // quarter-resolution requests (request sets only)
@@ -749,11 +779,26 @@ struct DeviceSet {
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// Side streams a set's launch uses: each kernel of its work list, and the
+// chain of reduced-resolution kernels, beside the others.  One after another
+// on a stream they leave the GPU half empty at each one's end.  Submissions
+// take the side streams of their session's stream: a stream and its events
+// made and destroyed for each cost a small decode about as much as the rest of
+// it (192 x 144 4:2:0, host to host: 234 us, 120 us without; 24 mixed requests
+// 383 us on two streams, 337 us on six).
+int side_streams(const DeviceSet &set) {
+    int n = set.q_count ? 1 : 0;
+    for (int k = 0; k < kSegments; k++) n += set.bounds[k + 1] > set.bounds[k];
+    return std::min(std::max(n - 1, 0), kMaxSides);
+}
+
 // Lay out, allocate and upload every input of `plans`; output pointers are
 // bound later by bind_output.  Copies run on `stream`; the host buffers are
 // read before this returns (a synchronize on pageable sources).
+// The set's kernels run beside each other on `sides`, or, without, on side
+// streams of its own.
 jxrb_status build_device_set(const jxrb_plan *const *plans, uint32_t count, cudaStream_t stream, DeviceSet &set,
-                             Staging *staging = nullptr) {
+                             Staging *staging = nullptr, Sides *sides = nullptr) {
     set.host_images.assign(count, ImageDev{});
     set.image_items.assign(count + 1, 0);
     set.output_offsets.assign(count, 0);
@@ -888,12 +933,8 @@ jxrb_status build_device_set(const jxrb_plan *const *plans, uint32_t count, cuda
                              stream), "upload work list");
     CUDA_TRY(cudaMemsetAsync(set.counters, 0, kCounterWords * sizeof(uint32_t), stream), "counter reset");
     CUDA_TRY(cudaMemsetAsync(set.status, 0, sizeof(uint32_t), stream), "status reset");
-    // the other tiles' kernel runs on a second stream beside the interior ones
-    if (set.bounds[kSegments] > set.bounds[kSideSegment0] && set.bounds[kSideSegment0] > 0 && !set.side) {
-        CUDA_TRY(cudaStreamCreateWithFlags(&set.side, cudaStreamNonBlocking), "cudaStreamCreate");
-        CUDA_TRY(cudaEventCreateWithFlags(&set.fork, cudaEventDisableTiming), "cudaEventCreate");
-        CUDA_TRY(cudaEventCreateWithFlags(&set.join, cudaEventDisableTiming), "cudaEventCreate");
-    }
+    set.sides = sides ? sides : &set.own_sides;
+    TRY(set.sides->grow(side_streams(set)));
     return JXRB_OK;
 }
 
@@ -938,7 +979,7 @@ jxrb_status bind_output(DeviceSet &set, uint8_t *dst, cudaStream_t stream) {
 struct jxrb_session {
     int device = 0;
     std::vector<cudaStream_t> streams;
-    std::vector<cudaStream_t> sides;   // per stream: where requests' edge-tile kernels run beside it
+    std::vector<Sides> sides;   // per stream: requests' kernels run on them beside it (under `lock`)
     std::atomic<uint32_t> next_stream{0};
     std::mutex lock;   // serialises encoding of submissions (runtime.rs:42)
     std::atomic<uint64_t> submissions{0}, uploaded{0}, read_back{0}, held{0}, launches{0};
@@ -957,10 +998,8 @@ size_t pick_stream(jxrb_session *s) {
     const size_t start = s->next_stream++ % n;
     for (size_t d = 0; d < n; d++) {
         const size_t k = (start + d) % n;
-        const cudaError_t a = cudaStreamQuery(s->streams[k]);
-        const cudaError_t b = a == cudaSuccess ? cudaStreamQuery(s->sides[k]) : a;
-        if (a != cudaSuccess || b != cudaSuccess) cudaGetLastError();   // not-ready is no error to report later
-        if (a == cudaSuccess && b == cudaSuccess) return k;
+        if (cudaStreamQuery(s->streams[k]) == cudaSuccess) return k;   // its side streams join it
+        cudaGetLastError();   // not-ready is no error to report later
     }
     return start;
 }
@@ -1042,27 +1081,45 @@ jxrb_status check_session(jxrb_session *s) {
 }
 
 void release_set(DeviceSet &set) {
-    if (set.side && set.own_side) {
-        cudaStreamSynchronize(set.side);
-        cudaStreamDestroy(set.side);
-    }
-    set.side = nullptr;
-    if (set.fork) cudaEventDestroy(set.fork);
-    if (set.join) cudaEventDestroy(set.join);
-    set.fork = set.join = nullptr;
+    set.own_sides.release();
+    set.sides = nullptr;
 }
 
 jxrb_status launch_set(jxrb_session *s, DeviceSet &set, cudaStream_t stream) {
-    cudaError_t e = launch_tiles(set.images, set.items, set.bounds, set.max_planes, set.status, set.counters, stream,
-                                 set.side, set.fork, set.join, &set.tune);
-    if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
-    for (int k = 0; k < kSegments; k++) s->launches += set.bounds[k + 1] > set.bounds[k];
-    if (set.q_count) {
-        e = launch_quarter(set.images, set.quarters, set.q_count, set.qplanes, set.q_planes, set.q_two_level,
-                           set.q_sixteenth_sums, set.q_max_mbs, set.q_max_samples, set.q_max_rows, set.status, stream);
-        if (e != cudaSuccess) return cuda_fail(e, "reduced-resolution launch");
-        s->launches += 3 + (set.q_two_level ? 3 : 0) + (set.q_sixteenth_sums ? 1 : 0);
+    // lanes: the side streams, then the set's own
+    const int sides = set.sides && set.tune.side_stream ? std::min(side_streams(set), (int)set.sides->streams.size()) : 0;
+    cudaStream_t lanes[kMaxSides + 1];
+    if (sides > 0) CUDA_TRY(cudaEventRecord(set.sides->fork, stream), "cudaEventRecord");
+    int forked = 0;
+    cudaError_t e = cudaSuccess;
+    while (forked < sides && e == cudaSuccess) {
+        e = cudaStreamWaitEvent(set.sides->streams[forked], set.sides->fork, 0);
+        if (e == cudaSuccess) {
+            lanes[forked] = set.sides->streams[forked];
+            forked++;
+        }
     }
+    lanes[forked] = stream;
+    const int n = forked + 1, first = set.q_count && n > 1 ? 1 : 0;
+    if (e == cudaSuccess && set.q_count) {
+        e = launch_quarter(set.images, set.quarters, set.q_count, set.qplanes, set.q_planes, set.q_two_level,
+                           set.q_sixteenth_sums, set.q_max_mbs, set.q_max_samples, set.q_max_rows, set.status, lanes[0]);
+        if (e == cudaSuccess) s->launches += 3 + (set.q_two_level ? 3 : 0) + (set.q_sixteenth_sums ? 1 : 0);
+    }
+    if (e == cudaSuccess) {
+        e = launch_tiles(set.images, set.items, set.bounds, set.max_planes, set.status, set.counters, lanes + first,
+                         n - first, &set.tune);
+        if (e == cudaSuccess)
+            for (int k = 0; k < kSegments; k++) s->launches += set.bounds[k + 1] > set.bounds[k];
+    }
+    // join whatever was forked, after a failed launch too: the set's memory is
+    // released in the order of `stream` alone
+    for (int k = 0; k < forked; k++) {
+        cudaError_t j = cudaEventRecord(set.sides->joins[k], set.sides->streams[k]);
+        if (j == cudaSuccess) j = cudaStreamWaitEvent(stream, set.sides->joins[k], 0);
+        if (e == cudaSuccess) e = j;
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "kernel launch");
     return JXRB_OK;
 }
 
@@ -1085,13 +1142,14 @@ jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32
         if (!plans[i]) return fail(JXRB_INVALID_PLAN, "null plan");
     std::unique_ptr<jxrb_submission> sub(new jxrb_submission);
     sub->session = s;
-    sub->stream = s->streams[pick_stream(s)];
+    const size_t lane = pick_stream(s);
+    sub->stream = s->streams[lane];
     std::lock_guard<std::mutex> guard(s->lock);
     CUDA_TRY(cudaEventCreate(&sub->begin), "cudaEventCreate");
     CUDA_TRY(cudaEventCreate(&sub->launched), "cudaEventCreate");
     CUDA_TRY(cudaEventRecord(sub->begin, sub->stream), "cudaEventRecord");
     if (!s->staging) s->staging.reset(new Staging);
-    TRY(build_device_set(plans, count, sub->stream, sub->set, s->staging.get()));
+    TRY(build_device_set(plans, count, sub->stream, sub->set, s->staging.get(), &s->sides[lane]));
     if (dst) {
         if (dst_len < sub->set.output_bytes) return fail(JXRB_INVALID_DESTINATION, "destination is smaller than the output");
         sub->output = static_cast<uint8_t *>(dst);
@@ -1359,12 +1417,11 @@ jxrb_status jxrb_session_create(int ordinal, const jxrb_session_options *options
     s->device = ordinal;
     const uint32_t streams = options && options->streams ? options->streams : 4;
     for (uint32_t i = 0; i < streams; i++) {
-        cudaStream_t st, side;
+        cudaStream_t st;
         CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
         s->streams.push_back(st);
-        CUDA_TRY(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking), "cudaStreamCreate");
-        s->sides.push_back(side);
     }
+    s->sides.resize(streams);
     CUDA_TRY(cudaStreamCreateWithFlags(&s->upload, cudaStreamNonBlocking), "cudaStreamCreate");
     *out = s.release();
     return JXRB_OK;
@@ -1374,11 +1431,10 @@ void jxrb_session_destroy(jxrb_session *s) {
     if (!s) return;
     cudaSetDevice(s->device);
     for (cudaStream_t st : s->streams) cudaStreamSynchronize(st);
-    for (cudaStream_t st : s->sides) cudaStreamSynchronize(st);
+    for (Sides &sd : s->sides) sd.release();
     if (s->upload) cudaStreamSynchronize(s->upload);
     s->staging.reset();
     for (cudaStream_t st : s->streams) cudaStreamDestroy(st);
-    for (cudaStream_t st : s->sides) cudaStreamDestroy(st);
     if (s->upload) cudaStreamDestroy(s->upload);
     delete s;
 }
@@ -2080,12 +2136,8 @@ jxrb_status build_request_set(jxrb_session *s, const jxrb_request *const *reqs, 
                                  stream), "upload quarter-resolution descriptors");
     CUDA_TRY(cudaMemsetAsync(set.counters, 0, kCounterWords * sizeof(uint32_t), stream), "counter reset");
     CUDA_TRY(cudaMemsetAsync(set.status, 0, sizeof(uint32_t), stream), "status reset");
-    if (set.bounds[kSegments] > set.bounds[kSideSegment0] && set.bounds[kSideSegment0] > 0) {
-        set.side = s->sides[side_index];
-        set.own_side = false;
-        CUDA_TRY(cudaEventCreateWithFlags(&set.fork, cudaEventDisableTiming), "cudaEventCreate");
-        CUDA_TRY(cudaEventCreateWithFlags(&set.join, cudaEventDisableTiming), "cudaEventCreate");
-    }
+    TRY(s->sides[side_index].grow(side_streams(set)));
+    set.sides = &s->sides[side_index];
     return JXRB_OK;
 }
 
@@ -2198,12 +2250,10 @@ void jxrb_image_destroy(jxrb_image *img) {
     // so far (requests on this image among it).  A serving loop evicting
     // images under its budget keeps its batches in flight meanwhile.
     bool ordered = img->mem != nullptr;
-    for (size_t k = 0; ordered && k < s->streams.size() + s->sides.size(); k++) {
-        cudaStream_t st = k < s->streams.size() ? s->streams[k] : s->sides[k - s->streams.size()];
-        if (st == s->streams[0]) continue;
+    for (size_t k = 1; ordered && k < s->streams.size(); k++) {   // side streams join theirs
         cudaEvent_t e = nullptr;
         ordered = cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess &&
-                  cudaEventRecord(e, st) == cudaSuccess && cudaStreamWaitEvent(s->streams[0], e, 0) == cudaSuccess;
+                  cudaEventRecord(e, s->streams[k]) == cudaSuccess && cudaStreamWaitEvent(s->streams[0], e, 0) == cudaSuccess;
         if (e) cudaEventDestroy(e);
     }
     if (img->mem) {
@@ -2211,7 +2261,6 @@ void jxrb_image_destroy(jxrb_image *img) {
             // the ordering could not be set up: wait for every stream instead
             cudaGetLastError();
             for (cudaStream_t st : s->streams) cudaStreamSynchronize(st);
-            for (cudaStream_t st : s->sides) cudaStreamSynchronize(st);
         }
         cudaFreeAsync(img->mem, s->streams[0]);
     }

@@ -3224,10 +3224,6 @@ static size_t segment_smem_bytes(int segment, int max_planes) {
     return tile_smem_bytes(max_planes);
 }
 
-// Launch the work list's segments (interior tiles with one to four
-// full-resolution planes, interior tiles of 4:2:0 images, every other tile).
-// `bounds` holds the kSegments + 1 segment boundaries; `counters` two words a
-// segment.
 // What the launcher learns about a device once: its SM count, which segment
 // kernels have their dynamic shared-memory limit raised on it (a function
 // attribute holds per device), and how many CTAs of each segment kernel fit
@@ -3271,25 +3267,18 @@ static cudaError_t segment_fit(int seg, int planes, size_t smem, int &sms, int &
     return cudaSuccess;
 }
 
+// Launch the work list's segments, each kernel on the next of `lanes` in turn.
+// `bounds` holds the kSegments + 1 segment boundaries; `counters` two words a
+// segment.  The other and edge tiles come first, so that their short,
+// latency-bound launches start with the interior ones.
 cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32_t *bounds, int max_planes,
-                         uint32_t *status, uint32_t *counters, cudaStream_t stream, cudaStream_t side,
-                         cudaEvent_t fork, cudaEvent_t join, const LaunchTuning *tune) {
+                         uint32_t *status, uint32_t *counters, const cudaStream_t *lanes, int lane_count,
+                         const LaunchTuning *tune) {
     const WorkItem *list = static_cast<const WorkItem *>(items);
-    // The edge and other tiles (segments kSideSegment0 ..) run beside the
-    // interior kernels on `side`, forked from and joined back to `stream`, so
-    // their short, latency-bound launches hide under the long ones.
-    const bool both = bounds[kSegments] > bounds[kSideSegment0] && bounds[kSideSegment0] > bounds[0] &&
-                      side != nullptr && (tune == nullptr || tune->side_stream);
-    if (both) {
-        cudaError_t e = cudaEventRecord(fork, stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
-        if (e != cudaSuccess) return e;
-    }
+    int lane = 0;
     for (int seg0 = 0; seg0 < kSegments; seg0++) {
-        // the side stream's kernels first, so that they start with the others
         const int seg = seg0 == 0 ? kSegmentOther : seg0 <= kSegmentOther - kSideSegment0 ? kSideSegment0 + seg0 - 1
                                                                                           : seg0 - (kSegmentOther - kSideSegment0) - 1;
-        cudaStream_t st = (both && seg >= kSideSegment0) ? side : stream;
         const uint32_t count = bounds[seg + 1] - bounds[seg];
         if (count == 0) continue;
         TileKernel k = segment_kernel(seg);
@@ -3304,14 +3293,10 @@ cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32
             per_sm = (int)tune->blocks_per_sm[slot];
         const long full = (long)sms * per_sm;
         const int blocks = (int)((long)count < full ? (long)count : full);
-        k<<<blocks, kThreads, smem, st>>>(images, list + bounds[seg], count, status, counters + 2 * seg);
+        k<<<blocks, kThreads, smem, lanes[lane]>>>(images, list + bounds[seg], count, status, counters + 2 * seg);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
-    }
-    if (both) {
-        cudaError_t e = cudaEventRecord(join, side);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, join, 0);
-        if (e != cudaSuccess) return e;
+        lane = lane + 1 < lane_count ? lane + 1 : 0;
     }
     return cudaSuccess;
 }
