@@ -98,7 +98,7 @@ struct ImageDev {
 // One plane of a reduced-resolution request (a quarter or a sixteenth of
 // the resolution).  Its pictures live in the submission's scratch.  A
 // quarter: the first-level kernel writes the block picture -- one sample a
-// block -- the overlap kernel filters it in place, the scale kernel scales it
+// block -- the overlap kernel filters it in place; its last writer scales it
 // and the output kernel reads it.  A sixteenth: one sample a macroblock, the
 // macroblock's DC written straight into the macroblock picture, or, with
 // two-level overlap, the block picture of the DC band filtered and summed

@@ -34,8 +34,8 @@ cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32
                          const LaunchTuning *tune);
 int tile_mbs();
 cudaError_t launch_quarter(const ImageDev *images, const QuarterImage *quarters, uint32_t count,
-                           const QuarterPlane *planes, uint32_t plane_count, bool two_level, bool sixteenth_sums,
-                           uint32_t max_mbs, uint32_t max_samples, uint32_t max_rows, uint32_t *status,
+                           const QuarterPlane *planes, uint32_t plane_count, bool two_level, bool subsampled,
+                           bool finish, uint32_t max_mbs, uint32_t max_samples, uint64_t max_pixels, uint32_t *status,
                            cudaStream_t stream);
 }  // namespace jxr
 
@@ -762,8 +762,9 @@ struct DeviceSet {
     // quarter-resolution requests (request sets only)
     QuarterImage *quarters = nullptr;
     QuarterPlane *qplanes = nullptr;
-    uint32_t q_count = 0, q_planes = 0, q_max_mbs = 0, q_max_samples = 0, q_max_rows = 0;
-    bool q_two_level = false, q_sixteenth_sums = false;
+    uint32_t q_count = 0, q_planes = 0, q_max_mbs = 0, q_max_samples = 0;
+    uint64_t q_max_pixels = 0;
+    bool q_two_level = false, q_subsampled = false, q_finish = false;   // launch_quarter's stages
     std::vector<uint8_t> host_quarter;  // descriptors and scale terms, uploaded in one copy
     std::vector<ImageDev> host_images;
     std::vector<WorkItemHost> host_items;
@@ -1103,8 +1104,9 @@ jxrb_status launch_set(jxrb_session *s, DeviceSet &set, cudaStream_t stream) {
     const int n = forked + 1, first = set.q_count && n > 1 ? 1 : 0;
     if (e == cudaSuccess && set.q_count) {
         e = launch_quarter(set.images, set.quarters, set.q_count, set.qplanes, set.q_planes, set.q_two_level,
-                           set.q_sixteenth_sums, set.q_max_mbs, set.q_max_samples, set.q_max_rows, set.status, lanes[0]);
-        if (e == cudaSuccess) s->launches += 3 + (set.q_two_level ? 3 : 0) + (set.q_sixteenth_sums ? 1 : 0);
+                           set.q_subsampled, set.q_finish, set.q_max_mbs, set.q_max_samples, set.q_max_pixels, set.status,
+                           lanes[0]);
+        if (e == cudaSuccess) s->launches += 2 + (set.q_subsampled ? 3 : set.q_two_level ? 1 : 0) + (set.q_finish ? 1 : 0);
     }
     if (e == cudaSuccess) {
         e = launch_tiles(set.images, set.items, set.bounds, set.max_planes, set.status, set.counters, lanes + first,
@@ -2056,7 +2058,7 @@ jxrb_status build_request_set(jxrb_session *s, const jxrb_request *const *reqs, 
             q.planes = (uint32_t)img.planes.size();
             q.width = sixteenth ? r.wx : r.wx * 4;
             q.height = sixteenth ? r.wy : r.wy * 4;
-            set.q_max_rows = std::max(set.q_max_rows, q.height);
+            set.q_max_pixels = std::max(set.q_max_pixels, (uint64_t)q.width * q.height);
             for (size_t k = 0; k < img.planes.size(); k++, qp++) {
                 const ImagePlane &ip = img.planes[k];
                 const QuarterScale &sc = *r.scales[k];
@@ -2091,7 +2093,8 @@ jxrb_status build_request_set(jxrb_session *s, const jxrb_request *const *reqs, 
                     d.rows = reinterpret_cast<const uint32_t *>(base + a.rows);
                 }
                 set.q_two_level |= ip.overlap == 2;
-                set.q_sixteenth_sums |= sixteenth && ip.overlap == 2;
+                set.q_subsampled |= ip.overlap == 2 && ip.bc != 4;
+                set.q_finish |= ip.overlap == 2 && (sixteenth || ip.bc != 4);
                 set.q_max_mbs = std::max(set.q_max_mbs, r.wx * r.wy);
                 set.q_max_samples = std::max(set.q_max_samples, r.wx * ip.bc * r.wy * ip.br);
             }

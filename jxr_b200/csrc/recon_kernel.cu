@@ -895,6 +895,70 @@ __device__ void output_generic(const ImageDev &im, const View *views, int X0, in
     }
 }
 
+// `n` little-endian words to any address: whole words where the destination
+// is aligned, the two ends in bytes and half-words.  The rows of images whose
+// width is no multiple of four start at every byte of a word; twelve single
+// bytes for such rows cost a 3999 x 2999 4:2:0 decode 13 us (107.5 us, 94.7 us here).
+template <int N>
+__device__ __forceinline__ void store_words(uint8_t *d, const uint32_t (&w)[N]) {
+    const uint32_t m = (uint32_t)reinterpret_cast<uintptr_t>(d) & 3;
+    uint32_t *q = reinterpret_cast<uint32_t *>(d + ((4 - m) & 3));
+    if (m == 0) {
+#pragma unroll
+        for (int k = 0; k < N; k++) q[k] = w[k];
+    } else if (m == 2) {
+        *reinterpret_cast<uint16_t *>(d) = (uint16_t)w[0];
+#pragma unroll
+        for (int k = 0; k + 1 < N; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 16);
+        *reinterpret_cast<uint16_t *>(d + 4 * N - 2) = (uint16_t)(w[N - 1] >> 16);
+    } else if (m == 1) {
+        d[0] = (uint8_t)w[0];
+        *reinterpret_cast<uint16_t *>(d + 1) = (uint16_t)(w[0] >> 8);
+#pragma unroll
+        for (int k = 0; k + 1 < N; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 24);
+        d[4 * N - 1] = (uint8_t)(w[N - 1] >> 24);
+    } else {
+        d[0] = (uint8_t)w[0];
+#pragma unroll
+        for (int k = 0; k + 1 < N; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 8);
+        *reinterpret_cast<uint16_t *>(d + 4 * N - 3) = (uint16_t)(w[N - 1] >> 8);
+        d[4 * N - 1] = (uint8_t)(w[N - 1] >> 24);
+    }
+}
+
+__device__ __forceinline__ void store12(uint8_t *d, const uint32_t px[4]) {
+    // R0 G0 B0 R1 | G1 B1 R2 G2 | B2 R3 G3 B3
+    const uint32_t w[3] = {(px[0] & 0xffffffu) | (px[1] << 24), ((px[1] >> 8) & 0xffffu) | (px[2] << 16),
+                           ((px[2] >> 16) & 0xffu) | ((px[3] & 0xffffffu) << 8)};
+    store_words(d, w);
+}
+
+__device__ __forceinline__ void store16(uint8_t *d, uint32_t a, uint32_t b, uint32_t c, uint32_t e) {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(d);
+    if ((p & 15) == 0) {
+        *reinterpret_cast<uint4 *>(d) = make_uint4(a, b, c, e);
+    } else if ((p & 7) == 0) {
+        *reinterpret_cast<uint2 *>(d) = make_uint2(a, b);
+        *reinterpret_cast<uint2 *>(d + 8) = make_uint2(c, e);
+    } else if ((p & 3) == 0) {
+        uint32_t *q = reinterpret_cast<uint32_t *>(d);
+        q[0] = a; q[1] = b; q[2] = c; q[3] = e;
+    } else {
+        const uint32_t w[4] = {a, b, c, e};
+#pragma unroll
+        for (int k = 0; k < 16; k++) d[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
+    }
+}
+
+__device__ __forceinline__ void store8(uint8_t *d, uint32_t a, uint32_t b) {
+    if ((reinterpret_cast<uintptr_t>(d) & 7) == 0) {
+        *reinterpret_cast<uint2 *>(d) = make_uint2(a, b);
+    } else {
+        const uint32_t w[2] = {a, b};
+        store_words(d, w);
+    }
+}
+
 // Output work is spread over row chunks: four horizontally adjacent pixels
 // of one block row (x = 4k .. 4k+3).  A chunk wholly inside the tile's output
 // region reads each full-resolution plane with one 128-bit shared load and
@@ -915,14 +979,33 @@ __device__ __forceinline__ bool chunk_range(const OutputDev &o, int X0, int X1, 
     return true;
 }
 
-// one 4-sample row chunk of a full-resolution plane
+// A picture in global memory, read like a tile's plane view.
+struct GlobalView {
+    const int32_t *p;
+    int w, h;
+    __device__ __forceinline__ int32_t at(int x, int y) const { return p[(size_t)y * w + x]; }
+    __device__ __forceinline__ int32_t clamped(int x, int y) const {
+        return at(min(max(x, 0), w - 1), min(max(y, 0), h - 1));
+    }
+};
+
+// one 4-sample row chunk of a full-resolution plane; of a picture in global
+// memory, whose rows are whole chunks unless it is a sixteenth, zeros past
+// the row's end
+__device__ __forceinline__ int4 row_chunk(const GlobalView &v, int kb, int y) {
+    const int32_t *row = v.p + (size_t)y * v.w;
+    const int x = 4 * kb;
+    if ((v.w & 3) == 0) return *reinterpret_cast<const int4 *>(row + x);
+    return make_int4(row[x], x + 1 < v.w ? row[x + 1] : 0, x + 2 < v.w ? row[x + 2] : 0, x + 3 < v.w ? row[x + 3] : 0);
+}
 __device__ __forceinline__ int4 row_chunk(const PlaneView &v, int kb, int y) {
     const TileView &t = v.tv;
     const int b = ((y >> 2) - t.by0) * t.nbx + (kb - t.bx0);
     return *reinterpret_cast<const int4 *>(&t.t[elem(b, y & 3, 0)]);
 }
 
-__device__ __forceinline__ void chunk_components(const ImageDev &im, const PlaneView *views, int kb, int y,
+template <class View>
+__device__ __forceinline__ void chunk_components(const ImageDev &im, const View *views, int kb, int y,
                                                  int32_t comp[3][4]) {
     const int4 yv = row_chunk(views[0], kb, y);
     comp[0][0] = yv.x; comp[0][1] = yv.y; comp[0][2] = yv.z; comp[0][3] = yv.w;
@@ -937,7 +1020,7 @@ __device__ __forceinline__ void chunk_components(const ImageDev &im, const Plane
     const int cx0 = 2 * kb;
 #pragma unroll
     for (int c = 1; c <= 2; c++) {
-        const PlaneView &v = views[c];
+        const View &v = views[c];
         int32_t col[4];
 #pragma unroll
         for (int d = 0; d < 4; d++) {
@@ -957,8 +1040,11 @@ __device__ __forceinline__ void chunk_components(const ImageDev &im, const Plane
     }
 }
 
-// 8-bit RGB / BGR (+ alpha) from YUV: the common photographic output.
-__device__ void output_rgb8(const ImageDev &im, const PlaneView *views, int X0, int X1, int Y0, int Y1, bool &bad) {
+// 8-bit RGB / BGR (+ alpha) from YUV: the common photographic output.  The
+// thread takes chunks `first`, `first` + `step`, ...
+template <class View>
+__device__ void output_rgb8(const ImageDev &im, const View *views, int X0, int X1, int Y0, int Y1, int first, int step,
+                            bool &bad) {
     const OutputDev &o = im.out;
     ChunkRange cr;
     if (!chunk_range(o, X0, X1, Y0, Y1, cr)) return;
@@ -970,7 +1056,7 @@ __device__ void output_rgb8(const ImageDev &im, const PlaneView *views, int X0, 
     const int ashift = alpha ? o.ch[3].shift : 0;
     const bool reverse = o.ch[0].source == 2;
     const int pb = o.channels;  // 3 or 4 bytes a pixel
-    for (int i = threadIdx.x; i < cr.nkb * cr.ny; i += blockDim.x) {
+    for (int i = first; i < cr.nkb * cr.ny; i += step) {
         const int kb = cr.kb0 + i % cr.nkb, y = cr.ay0 + i / cr.nkb;
         const int x0 = max(4 * kb, cr.ax0), x1 = min(4 * kb + 4, cr.ax1);
         int32_t comp[3][4];
@@ -1003,14 +1089,10 @@ __device__ void output_rgb8(const ImageDev &im, const PlaneView *views, int X0, 
         }
         uint8_t *dst = row + (uint64_t)(x0 - o.crop_x) * pb;
         const bool whole = x0 == 4 * kb && x1 == 4 * kb + 4;
-        if (whole && pb == 4 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(px[0], px[1], px[2], px[3]);
-        } else if (whole && pb == 3 && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
-            // 12 bytes: R0 G0 B0 R1 | G1 B1 R2 G2 | B2 R3 G3 B3
-            uint32_t *d = reinterpret_cast<uint32_t *>(dst);
-            d[0] = (px[0] & 0xffffffu) | (px[1] << 24);
-            d[1] = ((px[1] >> 8) & 0xffffu) | (px[2] << 16);
-            d[2] = ((px[2] >> 16) & 0xffu) | ((px[3] & 0xffffffu) << 8);
+        if (whole && pb == 4) {
+            store16(dst, px[0], px[1], px[2], px[3]);
+        } else if (whole && pb == 3) {
+            store12(dst, px);
         } else {
             for (int x = x0; x < x1; x++) {
                 const uint32_t w = px[x - 4 * kb];
@@ -1023,13 +1105,15 @@ __device__ void output_rgb8(const ImageDev &im, const PlaneView *views, int X0, 
 }
 
 // One channel straight from one plane (luma to U8 / U16 / I16 / I32).
-__device__ void output_direct(const ImageDev &im, const PlaneView *views, int X0, int X1, int Y0, int Y1, bool &bad) {
+template <class View>
+__device__ void output_direct(const ImageDev &im, const View *views, int X0, int X1, int Y0, int Y1, int first,
+                              int step, bool &bad) {
     const OutputDev &o = im.out;
     ChunkRange cr;
     if (!chunk_range(o, X0, X1, Y0, Y1, cr)) return;
     const ChannelScale &s = o.ch[0];
     const int eb = o.elem_bytes;
-    for (int i = threadIdx.x; i < cr.nkb * cr.ny; i += blockDim.x) {
+    for (int i = first; i < cr.nkb * cr.ny; i += step) {
         const int kb = cr.kb0 + i % cr.nkb, y = cr.ay0 + i / cr.nkb;
         const int x0 = max(4 * kb, cr.ax0), x1 = min(4 * kb + 4, cr.ax1);
         const int4 v4 = row_chunk(views[0], kb, y);
@@ -1040,12 +1124,13 @@ __device__ void output_direct(const ImageDev &im, const PlaneView *views, int X0
         uint8_t *row = o.base + (uint64_t)(y - o.crop_y) * o.row_stride;
         uint8_t *dst = row + (uint64_t)(x0 - o.crop_x) * eb;
         const bool whole = x0 == 4 * kb && x1 == 4 * kb + 4;
-        if (whole && eb == 2 && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
-            *reinterpret_cast<uint2 *>(dst) = make_uint2((w[0] & 0xffffu) | (w[1] << 16), (w[2] & 0xffffu) | (w[3] << 16));
-        } else if (whole && eb == 1 && (reinterpret_cast<uintptr_t>(dst) & 3) == 0) {
-            *reinterpret_cast<uint32_t *>(dst) = (w[0] & 0xffu) | ((w[1] & 0xffu) << 8) | ((w[2] & 0xffu) << 16) | (w[3] << 24);
-        } else if (whole && eb == 4 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-            *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
+        if (whole && eb == 2) {
+            store8(dst, (w[0] & 0xffffu) | (w[1] << 16), (w[2] & 0xffffu) | (w[3] << 16));
+        } else if (whole && eb == 1) {
+            const uint32_t q[1] = {(w[0] & 0xffu) | ((w[1] & 0xffu) << 8) | ((w[2] & 0xffu) << 16) | (w[3] << 24)};
+            store_words(dst, q);
+        } else if (whole && eb == 4) {
+            store16(dst, w[0], w[1], w[2], w[3]);
         } else {
             for (int x = x0; x < x1; x++) store_elem(row + (uint64_t)(x - o.crop_x) * eb, w[x - 4 * kb], eb);
         }
@@ -1128,70 +1213,6 @@ constexpr int kLpInts = 36 * 16;    // DC / low-pass coefficients of 6 x 6 macro
 template <int NP> __host__ __device__ constexpr int lp_stride() { return NP == 3 ? 20 : 16; }
 template <int NP> __host__ __device__ constexpr int lp_ints() { return 36 * lp_stride<NP>(); }
 constexpr int kMbcInts = 36 * 4;    // their 16-byte entries
-
-// `n` little-endian words to any address: whole words where the destination
-// is aligned, the two ends in bytes and half-words.  The rows of images whose
-// width is no multiple of four start at every byte of a word; twelve single
-// bytes for such rows cost a 3999 x 2999 4:2:0 decode 13 us (107.5 us, 94.7 us here).
-template <int N>
-__device__ __forceinline__ void store_words(uint8_t *d, const uint32_t (&w)[N]) {
-    const uint32_t m = (uint32_t)reinterpret_cast<uintptr_t>(d) & 3;
-    uint32_t *q = reinterpret_cast<uint32_t *>(d + ((4 - m) & 3));
-    if (m == 0) {
-#pragma unroll
-        for (int k = 0; k < N; k++) q[k] = w[k];
-    } else if (m == 2) {
-        *reinterpret_cast<uint16_t *>(d) = (uint16_t)w[0];
-#pragma unroll
-        for (int k = 0; k + 1 < N; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 16);
-        *reinterpret_cast<uint16_t *>(d + 4 * N - 2) = (uint16_t)(w[N - 1] >> 16);
-    } else if (m == 1) {
-        d[0] = (uint8_t)w[0];
-        *reinterpret_cast<uint16_t *>(d + 1) = (uint16_t)(w[0] >> 8);
-#pragma unroll
-        for (int k = 0; k + 1 < N; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 24);
-        d[4 * N - 1] = (uint8_t)(w[N - 1] >> 24);
-    } else {
-        d[0] = (uint8_t)w[0];
-#pragma unroll
-        for (int k = 0; k + 1 < N; k++) q[k] = __funnelshift_r(w[k], w[k + 1], 8);
-        *reinterpret_cast<uint16_t *>(d + 4 * N - 3) = (uint16_t)(w[N - 1] >> 8);
-        d[4 * N - 1] = (uint8_t)(w[N - 1] >> 24);
-    }
-}
-
-__device__ __forceinline__ void store12(uint8_t *d, const uint32_t px[4]) {
-    // R0 G0 B0 R1 | G1 B1 R2 G2 | B2 R3 G3 B3
-    const uint32_t w[3] = {(px[0] & 0xffffffu) | (px[1] << 24), ((px[1] >> 8) & 0xffffu) | (px[2] << 16),
-                           ((px[2] >> 16) & 0xffu) | ((px[3] & 0xffffffu) << 8)};
-    store_words(d, w);
-}
-
-__device__ __forceinline__ void store16(uint8_t *d, uint32_t a, uint32_t b, uint32_t c, uint32_t e) {
-    const uintptr_t p = reinterpret_cast<uintptr_t>(d);
-    if ((p & 15) == 0) {
-        *reinterpret_cast<uint4 *>(d) = make_uint4(a, b, c, e);
-    } else if ((p & 7) == 0) {
-        *reinterpret_cast<uint2 *>(d) = make_uint2(a, b);
-        *reinterpret_cast<uint2 *>(d + 8) = make_uint2(c, e);
-    } else if ((p & 3) == 0) {
-        uint32_t *q = reinterpret_cast<uint32_t *>(d);
-        q[0] = a; q[1] = b; q[2] = c; q[3] = e;
-    } else {
-        const uint32_t w[4] = {a, b, c, e};
-#pragma unroll
-        for (int k = 0; k < 16; k++) d[k] = (uint8_t)(w[k >> 2] >> (8 * (k & 3)));
-    }
-}
-
-__device__ __forceinline__ void store8(uint8_t *d, uint32_t a, uint32_t b) {
-    if ((reinterpret_cast<uintptr_t>(d) & 7) == 0) {
-        *reinterpret_cast<uint2 *>(d) = make_uint2(a, b);
-    } else {
-        const uint32_t w[2] = {a, b};
-        store_words(d, w);
-    }
-}
 
 // The 16 samples of sample cell b00 (lower-right quarter of block b00 and the
 // neighbouring quarters of the blocks right of and below it), second-level
@@ -2257,8 +2278,8 @@ __device__ void reconstruct_tile(const ImageDev &im, int tx, int ty, int32_t *sm
     }
     bool obad = false;
     switch (im.out.kind) {
-    case kOutRgb8: output_rgb8(im, views, X0, X1, Y0, Y1, obad); break;
-    case kOutDirect: output_direct(im, views, X0, X1, Y0, Y1, obad); break;
+    case kOutRgb8: output_rgb8(im, views, X0, X1, Y0, Y1, threadIdx.x, blockDim.x, obad); break;
+    case kOutDirect: output_direct(im, views, X0, X1, Y0, Y1, threadIdx.x, blockDim.x, obad); break;
     case kOutF16Wide: output_f16wide(im, views, X0, X1, Y0, Y1, obad); break;
     default: output_generic(im, views, X0, X1, Y0, Y1, obad); break;
     }
@@ -3309,8 +3330,42 @@ int tile_mbs() { return kTileMbs; }
 // sixteenth, reconstruct_sixteenth, 223-260).  The pictures are at most a
 // sixteenth of the full-resolution sample count, so each stage is its own
 // small kernel over pictures in global memory; blockIdx.y selects the plane
-// (or the request, for the output).
+// (or the request, for the output).  What a batch of them takes is the chain
+// of launches, each a few microseconds of latency: a sample is scaled to its
+// level by the kernel that gives it its last value, and kernels no plane of
+// the batch needs are left out.  16 thumbnails of 512..2048-pixel pictures,
+// submitted and waited for: 220 us with a pass of its own for the levels,
+// three overlap phases always and a pixel a thread in the output (seven
+// kernels, 118 us cold), 189 us here (four, 78 us cold).
 // ---------------------------------------------------------------------------
+
+// The earliest failing stage of the chain, as running its stages one after
+// another reports it.
+__device__ __forceinline__ void report_stage(uint32_t *status, uint32_t code) {
+    if (atomicCAS(status, 0u, code) > code) atomicMin(status, code);
+}
+
+// A sample scaled to the level it stands for: a shift without overlap
+// filtering, else the flat terms of the probe sample placed like it
+// (SampleScale::apply and FlatTerms::level, sample_scale.rs:250-350).
+__device__ __forceinline__ int32_t sample_level(const QuarterPlane &p, int32_t v, uint32_t x, uint32_t y, bool &bad) {
+    if (p.shift >= 0) return v >> p.shift;
+    if (v == 0) return 0;
+    const uint32_t t = __ldg(&p.rows[y]) * p.probe_stride + __ldg(&p.cols[x]);
+    const int64_t d = __ldg(&p.divisor[t]);
+    const int64_t num = (int64_t)v * p.gain - __ldg(&p.bias[t]);
+    int64_t q;
+    if (num == (int32_t)num && d == (int32_t)d) {   // the usual case: a 32-bit division
+        const int32_t n = (int32_t)num, e = (int32_t)d;
+        q = n / e;
+        if (n % e < 0) q -= 1;   // Euclidean division by a positive divisor
+    } else {
+        q = num / d;
+        if (num % d < 0) q -= 1;
+    }
+    bad |= q < INT32_MIN || q > INT32_MAX;
+    return (int32_t)q;
+}
 
 // The first level of every macroblock of the plane: dequantized DC and
 // low-pass values through the first-level inverse transform, doubled where
@@ -3318,61 +3373,94 @@ int tile_mbs() { return kTileMbs; }
 // A sixteenth leaves the low-pass values out (LowBands::Dc); without
 // two-level overlap it stops at the macroblock's DC, doubled where scaled,
 // written straight into the macroblock picture (macroblock_dc_plane, 387-409).
+// Four threads a macroblock: each loads a quarter of the values (at most four
+// dependent on nothing but the table entry), all of them run the transform,
+// and each scales and stores a row (4:2:0 chroma: a sample).  The pictures are
+// small enough for the loads and divisions of one thread's macroblock, one
+// after another, to be what the kernel takes: 16 thumbnails, cold caches, 32.8
+// us so, 29.3 us here.
 __global__ void __launch_bounds__(256) jxrb_quarter_first_level(const QuarterPlane *__restrict__ planes,
                                                                 uint32_t *status) {
     const QuarterPlane &p = planes[blockIdx.y];
     const uint32_t n = p.mbs_x * p.mbs_y;
-    const int count = p.bc * p.br;
+    const int count = p.bc * p.br, per = count >> 2;
     const size_t pw = (size_t)p.mbs_x * p.bc;
-    const bool dc_only = p.sixteenth != 0;
-    bool bad = false;
-    for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += gridDim.x * blockDim.x) {
+    const bool dc_only = p.sixteenth != 0, last = p.overlap != 2;   // no later kernel changes the values
+    const int j = threadIdx.x & 3;
+    bool bad = false, lbad = false;
+    // whole warps stay in the loop: they exchange values
+    for (uint32_t first = (blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) >> 2; first < n;
+         first += gridDim.x * blockDim.x >> 2) {
+        const uint32_t m = first + ((threadIdx.x & 31) >> 2);
+        const bool valid = m < n;
         const uint32_t mx = m % p.mbs_x, my = m / p.mbs_x;
-        const uint4 e = __ldg(&p.mbs[(size_t)my * p.mbs_stride + mx]);
+        uint4 e = make_uint4(0u, 0u, 0u, 0u);
+        if (valid) e = __ldg(&p.mbs[(size_t)my * p.mbs_stride + mx]);
         const int bands = (e.x >> 28) & 3;
         const int32_t *c = p.coeff + (e.x & 0x0fffffffu);
         const int stride = bands >= 2 ? 16 : 1;
-        int32_t v[16];
-        v[0] = dequant(__ldg(c), e.y, bad);
-        if (dc_only && p.overlap != 2) {
-            p.out[m] = p.scale2 ? dequant(v[0], 2, bad) : v[0];
+        if (dc_only && last) {
+            if (valid && j == 0) {
+                const int32_t v = dequant(__ldg(c), e.y, bad);
+                p.out[m] = sample_level(p, p.scale2 ? dequant(v, 2, bad) : v, mx, my, lbad);
+            }
             continue;
         }
+        // value k of the thread's share is coefficient j * per + k
+        int32_t own[4];
 #pragma unroll
-        for (int k = 1; k < 16; k++)
-            v[k] = (k < count && bands != 0 && !dc_only) ? dequant(__ldg(c + k * stride), e.z, bad) : 0;
-        int32_t *out = p.pic + (size_t)my * p.br * pw + (size_t)mx * p.bc;
-        if (count == 16) {
+        for (int k = 0; k < 4; k++) {
+            const int q = j * per + k;
+            own[k] = 0;
+            if (valid && k < per && (q == 0 || (bands != 0 && !dc_only)))
+                own[k] = dequant(__ldg(c + q * stride), q == 0 ? e.y : e.z, bad);
+        }
+        int32_t v[16], row[4];
+        const int lane0 = (threadIdx.x & 31) & ~3;
+        if (per == 4) {
+#pragma unroll
+            for (int k = 0; k < 16; k++) v[k] = __shfl_sync(0xffffffffu, own[k & 3], lane0 + (k >> 2));
             bad |= pct16(v);
 #pragma unroll
-            for (int k = 0; k < 16; k++) v[k] = p.scale2 ? dequant(v[k], 2, bad) : v[k];
+            for (int k = 0; k < 4; k++) row[k] = j == 0 ? v[k] : j == 1 ? v[4 + k] : j == 2 ? v[8 + k] : v[12 + k];
+        } else if (per == 2) {
+            int32_t w[8];
 #pragma unroll
-            for (int r = 0; r < 4; r++)
-#pragma unroll
-                for (int cc = 0; cc < 4; cc++) out[r * pw + cc] = v[r * 4 + cc];
-        } else if (count == 4) {
-            int32_t w[4] = {v[0], v[1], v[2], v[3]};
-            bad |= inverse_chroma_420<true>(w);
-#pragma unroll
-            for (int k = 0; k < 4; k++) w[k] = p.scale2 ? dequant(w[k], 2, bad) : w[k];
-            out[0] = w[0]; out[1] = w[1]; out[pw] = w[2]; out[pw + 1] = w[3];
-        } else {
-            int32_t w[8] = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]};
+            for (int k = 0; k < 8; k++) w[k] = __shfl_sync(0xffffffffu, own[k & 1], lane0 + (k >> 1));
             bad |= inverse_chroma_422<true>(w);
 #pragma unroll
-            for (int k = 0; k < 8; k++) w[k] = p.scale2 ? dequant(w[k], 2, bad) : w[k];
+            for (int k = 0; k < 2; k++) row[k] = j == 0 ? w[k] : j == 1 ? w[2 + k] : j == 2 ? w[4 + k] : w[6 + k];
+        } else {
+            int32_t w[4];
 #pragma unroll
-            for (int r = 0; r < 4; r++) { out[r * pw] = w[2 * r]; out[r * pw + 1] = w[2 * r + 1]; }
+            for (int k = 0; k < 4; k++) w[k] = __shfl_sync(0xffffffffu, own[0], lane0 + k);
+            bad |= inverse_chroma_420<true>(w);
+            row[0] = j == 0 ? w[0] : j == 1 ? w[1] : j == 2 ? w[2] : w[3];
         }
+        if (!valid) continue;
+        const uint32_t x = mx * p.bc + (per == 1 ? j & 1 : 0), y = my * p.br + (per == 1 ? j >> 1 : j);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            if (k >= per) break;
+            if (p.scale2) row[k] = dequant(row[k], 2, bad);
+            if (last) row[k] = sample_level(p, row[k], x + k, y, lbad);
+        }
+        int32_t *out = p.pic + (size_t)y * pw + x;
+        if (per == 4) *reinterpret_cast<int4 *>(out) = make_int4(row[0], row[1], row[2], row[3]);
+        else if (per == 2) *reinterpret_cast<int2 *>(out) = make_int2(row[0], row[1]);
+        else out[0] = row[0];
     }
-    if (bad) atomicCAS(status, 0u, (uint32_t)kStatusFirstTransform);
+    if (bad) report_stage(status, kStatusFirstTransform);
+    if (lbad) report_stage(status, kStatusSecondTransform);
 }
 
 // The first-level overlap filter over a two-level plane's picture, one cell a
 // thread.  Full resolution: 4x4 cells at origins 2 (mod 4), disjoint, one
-// pass (phase 0).  Subsampled chroma: 2x2 cells at odd origins in three
-// ordered phases (corners lose their neighbour, squares and pairs, corners
-// regain it), the schedule of crates/jxr-native/src/reconstruct/subsampled_overlap.rs:244-296.
+// pass (phase 0); each sample lies in one cell, so a quarter's are scaled to
+// their levels as they are written.  Subsampled chroma: 2x2 cells at odd
+// origins in three ordered phases (corners lose their neighbour, squares and
+// pairs, corners regain it), the schedule of
+// crates/jxr-native/src/reconstruct/subsampled_overlap.rs:244-296.
 __global__ void __launch_bounds__(256) jxrb_quarter_overlap(const QuarterPlane *__restrict__ planes, int phase,
                                                             uint32_t *status) {
     const QuarterPlane &p = planes[blockIdx.y];
@@ -3384,37 +3472,47 @@ __global__ void __launch_bounds__(256) jxrb_quarter_overlap(const QuarterPlane *
     auto inside = [&](int x, int y) { return x >= 0 && x < W && y >= 0 && y < H; };
     auto vb = [&](int x) { return boundary_at(x, W, lx, p.hard, p.col_start); };
     auto hb = [&](int y) { return boundary_at(y, H, ly, p.hard, p.row_start); };
-    bool bad = false;
+    bool bad = false, lbad = false;
     if (p.bc == 4) {
         if (phase != 0) return;
         const int ncx = W / 4 + 1, ncy = H / 4 + 1;
         for (int item = blockIdx.x * blockDim.x + threadIdx.x; item < ncx * ncy; item += gridDim.x * blockDim.x) {
             const int cx = -2 + 4 * (item % ncx), cy = -2 + 4 * (item / ncx);
             const bool vs = vb(cx + 2), hs = hb(cy + 2);
+            // each row of the cell as two pairs of samples (8-byte aligned:
+            // cx and W are even), those outside the picture left out
+            int32_t v[16];
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int x = cx + 2 * (k & 1), y = cy + (k >> 1);
+                const int2 q = inside(x, y) ? *reinterpret_cast<const int2 *>(&at(x, y)) : make_int2(0, 0);
+                v[2 * k] = q.x;
+                v[2 * k + 1] = q.y;
+            }
+            // zeros stand for what lies outside, and stay there: the strips
+            // and quarters that hold any hold nothing else
             if (!vs && !hs) {
-                int32_t v[16];
-#pragma unroll
-                for (int r = 0; r < 4; r++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++) v[r * 4 + c] = at(cx + c, cy + r);
                 bad |= pot16(v);
-#pragma unroll
-                for (int r = 0; r < 4; r++)
-#pragma unroll
-                    for (int c = 0; c < 4; c++) at(cx + c, cy + r) = v[r * 4 + c];
             } else if (vs && !hs) {
-                for (int c = 0; c < 4; c++)
-                    if (cx + c >= 0 && cx + c < W)
-                        bad |= inverse_pot4(at(cx + c, cy), at(cx + c, cy + 1), at(cx + c, cy + 2), at(cx + c, cy + 3));
+#pragma unroll
+                for (int c = 0; c < 4; c++) bad |= inverse_pot4(v[c], v[4 + c], v[8 + c], v[12 + c]);
             } else if (!vs && hs) {
-                for (int r = 0; r < 4; r++)
-                    if (cy + r >= 0 && cy + r < H)
-                        bad |= inverse_pot4(at(cx, cy + r), at(cx + 1, cy + r), at(cx + 2, cy + r), at(cx + 3, cy + r));
+#pragma unroll
+                for (int r = 0; r < 4; r++) bad |= inverse_pot4(v[4 * r], v[4 * r + 1], v[4 * r + 2], v[4 * r + 3]);
             } else {
+#pragma unroll
                 for (int k = 0; k < 4; k++) {
-                    const int x = cx + (k & 1) * 2, y = cy + (k >> 1) * 2;
-                    if (inside(x, y)) bad |= inverse_pot4(at(x, y), at(x + 1, y), at(x, y + 1), at(x + 1, y + 1));
+                    const int c = (k & 1) * 2 + (k >> 1) * 8;
+                    bad |= inverse_pot4(v[c], v[c + 1], v[c + 4], v[c + 5]);
                 }
+            }
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int x = cx + 2 * (k & 1), y = cy + (k >> 1);
+                if (!inside(x, y)) continue;
+                int2 q = make_int2(v[2 * k], v[2 * k + 1]);
+                if (!p.sixteenth) q = make_int2(sample_level(p, q.x, x, y, lbad), sample_level(p, q.y, x + 1, y, lbad));
+                *reinterpret_cast<int2 *>(&at(x, y)) = q;
             }
         }
     } else {
@@ -3458,109 +3556,90 @@ __global__ void __launch_bounds__(256) jxrb_quarter_overlap(const QuarterPlane *
             }
         }
     }
-    if (bad) atomicCAS(status, 0u, (uint32_t)kStatusOverlap);
+    if (bad) report_stage(status, kStatusOverlap);
+    if (lbad) report_stage(status, kStatusSecondTransform);
 }
 
-// A sixteenth of a two-level plane: each macroblock's filtered block values
-// summed, row by row, checked, into the macroblock picture (sum_macroblocks,
-// pipeline.rs:421-457).
-__global__ void __launch_bounds__(256) jxrb_sixteenth_sum(const QuarterPlane *__restrict__ planes, uint32_t *status) {
+// The last values of two-level planes' samples.  A sixteenth: each
+// macroblock's filtered block values summed, row by row, checked, into the
+// macroblock picture (sum_macroblocks, pipeline.rs:421-457), and scaled.  A
+// subsampled quarter: its picture scaled (the overlap kernel's ordered corners
+// write some samples twice).
+__global__ void __launch_bounds__(256) jxrb_quarter_finish(const QuarterPlane *__restrict__ planes, uint32_t *status) {
     const QuarterPlane &p = planes[blockIdx.y];
-    if (!p.sixteenth || p.overlap != 2) return;
-    const uint32_t n = p.mbs_x * p.mbs_y;
-    const size_t pw = (size_t)p.mbs_x * p.bc;
-    bool bad = false;
-    for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += gridDim.x * blockDim.x) {
-        const uint32_t mx = m % p.mbs_x, my = m / p.mbs_x;
-        const int32_t *b = p.pic + (size_t)my * p.br * pw + (size_t)mx * p.bc;
-        int32_t sum = 0;
-        for (int r = 0; r < p.br; r++)
-            for (int c = 0; c < p.bc; c++) sum = Ar<true>::add(sum, b[r * pw + c], bad);
-        p.out[m] = sum;
-    }
-    if (bad) atomicCAS(status, 0u, (uint32_t)kStatusSecondTransform);
-}
-
-// Each sample scaled to the level it stands for: a shift without overlap
-// filtering, else the flat terms of the probe sample placed like it
-// (SampleScale::apply and FlatTerms::level, sample_scale.rs:250-350).
-__global__ void __launch_bounds__(256) jxrb_quarter_scale(const QuarterPlane *__restrict__ planes, uint32_t *status) {
-    const QuarterPlane &p = planes[blockIdx.y];
-    const uint32_t W = p.sixteenth ? p.mbs_x : p.mbs_x * p.bc;
-    const uint32_t n = W * (p.sixteenth ? p.mbs_y : p.mbs_y * p.br);
+    if (p.overlap != 2 || (!p.sixteenth && p.bc == 4)) return;
+    const uint32_t pw = p.mbs_x * p.bc, W = p.sixteenth ? p.mbs_x : pw, n = W * (p.sixteenth ? p.mbs_y : p.mbs_y * p.br);
     bool bad = false;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int32_t v = p.out[i];
-        if (p.shift >= 0) {
-            p.out[i] = v >> p.shift;
-            continue;
+        const uint32_t x = i % W, y = i / W;
+        int32_t v = 0;
+        if (p.sixteenth) {
+            const int32_t *b = p.pic + (size_t)y * p.br * pw + (size_t)x * p.bc;
+            for (int r = 0; r < p.br; r++)
+                for (int c = 0; c < p.bc; c++) v = Ar<true>::add(v, b[(size_t)r * pw + c], bad);
+        } else {
+            v = p.out[i];
         }
-        if (v == 0) continue;
-        const uint32_t t = __ldg(&p.rows[i / W]) * p.probe_stride + __ldg(&p.cols[i % W]);
-        const int64_t d = __ldg(&p.divisor[t]);
-        const int64_t num = (int64_t)v * p.gain - __ldg(&p.bias[t]);
-        int64_t q = num / d;
-        if (num % d < 0) q -= 1;   // Euclidean division by a positive divisor
-        bad |= q < INT32_MIN || q > INT32_MAX;
-        p.out[i] = (int32_t)q;
+        p.out[i] = sample_level(p, v, x, y, bad);
     }
-    if (bad) atomicCAS(status, 0u, (uint32_t)kStatusSecondTransform);
+    if (bad) report_stage(status, kStatusSecondTransform);
 }
 
-// A picture in global memory, read like a tile's plane view.
-struct GlobalView {
-    const int32_t *p;
-    int w, h;
-    __device__ __forceinline__ int32_t at(int x, int y) const { return p[(size_t)y * w + x]; }
-    __device__ __forceinline__ int32_t clamped(int x, int y) const {
-        return at(min(max(x, 0), w - 1), min(max(y, 0), h - 1));
-    }
-};
-
 // Chroma upsampling, colour conversion, scaling and packing of the scaled
-// pictures: the full-resolution output path over bands of eight rows.
+// pictures: the full-resolution output paths, RGB8 and one-channel outputs
+// four pixels a thread, others over bands of eight rows.
 __global__ void __launch_bounds__(256) jxrb_quarter_output(const ImageDev *__restrict__ images,
                                                            const QuarterImage *__restrict__ quarters,
                                                            const QuarterPlane *__restrict__ planes, uint32_t *status) {
     const QuarterImage q = quarters[blockIdx.y];
     const ImageDev &im = images[q.image];
     GlobalView views[JXRB_MAX_PLANES];
-    for (uint32_t k = 0; k < q.planes && k < JXRB_MAX_PLANES; k++) {
+#pragma unroll
+    for (uint32_t k = 0; k < JXRB_MAX_PLANES; k++) {
+        if (k >= q.planes) break;
         const QuarterPlane &p = planes[q.first_plane + k];
         views[k] = p.sixteenth ? GlobalView{p.out, (int)p.mbs_x, (int)p.mbs_y}
                                : GlobalView{p.out, (int)(p.mbs_x * p.bc), (int)(p.mbs_y * p.br)};
     }
     bool bad = false;
-    const int bands = ((int)q.height + 7) / 8;
-    for (int b = blockIdx.x; b < bands; b += gridDim.x)
-        output_generic(im, views, 0, (int)q.width, b * 8, min((int)q.height, b * 8 + 8), bad);
-    if (bad) atomicCAS(status, 0u, (uint32_t)kStatusOutput);
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    if (im.out.kind == kOutRgb8) {
+        output_rgb8(im, views, 0, (int)q.width, 0, (int)q.height, first, step, bad);
+    } else if (im.out.kind == kOutDirect) {
+        output_direct(im, views, 0, (int)q.width, 0, (int)q.height, first, step, bad);
+    } else {
+        const int bands = ((int)q.height + 7) / 8;
+        for (int b = blockIdx.x; b < bands; b += gridDim.x)
+            output_generic(im, views, 0, (int)q.width, b * 8, min((int)q.height, b * 8 + 8), bad);
+    }
+    if (bad) report_stage(status, kStatusOutput);
 }
 
-// The reduced-resolution stages of a set: `planes` planes of `count`
+// The reduced-resolution stages of a set: `plane_count` planes of `count`
 // requests, the largest plane holding `max_mbs` macroblocks and `max_samples`
-// picture samples, the tallest request `max_rows` rows; `sixteenth_sums`: a
-// sixteenth of a two-level plane is among them.
+// picture samples, the largest request `max_pixels` pixels.  `two_level`: some
+// plane has two overlap levels; `subsampled`: some such plane is subsampled;
+// `finish`: some such plane is subsampled or a sixteenth's.
 cudaError_t launch_quarter(const ImageDev *images, const QuarterImage *quarters, uint32_t count,
-                           const QuarterPlane *planes, uint32_t plane_count, bool two_level, bool sixteenth_sums,
-                           uint32_t max_mbs, uint32_t max_samples, uint32_t max_rows, uint32_t *status,
+                           const QuarterPlane *planes, uint32_t plane_count, bool two_level, bool subsampled,
+                           bool finish, uint32_t max_mbs, uint32_t max_samples, uint64_t max_pixels, uint32_t *status,
                            cudaStream_t stream) {
     if (count == 0 || plane_count == 0) return cudaSuccess;
     auto blocks = [](uint64_t work) { return (unsigned)std::min<uint64_t>(std::max<uint64_t>((work + 255) / 256, 1), 1024); };
     // blockIdx.y selects a plane or request: at most 65535 of them a launch
     for (uint32_t base = 0; base < plane_count; base += 65535) {
         const unsigned n = (unsigned)std::min<uint32_t>(plane_count - base, 65535);
-        jxrb_quarter_first_level<<<dim3(blocks(max_mbs), n), 256, 0, stream>>>(planes + base, status);
-        if (two_level)
-            for (int phase = 0; phase < 3; phase++)
-                jxrb_quarter_overlap<<<dim3(blocks(max_samples / 4 + 64), n), 256, 0, stream>>>(planes + base, phase,
-                                                                                                status);
-        if (sixteenth_sums) jxrb_sixteenth_sum<<<dim3(blocks(max_mbs), n), 256, 0, stream>>>(planes + base, status);
-        jxrb_quarter_scale<<<dim3(blocks(max_samples), n), 256, 0, stream>>>(planes + base, status);
+        jxrb_quarter_first_level<<<dim3(blocks((uint64_t)max_mbs * 4), n), 256, 0, stream>>>(planes + base, status);
+        for (int phase = 0; phase < (subsampled ? 3 : two_level ? 1 : 0); phase++)
+            jxrb_quarter_overlap<<<dim3(blocks(max_samples / (subsampled ? 4 : 16) + 64), n), 256, 0, stream>>>(
+                planes + base, phase, status);
+        if (finish)
+            jxrb_quarter_finish<<<dim3(blocks(subsampled ? max_samples : max_mbs), n), 256, 0, stream>>>(planes + base,
+                                                                                                    status);
     }
     for (uint32_t base = 0; base < count; base += 65535) {
         const unsigned n = (unsigned)std::min<uint32_t>(count - base, 65535);
-        jxrb_quarter_output<<<dim3(std::max(1u, std::min((max_rows + 7) / 8, 256u)), n), 256, 0, stream>>>(
+        jxrb_quarter_output<<<dim3(std::min(blocks(max_pixels / 4 + 64), 512u), n), 256, 0, stream>>>(
             images, quarters + base, planes, status);
     }
     return cudaGetLastError();
