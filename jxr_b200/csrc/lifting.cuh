@@ -36,6 +36,10 @@ template <> struct Ar<false> {
     JXR_HD static int32_t sub(int32_t a, int32_t b, bool &) { return a - b; }
     JXR_HD static int32_t mul3(int32_t a, bool &) { return a * 3; }
     JXR_HD static int32_t neg(int32_t a, bool &) { return -a; }
+    // a + ((b + 1) >> 1) and a - ((b + 1) >> 1): the rounded half of b is minus
+    // the floored half of -b, which folds into one shift-and-add
+    JXR_HD static int32_t add_half(int32_t a, int32_t b, bool &) { return a - (-b >> 1); }
+    JXR_HD static int32_t sub_half(int32_t a, int32_t b, bool &) { return a + (-b >> 1); }
 };
 
 template <> struct Ar<true> {
@@ -54,6 +58,8 @@ template <> struct Ar<true> {
         bad |= w != (int64_t)(int32_t)w;
         return (int32_t)w;
     }
+    JXR_HD static int32_t add_half(int32_t a, int32_t b, bool &bad) { return add(a, add(b, 1, bad) >> 1, bad); }
+    JXR_HD static int32_t sub_half(int32_t a, int32_t b, bool &bad) { return sub(a, add(b, 1, bad) >> 1, bad); }
     JXR_HD static int32_t neg(int32_t a, bool &bad) {
         bad |= a == INT32_MIN;
         return (int32_t)(0u - (uint32_t)a);
@@ -64,6 +70,26 @@ template <> struct Ar<true> {
 // |v| - 1 otherwise; the OR of these bounds every magnitude below a power of
 // two (crates/jxr-native/src/reconstruct/pipeline.rs:557-577).
 JXR_HD uint32_t mag(int32_t v) { return (uint32_t)(v ^ (v >> 31)); }
+
+// The largest mag() of v[F] .. v[15].  On the GPU from the largest and the
+// smallest value, two values an instruction: sixteen instructions of the
+// half-rate pipe where a shift and an OR a value take thirty.
+template <int F>
+JXR_HD uint32_t mag_bound(const int32_t (&v)[16]) {
+#if defined(__CUDA_ARCH__)
+    int32_t hi = v[15], lo = v[15];
+#pragma unroll
+    for (int k = F; k < 15; k += 2) {
+        hi = k + 1 < 15 ? __vimax3_s32(hi, v[k], v[k + 1]) : max(hi, v[k]);
+        lo = k + 1 < 15 ? __vimin3_s32(lo, v[k], v[k + 1]) : min(lo, v[k]);
+    }
+    return (uint32_t)max(hi, ~lo);
+#else
+    uint32_t m = 0;
+    for (int k = F; k < 16; k++) m = m > mag(v[k]) ? m : mag(v[k]);
+    return m;
+#endif
+}
 
 // ---- core transform: crates/jxr-math/src/transform.rs -------------------
 
@@ -86,12 +112,12 @@ JXR_HD void inverse_todd(int32_t &a, int32_t &b, int32_t &c, int32_t &d, bool &b
     b = A::add(b, d, bad);
     a = A::sub(a, c, bad);
     d = A::sub(d, b >> 1, bad);
-    c = A::add(c, A::add(a, 1, bad) >> 1, bad);
+    c = A::add_half(c, a, bad);
     a = A::sub(a, A::add(A::mul3(b, bad), 4, bad) >> 3, bad);
     b = A::add(b, A::add(A::mul3(a, bad), 4, bad) >> 3, bad);
     c = A::sub(c, A::add(A::mul3(d, bad), 4, bad) >> 3, bad);
     d = A::add(d, A::add(A::mul3(c, bad), 4, bad) >> 3, bad);
-    c = A::sub(c, A::add(b, 1, bad) >> 1, bad);
+    c = A::sub_half(c, b, bad);
     d = A::sub(A::add(a, 1, bad) >> 1, d, bad);
     b = A::add(b, c, bad);
     a = A::sub(a, d, bad);
@@ -176,8 +202,8 @@ JXR_HD void inverse_scale(int32_t &a, int32_t &b, bool &bad) {
 template <bool CK>
 JXR_HD void inverse_rotate(int32_t &a, int32_t &b, bool &bad) {
     using A = Ar<CK>;
-    a = A::sub(a, A::add(b, 1, bad) >> 1, bad);
-    b = A::add(b, A::add(a, 1, bad) >> 1, bad);
+    a = A::sub_half(a, b, bad);
+    b = A::add_half(b, a, bad);
 }
 
 template <bool CK>
@@ -242,8 +268,8 @@ JXR_HD bool inverse_pot4_steps(int32_t &a, int32_t &b, int32_t &c, int32_t &d) {
     bool bad = false;
     a = A::add(a, d, bad);
     b = A::add(b, c, bad);
-    d = A::sub(d, A::add(a, 1, bad) >> 1, bad);
-    c = A::sub(c, A::add(b, 1, bad) >> 1, bad);
+    d = A::sub_half(d, a, bad);
+    c = A::sub_half(c, b, bad);
     inverse_scale<CK>(a, d, bad);
     inverse_scale<CK>(b, c, bad);
     a = A::add(a, A::add(A::mul3(d, bad), 4, bad) >> 3, bad);
@@ -255,8 +281,8 @@ JXR_HD bool inverse_pot4_steps(int32_t &a, int32_t &b, int32_t &c, int32_t &d) {
     d = A::neg(d, bad);
     c = A::neg(c, bad);
     inverse_rotate<CK>(c, d, bad);
-    d = A::add(d, A::add(a, 1, bad) >> 1, bad);
-    c = A::add(c, A::add(b, 1, bad) >> 1, bad);
+    d = A::add_half(d, a, bad);
+    c = A::add_half(c, b, bad);
     a = A::sub(a, d, bad);
     b = A::sub(b, c, bad);
     return bad;
@@ -285,11 +311,11 @@ JXR_HD bool inverse_pot2x2(int32_t &a, int32_t &b, int32_t &c, int32_t &d) {
     bool bad = false;
     a = A::add(a, d, bad);
     b = A::add(b, c, bad);
-    d = A::sub(d, A::add(a, 1, bad) >> 1, bad);
-    c = A::sub(c, A::add(b, 1, bad) >> 1, bad);
+    d = A::sub_half(d, a, bad);
+    c = A::sub_half(c, b, bad);
     bad |= inverse_pot2(a, b);
-    d = A::add(d, A::add(a, 1, bad) >> 1, bad);
-    c = A::add(c, A::add(b, 1, bad) >> 1, bad);
+    d = A::add_half(d, a, bad);
+    c = A::add_half(c, b, bad);
     a = A::sub(a, d, bad);
     b = A::sub(b, c, bad);
     return bad;
@@ -298,18 +324,12 @@ JXR_HD bool inverse_pot2x2(int32_t &a, int32_t &b, int32_t &c, int32_t &d) {
 // Bound dispatch: the wrapping form where every input is below the bound,
 // the checked form otherwise.
 JXR_HD bool pct16(int32_t (&v)[16]) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int i = 0; i < 16; i++) m |= mag(v[i]);
-    if (m < (uint32_t)kTransformBound) return inverse_pct<false>(v);
+    if (mag_bound<0>(v) < (uint32_t)kTransformBound) return inverse_pct<false>(v);
     return inverse_pct<true>(v);
 }
 
 JXR_HD bool pot16(int32_t (&v)[16]) {
-    uint32_t m = 0;
-#pragma unroll
-    for (int i = 0; i < 16; i++) m |= mag(v[i]);
-    if (m < (uint32_t)kOverlapBound) return inverse_pot4x4<false>(v);
+    if (mag_bound<0>(v) < (uint32_t)kOverlapBound) return inverse_pot4x4<false>(v);
     return inverse_pot4x4<true>(v);
 }
 

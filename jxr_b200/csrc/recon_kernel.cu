@@ -429,9 +429,7 @@ __device__ bool stage_block_transform(const PlaneDev &p, const PlaneGeom &g, int
         v[r * 4 + 0] = q.x; v[r * 4 + 1] = q.y; v[r * 4 + 2] = q.z; v[r * 4 + 3] = q.w;
     }
     bool bad = false;
-    uint32_t m = 0;
-#pragma unroll
-    for (int k = 1; k < 16; k++) m |= mag(v[k]);
+    const uint32_t m = mag_bound<1>(v);
     v[0] = dc[(by - g.my0 * p.br) * g.dw + (bx - g.mx0 * p.bc)];
     // |v| <= m + 1 for every coded coefficient, so (m + 1) * step bounds the
     // dequantized ones; below the transform bound with the DC, the wrapping
@@ -775,6 +773,7 @@ struct WorkItem {
 };
 
 struct TileShared {
+    int32_t plain;   // tile kernels: every macroblock entry of the tile is plain (plain_entry)
     uint32_t hard;   // edge kernels: hard tile starts, columns mx0 + 0..4 in bits 0..4, rows my0 + 0..4 in bits 8..12
     PlaneGeom geo[JXRB_MAX_PLANES];
     int bad;
@@ -1203,48 +1202,81 @@ __device__ void output_f16wide(const ImageDev &im, const PlaneView *views, int X
 // ---------------------------------------------------------------------------
 constexpr int kIB = 17;             // blocks across / down
 constexpr int kIDC = 24;            // DC tile side (macroblocks mx0-1 .. mx0+4)
-constexpr int kIBlocks = kIB * kIB;
-constexpr int kLpInts = 36 * 16;    // DC / low-pass coefficients of 6 x 6 macroblocks
-// The three-plane interior kernel keeps each macroblock's 16 low-pass values
-// 80 bytes apart: eight consecutive macroblocks' 16-byte reads then fall in
-// eight distinct bank groups (at 64 bytes, in two).  The others keep 64: the
-// four-plane kernel measured slower with the padding (C3 1.138 -> 1.18 ms a
-// step; its first level reads its own macroblocks' values from the blocks).
-template <int NP> __host__ __device__ constexpr int lp_stride() { return NP == 3 ? 20 : 16; }
-template <int NP> __host__ __device__ constexpr int lp_ints() { return 36 * lp_stride<NP>(); }
+
+// A plane's blocks in the interior and edge kernels: macroblock by
+// macroblock, each of the tile's own 4 x 4 as the run of 16 blocks it is in
+// the arena, 260 ints apart; then the right neighbours' first block columns,
+// the lower neighbours' first block rows, and the corner block.  A
+// macroblock's coefficients are copied as they lie.  The pitch puts
+// neighbouring macroblocks one 16-byte bank group apart, so that a
+// quarter-warp that takes one row piece of two blocks in each of four
+// macroblocks (block_of_thread) meets eight distinct groups.
+constexpr int kMbPitch = 260;
+constexpr int kHaloPitch = 68;
+constexpr int kRightAt = 16 * kMbPitch;
+constexpr int kBottomAt = kRightAt + 4 * kHaloPitch;
+constexpr int kCornerAt = kBottomAt + 4 * kHaloPitch;
+constexpr int kTileInts = kCornerAt + 16;
+
+// Block (i, j) of a tile, i, j = 0 .. 16.
+__device__ __forceinline__ int block_at(int i, int j) {
+    const int own = ((j >> 2) * 4 + (i >> 2)) * kMbPitch + ((j & 3) * 4 + (i & 3)) * 16;
+    const int right = kRightAt + (j >> 2) * kHaloPitch + (j & 3) * 16;
+    const int bottom = i < 16 ? kBottomAt + (i >> 2) * kHaloPitch + (i & 3) * 16 : kCornerAt;
+    return j == 16 ? bottom : i == 16 ? right : own;
+}
+// Sample (x, y) of a tile, 0 .. 67.
+__device__ __forceinline__ int sample_at(int x, int y) { return block_at(x >> 2, y >> 2) + ((y & 3) << 2) + (x & 3); }
+
+// The own block that thread t of a pass over them takes: across the four
+// macroblocks first (two bits), then the block column (two) and row (four).
+__device__ __forceinline__ void block_of_thread(int t, int &i, int &j) {
+    i = 4 * (t & 3) + ((t >> 2) & 3);
+    j = t >> 4;
+}
+
+// The ring's DC / low-pass values: 20 macroblocks of 16, 80 bytes apart, so
+// that eight consecutive macroblocks' 16-byte reads meet distinct bank groups.
+constexpr int kRingPitch = 20;
+constexpr int kRingInts = 20 * kRingPitch;
 constexpr int kMbcInts = 36 * 4;    // their 16-byte entries
 
-// The 16 samples of sample cell b00 (lower-right quarter of block b00 and the
+// The four blocks a sample cell takes its quarters from.
+struct CellBlocks {
+    int b00, b01, b10, b11;
+};
+__device__ __forceinline__ CellBlocks cell_blocks(int cx, int cy) {
+    return CellBlocks{block_at(cx, cy), block_at(cx + 1, cy), block_at(cx, cy + 1), block_at(cx + 1, cy + 1)};
+}
+// Sample (c, r) of the cell.
+__device__ __forceinline__ int32_t &cell_sample(int32_t *t, const CellBlocks &b, int c, int r) {
+    const int at = r < 2 ? (c < 2 ? b.b00 : b.b01) : (c < 2 ? b.b10 : b.b11);
+    return t[at + (((r + 2) & 3) << 2) + ((c + 2) & 3)];
+}
+
+// The 16 samples of a sample cell (lower-right quarter of block b00 and the
 // neighbouring quarters of the blocks right of and below it), second-level
 // overlap applied when the plane has it.  `small`: every block transform of
 // the tile had inputs below 2^16 in magnitude, so the cell's values are below
 // 35.3 * 2^16 and the wrapping operator needs no magnitude test (interval
 // bounds of the inverse transform and overlap steps: outputs below 2^27.8,
 // intermediates below 2^28.2).  Returns the overflow flag.
-__device__ __forceinline__ bool cell_samples(const int32_t *t, int b00, int overlap, int32_t (&w)[16],
+__device__ __forceinline__ bool cell_samples(const int32_t *t, const CellBlocks &b, int overlap, int32_t (&w)[16],
                                              bool small = false) {
-    const int b01 = b00 + 1, b10 = b00 + kIB, b11 = b10 + 1;
-    const int2 a0 = *reinterpret_cast<const int2 *>(&t[elem(b00, 2, 2)]);
-    const int2 a1 = *reinterpret_cast<const int2 *>(&t[elem(b01, 2, 0)]);
-    const int2 a2 = *reinterpret_cast<const int2 *>(&t[elem(b00, 3, 2)]);
-    const int2 a3 = *reinterpret_cast<const int2 *>(&t[elem(b01, 3, 0)]);
-    const int2 a4 = *reinterpret_cast<const int2 *>(&t[elem(b10, 0, 2)]);
-    const int2 a5 = *reinterpret_cast<const int2 *>(&t[elem(b11, 0, 0)]);
-    const int2 a6 = *reinterpret_cast<const int2 *>(&t[elem(b10, 1, 2)]);
-    const int2 a7 = *reinterpret_cast<const int2 *>(&t[elem(b11, 1, 0)]);
+    const int2 a0 = *reinterpret_cast<const int2 *>(t + b.b00 + 10);
+    const int2 a1 = *reinterpret_cast<const int2 *>(t + b.b01 + 8);
+    const int2 a2 = *reinterpret_cast<const int2 *>(t + b.b00 + 14);
+    const int2 a3 = *reinterpret_cast<const int2 *>(t + b.b01 + 12);
+    const int2 a4 = *reinterpret_cast<const int2 *>(t + b.b10 + 2);
+    const int2 a5 = *reinterpret_cast<const int2 *>(t + b.b11);
+    const int2 a6 = *reinterpret_cast<const int2 *>(t + b.b10 + 6);
+    const int2 a7 = *reinterpret_cast<const int2 *>(t + b.b11 + 4);
     w[0] = a0.x; w[1] = a0.y; w[2] = a1.x; w[3] = a1.y;
     w[4] = a2.x; w[5] = a2.y; w[6] = a3.x; w[7] = a3.y;
     w[8] = a4.x; w[9] = a4.y; w[10] = a5.x; w[11] = a5.y;
     w[12] = a6.x; w[13] = a6.y; w[14] = a7.x; w[15] = a7.y;
     if (overlap < 1) return false;
     return small ? inverse_pot4x4<false>(w) : pot16(w);
-}
-
-// Whether macroblock m of a tile's 6 x 6 ring-and-tile grid is one of the
-// tile's own 4 x 4.
-__device__ __forceinline__ bool inner_mb(int m) {
-    const int a = m % 6, b = m / 6;
-    return a >= 1 && a <= 4 && b >= 1 && b <= 4;
 }
 
 // Ring macroblock r (0..19) of the 6 x 6 grid: the top row, then the left
@@ -1262,30 +1294,6 @@ __device__ __forceinline__ void low_pass_run(const int32_t *coeff, uint4 e, int3
     for (int k = 0; k < 16; k++) v[k] = k == 0 || lp ? __ldg(src + k) : 0;
 }
 
-// The DC / low-pass values of a tile's own 4 x 4 macroblocks into their
-// low-pass slots (`stride` apart), one value a thread, for `planes` planes
-// of `plane_ints` tile ints each.  A macroblock that codes high-pass bands
-// has them as coefficient 0 of its 16 blocks, staged with the blocks; one
-// that codes none holds them alone in its coefficient run (one DC, or all
-// 16), read here directly.
-__device__ __forceinline__ void inner_low_pass(const ImageDev &im, const int32_t *tiles, int plane_ints,
-                                               const uint4 *mbc, int32_t *lps, int lp_ints, int stride, int planes) {
-    for (int k = threadIdx.x; k < planes * 256; k += kThreads) {
-        const int pi = k >> 8, q = k & 255, mi = q >> 4, kk = q & 15;
-        const int m = (1 + (mi >> 2)) * 6 + 1 + (mi & 3);
-        const uint4 e = mbc[pi * 36 + m];
-        const int bands = (e.x >> 28) & 3;
-        int32_t v;
-        if (bands >= 2) {
-            const int s = (4 * (mi >> 2) + (kk >> 2)) * kIB + 4 * (mi & 3) + (kk & 3);
-            v = tiles[pi * plane_ints + elem(s, 0, 0)];
-        } else {
-            v = kk == 0 || bands != 0 ? __ldg(im.plane[pi].coeff + (e.x & 0x0fffffffu) + kk) : 0;
-        }
-        lps[pi * lp_ints + m * stride + kk] = v;
-    }
-}
-
 // One 16-byte piece of a coded block into its slot: copied asynchronously
 // when the macroblock codes high-pass coefficients (and the piece is
 // aligned), zero when it codes none.
@@ -1298,6 +1306,121 @@ __device__ __forceinline__ void copy_chunk(int32_t *dst, const int32_t *coeff, u
     } else {
         *reinterpret_cast<int4 *>(dst) = make_int4(0, 0, 0, 0);
     }
+}
+
+// Whether a table entry's macroblock codes every band, at a 16-byte boundary:
+// the usual one, whose pieces are copied without a test each.
+__device__ __forceinline__ bool plain_entry(const int32_t *coeff, uint4 e) {
+    return ((e.x >> 29) & 1) && (reinterpret_cast<uintptr_t>(coeff + (e.x & 0x0fffffffu)) & 15) == 0;
+}
+
+// Clears `plain` when an entry of planes [0, planes) is none (one a thread).
+__device__ __forceinline__ void note_plain(const ImageDev &im, const uint4 *mbc, int planes, int32_t &plain) {
+    const int tid = threadIdx.x;
+    if (tid < planes * 36 && !plain_entry(im.plane[tid / 36].coeff, mbc[tid])) plain = 0;
+}
+
+// A full-resolution plane's coefficients of one tile, every one in flight at
+// once: the ring macroblocks' DC / low-pass values, 4 bytes each; the own
+// macroblocks, 1 KB of the arena each, 64 threads a macroblock, in order, their
+// low-pass values -- coefficient 0 of each block -- among them; and the halo:
+// the first block column of the macroblocks right of the tile, the first block
+// row of those below it, the corner block.  `plain`: every entry is.
+struct PlaneCopy {
+    // what a thread copies is the same in every plane
+    int ring0, ring1;     // ring macroblock values tid and 256 + tid: entry index | slot << 8
+    int halo_entry, halo_from, halo_to;
+    __device__ __forceinline__ PlaneCopy() {
+        const int tid = threadIdx.x, kk = tid & 15, r = tid >> 4;
+        ring0 = ring_mb(r) | (r * kRingPitch + kk) << 8;
+        ring1 = tid < 64 ? ring_mb(16 + r) | ((16 + r) * kRingPitch + kk) << 8 : 0;
+        const int hb = tid >> 2, piece = (tid & 3) << 2;
+        const int i = hb >= 16 && hb < 32 ? hb - 16 : 16, j = hb < 16 ? hb : 16;
+        halo_entry = ((j >> 2) + 1) * 6 + (i >> 2) + 1;
+        halo_from = (((j & 3) << 2) + (i & 3)) * 16 + piece;
+        halo_to = block_at(i, j) + piece;
+    }
+    __device__ __forceinline__ void run(const int32_t *coeff, const uint4 *ent, int32_t *tile, int32_t *ring,
+                                        bool plain) const {
+        const int tid = threadIdx.x, kk = tid & 15, c = (tid & 63) * 4;
+        if (plain) {
+            cp_async4(ring + (ring0 >> 8), coeff + (ent[ring0 & 255].x & 0x0fffffffu) + kk * 16);
+            if (tid < 64) cp_async4(ring + (ring1 >> 8), coeff + (ent[ring1 & 255].x & 0x0fffffffu) + kk * 16);
+#pragma unroll
+            for (int b = 0; b < 4; b++)
+                cp_async16(tile + (4 * b + (tid >> 6)) * kMbPitch + c,
+                           coeff + (ent[(b + 1) * 6 + (tid >> 6) + 1].x & 0x0fffffffu) + c);
+            if (tid < 33 * 4) cp_async16(tile + halo_to, coeff + (ent[halo_entry].x & 0x0fffffffu) + halo_from);
+            return;
+        }
+        for (int k = 0; k < 2; k++) {
+            if (k == 1 && tid >= 64) break;
+            const int at = k == 0 ? ring0 : ring1;
+            const uint4 e = ent[at & 255];
+            const int bands = (e.x >> 28) & 3;
+            if (kk == 0 || bands != 0)
+                cp_async4(ring + (at >> 8), coeff + (e.x & 0x0fffffffu) + (bands >= 2 ? kk * 16 : kk));
+            else
+                ring[at >> 8] = 0;
+        }
+        for (int b = 0; b < 4; b++)
+            copy_chunk(tile + (4 * b + (tid >> 6)) * kMbPitch + c, coeff, ent[(b + 1) * 6 + (tid >> 6) + 1], c);
+        if (tid < 33 * 4) copy_chunk(tile + halo_to, coeff, ent[halo_entry], halo_from);
+    }
+};
+
+// The DC / low-pass values of item k of a plane's 36 macroblocks -- the 16 own
+// ones, then the ring's 20 -- and its index in the 6 x 6 grid.  An own one that
+// codes high-pass bands has them as coefficient 0 of its blocks.
+__device__ __forceinline__ int first_level_mb(int k) {
+    return k < 16 ? ((k >> 2) + 1) * 6 + (k & 3) + 1 : ring_mb(k - 16);
+}
+__device__ __forceinline__ void first_level_values(int k, const int32_t *coeff, uint4 e, const int32_t *tile,
+                                                   const int32_t *ring, int32_t (&v)[16]) {
+    if (k >= 16) {
+        const int32_t *l = ring + (k - 16) * kRingPitch;
+#pragma unroll
+        for (int q = 0; q < 16; q += 4) {
+            const int4 w = *reinterpret_cast<const int4 *>(l + q);
+            v[q] = w.x; v[q + 1] = w.y; v[q + 2] = w.z; v[q + 3] = w.w;
+        }
+    } else if ((e.x >> 29) & 1) {
+        const int32_t *t = tile + k * kMbPitch;
+#pragma unroll
+        for (int q = 0; q < 16; q++) v[q] = t[q * 16];
+    } else {
+        low_pass_run(coeff, e, v);
+    }
+}
+
+// Stage C1 of a full-resolution plane: prediction line `line` of macroblock
+// (a, b), a, b = 0 .. 4; of the fifth column and row only the first block
+// column / row lies in the tile, along which the other direction of
+// prediction still runs.  Returns the overflow flag.
+__device__ __forceinline__ bool predict_line(int32_t *t, int a, int b, int line, int hp) {
+    using A = Ar<true>;
+    bool ov = false;
+    if (hp == 1) {
+        // from left along block row `line`: needs columns 1..3 (a < 4)
+        if (a == 4 || (b == 4 && line != 0)) return false;
+        int32_t *p = t + (b < 4 ? (4 * b + a) * kMbPitch + line * 64 : kBottomAt + a * kHaloPitch);
+#pragma unroll
+        for (int c = 16; c < 64; c += 16)
+#pragma unroll
+            for (int r = 4; r < 16; r += 4) p[c + r] = A::add(p[c + r], p[c + r - 16], ov);
+    } else {
+        // from top along block column `line`: needs rows 1..3 (b < 4)
+        if (b == 4 || (a == 4 && line != 0)) return false;
+        int32_t *p = t + (a < 4 ? (4 * b + a) * kMbPitch + line * 16 : kRightAt + b * kHaloPitch);
+        const int down = a < 4 ? 64 : 16;
+#pragma unroll
+        for (int r = 1; r < 4; r++) {
+            p += down;
+#pragma unroll
+            for (int c = 1; c < 4; c++) p[c] = A::add(p[c], p[c - down], ov);
+        }
+    }
+    return ov;
 }
 
 // The table entries of macroblocks mx0-1 .. mx0+4 x my0-1 .. my0+4 of every
@@ -1443,11 +1566,9 @@ __device__ __forceinline__ bool hard_overlap(const ImageDev &im, int32_t *tiles,
         const int cx = line < nv ? on : at_line, cy = line < nv ? at_line : on;
         const bool vs = hard_cell(cols, cx), hs = hard_cell(rows, cy);
         if (cx >= ncx || cy >= ncy || (line >= nv && vs)) continue;   // a crossing belongs to its column
-        int32_t *t = tiles + pi * kPlaneInts;
-        auto at = [&](int c, int r) -> int32_t & {
-            const int sx = 4 * cx + 2 + c, sy = 4 * cy + 2 + r;
-            return t[elem((sy >> 2) * kIB + (sx >> 2), sy & 3, sx & 3)];
-        };
+        int32_t *t = tiles + pi * kTileInts;
+        const CellBlocks cell = cell_blocks(cx, cy);
+        auto at = [&](int c, int r) -> int32_t & { return cell_sample(t, cell, c, r); };
         // sample k of the operator: down column o, along row o, or quarter o in raster order
         const int c0 = vs && hs ? 2 * (o & 1) : vs ? o : 0, r0 = vs && hs ? (o & 2) : vs ? 0 : o;
         const int c1 = vs && hs ? c0 + 1 : vs ? o : 1, r1 = vs && hs ? r0 : vs ? 1 : o;
@@ -1474,11 +1595,11 @@ __device__ __forceinline__ bool edge_overlap(const ImageDev &im, int32_t *tiles,
         if (im.plane[pi].overlap < 1) continue;
         int X, Y, c0, c1, r0, r1;
         edge_cell_at(ec, k, X, Y, c0, c1, r0, r1);
-        int32_t *t = tiles + pi * kPlaneInts;
-        auto at = [&](int x, int y) -> int32_t & {
-            const int sx = x - 16 * mx0, sy = y - 16 * my0;
-            return t[elem((sy >> 2) * kIB + (sx >> 2), sy & 3, sx & 3)];
-        };
+        int32_t *t = tiles + pi * kTileInts;
+        // (a cell cut on its left or upper side has no blocks there: only the
+        // others are read)
+        const CellBlocks cell = cell_blocks((X - 2 - 16 * mx0) >> 2, (Y - 2 - 16 * my0) >> 2);
+        auto at = [&](int x, int y) -> int32_t & { return cell_sample(t, cell, x - X, y - Y); };
         const bool vs = c1 - c0 < 4, hs = r1 - r0 < 4;
         if (hard && vs != hs) {
             // quarter o of the part inside the plane
@@ -1559,13 +1680,12 @@ __device__ __forceinline__ bool edge_pixels(const ImageDev &im, const int32_t *t
         if (x < (int)o.crop_x || x >= (int)(o.crop_x + o.crop_w) || y < (int)o.crop_y ||
             y >= (int)(o.crop_y + o.crop_h))
             continue;
-        const int sx = x - 16 * mx0, sy = y - 16 * my0;
-        const int e = elem((sy >> 2) * kIB + (sx >> 2), sy & 3, sx & 3);
+        const int e = sample_at(x - 16 * mx0, y - 16 * my0);
         int32_t comp[4] = {0, 0, 0, 0};
 #pragma unroll
         for (int pi = 0; pi < NP; pi++)
-            if (pi < im.nplanes && pi < 4) comp[pi] = tiles[pi * kPlaneInts + e];
-        const int32_t a = has_alpha ? tiles[(NP - 1) * kPlaneInts + e] : 0;
+            if (pi < im.nplanes && pi < 4) comp[pi] = tiles[pi * kTileInts + e];
+        const int32_t a = has_alpha ? tiles[(NP - 1) * kTileInts + e] : 0;
         uint8_t *dst = o.base + (uint64_t)(y - o.crop_y) * o.row_stride + (uint64_t)(x - o.crop_x) * pixel_bytes;
         if (!fast_pixel<NP>(im, comp, a, dst, bad)) format_pixel(o, comp, a, dst, chs, bad);
     }
@@ -1598,103 +1718,46 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
     // MODE 0: interior tiles only; 1: edge tiles only; 2: either, by position
     const bool edge = MODE == 1 || (MODE == 2 && (mx0 == 0 || my0 == 0 || mx0 + kTileMbs >= (int)im.plane[0].mbs_x ||
                                                   my0 + kTileMbs >= (int)im.plane[0].mbs_y));
-    int32_t *tiles = smem;                       // NP planes of kIBlocks slots
-    int32_t *dcs = smem + NP * kPlaneInts;       // NP DC tiles of kIDC x kIDC
-    int32_t *lps = dcs + NP * kDcInts;           // NP x 36 macroblocks x 16 DC / low-pass coefficients (lp_stride<NP>() apart)
+    int32_t *tiles = smem;                       // NP planes of blocks
+    int32_t *dcs = smem + NP * kTileInts;        // NP DC tiles of kIDC x kIDC
+    int32_t *rings = dcs + NP * kDcInts;         // NP rings of 20 macroblocks' DC / low-pass values
     if (tid == 0) sh.bad = 0;
     if (MODE == 1 && tid < 32) {
         const uint32_t starts = hard_starts(im, mx0, my0);
         if (tid == 0) sh.hard = starts;
     }
     int bad = 0;
-    // phase 1: every coefficient the tile reads, in flight at once.  The DC /
-    // low-pass coefficients of the ring of 20 macroblocks around the tile, 4
-    // bytes each; then the coded blocks, 16 bytes a thread.  Each of the
-    // tile's 4 x 4 macroblocks is 1 KB of the arena: 64 threads copy one, in
-    // order, and its low-pass coefficients -- coefficient 0 of each of its
-    // blocks -- arrive with it, so they are not gathered as 16 scattered
-    // words.  The halo follows: the first block column of the macroblocks
-    // right of the tile, the first block row of those below it, and the
-    // corner block.
-    for (int k = tid; k < NP * 320; k += kThreads) {
-        const int pi = k / 320, q = k - pi * 320, m = ring_mb(q >> 4), kk = q & 15;
-        const uint4 e = mbc[pi * 36 + m];
-        const int bands = (e.x >> 28) & 3;
-        int32_t *dst = lps + pi * lp_ints<NP>() + m * lp_stride<NP>() + kk;
-        if (kk == 0 || bands != 0)
-            cp_async4(dst, im.plane[pi].coeff + (e.x & 0x0fffffffu) + (bands >= 2 ? kk * 16 : kk));
-        else
-            *dst = 0;
-    }
-    // the planes one after another in the four-plane kernel, whose code size
-    // stalls instruction fetch (C3 1.004 -> 0.990 ms a step), unrolled in the
-    // others
-    constexpr int kCopyUnroll = NP == 4 ? 1 : NP;
+    // phase 1: every coefficient the tile reads (PlaneCopy)
+    {
+        const PlaneCopy copy;
+        const bool plain = sh.plain != 0;
+        // the planes one after another in the four-plane kernel, whose code
+        // size stalls instruction fetch (C3 1.004 -> 0.990 ms a step),
+        // unrolled in the others
+        constexpr int kCopyUnroll = NP == 4 ? 1 : NP;
 #pragma unroll kCopyUnroll
-    for (int pi = 0; pi < NP; pi++) {
-        const int32_t *coeff = im.plane[pi].coeff;
-        int32_t *tile = tiles + pi * kPlaneInts;
-        const uint4 *ent = mbc + pi * 36;
-#pragma unroll
-        for (int pass = 0; pass < 4; pass++) {
-            const int mb = pass * 4 + (tid >> 6), c = tid & 63;
-            const int a = mb & 3, b = mb >> 2, blk = c >> 2, r = c & 3;
-            const int sidx = (4 * b + (blk >> 2)) * kIB + 4 * a + (blk & 3);
-            copy_chunk(tile + sidx * 16 + ((r ^ swz(sidx)) << 2), coeff, ent[(b + 1) * 6 + a + 1], c * 4);
-        }
-        if (tid < 33 * 4) {
-            const int hb = tid >> 2, r = tid & 3;
-            const int i = hb < 16 ? 16 : hb < 32 ? hb - 16 : 16;
-            const int j = hb < 16 ? hb : 16;
-            const int sidx = j * kIB + i;
-            copy_chunk(tile + sidx * 16 + ((r ^ swz(sidx)) << 2), coeff, ent[((j >> 2) + 1) * 6 + (i >> 2) + 1],
-                       (((j & 3) << 2) + (i & 3)) * 16 + r * 4);
-        }
+        for (int pi = 0; pi < NP; pi++)
+            copy.run(im.plane[pi].coeff, mbc + pi * 36, tiles + pi * kTileInts, rings + pi * kRingInts, plain);
     }
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads();
-    // The tile's own low-pass values: with three planes copied into the
-    // padded slots first, one value a thread, so that stage A reads every
-    // macroblock's 16 values as four conflict-free 16-byte loads (C2
-    // 0.1694 -> 0.1668 ms a step); with four planes the extra pass and
-    // barrier cost more than the conflicts of reading them in stage A straight
-    // from the blocks (C3 1.131 -> 1.165 ms), so those read them there.
-    constexpr bool kCopyInner = NP == 3;
-    if (kCopyInner) {
-        inner_low_pass(im, tiles, kPlaneInts, mbc, lps, lp_ints<NP>(), lp_stride<NP>(), NP);
-        __syncthreads();
-    }
     // stage A: first level of macroblocks mx0-1 .. mx0+4 (every one exists)
+    // (the own ones of every plane first: warps then take one way of reading them)
     for (int item = tid; item < NP * 36; item += kThreads) {
-        const int pi = item / 36, m = item - pi * 36;
+        int pi, k;
+        if (item < NP * 16) { pi = item >> 4; k = item & 15; }
+        else { pi = (item - NP * 16) / 20; k = 16 + (item - NP * 16) - pi * 20; }
+        const int m = first_level_mb(k);
         const PlaneDev &p = im.plane[pi];
-        const uint4 e = mbc[item];
+        const uint4 e = mbc[pi * 36 + m];
         int32_t v[16];
         bool b = false;
-        if (!kCopyInner && inner_mb(m)) {
-            if (((e.x >> 28) & 3) >= 2) {
-                const int32_t *t = tiles + pi * kPlaneInts;
-                const int s0 = (4 * (m / 6) - 4) * kIB + 4 * (m % 6) - 4;
-#pragma unroll
-                for (int k = 0; k < 16; k++) v[k] = t[elem(s0 + (k >> 2) * kIB + (k & 3), 0, 0)];
-            } else {
-                low_pass_run(p.coeff, e, v);
-            }
-        } else {
-            const int32_t *l = lps + pi * lp_ints<NP>() + m * lp_stride<NP>();
-#pragma unroll
-            for (int k = 0; k < 16; k += 4) {
-                const int4 q = *reinterpret_cast<const int4 *>(l + k);
-                v[k] = q.x; v[k + 1] = q.y; v[k + 2] = q.z; v[k + 3] = q.w;
-            }
-        }
+        first_level_values(k, p.coeff, e, tiles + pi * kTileInts, rings + pi * kRingInts, v);
         // one magnitude test of the coded values: below the transform's bound
         // after dequantization, every product fits and the wrapping
         // transform is exact; otherwise the checked steps
-        uint32_t lm = 0;
-#pragma unroll
-        for (int k = 1; k < 16; k++) lm |= mag(v[k]);
+        const uint32_t lm = mag_bound<1>(v);
         if ((uint64_t)(lm + 1) * e.z < (uint64_t)kTransformBound &&
             (uint64_t)(mag(v[0]) + 1) * e.y < (uint64_t)kTransformBound) {
             v[0] *= (int32_t)e.y;
@@ -1717,7 +1780,10 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             *reinterpret_cast<int4 *>(out + r * kIDC) = make_int4(v[r * 4], v[r * 4 + 1], v[r * 4 + 2], v[r * 4 + 3]);
         if (b) bad |= kFlagFirst;
     }
-    if (tid == 0) sh.next = claimed;
+    if (tid == 0) {
+        sh.next = claimed;
+        sh.plain = 1;
+    }
     __syncthreads();
     // the next work item's macroblock entries, in flight through stage B
     const uint32_t next = sh.next;
@@ -1768,10 +1834,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 *reinterpret_cast<int2 *>(base + r * kIDC + 2) = make_int2(v[r * 4 + 2], v[r * 4 + 3]);
             }
         } else {
-            // stage C1: prediction within macroblocks mx0 .. mx0+4; of the fifth
-            // column and row of macroblocks only their first block column / row
-            // lies in the tile, along which the other direction of prediction
-            // still runs
+            // stage C1: prediction within macroblocks mx0 .. mx0+4
             const int item = k < kFirstB ? k : k - kItemsB;
             const int pi = item / 100, q = item - pi * 100;
             const int line = q & 3, m = q >> 2;
@@ -1780,72 +1843,43 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             const int hp = (e.x >> 30) & 3, bands = (e.x >> 28) & 3;
             if (hp == 0 || bands < 2) continue;
             if (hp == 3) { bad |= kFlagInvalid; continue; }
-            int32_t *t = tiles + pi * kPlaneInts;
-            using A = Ar<true>;
-            bool ov = false;
-            if (hp == 1) {
-                // from left along block row `line`: needs columns 1..3 (a < 4)
-                if (a == 4 || (b == 4 && line != 0)) continue;
-                const int j = 4 * b + line;
-#pragma unroll
-                for (int c = 1; c < 4; c++) {
-                    const int sidx = j * kIB + 4 * a + c;
-#pragma unroll
-                    for (int r = 1; r < 4; r++) t[elem(sidx, r, 0)] = A::add(t[elem(sidx, r, 0)], t[elem(sidx - 1, r, 0)], ov);
-                }
-            } else {
-                // from top along block column `line`: needs rows 1..3 (b < 4)
-                if (b == 4 || (a == 4 && line != 0)) continue;
-                const int i = 4 * a + line;
-#pragma unroll
-                for (int r = 1; r < 4; r++) {
-                    const int sidx = (4 * b + r) * kIB + i;
-#pragma unroll
-                    for (int c = 1; c < 4; c++) t[elem(sidx, 0, c)] = A::add(t[elem(sidx, 0, c)], t[elem(sidx - kIB, 0, c)], ov);
-                }
-            }
-            if (ov) bad |= kFlagPrediction;
+            if (predict_line(tiles + pi * kTileInts, a, b, line, hp)) bad |= kFlagPrediction;
         }
     }
     cp_async_wait_all();
     __syncthreads();
-    // stage C2: block transforms of the 17 x 17 blocks; an edge tile's items
-    // are only its blocks inside the plane (q / bcols as a multiply by
-    // ceil(2^16 / bcols), exact for q < 2^16 / 17)
-    int bcols = kIB, brows = kIB, bmagic = 0;
+    if (next < item_count) note_plain(imn, mbc_next, NP, sh.plain);
+    // stage C2: block transforms, a pass over each plane's 256 own blocks,
+    // then one over every plane's 33 halo blocks; an edge tile leaves out its
+    // blocks beyond the plane
+    int bcols = kIB, brows = kIB;
     if (edge) {
-        bcols = min(kIB, 4 * ((int)im.plane[0].mbs_x - mx0));
-        brows = min(kIB, 4 * ((int)im.plane[0].mbs_y - my0));
-        bmagic = (65536 + bcols - 1) / bcols;
+        bcols = 4 * ((int)im.plane[0].mbs_x - mx0);
+        brows = 4 * ((int)im.plane[0].mbs_y - my0);
     }
-    const int bcount = bcols * brows;
     bool small = true;   // every transform input of this thread's blocks below 2^16
-    for (int item = tid; item < NP * bcount; item += kThreads) {
-        int pi, s, i, j;
-        if (edge) {
-            int q = item;
-            for (pi = 0; q >= bcount; pi++) q -= bcount;
-            j = (q * bmagic) >> 16;
-            i = q - j * bcols;
-            s = j * kIB + i;
+#pragma unroll 1
+    for (int pass = 0; pass <= NP; pass++) {
+        int pi = pass, i, j;
+        if (pass < NP) {
+            block_of_thread(tid, i, j);
         } else {
-            pi = item / kIBlocks;
-            s = item - pi * kIBlocks;
-            i = s % kIB;
-            j = s / kIB;
+            if (tid >= NP * 33) break;
+            pi = tid / 33;
+            const int hb = tid - pi * 33;
+            i = hb >= 16 && hb < 32 ? hb - 16 : 16;
+            j = hb < 16 ? hb : 16;
         }
+        if (edge && (i >= bcols || j >= brows)) continue;
         const uint32_t step = mbc[pi * 36 + ((j >> 2) + 1) * 6 + (i >> 2) + 1].w;
-        int32_t *blk = tiles + pi * kPlaneInts + s * 16;
-        const int sw = swz(s);
+        int32_t *blk = tiles + pi * kTileInts + block_at(i, j);
         int32_t v[16];
 #pragma unroll
         for (int r = 0; r < 4; r++) {
-            const int4 q = *reinterpret_cast<const int4 *>(blk + ((r ^ sw) << 2));
+            const int4 q = *reinterpret_cast<const int4 *>(blk + (r << 2));
             v[r * 4 + 0] = q.x; v[r * 4 + 1] = q.y; v[r * 4 + 2] = q.z; v[r * 4 + 3] = q.w;
         }
-        uint32_t m = 0;
-#pragma unroll
-        for (int k = 1; k < 16; k++) m |= mag(v[k]);
+        const uint32_t m = mag_bound<1>(v);
         v[0] = dcs[pi * kDcInts + (j + 4) * kIDC + i + 4];
         bool b = false;
         small &= (uint64_t)(m + 1) * step <= (1u << 16) && mag(v[0]) < (1u << 16);
@@ -1861,7 +1895,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         if (b) bad |= kFlagSecond;
 #pragma unroll
         for (int r = 0; r < 4; r++)
-            *reinterpret_cast<int4 *>(blk + ((r ^ sw) << 2)) = make_int4(v[r * 4], v[r * 4 + 1], v[r * 4 + 2], v[r * 4 + 3]);
+            *reinterpret_cast<int4 *>(blk + (r << 2)) = make_int4(v[r * 4], v[r * 4 + 1], v[r * 4 + 2], v[r * 4 + 3]);
     }
     const bool tile_small = __syncthreads_and(small) != 0;
     bool grid_cell = true, cut = false;
@@ -1883,7 +1917,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
     // stage D + E: the thread's sample cell, every plane, then its 16 pixels
     if (grid_cell) {
         const int cx = gcx, cy = gcy;
-        const int b00 = cy * kIB + cx;
+        const CellBlocks cell = cell_blocks(cx, cy);
         const OutputDev &o = im.out;
         const int x0 = 16 * mx0 + 2 + 4 * cx, y0 = 16 * my0 + 2 + 4 * cy;
         const bool inside = x0 >= (int)o.crop_x && x0 + 4 <= (int)(o.crop_x + o.crop_w) && y0 >= (int)o.crop_y &&
@@ -1893,9 +1927,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         bool obad = false, done = false;
         if (inside && kind == kOutRgb8 && NP >= 3 && !o.premultiply) {
             int32_t y[16], u[16], v[16];
-            bool ov = cell_samples(tiles, b00, overlap_of(0), y, tile_small);
-            ov |= cell_samples(tiles + kPlaneInts, b00, overlap_of(1), u, tile_small);
-            ov |= cell_samples(tiles + 2 * kPlaneInts, b00, overlap_of(2), v, tile_small);
+            bool ov = cell_samples(tiles, cell, overlap_of(0), y, tile_small);
+            ov |= cell_samples(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
+            ov |= cell_samples(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
             if (ov) bad |= kFlagOverlap;
             uint32_t m = 0;
             if (!tile_small) {
@@ -1921,7 +1955,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 bool alpha_ok = true;
                 if (NP == 4 && has_alpha) {
                     int32_t a[16];
-                    if (cell_samples(tiles + 3 * kPlaneInts, b00, overlap_of(3), a, tile_small))
+                    if (cell_samples(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small))
                         bad |= kFlagOverlap;
                     const ChannelScale &sa = o.ch[3];
                     const int32_t aadd = sa.shifted_bias + sa.rounding;
@@ -1946,7 +1980,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             }
         } else if (inside && kind == kOutDirect && NP == 1) {
             int32_t y[16];
-            if (cell_samples(tiles, b00, overlap_of(0), y, tile_small)) bad |= kFlagOverlap;
+            if (cell_samples(tiles, cell, overlap_of(0), y, tile_small)) bad |= kFlagOverlap;
             const ChannelScale &s = o.ch[0];
             const int eb = o.elem_bytes;
 #pragma unroll
@@ -1966,9 +2000,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         } else if (inside && kind == kOutF16Wide && o.nchw && NP == 4 && o.channels <= NP) {
             // colour channel planes first, then alpha
             int32_t y[16], u[16], v[16];
-            bool ov = cell_samples(tiles, b00, overlap_of(0), y, tile_small);
-            ov |= cell_samples(tiles + kPlaneInts, b00, overlap_of(1), u, tile_small);
-            ov |= cell_samples(tiles + 2 * kPlaneInts, b00, overlap_of(2), v, tile_small);
+            bool ov = cell_samples(tiles, cell, overlap_of(0), y, tile_small);
+            ov |= cell_samples(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
+            ov |= cell_samples(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
             if (ov) bad |= kFlagOverlap;
             uint8_t *base = o.base + (uint64_t)(y0 - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * 4;
             const int primaries = has_alpha ? o.channels - 1 : o.channels;
@@ -2031,7 +2065,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             }
             if (has_alpha && NP == 4) {
                 int32_t a[16];
-                if (cell_samples(tiles + 3 * kPlaneInts, b00, overlap_of(3), a, tile_small)) bad |= kFlagOverlap;
+                if (cell_samples(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small)) bad |= kFlagOverlap;
                 const ChannelScale &s = o.ch[o.channels - 1];
                 bool alean = s.post_shift < 0 && mag(s.shifted_bias) < (1u << 28) && mag(s.rounding) < (1u << 28);
                 if (alean && !tile_small) {
@@ -2055,9 +2089,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         } else if (inside && kind == kOutF16Wide && o.nchw && NP == 3 && o.channels <= NP) {
             // colour channel planes first, then alpha
             int32_t y[16], u[16], v[16];
-            bool ov = cell_samples(tiles, b00, overlap_of(0), y, tile_small);
-            ov |= cell_samples(tiles + kPlaneInts, b00, overlap_of(1), u, tile_small);
-            ov |= cell_samples(tiles + 2 * kPlaneInts, b00, overlap_of(2), v, tile_small);
+            bool ov = cell_samples(tiles, cell, overlap_of(0), y, tile_small);
+            ov |= cell_samples(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
+            ov |= cell_samples(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
             if (ov) bad |= kFlagOverlap;
             uint8_t *base = o.base + (uint64_t)(y0 - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * 4;
             const int primaries = has_alpha ? o.channels - 1 : o.channels;
@@ -2086,7 +2120,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             }
             if (has_alpha && NP == 4) {
                 int32_t a[16];
-                if (cell_samples(tiles + 3 * kPlaneInts, b00, overlap_of(3), a, tile_small)) bad |= kFlagOverlap;
+                if (cell_samples(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small)) bad |= kFlagOverlap;
                 const ChannelScale &s = o.ch[o.channels - 1];
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
@@ -2108,7 +2142,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             int32_t w[NP][16];
 #pragma unroll
             for (int pi = 0; pi < NP; pi++)
-                if (cell_samples(tiles + pi * kPlaneInts, b00, overlap_of(pi), w[pi], tile_small))
+                if (cell_samples(tiles + pi * kTileInts, cell, overlap_of(pi), w[pi], tile_small))
                     bad |= kFlagOverlap;
             const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
             const uint64_t chs = o.nchw ? o.plane_stride : (uint64_t)o.elem_bytes;
@@ -2370,7 +2404,7 @@ struct ChromaTile {
     static constexpr int kSquare0 = CV == 2 ? 1 : 3;         // DC row of the first
     static constexpr int kCells = CV == 2 ? 9 : 17;          // cells down; 4:2:2's first is the plane's top edge only
     static constexpr int kSmemInts =
-        kPlaneInts + jxr::kDcInts + jxr::kLpInts + 2 * (kInts + kDcInts + kLpInts) + 2 * 3 * kMbcInts;
+        kTileInts + jxr::kDcInts + kRingInts + 2 * (kInts + kDcInts + kLpInts) + 2 * 3 * kMbcInts;
     // plane row of the tile's first sample, and of cell row 0
     __device__ static int sample0(int my0) { return CV == 2 ? 8 * my0 - 8 : 16 * my0; }
     __device__ static int cell0(int my0) { return 4 * CV * my0 - 2; }
@@ -2473,7 +2507,7 @@ __device__ bool edge_pixels_chroma(const ImageDev &im, const int32_t *ytile, con
             y >= (int)(o.crop_y + o.crop_h))
             continue;
         const int sx = x - 16 * mx0, sy = y - 16 * my0;
-        int32_t comp[4] = {ytile[elem((sy >> 2) * kIB + (sx >> 2), sy & 3, sx & 3)], 0, 0, 0};
+        int32_t comp[4] = {ytile[sample_at(sx, sy)], 0, 0, 0};
         const int cx = x >> 1, cy = CV == 2 ? y >> 1 : y;
 #pragma unroll
         for (int pc = 0; pc < 2; pc++) {
@@ -2516,9 +2550,9 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
     const bool edge = MODE == 1 || (MODE == 2 && (mx0 == 0 || my0 == 0 || mx0 + kTileMbs >= (int)im.plane[0].mbs_x ||
                                                   my0 + kTileMbs >= (int)im.plane[0].mbs_y));
     int32_t *ytile = smem;                              // luma: 17 x 17 blocks
-    int32_t *ydc = ytile + kPlaneInts;                  // 24 x 24
-    int32_t *ylp = ydc + kDcInts;                       // 36 x 16
-    int32_t *ctile = ylp + kLpInts;                     // chroma: 2 x 11 x 11 or 17 blocks
+    int32_t *ydc = ytile + kTileInts;                   // 24 x 24
+    int32_t *yring = ydc + kDcInts;                     // 20 macroblocks' DC / low-pass values
+    int32_t *ctile = yring + kRingInts;                 // chroma: 2 x 11 x 11 or 17 blocks
     int32_t *cdc = ctile + 2 * CT::kInts;               // 2 x 12 x 12 or 24
     int32_t *clp = cdc + 2 * CT::kDcInts;               // 2 x 36 x 4 or 8
     if (tid == 0) sh.bad = 0;
@@ -2527,39 +2561,17 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
         if (tid == 0) sh.hard = starts;
     }
     int bad = 0;
-    // phase 1: the DC / low-pass values (luma 16, chroma 4 or 8 a macroblock) of
-    // the ring of luma macroblocks and of the 6 x 6 chroma macroblocks, then
-    // the blocks.  Those of the tile's own luma macroblocks arrive with their
-    // blocks (coefficient 0 of each) and are read from the slots.
-    for (int k = tid; k < 320 + 2 * CT::kLpInts; k += kThreads) {
-        int pi, m, kk;
-        int32_t *dst;
-        if (k < 320) { pi = 0; m = ring_mb(k >> 4); kk = k & 15; dst = ylp + m * 16 + kk; }
-        else { const int q = k - 320; pi = 1 + q / CT::kLpInts; const int r = q - (pi - 1) * CT::kLpInts; m = r / CT::kLow; kk = r % CT::kLow; dst = clp + q; }
+    // phase 1: luma as in the full-resolution tile; the DC / low-pass values
+    // (4 or 8 a macroblock) of the 6 x 6 chroma macroblocks, and their blocks
+    PlaneCopy().run(im.plane[0].coeff, mbc, ytile, yring, sh.plain != 0);
+    for (int k = tid; k < 2 * CT::kLpInts; k += kThreads) {
+        const int pi = 1 + k / CT::kLpInts, r = k - (pi - 1) * CT::kLpInts, m = r / CT::kLow, kk = r % CT::kLow;
         const uint4 e = mbc[pi * 36 + m];
         const int bands = (e.x >> 28) & 3;
         if (kk == 0 || bands != 0)
-            cp_async4(dst, im.plane[pi].coeff + (e.x & 0x0fffffffu) + (bands >= 2 ? kk * 16 : kk));
+            cp_async4(clp + k, im.plane[pi].coeff + (e.x & 0x0fffffffu) + (bands >= 2 ? kk * 16 : kk));
         else
-            *dst = 0;
-    }
-    {
-        const int32_t *coeff = im.plane[0].coeff;
-#pragma unroll
-        for (int pass = 0; pass < 4; pass++) {
-            const int mb = pass * 4 + (tid >> 6), c = tid & 63;
-            const int a = mb & 3, b = mb >> 2, blk = c >> 2, r = c & 3;
-            const int sidx = (4 * b + (blk >> 2)) * kIB + 4 * a + (blk & 3);
-            copy_chunk(ytile + sidx * 16 + ((r ^ swz(sidx)) << 2), coeff, mbc[(b + 1) * 6 + a + 1], c * 4);
-        }
-        if (tid < 33 * 4) {
-            const int hb = tid >> 2, r = tid & 3;
-            const int i = hb < 16 ? 16 : hb < 32 ? hb - 16 : 16;
-            const int j = hb < 16 ? hb : 16;
-            const int sidx = j * kIB + i;
-            copy_chunk(ytile + sidx * 16 + ((r ^ swz(sidx)) << 2), coeff, mbc[((j >> 2) + 1) * 6 + (i >> 2) + 1],
-                       (((j & 3) << 2) + (i & 3)) * 16 + r * 4);
-        }
+            clp[k] = 0;
     }
     for (int k = tid; k < 2 * CT::kInts / 4; k += kThreads) {
         const int pc = k / (CT::kInts / 4), q = k - pc * (CT::kInts / 4), sidx = q >> 2, r = q & 3;
@@ -2573,31 +2585,14 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
     __syncthreads();
     // stage A: first level of the 6 x 6 macroblocks of every plane
     for (int item = tid; item < 3 * 36; item += kThreads) {
-        const int pi = item / 36, m = item - pi * 36;
+        const int pi = item / 36, k36 = item - pi * 36, m = pi == 0 ? first_level_mb(k36) : k36;
         const PlaneDev &p = im.plane[pi];
-        const uint4 e = mbc[item];
+        const uint4 e = mbc[pi * 36 + m];
         bool b = false;
         if (pi == 0) {
             int32_t v[16];
-            if (inner_mb(m)) {
-                if (((e.x >> 28) & 3) >= 2) {
-                    const int s0 = (4 * (m / 6) - 4) * kIB + 4 * (m % 6) - 4;
-#pragma unroll
-                    for (int k = 0; k < 16; k++) v[k] = ytile[elem(s0 + (k >> 2) * kIB + (k & 3), 0, 0)];
-                } else {
-                    low_pass_run(p.coeff, e, v);
-                }
-            } else {
-                const int32_t *l = ylp + m * 16;
-#pragma unroll
-                for (int k = 0; k < 16; k += 4) {
-                    const int4 q = *reinterpret_cast<const int4 *>(l + k);
-                    v[k] = q.x; v[k + 1] = q.y; v[k + 2] = q.z; v[k + 3] = q.w;
-                }
-            }
-            uint32_t lm = 0;   // one magnitude test, as in the full-resolution tile
-#pragma unroll
-            for (int k = 1; k < 16; k++) lm |= mag(v[k]);
+            first_level_values(k36, p.coeff, e, ytile, yring, v);
+            const uint32_t lm = mag_bound<1>(v);   // one magnitude test, as in the full-resolution tile
             if ((uint64_t)(lm + 1) * e.z < (uint64_t)kTransformBound &&
                 (uint64_t)(mag(v[0]) + 1) * e.y < (uint64_t)kTransformBound) {
                 v[0] *= (int32_t)e.y;
@@ -2639,13 +2634,15 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
         }
         if (b) bad |= kFlagFirst;
     }
-    if (tid == 0) sh.next = claimed;
+    if (tid == 0) {
+        sh.next = claimed;
+        sh.plain = 1;
+    }
     __syncthreads();
     const uint32_t next = sh.next;
-    if (next < item_count) {
-        const WorkItem wn = items[next];
-        load_entries<3, MODE != 0>(images[wn.image & kImageMask], wn.tx, wn.ty, mbc_next);
-    }
+    const WorkItem wnext = next < item_count ? items[next] : WorkItem{0, 0, 0};
+    const ImageDev &imn = images[wnext.image & kImageMask];
+    if (next < item_count) load_entries<3, MODE != 0>(imn, wnext.tx, wnext.ty, mbc_next);
     // stages B and C1 in one pass (disjoint data: the DC tiles; the first
     // rows and columns of the high-pass blocks); the overlap items go to
     // threads that get no second item.
@@ -2714,27 +2711,7 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
                 const int hp = (e.x >> 30) & 3, bands = (e.x >> 28) & 3;
                 if (hp == 0 || bands < 2) continue;
                 if (hp == 3) { bad |= kFlagInvalid; continue; }
-                if (hp == 1) {
-                    if (a == 4 || (b == 4 && line != 0)) continue;
-                    const int j = 4 * b + line;
-#pragma unroll
-                    for (int c = 1; c < 4; c++) {
-                        const int sidx = j * kIB + 4 * a + c;
-#pragma unroll
-                        for (int r = 1; r < 4; r++)
-                            ytile[elem(sidx, r, 0)] = A::add(ytile[elem(sidx, r, 0)], ytile[elem(sidx - 1, r, 0)], ov);
-                    }
-                } else {
-                    if (b == 4 || (a == 4 && line != 0)) continue;
-                    const int i = 4 * a + line;
-#pragma unroll
-                    for (int r = 1; r < 4; r++) {
-                        const int sidx = (4 * b + r) * kIB + i;
-#pragma unroll
-                        for (int c = 1; c < 4; c++)
-                            ytile[elem(sidx, 0, c)] = A::add(ytile[elem(sidx, 0, c)], ytile[elem(sidx - kIB, 0, c)], ov);
-                    }
-                }
+                ov = predict_line(ytile, a, b, line, hp);
             } else {
                 const int q = item - 100, pc = q / kPred, rem = q - pc * kPred, line = rem % CV, m = rem / CV;
                 const int a = m % 6, b = m / 6;
@@ -2771,17 +2748,18 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
     // rows 1..10 (4:2:2: 0..16);
     // an edge tile's items are only its blocks inside the plane (divisions
     // as multiplies by ceil(2^16 / n), exact for these small quotients)
-    int lcols = kIB, lrows = kIB, lmagic = 0, ccols = 10, crows = CT::kTransRows, cmagic = 0;
+    if (next < item_count) note_plain(imn, mbc_next, 1, sh.plain);
+    int lcols = kIB, lrows = kIB, ccols = 10, crows = CT::kTransRows, cmagic = 0;
     if (edge) {
         const int rx = (int)im.plane[0].mbs_x - mx0, ry = (int)im.plane[0].mbs_y - my0;
-        lcols = min(kIB, 4 * rx);
-        lrows = min(kIB, 4 * ry);
+        lcols = 4 * rx;
+        lrows = 4 * ry;
         ccols = min(10, 2 * rx + 1);
         crows = CV == 2 ? min(10, 2 * ry + 1) : min(17, 4 * ry);
-        lmagic = (65536 + lcols - 1) / lcols;
         cmagic = (65536 + ccols - 1) / ccols;
     }
-    const int lcount = lcols * lrows, ccount = ccols * crows;
+    constexpr int lcount = 256 + 33;   // own blocks, a pass of the threads, then the halo
+    const int ccount = ccols * crows;
     bool small = true;   // every transform input of this thread's blocks below 2^16 (as in interior_tile)
     for (int item = tid; item < lcount + 2 * ccount; item += kThreads) {
         int32_t *blk;
@@ -2790,17 +2768,17 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
         int sw;
         if (item < lcount) {
             int i, j;
-            if (edge) {
-                j = (item * lmagic) >> 16;
-                i = item - j * lcols;
+            if (item < 256) {
+                block_of_thread(item, i, j);
             } else {
-                i = item % kIB;
-                j = item / kIB;
+                const int hb = item - 256;
+                i = hb >= 16 && hb < 32 ? hb - 16 : 16;
+                j = hb < 16 ? hb : 16;
             }
-            const int s = j * kIB + i;
+            if (edge && (i >= lcols || j >= lrows)) continue;
             step = mbc[((j >> 2) + 1) * 6 + (i >> 2) + 1].w;
-            blk = ytile + s * 16;
-            sw = swz(s);
+            blk = ytile + block_at(i, j);
+            sw = 0;
             dcv = ydc[(j + 4) * kIDC + i + 4];
         } else {
             const int q = item - lcount;
@@ -2828,9 +2806,7 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
             const int4 q = *reinterpret_cast<const int4 *>(blk + ((r ^ sw) << 2));
             v[r * 4 + 0] = q.x; v[r * 4 + 1] = q.y; v[r * 4 + 2] = q.z; v[r * 4 + 3] = q.w;
         }
-        uint32_t m = 0;
-#pragma unroll
-        for (int k = 1; k < 16; k++) m |= mag(v[k]);
+        const uint32_t m = mag_bound<1>(v);
         v[0] = dcv;
         bool b = false;
         small &= (uint64_t)(m + 1) * step <= (1u << 16) && mag(v[0]) < (1u << 16);
@@ -2901,7 +2877,7 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
                             y0 + 4 <= (int)(o.crop_y + o.crop_h);
         bool obad = false, done = false;
         int32_t y[16];
-        if (cell_rw(ytile, cy * kIB + cx, kIB, MODE == 1 && cut ? 0 : im.plane[0].overlap, y, false, tile_small)) bad |= kFlagOverlap;
+        if (cell_samples(ytile, cell_blocks(cx, cy), MODE == 1 && cut ? 0 : im.plane[0].overlap, y, tile_small)) bad |= kFlagOverlap;
         // chroma columns (tile coordinates) 8 + 2cx .. 11 + 2cx, rows 8 + 2cy .. 11 + 2cy (4:2:2: 2 + 4cy .. 5 + 4cy)
         if (tile_small && !edge && inside && o.kind == kOutRgb8 && !o.premultiply &&
             (o.channels == 3 || o.ch[3].padding)) {
@@ -3118,7 +3094,10 @@ jxrb_interior_chroma_tiles(const ImageDev *__restrict__ images, const WorkItem *
         {
             const WorkItem w = items[i];
             load_entries<3, MODE != 0>(images[w.image & kImageMask], w.tx, w.ty, mbc[0]);
+            if (threadIdx.x == 0) sh.plain = 1;
             cp_async_wait_all();
+            __syncthreads();
+            note_plain(images[w.image & kImageMask], mbc[0], 1, sh.plain);
             __syncthreads();
         }
         __shared__ ImageDev simg;
@@ -3152,13 +3131,16 @@ jxrb_interior_tiles(const ImageDev *__restrict__ images, const WorkItem *__restr
     extern __shared__ __align__(16) int32_t smem_interior[];
     __shared__ TileShared sh;
     uint4 *mbc[2];
-    mbc[0] = reinterpret_cast<uint4 *>(smem_interior + NP * (kPlaneInts + kDcInts + lp_ints<NP>()));
+    mbc[0] = reinterpret_cast<uint4 *>(smem_interior + NP * (kTileInts + kDcInts + kRingInts));
     mbc[1] = mbc[0] + NP * 36;
     uint32_t i;
     if (claim(counters, item_count, i)) {
         const WorkItem w = items[i];
         load_entries<NP, MODE != 0>(images[w.image & kImageMask], w.tx, w.ty, mbc[0]);
+        if (threadIdx.x == 0) sh.plain = 1;
         cp_async_wait_all();
+        __syncthreads();
+        note_plain(images[w.image & kImageMask], mbc[0], NP, sh.plain);
         __syncthreads();
         __shared__ ImageDev simg;
         uint32_t held = 0xffffffffu;
@@ -3185,14 +3167,11 @@ jxrb_interior_tiles(const ImageDev *__restrict__ images, const WorkItem *__restr
 namespace jxr {
 
 size_t tile_smem_bytes(int planes) {
-    return (size_t)planes * (kPlaneInts + kDcInts + kLpInts + kMbcInts) * sizeof(int32_t);
+    return (size_t)planes * (kPlaneInts + kDcInts) * sizeof(int32_t);
 }
 
-// Interior tiles keep padded low-pass slots and a second set of macroblock
-// entries (the next tile's).
 static size_t interior_smem_bytes(int planes) {
-    const int lp = planes == 3 ? lp_ints<3>() : lp_ints<1>();
-    return (size_t)planes * (kPlaneInts + kDcInts + lp + 2 * kMbcInts) * sizeof(int32_t);
+    return (size_t)planes * (kTileInts + kDcInts + kRingInts + 2 * kMbcInts) * sizeof(int32_t);
 }
 
 typedef void (*TileKernel)(const ImageDev *, const WorkItem *, uint32_t, uint32_t *, uint32_t *);
