@@ -1241,6 +1241,46 @@ constexpr int kRingPitch = 20;
 constexpr int kRingInts = 20 * kRingPitch;
 constexpr int kMbcInts = 36 * 4;    // their 16-byte entries
 
+// The checked forms of the tile kernels' block operators, out of line: few
+// blocks take them, and inline, once at each use, they spread the code that
+// every block runs over several times the instruction cache.  A caller's
+// values go through a copy, so that its own stay in registers.
+__device__ __noinline__ bool checked_transform_of(int32_t (&v)[16], int first, uint32_t step) {
+    bool bad = false;
+    for (int k = first; k < 16; k++) v[k] = dequant(v[k], step, bad);
+    bad |= pct16(v);
+    return bad;
+}
+__device__ __noinline__ bool checked_overlap_of(int32_t (&v)[16]) { return inverse_pot4x4<true>(v); }
+__device__ __forceinline__ bool checked_transform(int32_t (&v)[16], int first, uint32_t step) {
+    int32_t w[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) w[k] = v[k];
+    const bool bad = checked_transform_of(w, first, step);
+#pragma unroll
+    for (int k = 0; k < 16; k++) v[k] = w[k];
+    return bad;
+}
+__device__ __forceinline__ bool checked_first_level(int32_t (&v)[16], uint32_t dc_step, uint32_t step, int scale2) {
+    bool bad = false;
+    v[0] = dequant(v[0], dc_step, bad);
+    bad |= checked_transform(v, 1, step);
+    if (scale2) {
+#pragma unroll
+        for (int k = 0; k < 16; k++) v[k] = dequant(v[k], 2, bad);
+    }
+    return bad;
+}
+__device__ __forceinline__ bool checked_overlap(int32_t (&v)[16]) {
+    int32_t w[16];
+#pragma unroll
+    for (int k = 0; k < 16; k++) w[k] = v[k];
+    const bool bad = checked_overlap_of(w);
+#pragma unroll
+    for (int k = 0; k < 16; k++) v[k] = w[k];
+    return bad;
+}
+
 // The four blocks a sample cell takes its quarters from.
 struct CellBlocks {
     int b00, b01, b10, b11;
@@ -1255,14 +1295,9 @@ __device__ __forceinline__ int32_t &cell_sample(int32_t *t, const CellBlocks &b,
 }
 
 // The 16 samples of a sample cell (lower-right quarter of block b00 and the
-// neighbouring quarters of the blocks right of and below it), second-level
-// overlap applied when the plane has it.  `small`: every block transform of
-// the tile had inputs below 2^16 in magnitude, so the cell's values are below
-// 35.3 * 2^16 and the wrapping operator needs no magnitude test (interval
-// bounds of the inverse transform and overlap steps: outputs below 2^27.8,
-// intermediates below 2^28.2).  Returns the overflow flag.
-__device__ __forceinline__ bool cell_samples(const int32_t *t, const CellBlocks &b, int overlap, int32_t (&w)[16],
-                                             bool small = false) {
+// neighbouring quarters of the blocks right of and below it) as the block
+// transforms left them.
+__device__ __forceinline__ void cell_load(const int32_t *t, const CellBlocks &b, int32_t (&w)[16]) {
     const int2 a0 = *reinterpret_cast<const int2 *>(t + b.b00 + 10);
     const int2 a1 = *reinterpret_cast<const int2 *>(t + b.b01 + 8);
     const int2 a2 = *reinterpret_cast<const int2 *>(t + b.b00 + 14);
@@ -1275,8 +1310,30 @@ __device__ __forceinline__ bool cell_samples(const int32_t *t, const CellBlocks 
     w[4] = a2.x; w[5] = a2.y; w[6] = a3.x; w[7] = a3.y;
     w[8] = a4.x; w[9] = a4.y; w[10] = a5.x; w[11] = a5.y;
     w[12] = a6.x; w[13] = a6.y; w[14] = a7.x; w[15] = a7.y;
-    if (overlap < 1) return false;
-    return small ? inverse_pot4x4<false>(w) : pot16(w);
+}
+
+// The same, second-level overlap applied when the plane has it.  `small`:
+// every block transform of the tile had inputs below 2^16 in magnitude, so the
+// cell's values are below 35.3 * 2^16 and the wrapping operator needs no
+// magnitude test (interval bounds of the inverse transform and overlap steps:
+// outputs below 2^27.8, intermediates below 2^28.2).  False, the values as they
+// were, when the cell needs the checked operator: the specialised outputs then
+// leave the cell to the general store, which has it (with every plane's cell
+// held, a call here would spill).
+__device__ __forceinline__ bool cell_samples_fast(const int32_t *t, const CellBlocks &b, int overlap, int32_t (&w)[16],
+                                                  bool small) {
+    cell_load(t, b, w);
+    if (overlap < 1) return true;
+    if (!small && mag_bound<0>(w) >= (uint32_t)kOverlapBound) return false;
+    inverse_pot4x4<false>(w);
+    return true;
+}
+
+// Any cell; returns the overflow flag.
+__device__ __forceinline__ bool cell_samples(const int32_t *t, const CellBlocks &b, int overlap, int32_t (&w)[16],
+                                             bool small = false) {
+    if (cell_samples_fast(t, b, overlap, w, small)) return false;
+    return checked_overlap(w);
 }
 
 // Ring macroblock r (0..19) of the 6 x 6 grid: the top row, then the left
@@ -1692,6 +1749,29 @@ __device__ __forceinline__ bool edge_pixels(const ImageDev &im, const int32_t *t
     return bad;
 }
 
+// Samples and terms of a channel below this leave no checked scaling step
+// room to overflow: 2^28, less what the shift up after the rounding takes.
+__device__ __forceinline__ uint32_t lean_limit(const ChannelScale &s) {
+    return s.post_shift < 28 ? (1u << 28) >> max(s.post_shift, 0) : 0u;
+}
+__device__ __forceinline__ bool lean_channel(const ChannelScale &s) {
+    return mag(s.shifted_bias) < lean_limit(s) && mag(s.rounding) < lean_limit(s);
+}
+// Whether the three colour channels are R, G and B from YUV in some order,
+// each lean and without a shift up; `at`: two bits a component, its channel.
+__device__ __forceinline__ bool lean_rgb(const OutputDev &o, int colours, uint32_t &at) {
+    bool lean = o.conv == kConvYuvToRgb && !o.packed_swap && colours == 3;
+    uint32_t seen = 0;
+    at = 0;
+    for (int ch = 0; ch < 3; ch++) {
+        const ChannelScale &s = o.ch[ch];
+        lean &= !s.padding && s.post_shift < 0 && lean_channel(s);
+        seen |= 1u << (s.source & 31);
+        at |= (uint32_t)ch << (2 * (s.source & 3));
+    }
+    return lean && seen == 7u;
+}
+
 // One interior tile.  Its macroblock entries are already in `mbc` (copied
 // while the previous tile ran); while it runs, the entries of the next work
 // item go into `mbc_next`.  `claimed` is thread 0's claim of that next item.
@@ -1758,21 +1838,19 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         // after dequantization, every product fits and the wrapping
         // transform is exact; otherwise the checked steps
         const uint32_t lm = mag_bound<1>(v);
-        if ((uint64_t)(lm + 1) * e.z < (uint64_t)kTransformBound &&
-            (uint64_t)(mag(v[0]) + 1) * e.y < (uint64_t)kTransformBound) {
+        // (half the bound: the outputs, below 35.3 * 2^24, are doubled where
+        // the plane is scaled)
+        if ((uint64_t)(lm + 1) * e.z < (uint64_t)kTransformBound / 2 &&
+            (uint64_t)(mag(v[0]) + 1) * e.y < (uint64_t)kTransformBound / 2) {
             v[0] *= (int32_t)e.y;
 #pragma unroll
             for (int k = 1; k < 16; k++) v[k] *= (int32_t)e.z;
             inverse_pct<false>(v);
+            const int up = p.scale2 ? 1 : 0;
+#pragma unroll
+            for (int k = 0; k < 16; k++) v[k] <<= up;
         } else {
-            v[0] = dequant(v[0], e.y, b);
-#pragma unroll
-            for (int k = 1; k < 16; k++) v[k] = dequant(v[k], e.z, b);
-            b |= pct16(v);
-        }
-        if (p.scale2) {
-#pragma unroll
-            for (int k = 0; k < 16; k++) v[k] = dequant(v[k], 2, b);
+            b = checked_first_level(v, e.y, e.z, p.scale2);
         }
         int32_t *out = dcs + pi * kDcInts + (m / 6) * 4 * kIDC + (m % 6) * 4;
 #pragma unroll
@@ -1827,7 +1905,8 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 const int2 b = *reinterpret_cast<const int2 *>(base + r * kIDC + 2);
                 v[r * 4] = a.x; v[r * 4 + 1] = a.y; v[r * 4 + 2] = b.x; v[r * 4 + 3] = b.y;
             }
-            if (pot16(v)) bad |= kFlagOverlap;
+            if (mag_bound<0>(v) < (uint32_t)kOverlapBound) inverse_pot4x4<false>(v);
+            else if (checked_overlap(v)) bad |= kFlagOverlap;
 #pragma unroll
             for (int r = 0; r < 4; r++) {
                 *reinterpret_cast<int2 *>(base + r * kIDC) = make_int2(v[r * 4], v[r * 4 + 1]);
@@ -1888,9 +1967,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             for (int k = 1; k < 16; k++) v[k] = v[k] * (int32_t)step;
             inverse_pct<false>(v);
         } else {
-#pragma unroll
-            for (int k = 1; k < 16; k++) v[k] = dequant(v[k], step, b);
-            b |= pct16(v);
+            b = checked_transform(v, 1, step);
         }
         if (b) bad |= kFlagSecond;
 #pragma unroll
@@ -1925,18 +2002,14 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         const int kind = o.kind;
         const bool has_alpha = im.alpha >= 0;
         bool obad = false, done = false;
+        uint32_t rgb_at = 0;
         if (inside && kind == kOutRgb8 && NP >= 3 && !o.premultiply) {
             int32_t y[16], u[16], v[16];
-            bool ov = cell_samples(tiles, cell, overlap_of(0), y, tile_small);
-            ov |= cell_samples(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
-            ov |= cell_samples(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
-            if (ov) bad |= kFlagOverlap;
-            uint32_t m = 0;
-            if (!tile_small) {
-#pragma unroll
-                for (int k = 0; k < 16; k++) m |= mag(y[k]) | mag(u[k]) | mag(v[k]);
-            }
-            if (m < (1u << 28)) {
+            bool fast = cell_samples_fast(tiles, cell, overlap_of(0), y, tile_small);
+            fast &= cell_samples_fast(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
+            fast &= cell_samples_fast(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
+            if (!tile_small) fast &= max(max(mag_bound<0>(y), mag_bound<0>(u)), mag_bound<0>(v)) < (1u << 28);
+            if (fast) {
                 const ChannelScale &sc = o.ch[0];
                 const int32_t add = sc.shifted_bias + sc.rounding;
                 const int shift = sc.shift;
@@ -1955,17 +2028,12 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 bool alpha_ok = true;
                 if (NP == 4 && has_alpha) {
                     int32_t a[16];
-                    if (cell_samples(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small))
-                        bad |= kFlagOverlap;
+                    alpha_ok = cell_samples_fast(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small);
+                    if (!tile_small) alpha_ok &= mag_bound<0>(a) < (1u << 28);
                     const ChannelScale &sa = o.ch[3];
                     const int32_t aadd = sa.shifted_bias + sa.rounding;
-                    uint32_t am = 0;
 #pragma unroll
-                    for (int k = 0; k < 16; k++) {
-                        am |= mag(a[k]);
-                        px[k] |= clamp_u8((a[k] + aadd) >> sa.shift) << 24;
-                    }
-                    alpha_ok = tile_small || am < (1u << 28);
+                    for (int k = 0; k < 16; k++) px[k] |= clamp_u8((a[k] + aadd) >> sa.shift) << 24;
                 }
                 if (alpha_ok) {
 #pragma unroll
@@ -1978,169 +2046,98 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                     done = true;
                 }
             }
-        } else if (inside && kind == kOutDirect && NP == 1) {
+        } else if (inside && kind == kOutDirect && NP == 1 && lean_channel(o.ch[0])) {
+            // samples and terms below the lean limit: no scaling step can
+            // overflow, so the unchecked ones give the same values
             int32_t y[16];
-            if (cell_samples(tiles, cell, overlap_of(0), y, tile_small)) bad |= kFlagOverlap;
-            const ChannelScale &s = o.ch[0];
-            const int eb = o.elem_bytes;
+            const bool fast = cell_samples_fast(tiles, cell, overlap_of(0), y, tile_small);
+            if (fast && ((tile_small && o.ch[0].post_shift <= 0) || mag_bound<0>(y) < lean_limit(o.ch[0]))) {
+                const ChannelScale &s = o.ch[0];
+                const int eb = o.elem_bytes;
+                const int32_t add = s.shifted_bias + s.rounding, shift = s.shift, up = max(s.post_shift, 0), lo = s.lo, hi = s.hi;
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
-                uint32_t q[4];
+                for (int r = 0; r < 4; r++) {
+                    uint32_t q[4];
 #pragma unroll
-                for (int c = 0; c < 4; c++) q[c] = (uint32_t)min(max(apply_scale(s, y[r * 4 + c], obad), s.lo), s.hi);
-                uint8_t *dst = o.base + (uint64_t)(y0 + r - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * eb;
-                if (eb == 2) store8(dst, (q[0] & 0xffffu) | (q[1] << 16), (q[2] & 0xffffu) | (q[3] << 16));
-                else if (eb == 4) store16(dst, q[0], q[1], q[2], q[3]);
-                else {
-                    const uint32_t w[1] = {(q[0] & 0xffu) | ((q[1] & 0xffu) << 8) | ((q[2] & 0xffu) << 16) | (q[3] << 24)};
-                    store_words(dst, w);
+                    for (int c = 0; c < 4; c++) q[c] = (uint32_t)min(max(((y[r * 4 + c] + add) >> shift) << up, lo), hi);
+                    uint8_t *dst = o.base + (uint64_t)(y0 + r - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * eb;
+                    if (eb == 2) store8(dst, (q[0] & 0xffffu) | (q[1] << 16), (q[2] & 0xffffu) | (q[3] << 16));
+                    else if (eb == 4) store16(dst, q[0], q[1], q[2], q[3]);
+                    else {
+                        const uint32_t w[1] = {(q[0] & 0xffu) | ((q[1] & 0xffu) << 8) | ((q[2] & 0xffu) << 16) | (q[3] << 24)};
+                        store_words(dst, w);
+                    }
                 }
+                done = true;
             }
-            done = true;
-        } else if (inside && kind == kOutF16Wide && o.nchw && NP == 4 && o.channels <= NP) {
-            // colour channel planes first, then alpha
-            int32_t y[16], u[16], v[16];
-            bool ov = cell_samples(tiles, cell, overlap_of(0), y, tile_small);
-            ov |= cell_samples(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
-            ov |= cell_samples(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
-            if (ov) bad |= kFlagOverlap;
+        } else if (NP >= 3 && inside && kind == kOutF16Wide && o.nchw && o.channels <= NP &&
+                   lean_rgb(o, has_alpha ? o.channels - 1 : o.channels, rgb_at) &&
+                   (!has_alpha || (o.ch[o.channels - 1].post_shift < 0 && lean_channel(o.ch[o.channels - 1])))) {
+            // R, G and B to their channel planes, alpha to the last.  YUV
+            // below 2^28 keeps the inverse RCT below 2^30 and, with terms below
+            // 2^28, every scaling step below 2^31: no checked step can
+            // overflow, so the unchecked ones give the same values.  Larger
+            // samples and other conversions take the general store: unrolled
+            // beside this form, their code alone stalled instruction fetch
+            // (3072 x 3072 half with alpha: 165 -> 134 us without it, 4096 x
+            // 4096 RGB8, the same code in the three-plane kernel, 136 -> 128;
+            // with the checked operators out of line too, 125 and 130).
             uint8_t *base = o.base + (uint64_t)(y0 - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * 4;
-            const int primaries = has_alpha ? o.channels - 1 : o.channels;
             const uint64_t rs = o.row_stride, ps = o.plane_stride;
-            // The channels' terms in registers (the stores may alias the
-            // descriptor).  YUV below 2^28 keeps the inverse RCT below 2^30,
-            // and terms below 2^28 keep every scaling step below 2^31: no
-            // checked step can overflow, so the unchecked forms give the same
-            // values.  A tile whose transform inputs were all below 2^16 has
-            // its overlap outputs below 2^27.8, so its cells skip that test.
-            // The lean form takes R, G and B to channels 0, 1, 2 with no
-            // padding channel; other orders take the general form.
-            // Four-plane kernels only: in the three-plane one the extra code
-            // costs the RGB8 path more than it saves here.
-            int32_t cadd[3], cshift[3];
-            bool lean = o.conv == kConvYuvToRgb && !o.packed_swap;
+            bool lean = true;
+            if (has_alpha && NP == 4) {
+                int32_t a[16];
+                lean = cell_samples_fast(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small) &&
+                       (tile_small || mag_bound<0>(a) < (1u << 28));
+                if (lean) {
+                    const ChannelScale &s = o.ch[o.channels - 1];
+                    const int32_t add = s.shifted_bias + s.rounding, shift = s.shift;
+                    uint8_t *abase = base + (uint64_t)(o.channels - 1) * ps;
 #pragma unroll
-            for (int ch = 0; ch < 3; ch++) {
-                const ChannelScale &s = o.ch[ch];
-                cadd[ch] = s.shifted_bias + s.rounding;
-                cshift[ch] = s.shift;
-                lean &= s.source == ch && !s.padding && s.post_shift < 0 && mag(s.shifted_bias) < (1u << 28) &&
-                        mag(s.rounding) < (1u << 28);
+                    for (int r = 0; r < 4; r++)
+                        store16(abase + r * rs, f16_widened((a[r * 4] + add) >> shift), f16_widened((a[r * 4 + 1] + add) >> shift),
+                                f16_widened((a[r * 4 + 2] + add) >> shift), f16_widened((a[r * 4 + 3] + add) >> shift));
+                }
             }
-            if (lean && !tile_small) {
-                uint32_t m = 0;
+            if (lean) {
+                int32_t y[16], u[16], v[16];
+                bool fast = cell_samples_fast(tiles, cell, overlap_of(0), y, tile_small);
+                fast &= cell_samples_fast(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
+                fast &= cell_samples_fast(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
+                if (fast && (tile_small || max(max(mag_bound<0>(y), mag_bound<0>(u)), mag_bound<0>(v)) < (1u << 28))) {
+                    int32_t cadd[3], cshift[3];
+                    uint8_t *plane[3];
 #pragma unroll
-                for (int k = 0; k < 16; k++) m |= mag(y[k]) | mag(u[k]) | mag(v[k]);
-                lean = m < (1u << 28);
-            }
+                    for (int c = 0; c < 3; c++) {
+                        const int ch = (rgb_at >> (2 * c)) & 3;
+                        cadd[c] = o.ch[ch].shifted_bias + o.ch[ch].rounding;
+                        cshift[c] = o.ch[ch].shift;
+                        plane[c] = base + ch * ps;
+                    }
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
-                uint32_t q[3][4];
+                    for (int r = 0; r < 4; r++) {
+                        uint32_t q[3][4];
 #pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int k = r * 4 + c;
-                    if (lean) {
-                        int32_t R, G, B;
-                        yuv_to_rgb_fast(y[k], u[k], v[k], R, G, B);
-                        q[0][c] = f16_widened((R + cadd[0]) >> cshift[0]);
-                        q[1][c] = f16_widened((G + cadd[1]) >> cshift[1]);
-                        q[2][c] = f16_widened((B + cadd[2]) >> cshift[2]);
-                    } else {
-                        const int32_t in[4] = {y[k], u[k], v[k], 0};
-                        int32_t conv[4];
-                        convert(o, in, conv, obad);
-#pragma unroll
-                        for (int ch = 0; ch < 3; ch++) {
-                            const ChannelScale &s = o.ch[ch];
-                            const int src = s.source;
-                            const int32_t val = apply_scale(s, src == 0 ? conv[0] : src == 1 ? conv[1] : conv[2], obad);
-                            const uint32_t mm = min((uint32_t)(val < 0 ? -(int64_t)val : val), 32767u);
-                            q[ch][c] = widen_f16(s.padding ? 0u : ((val < 0 ? 0x8000u : 0u) | mm));
+                        for (int c = 0; c < 4; c++) {
+                            const int k = r * 4 + c;
+                            int32_t R, G, B;
+                            yuv_to_rgb_fast(y[k], u[k], v[k], R, G, B);
+                            q[0][c] = f16_widened((R + cadd[0]) >> cshift[0]);
+                            q[1][c] = f16_widened((G + cadd[1]) >> cshift[1]);
+                            q[2][c] = f16_widened((B + cadd[2]) >> cshift[2]);
                         }
+#pragma unroll
+                        for (int c = 0; c < 3; c++) store16(plane[c] + r * rs, q[c][0], q[c][1], q[c][2], q[c][3]);
                     }
-                }
-#pragma unroll
-                for (int ch = 0; ch < 3; ch++)
-                    if (ch < primaries) store16(base + r * rs + ch * ps, q[ch][0], q[ch][1], q[ch][2], q[ch][3]);
-            }
-            if (has_alpha && NP == 4) {
-                int32_t a[16];
-                if (cell_samples(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small)) bad |= kFlagOverlap;
-                const ChannelScale &s = o.ch[o.channels - 1];
-                bool alean = s.post_shift < 0 && mag(s.shifted_bias) < (1u << 28) && mag(s.rounding) < (1u << 28);
-                if (alean && !tile_small) {
-                    uint32_t am = 0;
-#pragma unroll
-                    for (int k = 0; k < 16; k++) am |= mag(a[k]);
-                    alean = am < (1u << 29);
-                }
-                const int32_t aadd = s.shifted_bias + s.rounding, ashift = s.shift;
-                uint8_t *abase = base + (uint64_t)(o.channels - 1) * ps;
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    uint32_t q[4];
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        q[c] = f16_widened(alean ? (a[r * 4 + c] + aadd) >> ashift : apply_scale(s, a[r * 4 + c], obad));
-                    store16(abase + r * rs, q[0], q[1], q[2], q[3]);
+                    done = true;
                 }
             }
-            done = true;
-        } else if (inside && kind == kOutF16Wide && o.nchw && NP == 3 && o.channels <= NP) {
-            // colour channel planes first, then alpha
-            int32_t y[16], u[16], v[16];
-            bool ov = cell_samples(tiles, cell, overlap_of(0), y, tile_small);
-            ov |= cell_samples(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
-            ov |= cell_samples(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
-            if (ov) bad |= kFlagOverlap;
-            uint8_t *base = o.base + (uint64_t)(y0 - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * 4;
-            const int primaries = has_alpha ? o.channels - 1 : o.channels;
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                uint32_t q[3][4];
-#pragma unroll
-                for (int c = 0; c < 4; c++) {
-                    const int k = r * 4 + c;
-                    const int32_t in[4] = {y[k], u[k], v[k], 0};
-                    int32_t conv[4];
-                    convert(o, in, conv, obad);
-#pragma unroll
-                    for (int ch = 0; ch < 3; ch++) {
-                        const ChannelScale &s = o.ch[ch];
-                        const int src = s.source;
-                        const int32_t val = apply_scale(s, src == 0 ? conv[0] : src == 1 ? conv[1] : conv[2], obad);
-                        const uint32_t mm = min((uint32_t)(val < 0 ? -(int64_t)val : val), 32767u);
-                        q[ch][c] = widen_f16(s.padding ? 0u : ((val < 0 ? 0x8000u : 0u) | mm));
-                    }
-                }
-#pragma unroll
-                for (int ch = 0; ch < 3; ch++)
-                    if (ch < primaries)
-                        store16(base + r * o.row_stride + ch * o.plane_stride, q[ch][0], q[ch][1], q[ch][2], q[ch][3]);
-            }
-            if (has_alpha && NP == 4) {
-                int32_t a[16];
-                if (cell_samples(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small)) bad |= kFlagOverlap;
-                const ChannelScale &s = o.ch[o.channels - 1];
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    uint32_t q[4];
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const int32_t val = apply_scale(s, a[r * 4 + c], obad);
-                        const uint32_t mm = min((uint32_t)(val < 0 ? -(int64_t)val : val), 32767u);
-                        q[c] = widen_f16((val < 0 ? 0x8000u : 0u) | mm);
-                    }
-                    store16(base + r * o.row_stride + (o.channels - 1) * o.plane_stride, q[0], q[1], q[2], q[3]);
-                }
-            }
-            done = true;
         }
         if (!done) {
             // any other output, or pixels at the crop edge: the general store,
             // pixel by pixel, from every plane's cell samples
             int32_t w[NP][16];
-#pragma unroll
+#pragma unroll 1
             for (int pi = 0; pi < NP; pi++)
                 if (cell_samples(tiles + pi * kTileInts, cell, overlap_of(pi), w[pi], tile_small))
                     bad |= kFlagOverlap;
@@ -2426,7 +2423,11 @@ __device__ __forceinline__ bool cell_rw(int32_t *t, int b00, int stride, int ove
         w[2 * k] = a.x;
         w[2 * k + 1] = a.y;
     }
-    const bool bad = overlap < 1 ? false : small ? inverse_pot4x4<false>(w) : pot16(w);
+    bool bad = false;
+    if (overlap >= 1) {
+        if (small || mag_bound<0>(w) < (uint32_t)kOverlapBound) inverse_pot4x4<false>(w);
+        else bad = checked_overlap(w);
+    }
     if (store) {
 #pragma unroll
         for (int k = 0; k < 8; k++) *q[k] = make_int2(w[2 * k], w[2 * k + 1]);
@@ -2593,21 +2594,19 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
             int32_t v[16];
             first_level_values(k36, p.coeff, e, ytile, yring, v);
             const uint32_t lm = mag_bound<1>(v);   // one magnitude test, as in the full-resolution tile
-            if ((uint64_t)(lm + 1) * e.z < (uint64_t)kTransformBound &&
-                (uint64_t)(mag(v[0]) + 1) * e.y < (uint64_t)kTransformBound) {
+            // (half the bound: the outputs, below 35.3 * 2^24, are doubled where
+            // the plane is scaled)
+            if ((uint64_t)(lm + 1) * e.z < (uint64_t)kTransformBound / 2 &&
+                (uint64_t)(mag(v[0]) + 1) * e.y < (uint64_t)kTransformBound / 2) {
                 v[0] *= (int32_t)e.y;
 #pragma unroll
                 for (int k = 1; k < 16; k++) v[k] *= (int32_t)e.z;
                 inverse_pct<false>(v);
+                const int up = p.scale2 ? 1 : 0;
+#pragma unroll
+                for (int k = 0; k < 16; k++) v[k] <<= up;
             } else {
-                v[0] = dequant(v[0], e.y, b);
-#pragma unroll
-                for (int k = 1; k < 16; k++) v[k] = dequant(v[k], e.z, b);
-                b |= pct16(v);
-            }
-            if (p.scale2) {
-#pragma unroll
-                for (int k = 0; k < 16; k++) v[k] = dequant(v[k], 2, b);
+                b = checked_first_level(v, e.y, e.z, p.scale2);
             }
             int32_t *out = ydc + (m / 6) * 4 * kIDC + (m % 6) * 4;
 #pragma unroll
@@ -2689,7 +2688,8 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
                     const int2 d = *reinterpret_cast<const int2 *>(base + r * kIDC + 2);
                     v[r * 4] = a.x; v[r * 4 + 1] = a.y; v[r * 4 + 2] = d.x; v[r * 4 + 3] = d.y;
                 }
-                b = pot16(v);
+                if (mag_bound<0>(v) < (uint32_t)kOverlapBound) b = inverse_pot4x4<false>(v);
+                else b = checked_overlap(v);
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
                     *reinterpret_cast<int2 *>(base + r * kIDC) = make_int2(v[r * 4], v[r * 4 + 1]);
@@ -2815,9 +2815,7 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
             for (int k = 1; k < 16; k++) v[k] = v[k] * (int32_t)step;
             inverse_pct<false>(v);
         } else {
-#pragma unroll
-            for (int k = 1; k < 16; k++) v[k] = dequant(v[k], step, b);
-            b |= pct16(v);
+            b = checked_transform(v, 1, step);
         }
         if (b) bad |= kFlagSecond;
 #pragma unroll
