@@ -145,6 +145,7 @@ constexpr int kKinds = 6;
 constexpr uint32_t kTag420 = 5, kTag422 = 6;
 constexpr uint32_t kTagEdge = kKinds;
 constexpr uint32_t kTagHard = 2 * kKinds;
+constexpr int kTags = 3 * kKinds + 1;
 constexpr int kTagShift = 27;
 constexpr uint32_t kImageMask = (1u << kTagShift) - 1;
 constexpr int kSideSegment0 = kKinds;          // segments run beside the interior ones
@@ -152,8 +153,18 @@ constexpr int kSegments = 2 * kKinds + 1;
 constexpr int kSegmentOther = kSegments - 1;
 // Edge tiles that the interior kernel of the same images takes instead of an
 // edge kernel (one launch, edge tiles first in it), by kind; their edge
-// segment then holds their hard tiles alone.
-constexpr bool kFoldEdges[kKinds] = {false, false, true, false, false, false};
+// segment then holds their hard tiles alone.  The one-plane kernel stays small
+// enough with them (2047 x 1535 16-bit gray 13.5 us apart, 12.1 folded); in the
+// others their code costs every interior tile more fetches than the launch
+// saves (4096 x 4096 RGB8 129.7 us folded, 126.4 apart; 3999 x 2999 4:2:0 95.0
+// and 87.5).
+constexpr bool kFoldEdges[kKinds] = {true, false, false, false, false, false};
+// Up to this many tiles of a kind in a set, its interior tiles run in the edge
+// kernel with the others: one launch, no fork and join.  64 tiles (512 x 512)
+// of RGB8 4:4:4, 4:2:0, RGBA: 11.3, 11.4, 11.4 us in two kernels, 10.0, 10.3,
+// 10.3 in one; 256 tiles (1024 x 1024): 13.9, 14.4, 16.9 against 15.2, 16.4,
+// 16.5.
+constexpr uint32_t kMergeTiles = 128;
 constexpr int kCounterWords = 2 * kSegments;   // two scheduling words a segment
 
 // Side streams a set's kernels may run on beside its own: with the set's

@@ -152,19 +152,37 @@ uint32_t tile_tag(uint32_t kind, uint32_t tx, uint32_t ty, uint32_t T, uint32_t 
 bool folded_edge_tag(uint32_t tag) {
     return tag > kTagEdge && tag <= kTagHard && kFoldEdges[tag - kTagEdge - 1];
 }
-int segment_of_tag(uint32_t tag) {
+// `merged`: the kinds (bit kind - 1) whose interior tiles run in the edge
+// kernel (merged_kinds).
+int segment_of_tag(uint32_t tag, uint32_t merged) {
     if (tag == 0) return kSegmentOther;
     if (tag > kTagHard) return kSideSegment0 + (int)(tag - kTagHard) - 1;
-    return folded_edge_tag(tag) ? (int)(tag - kTagEdge) - 1 : (int)tag - 1;
+    if (tag > kTagEdge) return folded_edge_tag(tag) ? (int)(tag - kTagEdge) - 1 : (int)tag - 1;
+    return (merged >> (tag - 1)) & 1 ? kSideSegment0 + (int)tag - 1 : (int)tag - 1;
 }
+
+// The kinds whose interior and edge kernels would both run, over no more than
+// kMergeTiles tiles together.  `count`: tiles by tag.
+uint32_t merged_kinds(const uint32_t *count) {
+    uint32_t merged = 0;
+    for (uint32_t k = 1; k <= (uint32_t)kKinds; k++) {
+        const uint32_t edge = (folded_edge_tag(kTagEdge + k) ? 0 : count[kTagEdge + k]) + count[kTagHard + k];
+        if (count[k] > 0 && edge > 0 && count[k] + edge <= kMergeTiles) merged |= 1u << (k - 1);
+    }
+    return merged;
+}
+
 int rank_of_tag(uint32_t tag) { return folded_edge_tag(tag) ? 0 : 1; }
 
 // Stable order of a work list by segment (a counting sort: one pass to count,
 // one to place); `bounds` receives the kSegments + 1 segment boundaries.
 void order_by_segment(std::vector<WorkItemHost> &items, uint32_t *bounds) {
-    auto key = [](const WorkItemHost &w) {
+    uint32_t tags[kTags] = {};
+    for (const WorkItemHost &w : items) tags[w.image >> kTagShift]++;
+    const uint32_t merged = merged_kinds(tags);
+    auto key = [&](const WorkItemHost &w) {
         const uint32_t tag = w.image >> kTagShift;
-        return segment_of_tag(tag) * 2 + rank_of_tag(tag);
+        return segment_of_tag(tag, merged) * 2 + rank_of_tag(tag);
     };
     uint32_t cursor[2 * kSegments] = {};
     for (const WorkItemHost &w : items) cursor[key(w)]++;
@@ -1353,10 +1371,11 @@ jxrb_status stage_plan(const jxrb_plan *plan, const int32_t *coefficients, const
     const bool two_level = p0.overlap == 2;
     const uint8_t *sx = p0.hard ? p0.col_start.data() : nullptr, *sy = p0.hard ? p0.row_start.data() : nullptr;
     // count the tiles of each segment, then place each at its segment's cursor
-    uint32_t count[kSegments] = {};
+    uint32_t count[kSegments] = {}, tags[kTags] = {};
     for (uint32_t ty = 0; ty < tiles_y; ty++)
-        for (uint32_t tx = 0; tx < tiles_x; tx++)
-            count[segment_of_tag(tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level))]++;
+        for (uint32_t tx = 0; tx < tiles_x; tx++) tags[tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level)]++;
+    const uint32_t merged = merged_kinds(tags);
+    for (uint32_t tag = 0; tag < (uint32_t)kTags; tag++) count[segment_of_tag(tag, merged)] += tags[tag];
     uint32_t cursor[kSegments];
     layout.bounds[0] = 0;
     for (int s = 0; s < kSegments; s++) {
@@ -1368,7 +1387,7 @@ jxrb_status stage_plan(const jxrb_plan *plan, const int32_t *coefficients, const
     for (uint32_t ty = 0; ty < tiles_y; ty++)
         for (uint32_t tx = 0; tx < tiles_x; tx++) {
             const uint32_t tag = tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level);
-            list[cursor[segment_of_tag(tag)]++] = WorkItemHost{tag << kTagShift, (uint16_t)tx, (uint16_t)ty};
+            list[cursor[segment_of_tag(tag, merged)]++] = WorkItemHost{tag << kTagShift, (uint16_t)tx, (uint16_t)ty};
         }
     return JXRB_OK;
 }
