@@ -1329,6 +1329,17 @@ __device__ __forceinline__ bool cell_samples_fast(const int32_t *t, const CellBl
     return true;
 }
 
+__device__ __forceinline__ void cell_store(int32_t *t, const CellBlocks &b, const int32_t (&w)[16]) {
+    *reinterpret_cast<int2 *>(t + b.b00 + 10) = make_int2(w[0], w[1]);
+    *reinterpret_cast<int2 *>(t + b.b01 + 8) = make_int2(w[2], w[3]);
+    *reinterpret_cast<int2 *>(t + b.b00 + 14) = make_int2(w[4], w[5]);
+    *reinterpret_cast<int2 *>(t + b.b01 + 12) = make_int2(w[6], w[7]);
+    *reinterpret_cast<int2 *>(t + b.b10 + 2) = make_int2(w[8], w[9]);
+    *reinterpret_cast<int2 *>(t + b.b11) = make_int2(w[10], w[11]);
+    *reinterpret_cast<int2 *>(t + b.b10 + 6) = make_int2(w[12], w[13]);
+    *reinterpret_cast<int2 *>(t + b.b11 + 4) = make_int2(w[14], w[15]);
+}
+
 // Any cell; returns the overflow flag.
 __device__ __forceinline__ bool cell_samples(const int32_t *t, const CellBlocks &b, int overlap, int32_t (&w)[16],
                                              bool small = false) {
@@ -1772,6 +1783,149 @@ __device__ __forceinline__ bool lean_rgb(const OutputDev &o, int colours, uint32
     return lean && seen == 7u;
 }
 
+// Stages D and E of one cell (gcx, gcy) of the grid: the second-level overlap
+// plane after plane, in place (unless a hard boundary cut the cell: `cut`),
+// with one copy of the operator, then the 16 pixels row by row, through every
+// output the image may have.  The edge and four-plane kernels take all their
+// cells this way: a third of the code of the form that holds every plane's cell
+// in registers, and no values kept across it (2500 x 1900 hard tiles 58.4 ->
+// 55.3 us, mixed batch 137.3 -> 135.5).  The interior kernels of up to three
+// planes keep that form for the usual outputs (4096 x 4096 RGB8 127.3 us, 133.5
+// this way: eight more loads and stores a plane) and come here with the rest.
+// Returns the tile flags.
+template <int NP>
+__device__ __forceinline__ int cell_rows(const ImageDev &im, int32_t *tiles, int mx0, int my0, int gcx, int gcy, bool cut,
+                                         bool tile_small) {
+    const CellBlocks cell = cell_blocks(gcx, gcy);
+    int bad = 0;
+#pragma unroll 1
+    for (int pi = 0; pi < NP; pi++) {
+        if (cut || im.plane[pi].overlap < 1) continue;
+        int32_t w[16];
+        if (cell_samples(tiles + pi * kTileInts, cell, 1, w, tile_small)) bad |= kFlagOverlap;
+        cell_store(tiles + pi * kTileInts, cell, w);
+    }
+    const OutputDev &o = im.out;
+    const int x0 = 16 * mx0 + 2 + 4 * gcx, y0 = 16 * my0 + 2 + 4 * gcy;
+    const bool inside = x0 >= (int)o.crop_x && x0 + 4 <= (int)(o.crop_x + o.crop_w) && y0 >= (int)o.crop_y &&
+                        y0 + 4 <= (int)(o.crop_y + o.crop_h);
+    const int kind = o.kind;
+    const bool has_alpha = im.alpha >= 0;
+    bool obad = false;
+    uint32_t rgb_at = 0;
+    // the specialised outputs this image's cells may take
+    const bool rgb8 = NP >= 3 && inside && kind == kOutRgb8 && !o.premultiply;
+    const bool direct = NP == 1 && inside && kind == kOutDirect && lean_channel(o.ch[0]);
+    const bool f16 = NP >= 3 && inside && kind == kOutF16Wide && o.nchw && o.channels <= NP &&
+                     lean_rgb(o, has_alpha ? o.channels - 1 : o.channels, rgb_at) &&
+                     (!has_alpha || (o.ch[o.channels - 1].post_shift < 0 && lean_channel(o.ch[o.channels - 1])));
+    const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
+    const uint64_t chs = o.nchw ? o.plane_stride : (uint64_t)o.elem_bytes;
+    uint8_t *dst = o.base + (int64_t)(y0 - (int)o.crop_y) * (int64_t)o.row_stride + (int64_t)(x0 - (int)o.crop_x) * (int64_t)pixel_bytes;
+#pragma unroll 1
+    for (int r = 0; r < 4; r++, dst += o.row_stride) {
+        int32_t w[NP][4];
+        const int left = (r < 2 ? cell.b00 + 8 : cell.b10 - 8) + 4 * r + 2, right = (r < 2 ? cell.b01 + 8 : cell.b11 - 8) + 4 * r;
+#pragma unroll
+        for (int pi = 0; pi < NP; pi++) {
+            const int2 l = *reinterpret_cast<const int2 *>(tiles + pi * kTileInts + left);
+            const int2 q = *reinterpret_cast<const int2 *>(tiles + pi * kTileInts + right);
+            w[pi][0] = l.x; w[pi][1] = l.y; w[pi][2] = q.x; w[pi][3] = q.y;
+        }
+        uint32_t m = 0;
+        if (!tile_small) {
+#pragma unroll
+            for (int pi = 0; pi < NP; pi++)
+#pragma unroll
+                for (int c = 0; c < 4; c++) m |= mag(w[pi][c]);
+        }
+        if (rgb8 && m < (1u << 28)) {
+            const ChannelScale &sc = o.ch[0];
+            const int32_t add = sc.shifted_bias + sc.rounding;
+            const int shift = sc.shift;
+            // byte order of the packed pixel: R G B, or B G R
+            const uint32_t order = sc.source == 2 ? 0x7014u : 0x7410u;
+            uint32_t px[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                // each colour is luma plus terms in u and v, so adding the
+                // output bias to luma adds it to all three (no
+                // intermediate nears int32 below 2^28)
+                int32_t R, G, B;
+                yuv_to_rgb_fast(w[0][c] + add, w[NP > 1 ? 1 : 0][c], w[NP > 2 ? 2 : 0][c], R, G, B);
+                px[c] = pack_rgb8(clamp_u8(R >> shift), clamp_u8(G >> shift), clamp_u8(B >> shift), order);
+                if (NP == 4 && has_alpha) {
+                    const ChannelScale &sa = o.ch[3];
+                    px[c] |= clamp_u8((w[NP - 1][c] + sa.shifted_bias + sa.rounding) >> sa.shift) << 24;
+                }
+            }
+            if (o.channels == 4) store16(dst, px[0], px[1], px[2], px[3]);
+            else store12(dst, px);
+        } else if (direct && m < lean_limit(o.ch[0]) && (o.ch[0].post_shift <= 0 || !tile_small)) {
+            const ChannelScale &s = o.ch[0];
+            const int eb = o.elem_bytes, up = max(s.post_shift, 0);
+            uint32_t q[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                q[c] = (uint32_t)min(max(((w[0][c] + s.shifted_bias + s.rounding) >> s.shift) << up, s.lo), s.hi);
+            if (eb == 2) store8(dst, (q[0] & 0xffffu) | (q[1] << 16), (q[2] & 0xffffu) | (q[3] << 16));
+            else if (eb == 4) store16(dst, q[0], q[1], q[2], q[3]);
+            else {
+                const uint32_t b[1] = {(q[0] & 0xffu) | ((q[1] & 0xffu) << 8) | ((q[2] & 0xffu) << 16) | (q[3] << 24)};
+                store_words(dst, b);
+            }
+        } else if (f16 && m < (1u << 28)) {
+            // R, G and B to their channel planes, alpha to the last.  YUV
+            // below 2^28 keeps the inverse RCT below 2^30 and, with terms
+            // below 2^28, every scaling step below 2^31: no checked step
+            // can overflow, so the unchecked ones give the same values.
+            int32_t rgb[3][4];
+#pragma unroll
+            for (int c = 0; c < 4; c++)
+                yuv_to_rgb_fast(w[0][c], w[NP > 1 ? 1 : 0][c], w[NP > 2 ? 2 : 0][c], rgb[0][c], rgb[1][c], rgb[2][c]);
+#pragma unroll
+            for (int c = 0; c < 3; c++) {
+                const int ch = (rgb_at >> (2 * c)) & 3;
+                const ChannelScale &s = o.ch[ch];
+                const int32_t add = s.shifted_bias + s.rounding;
+                store16(dst + ch * chs, f16_widened((rgb[c][0] + add) >> s.shift), f16_widened((rgb[c][1] + add) >> s.shift),
+                        f16_widened((rgb[c][2] + add) >> s.shift), f16_widened((rgb[c][3] + add) >> s.shift));
+            }
+            if (has_alpha && NP == 4) {
+                const ChannelScale &s = o.ch[o.channels - 1];
+                const int32_t add = s.shifted_bias + s.rounding;
+                store16(dst + (o.channels - 1) * chs, f16_widened((w[NP - 1][0] + add) >> s.shift),
+                        f16_widened((w[NP - 1][1] + add) >> s.shift), f16_widened((w[NP - 1][2] + add) >> s.shift),
+                        f16_widened((w[NP - 1][3] + add) >> s.shift));
+            }
+        } else {
+            // any other output, or pixels at the crop edge: the general
+            // store, pixel by pixel
+            const int yy = y0 + r;
+            if (yy < (int)o.crop_y || yy >= (int)(o.crop_y + o.crop_h)) continue;
+#pragma unroll 1
+            for (int c = 0; c < 4; c++) {
+                const int x = x0 + c;
+                if (x < (int)o.crop_x || x >= (int)(o.crop_x + o.crop_w)) continue;
+                const int at = (c < 2 ? left + c : right + c - 2);
+                int32_t comp[4] = {0, 0, 0, 0};
+#pragma unroll
+                for (int pi = 0; pi < NP; pi++)
+                    if (pi < im.nplanes && pi < 4) comp[pi] = tiles[pi * kTileInts + at];
+                const int32_t a = has_alpha ? tiles[(NP - 1) * kTileInts + at] : 0;
+                format_pixel(o, comp, a, dst + (int64_t)c * (int64_t)pixel_bytes, chs, obad);
+            }
+        }
+    }
+    if (obad) bad |= kFlagOutput;
+    return bad;
+}
+template <int NP>
+__device__ __noinline__ int cell_rows_call(const ImageDev &im, int32_t *tiles, int mx0, int my0, int gcx, int gcy,
+                                           bool cut, bool tile_small) {
+    return cell_rows<NP>(im, tiles, mx0, my0, gcx, gcy, cut, tile_small);
+}
+
 // One interior tile.  Its macroblock entries are already in `mbc` (copied
 // while the previous tile ran); while it runs, the entries of the next work
 // item go into `mbc_next`.  `claimed` is thread 0's claim of that next item.
@@ -1990,9 +2144,11 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         // cells that a hard boundary cuts have their operators behind them
         cut = hard && (hard_cell(hard & 0x1fu, gcx) || hard_cell((hard >> 8) & 0x1fu, gcy));
     }
-    auto overlap_of = [&](int pi) { return MODE == 1 && cut ? 0 : im.plane[pi].overlap; };
-    // stage D + E: the thread's sample cell, every plane, then its 16 pixels
-    if (grid_cell) {
+    // stages D and E: the thread's sample cell, every plane, then its 16 pixels
+    constexpr bool kRows = MODE == 1 || NP == 4;
+    if (grid_cell && kRows) {
+        bad |= cell_rows<NP>(im, tiles, mx0, my0, gcx, gcy, cut, tile_small);
+    } else if (grid_cell) {
         const int cx = gcx, cy = gcy;
         const CellBlocks cell = cell_blocks(cx, cy);
         const OutputDev &o = im.out;
@@ -2001,13 +2157,13 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                             y0 + 4 <= (int)(o.crop_y + o.crop_h);
         const int kind = o.kind;
         const bool has_alpha = im.alpha >= 0;
-        bool obad = false, done = false;
+        bool done = false;
         uint32_t rgb_at = 0;
         if (inside && kind == kOutRgb8 && NP >= 3 && !o.premultiply) {
             int32_t y[16], u[16], v[16];
-            bool fast = cell_samples_fast(tiles, cell, overlap_of(0), y, tile_small);
-            fast &= cell_samples_fast(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
-            fast &= cell_samples_fast(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
+            bool fast = cell_samples_fast(tiles, cell, im.plane[0].overlap, y, tile_small);
+            fast &= cell_samples_fast(tiles + kTileInts, cell, im.plane[1].overlap, u, tile_small);
+            fast &= cell_samples_fast(tiles + 2 * kTileInts, cell, im.plane[2].overlap, v, tile_small);
             if (!tile_small) fast &= max(max(mag_bound<0>(y), mag_bound<0>(u)), mag_bound<0>(v)) < (1u << 28);
             if (fast) {
                 const ChannelScale &sc = o.ch[0];
@@ -2028,7 +2184,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 bool alpha_ok = true;
                 if (NP == 4 && has_alpha) {
                     int32_t a[16];
-                    alpha_ok = cell_samples_fast(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small);
+                    alpha_ok = cell_samples_fast(tiles + 3 * kTileInts, cell, im.plane[3].overlap, a, tile_small);
                     if (!tile_small) alpha_ok &= mag_bound<0>(a) < (1u << 28);
                     const ChannelScale &sa = o.ch[3];
                     const int32_t aadd = sa.shifted_bias + sa.rounding;
@@ -2050,7 +2206,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             // samples and terms below the lean limit: no scaling step can
             // overflow, so the unchecked ones give the same values
             int32_t y[16];
-            const bool fast = cell_samples_fast(tiles, cell, overlap_of(0), y, tile_small);
+            const bool fast = cell_samples_fast(tiles, cell, im.plane[0].overlap, y, tile_small);
             if (fast && ((tile_small && o.ch[0].post_shift <= 0) || mag_bound<0>(y) < lean_limit(o.ch[0]))) {
                 const ChannelScale &s = o.ch[0];
                 const int eb = o.elem_bytes;
@@ -2087,7 +2243,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             bool lean = true;
             if (has_alpha && NP == 4) {
                 int32_t a[16];
-                lean = cell_samples_fast(tiles + 3 * kTileInts, cell, overlap_of(3), a, tile_small) &&
+                lean = cell_samples_fast(tiles + 3 * kTileInts, cell, im.plane[3].overlap, a, tile_small) &&
                        (tile_small || mag_bound<0>(a) < (1u << 28));
                 if (lean) {
                     const ChannelScale &s = o.ch[o.channels - 1];
@@ -2101,9 +2257,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             }
             if (lean) {
                 int32_t y[16], u[16], v[16];
-                bool fast = cell_samples_fast(tiles, cell, overlap_of(0), y, tile_small);
-                fast &= cell_samples_fast(tiles + kTileInts, cell, overlap_of(1), u, tile_small);
-                fast &= cell_samples_fast(tiles + 2 * kTileInts, cell, overlap_of(2), v, tile_small);
+                bool fast = cell_samples_fast(tiles, cell, im.plane[0].overlap, y, tile_small);
+                fast &= cell_samples_fast(tiles + kTileInts, cell, im.plane[1].overlap, u, tile_small);
+                fast &= cell_samples_fast(tiles + 2 * kTileInts, cell, im.plane[2].overlap, v, tile_small);
                 if (fast && (tile_small || max(max(mag_bound<0>(y), mag_bound<0>(u)), mag_bound<0>(v)) < (1u << 28))) {
                     int32_t cadd[3], cshift[3];
                     uint8_t *plane[3];
@@ -2133,33 +2289,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 }
             }
         }
-        if (!done) {
-            // any other output, or pixels at the crop edge: the general store,
-            // pixel by pixel, from every plane's cell samples
-            int32_t w[NP][16];
-#pragma unroll 1
-            for (int pi = 0; pi < NP; pi++)
-                if (cell_samples(tiles + pi * kTileInts, cell, overlap_of(pi), w[pi], tile_small))
-                    bad |= kFlagOverlap;
-            const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
-            const uint64_t chs = o.nchw ? o.plane_stride : (uint64_t)o.elem_bytes;
-            for (int r = 0; r < 4; r++)
-                for (int c = 0; c < 4; c++) {
-                    const int x = x0 + c, yy = y0 + r;
-                    if (x < (int)o.crop_x || x >= (int)(o.crop_x + o.crop_w) || yy < (int)o.crop_y ||
-                        yy >= (int)(o.crop_y + o.crop_h))
-                        continue;
-                    const int k = r * 4 + c;
-                    int32_t comp[4] = {0, 0, 0, 0};
-#pragma unroll
-                    for (int pi = 0; pi < NP; pi++)
-                        if (pi < im.nplanes && pi < 4) comp[pi] = w[pi][k];
-                    const int32_t a = has_alpha ? w[NP - 1][k] : 0;
-                    uint8_t *dst = o.base + (uint64_t)(yy - o.crop_y) * o.row_stride + (uint64_t)(x - o.crop_x) * pixel_bytes;
-                    format_pixel(o, comp, a, dst, chs, obad);
-                }
-        }
-        if (obad) bad |= kFlagOutput;
+        // any other output, cells that need the checked operator, or pixels at
+        // the crop edge
+        if (!done) bad |= cell_rows_call<NP>(im, tiles, mx0, my0, gcx, gcy, false, tile_small);
     }
     if (edge && edge_pixels<NP>(im, tiles, mx0, my0, ec)) bad |= kFlagOutput;
     if (bad) atomicOr(&sh.bad, bad);
