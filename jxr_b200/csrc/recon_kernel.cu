@@ -1394,26 +1394,33 @@ __device__ __forceinline__ void note_plain(const ImageDev &im, const uint4 *mbc,
 // low-pass values -- coefficient 0 of each block -- among them; and the halo:
 // the first block column of the macroblocks right of the tile, the first block
 // row of those below it, the corner block.  `plain`: every entry is.
+__device__ __forceinline__ bool far_mb(int m) { return m < 6 || m % 6 == 0; }
 struct PlaneCopy {
     // what a thread copies is the same in every plane
     int ring0, ring1;     // ring macroblock values tid and 256 + tid: entry index | slot << 8
+    bool far0, far1;      // theirs a macroblock that only the first-level overlap reads
     int halo_entry, halo_from, halo_to;
     __device__ __forceinline__ PlaneCopy() {
         const int tid = threadIdx.x, kk = tid & 15, r = tid >> 4;
         ring0 = ring_mb(r) | (r * kRingPitch + kk) << 8;
         ring1 = tid < 64 ? ring_mb(16 + r) | ((16 + r) * kRingPitch + kk) << 8 : 0;
+        far0 = far_mb(ring0 & 255);
+        far1 = tid >= 64 || far_mb(ring1 & 255);
         const int hb = tid >> 2, piece = (tid & 3) << 2;
         const int i = hb >= 16 && hb < 32 ? hb - 16 : 16, j = hb < 16 ? hb : 16;
         halo_entry = ((j >> 2) + 1) * 6 + (i >> 2) + 1;
         halo_from = (((j & 3) << 2) + (i & 3)) * 16 + piece;
         halo_to = block_at(i, j) + piece;
     }
+    // `two_level`: the plane has a first-level overlap, which alone reads the
+    // macroblocks left of and above the tile.
     __device__ __forceinline__ void run(const int32_t *coeff, const uint4 *ent, int32_t *tile, int32_t *ring,
-                                        bool plain) const {
+                                        bool plain, bool two_level) const {
         const int tid = threadIdx.x, kk = tid & 15, c = (tid & 63) * 4;
+        const bool want0 = two_level || !far0, want1 = tid < 64 && (two_level || !far1);
         if (plain) {
-            cp_async4(ring + (ring0 >> 8), coeff + (ent[ring0 & 255].x & 0x0fffffffu) + kk * 16);
-            if (tid < 64) cp_async4(ring + (ring1 >> 8), coeff + (ent[ring1 & 255].x & 0x0fffffffu) + kk * 16);
+            if (want0) cp_async4(ring + (ring0 >> 8), coeff + (ent[ring0 & 255].x & 0x0fffffffu) + kk * 16);
+            if (want1) cp_async4(ring + (ring1 >> 8), coeff + (ent[ring1 & 255].x & 0x0fffffffu) + kk * 16);
 #pragma unroll
             for (int b = 0; b < 4; b++)
                 cp_async16(tile + (4 * b + (tid >> 6)) * kMbPitch + c,
@@ -1422,7 +1429,7 @@ struct PlaneCopy {
             return;
         }
         for (int k = 0; k < 2; k++) {
-            if (k == 1 && tid >= 64) break;
+            if (!(k == 0 ? want0 : want1)) continue;
             const int at = k == 0 ? ring0 : ring1;
             const uint4 e = ent[at & 255];
             const int bands = (e.x >> 28) & 3;
@@ -1961,6 +1968,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         if (tid == 0) sh.hard = starts;
     }
     int bad = 0;
+    // four-plane images have two overlap levels as a rule: their kernel does
+    // without the test (1 % of its time)
+    constexpr bool kAllRing = NP == 4;
     // phase 1: every coefficient the tile reads (PlaneCopy)
     {
         const PlaneCopy copy;
@@ -1971,7 +1981,8 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         constexpr int kCopyUnroll = NP == 4 ? 1 : NP;
 #pragma unroll kCopyUnroll
         for (int pi = 0; pi < NP; pi++)
-            copy.run(im.plane[pi].coeff, mbc + pi * 36, tiles + pi * kTileInts, rings + pi * kRingInts, plain);
+            copy.run(im.plane[pi].coeff, mbc + pi * 36, tiles + pi * kTileInts, rings + pi * kRingInts, plain,
+                     kAllRing || im.plane[pi].overlap == 2);
     }
     cp_async_commit();
     cp_async_wait_all();
@@ -1984,6 +1995,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         else { pi = (item - NP * 16) / 20; k = 16 + (item - NP * 16) - pi * 20; }
         const int m = first_level_mb(k);
         const PlaneDev &p = im.plane[pi];
+        if (!kAllRing && p.overlap != 2 && far_mb(m)) continue;   // not copied, not read
         const uint4 e = mbc[pi * 36 + m];
         int32_t v[16];
         bool b = false;
@@ -2514,6 +2526,13 @@ jxrb_reconstruct_tiles(const ImageDev *__restrict__ images, const WorkItem *__re
 // ---------------------------------------------------------------------------
 constexpr int kCB = 11;                          // chroma blocks across
 constexpr int kCDC = 12;                         // chroma DC tile columns
+// Chroma blocks are 80 bytes apart: eight consecutive ones' row pieces meet
+// eight distinct 16-byte bank groups.
+constexpr int kCPitch = 20;
+__device__ __forceinline__ int chroma_block(int i, int j) { return (j * kCB + i) * kCPitch; }
+__device__ __forceinline__ int chroma_sample(int x, int y) {
+    return chroma_block(x >> 2, y >> 2) + ((y & 3) << 2) + (x & 3);
+}
 
 // The chroma tile by block rows a macroblock (CV: 2 for 4:2:0, 4 for 4:2:2).
 template <int CV>
@@ -2521,12 +2540,17 @@ struct ChromaTile {
     static constexpr int kFirstMb = CV == 2 ? -1 : 0;        // first macroblock row held, from my0
     static constexpr int kMbRows = CV == 2 ? 6 : 5;          // the last one's first block row alone
     static constexpr int kRows = CV * (kMbRows - 1) + 1;     // blocks down: 11 or 17
-    static constexpr int kInts = kCB * kRows * 16;
+    static constexpr int kBlocks = kCB * kRows;
+    static constexpr int kInts = kBlocks * kCPitch;
     static constexpr int kDcRows = 6 * CV;                   // macroblocks my0-1 .. my0+4
     static constexpr int kDcInts = kCDC * kDcRows;
     static constexpr int kDcRow0 = CV == 2 ? 0 : CV;         // DC row of block row 0
     static constexpr int kLow = 2 * CV;                      // DC / low-pass values a macroblock
-    static constexpr int kLpInts = 36 * kLow;
+    // macroblocks of the 6 x 6 whose blocks the tile does not hold whole, their
+    // DC / low-pass values gathered: the right column and the bottom row, and
+    // 4:2:2's top row
+    static constexpr int kGather = CV == 2 ? 11 : 16;
+    static constexpr int kLpInts = kGather * kLow;
     static constexpr int kRow0 = CV == 2 ? 1 : 0;            // block rows reconstructed
     static constexpr int kTransRows = CV == 2 ? 10 : 17;
     static constexpr int kSquares = CV == 2 ? 5 : 9;         // first-level squares down
@@ -2534,38 +2558,19 @@ struct ChromaTile {
     static constexpr int kCells = CV == 2 ? 9 : 17;          // cells down; 4:2:2's first is the plane's top edge only
     static constexpr int kSmemInts =
         kTileInts + jxr::kDcInts + kRingInts + 2 * (kInts + kDcInts + kLpInts) + 2 * 3 * kMbcInts;
+    __device__ static int gather_mb(int g) {   // its index in the 6 x 6 grid
+        if (CV == 2) return g < 6 ? g * 6 + 5 : 30 + g - 6;
+        return g < 6 ? g : g < 12 ? 30 + g - 6 : (g - 11) * 6 + 5;
+    }
+    __device__ static bool held(int a, int b) { return a < 5 && b < 5 && (CV == 2 || b > 0); }
+    __device__ static int gather_slot(int a, int b) {
+        if (CV == 2) return a == 5 ? b : 6 + a;
+        return b == 0 ? a : b == 5 ? 6 + a : 11 + b;
+    }
     // plane row of the tile's first sample, and of cell row 0
     __device__ static int sample0(int my0) { return CV == 2 ? 8 * my0 - 8 : 16 * my0; }
     __device__ static int cell0(int my0) { return 4 * CV * my0 - 2; }
 };
-
-// The 16 samples of the 4 x 4 cell whose upper-left quarter is the lower-right
-// quarter of block b00 of a tile `stride` blocks wide; second-level overlap
-// applied when the plane has it, and written back when `store` is set.
-__device__ __forceinline__ bool cell_rw(int32_t *t, int b00, int stride, int overlap, int32_t (&w)[16], bool store,
-                                        bool small = false) {
-    const int b01 = b00 + 1, b10 = b00 + stride, b11 = b10 + 1;
-    int2 *q[8] = {reinterpret_cast<int2 *>(&t[elem(b00, 2, 2)]), reinterpret_cast<int2 *>(&t[elem(b01, 2, 0)]),
-                  reinterpret_cast<int2 *>(&t[elem(b00, 3, 2)]), reinterpret_cast<int2 *>(&t[elem(b01, 3, 0)]),
-                  reinterpret_cast<int2 *>(&t[elem(b10, 0, 2)]), reinterpret_cast<int2 *>(&t[elem(b11, 0, 0)]),
-                  reinterpret_cast<int2 *>(&t[elem(b10, 1, 2)]), reinterpret_cast<int2 *>(&t[elem(b11, 1, 0)])};
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const int2 a = *q[k];
-        w[2 * k] = a.x;
-        w[2 * k + 1] = a.y;
-    }
-    bool bad = false;
-    if (overlap >= 1) {
-        if (small || mag_bound<0>(w) < (uint32_t)kOverlapBound) inverse_pot4x4<false>(w);
-        else bad = checked_overlap(w);
-    }
-    if (store) {
-#pragma unroll
-        for (int k = 0; k < 8; k++) *q[k] = make_int2(w[2 * k], w[2 * k + 1]);
-    }
-    return bad;
-}
 
 // A first-level chroma square of a subsampled edge tile whose centre lies on the
 // plane's edge (subsampled_overlap.rs:244-296): the two-sample operator on
@@ -2602,7 +2607,7 @@ __device__ bool chroma_edge_square(int32_t *cd, int wx, int wy, bool vs, bool hs
 __device__ bool chroma_cut_cell(int32_t *t, int X, int Y, int ox, int oy, int Wc, int Hc, bool vs, bool hs) {
     auto at = [&](int x, int y) -> int32_t & {
         const int sx = x - ox, sy = y - oy;
-        return t[elem((sy >> 2) * kCB + (sx >> 2), sy & 3, sx & 3)];
+        return t[chroma_sample(sx, sy)];
     };
     const int c0 = max(X, 0), c1 = min(X + 4, Wc), r0 = max(Y, 0), r1 = min(Y + 4, Hc);
     bool bad = false;
@@ -2617,17 +2622,44 @@ __device__ bool chroma_cut_cell(int32_t *t, int X, int Y, int ox, int oy, int Wc
     return bad;
 }
 
-// Stage E at the plane's edge of a 4:2:0 or 4:2:2 tile: the pixels of the cut luma
-// cells, one a thread; chroma interpolated with its reads clamped to the
-// plane, as the general path does.  Returns the output flag.
+// Pixel (x, y) of a 4:2:0 or 4:2:2 tile through the general store, or a
+// specialised one that takes it: chroma interpolated in the checked split form
+// with its reads clamped to the plane, as the general path does.  Returns the
+// output flag.
 template <int CV>
-__device__ bool edge_pixels_chroma(const ImageDev &im, const int32_t *ytile, const int32_t *ctile, int mx0, int my0,
-                                const EdgeCells &ec) {
+__device__ __noinline__ bool chroma_pixel(const ImageDev &im, const int32_t *ytile, const int32_t *ctile, int mx0,
+                                          int my0, int x, int y) {
+    using CT = ChromaTile<CV>;
     const OutputDev &o = im.out;
     const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
     const uint64_t chs = o.nchw ? o.plane_stride : (uint64_t)o.elem_bytes;
-    using CT = ChromaTile<CV>;
-    const int Wc = ec.W >> 1, Hc = CV == 2 ? ec.H >> 1 : ec.H, ox = 8 * mx0 - 8, oy = CT::sample0(my0);
+    const int Wc = 8 * (int)im.plane[0].mbs_x, Hc = 4 * CV * (int)im.plane[0].mbs_y, ox = 8 * mx0 - 8, oy = CT::sample0(my0);
+    int32_t comp[4] = {ytile[sample_at(x - 16 * mx0, y - 16 * my0)], 0, 0, 0};
+    const int cx = x >> 1, cy = CV == 2 ? y >> 1 : y;
+#pragma unroll
+    for (int pc = 0; pc < 2; pc++) {
+        const int32_t *t = ctile + pc * CT::kInts;
+        auto C = [&](int a, int b) { return t[chroma_sample(min(max(a, 0), Wc - 1) - ox, min(max(b, 0), Hc - 1) - oy)]; };
+        int32_t col[3];
+#pragma unroll
+        for (int d = -1; d <= 1; d++)
+            col[d + 1] = CV == 4 ? C(cx + d, cy)
+                       : (y & 1) ? up_odd(C(cx + d, cy), C(cx + d, cy + 1), im.centering_y)
+                                 : up_even(C(cx + d, cy - 1), C(cx + d, cy), im.centering_y);
+        comp[1 + pc] = (x & 1) ? up_odd(col[1], col[2], im.centering_x) : up_even(col[0], col[1], im.centering_x);
+    }
+    bool bad = false;
+    uint8_t *dst = o.base + (uint64_t)(y - o.crop_y) * o.row_stride + (uint64_t)(x - o.crop_x) * pixel_bytes;
+    if (!fast_pixel<3>(im, comp, 0, dst, bad)) format_pixel(o, comp, 0, dst, chs, bad);
+    return bad;
+}
+
+// Stage E at the plane's edge of a 4:2:0 or 4:2:2 tile: the pixels of the cut
+// luma cells, one a thread.  Returns the output flag.
+template <int CV>
+__device__ bool edge_pixels_chroma(const ImageDev &im, const int32_t *ytile, const int32_t *ctile, int mx0, int my0,
+                                   const EdgeCells &ec) {
+    const OutputDev &o = im.out;
     const int cells = ec.n[0] + ec.n[1] + ec.n[2] + ec.n[3];
     bool bad = false;
     for (int item = threadIdx.x; item < cells * 8; item += kThreads) {
@@ -2639,26 +2671,7 @@ __device__ bool edge_pixels_chroma(const ImageDev &im, const int32_t *ytile, con
         if (x < (int)o.crop_x || x >= (int)(o.crop_x + o.crop_w) || y < (int)o.crop_y ||
             y >= (int)(o.crop_y + o.crop_h))
             continue;
-        const int sx = x - 16 * mx0, sy = y - 16 * my0;
-        int32_t comp[4] = {ytile[sample_at(sx, sy)], 0, 0, 0};
-        const int cx = x >> 1, cy = CV == 2 ? y >> 1 : y;
-#pragma unroll
-        for (int pc = 0; pc < 2; pc++) {
-            const int32_t *t = ctile + pc * CT::kInts;
-            auto C = [&](int a, int b) {
-                const int ta = min(max(a, 0), Wc - 1) - ox, tb = min(max(b, 0), Hc - 1) - oy;
-                return t[elem((tb >> 2) * kCB + (ta >> 2), tb & 3, ta & 3)];
-            };
-            int32_t col[3];
-#pragma unroll
-            for (int d = -1; d <= 1; d++)
-                col[d + 1] = CV == 4 ? C(cx + d, cy)
-                           : (y & 1) ? up_odd(C(cx + d, cy), C(cx + d, cy + 1), im.centering_y)
-                                     : up_even(C(cx + d, cy - 1), C(cx + d, cy), im.centering_y);
-            comp[1 + pc] = (x & 1) ? up_odd(col[1], col[2], im.centering_x) : up_even(col[0], col[1], im.centering_x);
-        }
-        uint8_t *dst = o.base + (uint64_t)(y - o.crop_y) * o.row_stride + (uint64_t)(x - o.crop_x) * pixel_bytes;
-        if (!fast_pixel<3>(im, comp, 0, dst, bad)) format_pixel(o, comp, 0, dst, chs, bad);
+        bad |= chroma_pixel<CV>(im, ytile, ctile, mx0, my0, x, y);
     }
     return bad;
 }
@@ -2687,31 +2700,43 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
     int32_t *yring = ydc + kDcInts;                     // 20 macroblocks' DC / low-pass values
     int32_t *ctile = yring + kRingInts;                 // chroma: 2 x 11 x 11 or 17 blocks
     int32_t *cdc = ctile + 2 * CT::kInts;               // 2 x 12 x 12 or 24
-    int32_t *clp = cdc + 2 * CT::kDcInts;               // 2 x 36 x 4 or 8
+    int32_t *clp = cdc + 2 * CT::kDcInts;               // gathered DC / low-pass values
     if (tid == 0) sh.bad = 0;
     if (MODE == 1 && tid < 32) {
         const uint32_t starts = hard_starts(im, mx0, my0);
         if (tid == 0) sh.hard = starts;
     }
     int bad = 0;
-    // phase 1: luma as in the full-resolution tile; the DC / low-pass values
-    // (4 or 8 a macroblock) of the 6 x 6 chroma macroblocks, and their blocks
-    PlaneCopy().run(im.plane[0].coeff, mbc, ytile, yring, sh.plain != 0);
-    for (int k = tid; k < 2 * CT::kLpInts; k += kThreads) {
-        const int pi = 1 + k / CT::kLpInts, r = k - (pi - 1) * CT::kLpInts, m = r / CT::kLow, kk = r % CT::kLow;
-        const uint4 e = mbc[pi * 36 + m];
-        const int bands = (e.x >> 28) & 3;
-        if (kk == 0 || bands != 0)
-            cp_async4(clp + k, im.plane[pi].coeff + (e.x & 0x0fffffffu) + (bands >= 2 ? kk * 16 : kk));
-        else
-            clp[k] = 0;
-    }
-    for (int k = tid; k < 2 * CT::kInts / 4; k += kThreads) {
-        const int pc = k / (CT::kInts / 4), q = k - pc * (CT::kInts / 4), sidx = q >> 2, r = q & 3;
-        const int i = sidx % kCB, j = sidx / kCB;
-        copy_chunk(ctile + pc * CT::kInts + sidx * 16 + ((r ^ swz(sidx)) << 2), im.plane[1 + pc].coeff,
-                   mbc[(1 + pc) * 36 + (j / CV + 1 + CT::kFirstMb) * 6 + (i >> 1)],
-                   (((j % CV) << 1) + (i & 1)) * 16 + r * 4);
+    // phase 1: luma as in the full-resolution tile; the chroma planes' blocks,
+    // and the DC / low-pass values of the macroblocks they do not hold whole
+    const bool plain = sh.plain != 0;
+    PlaneCopy().run(im.plane[0].coeff, mbc, ytile, yring, plain, im.plane[0].overlap == 2);
+    {
+        const int32_t *coeff[2] = {im.plane[1].coeff, im.plane[2].coeff};
+        if (tid < CT::kLpInts) {
+            const int m = CT::gather_mb(tid / CT::kLow), kk = tid % CT::kLow;
+#pragma unroll
+            for (int pc = 0; pc < 2; pc++) {
+                const uint4 e = mbc[(1 + pc) * 36 + m];
+                const int bands = (e.x >> 28) & 3;
+                if (kk == 0 || bands != 0)
+                    cp_async4(clp + pc * CT::kLpInts + tid, coeff[pc] + (e.x & 0x0fffffffu) + (bands >= 2 ? kk * 16 : kk));
+                else
+                    clp[pc * CT::kLpInts + tid] = 0;
+            }
+        }
+        const int piece = (tid & 3) << 2;
+        for (int q = tid >> 2; q < CT::kBlocks; q += kThreads / 4) {
+            const int j = q / kCB, i = q - j * kCB;
+            const int entry = (j / CV + 1 + CT::kFirstMb) * 6 + (i >> 1);
+            const int from = (((j % CV) << 1) + (i & 1)) * 16 + piece;
+#pragma unroll
+            for (int pc = 0; pc < 2; pc++) {
+                int32_t *to = ctile + pc * CT::kInts + q * kCPitch + piece;
+                if (plain) cp_async16(to, coeff[pc] + (mbc[(1 + pc) * 36 + entry].x & 0x0fffffffu) + from);
+                else copy_chunk(to, coeff[pc], mbc[(1 + pc) * 36 + entry], from);
+            }
+        }
     }
     cp_async_commit();
     cp_async_wait_all();
@@ -2720,6 +2745,7 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
     for (int item = tid; item < 3 * 36; item += kThreads) {
         const int pi = item / 36, k36 = item - pi * 36, m = pi == 0 ? first_level_mb(k36) : k36;
         const PlaneDev &p = im.plane[pi];
+        if (pi == 0 && p.overlap != 2 && far_mb(m)) continue;   // not copied, not read
         const uint4 e = mbc[pi * 36 + m];
         bool b = false;
         if (pi == 0) {
@@ -2745,16 +2771,27 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
             for (int r = 0; r < 4; r++)
                 *reinterpret_cast<int4 *>(out + r * kIDC) = make_int4(v[r * 4], v[r * 4 + 1], v[r * 4 + 2], v[r * 4 + 3]);
         } else {
-            const int32_t *l = clp + (pi - 1) * CT::kLpInts + m * CT::kLow;
+            const int ma = m % 6, mb = m / 6, bands = (e.x >> 28) & 3;
             int32_t w[CT::kLow];
+            if (!CT::held(ma, mb)) {
+                const int32_t *l = clp + (pi - 1) * CT::kLpInts + CT::gather_slot(ma, mb) * CT::kLow;
 #pragma unroll
-            for (int k = 0; k < CT::kLow; k += 4) {
-                const int4 q = *reinterpret_cast<const int4 *>(l + k);
-                w[k] = dequant(q.x, k == 0 ? e.y : e.z, b);
-                w[k + 1] = dequant(q.y, e.z, b);
-                w[k + 2] = dequant(q.z, e.z, b);
-                w[k + 3] = dequant(q.w, e.z, b);
+                for (int k = 0; k < CT::kLow; k += 4) {
+                    const int4 q = *reinterpret_cast<const int4 *>(l + k);
+                    w[k] = q.x; w[k + 1] = q.y; w[k + 2] = q.z; w[k + 3] = q.w;
+                }
+            } else if (bands >= 2) {
+                // coefficient 0 of its blocks
+                const int32_t *t = ctile + (pi - 1) * CT::kInts + chroma_block(2 * ma, CV * (mb - 1 - CT::kFirstMb));
+#pragma unroll
+                for (int k = 0; k < CT::kLow; k++) w[k] = t[chroma_block(k & 1, k >> 1)];
+            } else {
+                const int32_t *src = p.coeff + (e.x & 0x0fffffffu);
+#pragma unroll
+                for (int k = 0; k < CT::kLow; k++) w[k] = k == 0 || bands != 0 ? __ldg(src + k) : 0;
             }
+#pragma unroll
+            for (int k = 0; k < CT::kLow; k++) w[k] = dequant(w[k], k == 0 ? e.y : e.z, b);
             if constexpr (CV == 2) b |= inverse_chroma_420<true>(w);
             else b |= inverse_chroma_422<true>(w);
 #pragma unroll
@@ -2856,18 +2893,17 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
                 if (hp == 1) {
                     // block row CV b + line: column 2a + 1 from column 2a
                     if (a == 5 || (b == last && line != 0)) continue;
-                    const int sidx = (CV * b + line) * kCB + 2 * a + 1;
+                    int32_t *q = t + chroma_block(2 * a + 1, CV * b + line);
 #pragma unroll
-                    for (int r = 1; r < 4; r++) t[elem(sidx, r, 0)] = A::add(t[elem(sidx, r, 0)], t[elem(sidx - 1, r, 0)], ov);
+                    for (int r = 4; r < 16; r += 4) q[r] = A::add(q[r], q[r - kCPitch], ov);
                 } else {
                     // block column 2a + line: rows CV b + 1 .. from the row above
                     if (line > 1 || b == last || (a == 5 && line != 0)) continue;
 #pragma unroll
                     for (int r = 1; r < CV; r++) {
-                        const int sidx = (CV * b + r) * kCB + 2 * a + line;
+                        int32_t *q = t + chroma_block(2 * a + line, CV * b + r);
 #pragma unroll
-                        for (int c = 1; c < 4; c++)
-                            t[elem(sidx, 0, c)] = A::add(t[elem(sidx, 0, c)], t[elem(sidx - kCB, 0, c)], ov);
+                        for (int c = 1; c < 4; c++) q[c] = A::add(q[c], q[c - kCB * kCPitch], ov);
                     }
                 }
             }
@@ -2880,7 +2916,7 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
     // rows 1..10 (4:2:2: 0..16);
     // an edge tile's items are only its blocks inside the plane (divisions
     // as multiplies by ceil(2^16 / n), exact for these small quotients)
-    if (next < item_count) note_plain(imn, mbc_next, 1, sh.plain);
+    if (next < item_count) note_plain(imn, mbc_next, 3, sh.plain);
     int lcols = kIB, lrows = kIB, ccols = 10, crows = CT::kTransRows, cmagic = 0;
     if (edge) {
         const int rx = (int)im.plane[0].mbs_x - mx0, ry = (int)im.plane[0].mbs_y - my0;
@@ -2897,7 +2933,6 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
         int32_t *blk;
         uint32_t step;
         int32_t dcv;
-        int sw;
         if (item < lcount) {
             int i, j;
             if (item < 256) {
@@ -2910,7 +2945,6 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
             if (edge && (i >= lcols || j >= lrows)) continue;
             step = mbc[((j >> 2) + 1) * 6 + (i >> 2) + 1].w;
             blk = ytile + block_at(i, j);
-            sw = 0;
             dcv = ydc[(j + 4) * kIDC + i + 4];
         } else {
             const int q = item - lcount;
@@ -2926,16 +2960,14 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
                 i = 1 + rem % 10;
                 j = CT::kRow0 + rem / 10;
             }
-            const int sidx = j * kCB + i;
             step = mbc[(1 + pc) * 36 + (j / CV + 1 + CT::kFirstMb) * 6 + (i >> 1)].w;
-            blk = ctile + pc * CT::kInts + sidx * 16;
-            sw = swz(sidx);
+            blk = ctile + pc * CT::kInts + chroma_block(i, j);
             dcv = cdc[pc * CT::kDcInts + (j + CT::kDcRow0) * kCDC + i];
         }
         int32_t v[16];
 #pragma unroll
         for (int r = 0; r < 4; r++) {
-            const int4 q = *reinterpret_cast<const int4 *>(blk + ((r ^ sw) << 2));
+            const int4 q = *reinterpret_cast<const int4 *>(blk + (r << 2));
             v[r * 4 + 0] = q.x; v[r * 4 + 1] = q.y; v[r * 4 + 2] = q.z; v[r * 4 + 3] = q.w;
         }
         const uint32_t m = mag_bound<1>(v);
@@ -2952,43 +2984,16 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
         if (b) bad |= kFlagSecond;
 #pragma unroll
         for (int r = 0; r < 4; r++)
-            *reinterpret_cast<int4 *>(blk + ((r ^ sw) << 2)) = make_int4(v[r * 4], v[r * 4 + 1], v[r * 4 + 2], v[r * 4 + 3]);
+            *reinterpret_cast<int4 *>(blk + (r << 2)) = make_int4(v[r * 4], v[r * 4 + 1], v[r * 4 + 2], v[r * 4 + 3]);
     }
     // a small tile's overlap outputs stay below 2^27.8, and the chroma
     // interpolated from them below 2^28: no magnitude tests below
     const bool tile_small = __syncthreads_and(small) != 0;
-    // stage D (chroma): the 9 x 9 (4:2:2: 9 x 16) second-level cells of each
-    // chroma plane, in place; cell column k of the luma tile's macroblock
-    // boundary a is 2a, cell row likewise, 4:2:2's 4b
-    for (int item = tid; item < 2 * 9 * CT::kCells; item += kThreads) {
-        const int pc = item / (9 * CT::kCells), c = item - pc * (9 * CT::kCells);
-        if (CV == 4 && c < 9 && !(edge && my0 == 0)) continue;   // the row above is another tile's
-        int32_t *t = ctile + pc * CT::kInts;
-        if (edge) {
-            // cells past the chroma plane's edge, or cut by it
-            const int Wc = 8 * (int)im.plane[1].mbs_x, Hc = 4 * CV * (int)im.plane[1].mbs_y;
-            const int X = 8 * mx0 - 2 + 4 * (c % 9), Y = CT::cell0(my0) + 4 * (c / 9);
-            if (X >= Wc || Y >= Hc) continue;
-            bool vs = X + 2 == 0 || X + 2 == Wc, hs = Y + 2 == 0 || Y + 2 == Hc;
-            if (MODE == 1) {
-                vs |= (c % 9) % 2 == 0 && ((sh.hard >> ((c % 9) / 2)) & 1);
-                hs |= (c / 9) % CV == 0 && ((sh.hard >> (8 + (c / 9) / CV)) & 1);
-            }
-            if (vs || hs) {
-                if (im.plane[1 + pc].overlap >= 1 && chroma_cut_cell(t, X, Y, 8 * mx0 - 8, CT::sample0(my0), Wc, Hc, vs, hs))
-                    bad |= kFlagOverlap;
-                continue;
-            }
-        }
-        int32_t w[16];
-        if (cell_rw(t, (CV == 2 ? 1 + c / 9 : c / 9 - 1) * kCB + 1 + c % 9, kCB, im.plane[1 + pc].overlap, w, true, tile_small))
-            bad |= kFlagOverlap;
-    }
     EdgeCells ec;
     bool grid_cell = true, cut = false;
     int gcx = tid & 15, gcy = tid >> 4;   // the thread's cell of the 16 x 16 grid
     if (edge) {
-        // stage D for the luma cells the plane's edge cuts, in place
+        // stage D for the luma cells that the plane's edge or a hard boundary cuts
         ec = edge_cells(im, mx0, my0);
         const uint32_t hard = MODE == 1 ? sh.hard : 0;
         if (edge_overlap<1>(im, ytile, mx0, my0, ec, hard)) bad |= kFlagOverlap;
@@ -2996,185 +3001,141 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
         edge_grid(ec, mx0, my0, gcx, gcy, grid_cell);
         cut = hard && (hard_cell(hard & 0x1fu, gcx) || hard_cell((hard >> 8) & 0x1fu, gcy));
     }
+    // stage D, in place, with one copy of the operator: the thread's luma cell,
+    // then the 9 x 9 (4:2:2: 9 x 16) cells of each chroma plane; chroma cell
+    // column k of the luma tile's macroblock boundary a is 2a, cell row
+    // likewise, 4:2:2's 4b
+#pragma unroll 1
+    for (int item = tid; item < kThreads + 2 * 9 * CT::kCells; item += kThreads) {
+        int32_t *t = ytile;
+        CellBlocks cell;
+        int pi = 0;
+        if (item < kThreads) {
+            if (!grid_cell || cut) continue;
+            cell = cell_blocks(gcx, gcy);
+        } else {
+            const int pc = (item - kThreads) / (9 * CT::kCells), c = item - kThreads - pc * (9 * CT::kCells);
+            const int ci = c % 9, cj = c / 9;
+            if (CV == 4 && cj == 0 && !(edge && my0 == 0)) continue;   // the row above is another tile's
+            pi = 1 + pc;
+            t = ctile + pc * CT::kInts;
+            if (edge) {
+                // cells past the chroma plane's edge, or cut by it
+                const int Wc = 8 * (int)im.plane[1].mbs_x, Hc = 4 * CV * (int)im.plane[1].mbs_y;
+                const int X = 8 * mx0 - 2 + 4 * ci, Y = CT::cell0(my0) + 4 * cj;
+                if (X >= Wc || Y >= Hc) continue;
+                bool vs = X + 2 == 0 || X + 2 == Wc, hs = Y + 2 == 0 || Y + 2 == Hc;
+                if (MODE == 1) {
+                    vs |= ci % 2 == 0 && ((sh.hard >> (ci / 2)) & 1);
+                    hs |= cj % CV == 0 && ((sh.hard >> (8 + cj / CV)) & 1);
+                }
+                if (vs || hs) {
+                    if (im.plane[pi].overlap >= 1 && chroma_cut_cell(t, X, Y, 8 * mx0 - 8, CT::sample0(my0), Wc, Hc, vs, hs))
+                        bad |= kFlagOverlap;
+                    continue;
+                }
+            }
+            const int b00 = chroma_block(1 + ci, CV == 2 ? 1 + cj : cj - 1);
+            cell = CellBlocks{b00, b00 + kCPitch, b00 + kCB * kCPitch, b00 + (kCB + 1) * kCPitch};
+        }
+        if (im.plane[pi].overlap < 1) continue;
+        int32_t w[16];
+        if (cell_samples(t, cell, 1, w, tile_small)) bad |= kFlagOverlap;
+        cell_store(t, cell, w);
+    }
     __syncthreads();
-    // stage E: each thread's luma cell, the chroma around it interpolated
-    // (T.832 Table 180, vertical then horizontal), converted and stored
+    // stage E: each thread's luma cell row by row, the chroma around it
+    // interpolated (T.832 Table 180, vertical then horizontal), converted and
+    // stored
     if (grid_cell) {
         const int cx = gcx, cy = gcy;
+        const CellBlocks cell = cell_blocks(cx, cy);
         const OutputDev &o = im.out;
         const int x0 = 16 * mx0 + 2 + 4 * cx, y0 = 16 * my0 + 2 + 4 * cy;
         const bool inside = x0 >= (int)o.crop_x && x0 + 4 <= (int)(o.crop_x + o.crop_w) && y0 >= (int)o.crop_y &&
                             y0 + 4 <= (int)(o.crop_y + o.crop_h);
-        bool obad = false, done = false;
-        int32_t y[16];
-        if (cell_samples(ytile, cell_blocks(cx, cy), MODE == 1 && cut ? 0 : im.plane[0].overlap, y, tile_small)) bad |= kFlagOverlap;
-        // chroma columns (tile coordinates) 8 + 2cx .. 11 + 2cx, rows 8 + 2cy .. 11 + 2cy (4:2:2: 2 + 4cy .. 5 + 4cy)
-        if (tile_small && !edge && inside && o.kind == kOutRgb8 && !o.premultiply &&
-            (o.channels == 3 || o.ch[3].padding)) {
-            // RGB8 of an interior small tile, row by row: each luma row's
-            // chroma from the two chroma rows it lies between, read afresh,
-            // so that no cell holds both chroma planes' 4 x 4 neighbourhoods
-            // (every sample is below 2^28: no tests, the one-division form)
-            const ChannelScale &sc = o.ch[0];
-            const int32_t add = sc.shifted_bias + sc.rounding;
-            const int shift = sc.shift;
-            const uint32_t order = sc.source == 2 ? 0x7014u : 0x7410u;
-            const int cyc = im.centering_y, cxc = im.centering_x;
+        // RGB8 from YUV; a fourth byte can only be padding (no alpha plane)
+        const bool rgb8 = inside && o.kind == kOutRgb8 && !o.premultiply && (o.channels == 3 || o.ch[3].padding);
+        const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
+        uint8_t *dst = o.base + (int64_t)(y0 - (int)o.crop_y) * (int64_t)o.row_stride +
+                       (int64_t)(x0 - (int)o.crop_x) * (int64_t)pixel_bytes;
+        // chroma columns (tile coordinates) 8 + 2cx .. 11 + 2cx, in two pairs
+        const int sx = 8 + 2 * cx;
+        const int at0 = (sx >> 2) * kCPitch + (sx & 3), at1 = ((sx + 2) >> 2) * kCPitch + ((sx + 2) & 3);
+        const int cxc = im.centering_x, cyc = im.centering_y;
+        bool obad = false;
+#pragma unroll 1
+        for (int r = 0; r < 4; r++, dst += o.row_stride) {
+            int32_t y[4];
+            {
+                const int2 l = *reinterpret_cast<const int2 *>(ytile + (r < 2 ? cell.b00 + 8 : cell.b10 - 8) + 4 * r + 2);
+                const int2 q = *reinterpret_cast<const int2 *>(ytile + (r < 2 ? cell.b01 + 8 : cell.b11 - 8) + 4 * r);
+                y[0] = l.x; y[1] = l.y; y[2] = q.x; y[3] = q.y;
+            }
+            uint32_t m = 0;
+            if (!tile_small) {
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
-                // luma row y0 + r takes chroma rows a and a + 1 of the
-                // neighbourhood, as the 4 x 4 form below does
-                const int a = (r + 1) >> 1;
-                int32_t ch[2][4];
+                for (int c = 0; c < 4; c++) m |= mag(y[c]);
+            }
+            // the chroma row, or for 4:2:0 the two chroma rows it lies between,
+            // weighted; a small tile's samples, and others that test so, are
+            // below 2^28: the one-division form
+            int32_t ch[2][4];
+            const int ya = CV == 2 ? 8 + 2 * cy + ((r + 1) >> 1) : 2 + 4 * cy + r;
+            const int row_a = (ya >> 2) * (kCB * kCPitch) + ((ya & 3) << 2);
+            const int row_b = ((ya + 1) >> 2) * (kCB * kCPitch) + (((ya + 1) & 3) << 2);
+            const int wa = (r & 1) ? 4 + cyc : cyc, wb = 8 - wa;
 #pragma unroll
-                for (int pc = 0; pc < 2; pc++) {
-                    const int32_t *t = ctile + pc * CT::kInts;
-                    int32_t col[4];
-                    if (CV == 4) {
-#pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            const int sx = 8 + 2 * cx + 2 * h, sy = 2 + 4 * cy + r;
-                            const int2 p = *reinterpret_cast<const int2 *>(&t[elem((sy >> 2) * kCB + (sx >> 2), sy & 3, sx & 3)]);
-                            col[2 * h] = p.x; col[2 * h + 1] = p.y;
-                        }
-                    } else {
-                    int32_t sa[4], sb[4];
-#pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        const int sx = 8 + 2 * cx + 2 * h, ya = 8 + 2 * cy + a, yb = ya + 1;
-                        const int2 pa = *reinterpret_cast<const int2 *>(&t[elem((ya >> 2) * kCB + (sx >> 2), ya & 3, sx & 3)]);
-                        const int2 pb = *reinterpret_cast<const int2 *>(&t[elem((yb >> 2) * kCB + (sx >> 2), yb & 3, sx & 3)]);
-                        sa[2 * h] = pa.x; sa[2 * h + 1] = pa.y;
-                        sb[2 * h] = pb.x; sb[2 * h + 1] = pb.y;
-                    }
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        col[k] = (r & 1) ? up_odd_small(sa[k], sb[k], cyc) : up_even_small(sa[k], sb[k], cyc);
-                    }
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        ch[pc][c] = (c & 1) ? up_odd_small(col[1 + (c >> 1)], col[2 + (c >> 1)], cxc)
-                                            : up_even_small(col[(c >> 1)], col[1 + (c >> 1)], cxc);
+            for (int pc = 0; pc < 2; pc++) {
+                const int32_t *t = ctile + pc * CT::kInts;
+                int32_t col[4];
+                const int2 a0 = *reinterpret_cast<const int2 *>(t + row_a + at0), a1 = *reinterpret_cast<const int2 *>(t + row_a + at1);
+                col[0] = a0.x; col[1] = a0.y; col[2] = a1.x; col[3] = a1.y;
+                if (!tile_small) m |= mag(col[0]) | mag(col[1]) | mag(col[2]) | mag(col[3]);
+                if (CV == 2) {
+                    const int2 b0 = *reinterpret_cast<const int2 *>(t + row_b + at0), b1 = *reinterpret_cast<const int2 *>(t + row_b + at1);
+                    if (!tile_small) m |= mag(b0.x) | mag(b0.y) | mag(b1.x) | mag(b1.y);
+                    col[0] = (col[0] * wa + b0.x * wb + 4) >> 3;
+                    col[1] = (col[1] * wa + b0.y * wb + 4) >> 3;
+                    col[2] = (col[2] * wa + b1.x * wb + 4) >> 3;
+                    col[3] = (col[3] * wa + b1.y * wb + 4) >> 3;
                 }
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+                    ch[pc][c] = (c & 1) ? up_odd_small(col[1 + (c >> 1)], col[2 + (c >> 1)], cxc)
+                                        : up_even_small(col[(c >> 1)], col[1 + (c >> 1)], cxc);
+            }
+            if (rgb8 && m < (1u << 28)) {
+                const ChannelScale &sc = o.ch[0];
+                const int32_t add = sc.shifted_bias + sc.rounding;
+                const int shift = sc.shift;
+                const uint32_t order = sc.source == 2 ? 0x7014u : 0x7410u;
                 uint32_t px[4];
 #pragma unroll
                 for (int c = 0; c < 4; c++) {
                     int32_t R, G, B;
-                    yuv_to_rgb_fast(y[r * 4 + c] + add, ch[0][c], ch[1][c], R, G, B);
+                    yuv_to_rgb_fast(y[c] + add, ch[0][c], ch[1][c], R, G, B);
                     px[c] = pack_rgb8(clamp_u8(R >> shift), clamp_u8(G >> shift), clamp_u8(B >> shift), order);
                 }
-                uint8_t *dst = o.base + (uint64_t)(y0 + r - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * o.channels;
                 if (o.channels == 4) store16(dst, px[0], px[1], px[2], px[3]);
                 else store12(dst, px);
+                continue;
             }
-            done = true;
-        }
-        int32_t u[16], v[16];
-#pragma unroll
-        for (int pc = 0; pc < 2 && !done; pc++) {
-            const int32_t *t = ctile + pc * CT::kInts;
-            int32_t s[4][4];
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const int sy = CV == 2 ? 8 + 2 * cy + r : 2 + 4 * cy + r;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int sx = 8 + 2 * cx + 2 * h;
-                    const int2 a = *reinterpret_cast<const int2 *>(&t[elem((sy >> 2) * kCB + (sx >> 2), sy & 3, sx & 3)]);
-                    s[r][2 * h] = a.x;
-                    s[r][2 * h + 1] = a.y;
-                }
-            }
-            int32_t *dst = pc == 0 ? u : v;
-            // chroma samples below 2^28 take the one-division form: in an
-            // interior small tile they all are (overlap outputs below
-            // 2^27.8); elsewhere the 16 read are tested
-            bool fast = tile_small && !edge;
-            if (!fast) {
-                uint32_t cm = 0;
-#pragma unroll
-                for (int r = 0; r < 4; r++)
-#pragma unroll
-                    for (int k = 0; k < 4; k++) cm |= mag(s[r][k]);
-                fast = cm < (1u << 28);
-            }
-            if (fast) {
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    int32_t col[4];
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        col[k] = CV == 4 ? s[r][k]
-                               : (r & 1) ? up_odd_small(s[1 + (r >> 1)][k], s[2 + (r >> 1)][k], im.centering_y)
-                                         : up_even_small(s[(r >> 1)][k], s[1 + (r >> 1)][k], im.centering_y);
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        dst[r * 4 + c] = (c & 1) ? up_odd_small(col[1 + (c >> 1)], col[2 + (c >> 1)], im.centering_x)
-                                                 : up_even_small(col[(c >> 1)], col[1 + (c >> 1)], im.centering_x);
-                }
-            } else {
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    // luma row y0 + r: chroma row (y0 + r) >> 1 = tile row 9 + 2cy + (r >> 1)
-                    int32_t col[4];
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        col[k] = CV == 4 ? s[r][k]
-                               : (r & 1) ? up_odd(s[1 + (r >> 1)][k], s[2 + (r >> 1)][k], im.centering_y)
-                                         : up_even(s[(r >> 1)][k], s[1 + (r >> 1)][k], im.centering_y);
-#pragma unroll
-                    for (int c = 0; c < 4; c++)
-                        dst[r * 4 + c] = (c & 1) ? up_odd(col[1 + (c >> 1)], col[2 + (c >> 1)], im.centering_x)
-                                                 : up_even(col[(c >> 1)], col[1 + (c >> 1)], im.centering_x);
-                }
-            }
-        }
-        // RGB8 from YUV; a fourth byte can only be padding (no alpha plane)
-        if (!done && inside && o.kind == kOutRgb8 && !o.premultiply && (o.channels == 3 || o.ch[3].padding)) {
-            uint32_t m = 0;
-            if (!tile_small) {
-#pragma unroll
-                for (int k = 0; k < 16; k++) m |= mag(y[k]) | mag(u[k]) | mag(v[k]);
-            }
-            if (m < (1u << 28)) {
-                const ChannelScale &sc = o.ch[0];
-                const int32_t add = sc.shifted_bias + sc.rounding;
-                const int shift = sc.shift;
-                // byte order of the packed pixel: R G B, or B G R
-                const uint32_t order = sc.source == 2 ? 0x7014u : 0x7410u;
-                uint32_t px[16];
-#pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    // each colour is luma plus terms in u and v, so adding the
-                    // output bias to luma adds it to all three (no
-                    // intermediate nears int32 below 2^28)
-                    int32_t R, G, B;
-                    yuv_to_rgb_fast(y[k] + add, u[k], v[k], R, G, B);
-                    px[k] = pack_rgb8(clamp_u8(R >> shift), clamp_u8(G >> shift), clamp_u8(B >> shift), order);
-                }
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    uint8_t *dst = o.base + (uint64_t)(y0 + r - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * o.channels;
-                    if (o.channels == 4) store16(dst, px[4 * r], px[4 * r + 1], px[4 * r + 2], px[4 * r + 3]);
-                    else store12(dst, &px[4 * r]);
-                }
-                done = true;
-            }
-        }
-        if (!done) {
-            const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
+            const int yy = y0 + r;
+            if (yy < (int)o.crop_y || yy >= (int)(o.crop_y + o.crop_h)) continue;
             const uint64_t chs = o.nchw ? o.plane_stride : (uint64_t)o.elem_bytes;
-            for (int r = 0; r < 4; r++)
-                for (int c = 0; c < 4; c++) {
-                    const int x = x0 + c, yy = y0 + r;
-                    if (x < (int)o.crop_x || x >= (int)(o.crop_x + o.crop_w) || yy < (int)o.crop_y ||
-                        yy >= (int)(o.crop_y + o.crop_h))
-                        continue;
-                    const int k = r * 4 + c;
-                    const int32_t comp[4] = {y[k], u[k], v[k], 0};
-                    uint8_t *dst = o.base + (uint64_t)(yy - o.crop_y) * o.row_stride + (uint64_t)(x - o.crop_x) * pixel_bytes;
-                    format_pixel(o, comp, 0, dst, chs, obad);
+#pragma unroll 1
+            for (int c = 0; c < 4; c++) {
+                if (x0 + c < (int)o.crop_x || x0 + c >= (int)(o.crop_x + o.crop_w)) continue;
+                if (m < (1u << 28)) {
+                    const int32_t comp[4] = {c == 0 ? y[0] : c == 1 ? y[1] : c == 2 ? y[2] : y[3],
+                                             c == 0 ? ch[0][0] : c == 1 ? ch[0][1] : c == 2 ? ch[0][2] : ch[0][3],
+                                             c == 0 ? ch[1][0] : c == 1 ? ch[1][1] : c == 2 ? ch[1][2] : ch[1][3], 0};
+                    format_pixel(o, comp, 0, dst + (int64_t)c * (int64_t)pixel_bytes, chs, obad);
+                } else {
+                    obad |= chroma_pixel<CV>(im, ytile, ctile, mx0, my0, x0 + c, yy);
                 }
+            }
         }
         if (obad) bad |= kFlagOutput;
     }
@@ -3210,8 +3171,11 @@ __device__ __forceinline__ void hold_image(const ImageDev *__restrict__ images, 
 
 // Tiles of YUV 4:2:0 (CV 2) and 4:2:2 (CV 4) images: interior (MODE 0), edge
 // (MODE 1) or both (MODE 2).
+// Four 4:2:0 interior tiles an SM (64 registers, a few spilled), three edge
+// tiles and three of 4:2:2's larger ones: 3999 x 2999 4:2:0 87.1 us, the mixed
+// batch 127.6, against 89.0 and 129.6 with three of each.
 template <int MODE, int CV>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, CV == 2 && MODE == 0 ? 4 : 3)
 jxrb_interior_chroma_tiles(const ImageDev *__restrict__ images, const WorkItem *__restrict__ items, uint32_t item_count,
                        uint32_t *status, uint32_t *counters) {
     extern __shared__ __align__(16) int32_t smem_chroma[];
@@ -3227,7 +3191,7 @@ jxrb_interior_chroma_tiles(const ImageDev *__restrict__ images, const WorkItem *
             if (threadIdx.x == 0) sh.plain = 1;
             cp_async_wait_all();
             __syncthreads();
-            note_plain(images[w.image & kImageMask], mbc[0], 1, sh.plain);
+            note_plain(images[w.image & kImageMask], mbc[0], 3, sh.plain);
             __syncthreads();
         }
         __shared__ ImageDev simg;
