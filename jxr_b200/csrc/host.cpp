@@ -729,6 +729,136 @@ private:
     CopyPool pool_{staging_threads()};
 };
 
+// What a session keeps for its submissions instead of making it for each: a
+// ring of page-locked buffers their descriptors are uploaded from in one copy,
+// page-locked words their status comes back to, and their events.  A pageable
+// copy, memset or status read apiece, and an event made and destroyed, took
+// more of a small submission than its kernels did (192 x 144 4:2:0, host to
+// host: 113 us so, 93 us here; 24 mixed requests 320 and 308).  upload() is called
+// under the session's lock; the rest has its own.
+class SubmissionPool {
+public:
+    static constexpr size_t kBytes = size_t(256) << 10;
+    static constexpr int kSlots = 8;
+    static constexpr uint32_t kWords = 1024;
+    static constexpr int kBounces = 4;         // buffers small outputs come back through
+    static constexpr size_t kMaxEvents = 256;
+
+    ~SubmissionPool() {
+        for (Slot &sl : slots_)
+            if (sl.done) {
+                cudaEventSynchronize(sl.done);
+                cudaEventDestroy(sl.done);
+            }
+        for (auto &list : events_)
+            for (cudaEvent_t e : list) cudaEventDestroy(e);
+        if (host_) cudaFreeHost(host_);
+    }
+    // `bytes` of pageable memory at `src` to device memory at `dst` on
+    // `stream`; false (nothing done) when they do not fit a buffer or every
+    // buffer is in flight
+    bool upload(uint8_t *dst, const void *src, size_t bytes, cudaStream_t stream, jxrb_status &result) {
+        result = JXRB_OK;
+        if (bytes > kBytes || !reserve()) return false;
+        for (int k = 0; k < kSlots; k++) {
+            Slot &sl = slots_[next_];
+            uint8_t *host = host_ + kBytes * next_;
+            next_ = (next_ + 1) % kSlots;
+            if (sl.pending && cudaEventQuery(sl.done) != cudaSuccess) {
+                cudaGetLastError();   // not-ready is no error to report later
+                continue;
+            }
+            std::memcpy(host, src, bytes);
+            result = send(dst, host, bytes, stream, sl);
+            return true;
+        }
+        return false;
+    }
+    // A word the status is copied to; null when none is free.
+    volatile uint32_t *take_word() {
+        std::lock_guard<std::mutex> guard(lock_);
+        if (!host_ || free_words_.empty()) return nullptr;
+        volatile uint32_t *w = words() + free_words_.back();
+        free_words_.pop_back();
+        return w;
+    }
+    void give_word(volatile uint32_t *w) {
+        if (!w) return;
+        std::lock_guard<std::mutex> guard(lock_);
+        free_words_.push_back((uint32_t)(w - words()));
+    }
+    // A page-locked buffer of kBytes; null when none is free.
+    uint8_t *take_bounce() {
+        std::lock_guard<std::mutex> guard(lock_);
+        if (!host_ || free_bounces_.empty()) return nullptr;
+        uint8_t *b = free_bounces_.back();
+        free_bounces_.pop_back();
+        return b;
+    }
+    void give_bounce(uint8_t *b) {
+        std::lock_guard<std::mutex> guard(lock_);
+        free_bounces_.push_back(b);
+    }
+    // An event, with or without timing.
+    jxrb_status take_event(bool timing, cudaEvent_t &e) {
+        {
+            std::lock_guard<std::mutex> guard(lock_);
+            if (!events_[timing].empty()) {
+                e = events_[timing].back();
+                events_[timing].pop_back();
+                return JXRB_OK;
+            }
+        }
+        CUDA_TRY(cudaEventCreateWithFlags(&e, timing ? cudaEventDefault : cudaEventDisableTiming), "cudaEventCreate");
+        return JXRB_OK;
+    }
+    void give_event(bool timing, cudaEvent_t e) {
+        if (!e) return;
+        {
+            std::lock_guard<std::mutex> guard(lock_);
+            if (events_[timing].size() < kMaxEvents) {
+                events_[timing].push_back(e);
+                return;
+            }
+        }
+        cudaEventDestroy(e);
+    }
+
+private:
+    struct Slot {
+        cudaEvent_t done = nullptr;
+        bool pending = false;
+    };
+    volatile uint32_t *words() { return reinterpret_cast<volatile uint32_t *>(host_ + kBytes * (kSlots + kBounces)); }
+    bool reserve() {
+        if (host_) return true;
+        void *p = nullptr;
+        if (cudaHostAlloc(&p, kBytes * (kSlots + kBounces) + kWords * sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        std::lock_guard<std::mutex> guard(lock_);
+        host_ = static_cast<uint8_t *>(p);
+        for (uint32_t k = 0; k < kWords; k++) free_words_.push_back(k);
+        for (int k = 0; k < kBounces; k++) free_bounces_.push_back(host_ + kBytes * (kSlots + k));
+        return true;
+    }
+    jxrb_status send(uint8_t *dst, const uint8_t *host, size_t bytes, cudaStream_t stream, Slot &sl) {
+        if (!sl.done) CUDA_TRY(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming), "cudaEventCreate");
+        CUDA_TRY(cudaMemcpyAsync(dst, host, bytes, cudaMemcpyHostToDevice, stream), "upload descriptors");
+        sl.pending = true;
+        CUDA_TRY(cudaEventRecord(sl.done, stream), "cudaEventRecord");
+        return JXRB_OK;
+    }
+    uint8_t *host_ = nullptr;
+    Slot slots_[kSlots];
+    int next_ = 0;
+    std::mutex lock_;
+    std::vector<uint32_t> free_words_;
+    std::vector<uint8_t *> free_bounces_;
+    std::vector<cudaEvent_t> events_[2];
+};
+
 // ---------------------------------------------------------------------------
 // device buffers of one launch set (one or more images)
 // ---------------------------------------------------------------------------
@@ -783,7 +913,10 @@ struct DeviceSet {
     uint32_t q_count = 0, q_planes = 0, q_max_mbs = 0, q_max_samples = 0;
     uint64_t q_max_pixels = 0;
     bool q_two_level = false, q_subsampled = false, q_finish = false;   // launch_quarter's stages
-    std::vector<uint8_t> host_quarter;  // descriptors and scale terms, uploaded in one copy
+    // everything of the set below its coefficients and pictures -- image
+    // descriptors first, work list, zeroed status and counters, tables or the
+    // reduced-resolution descriptors -- as it goes to the device in one copy
+    std::vector<uint8_t> host_blob;
     std::vector<ImageDev> host_images;
     std::vector<WorkItemHost> host_items;
     // the callers' coefficients, copied by upload_coefficients after every
@@ -812,12 +945,11 @@ int side_streams(const DeviceSet &set) {
 }
 
 // Lay out, allocate and upload every input of `plans`; output pointers are
-// bound later by bind_output.  Copies run on `stream`; the host buffers are
-// read before this returns (a synchronize on pageable sources).
-// The set's kernels run beside each other on `sides`, or, without, on side
+// bound later by bind_output, which also uploads the blob built here.  The
+// set's kernels run beside each other on `sides`, or, without, on side
 // streams of its own.
 jxrb_status build_device_set(const jxrb_plan *const *plans, uint32_t count, cudaStream_t stream, DeviceSet &set,
-                             Staging *staging = nullptr, Sides *sides = nullptr) {
+                             Sides *sides = nullptr) {
     set.host_images.assign(count, ImageDev{});
     set.image_items.assign(count + 1, 0);
     set.output_offsets.assign(count, 0);
@@ -935,23 +1067,13 @@ jxrb_status build_device_set(const jxrb_plan *const *plans, uint32_t count, cuda
                 set.host_items[it++] = WorkItemHost{i | tag << kTagShift, (uint16_t)tx, (uint16_t)ty};
             }
     }
-    {
-        std::vector<uint8_t> tables(tables_end - tables_at, 0);
-        for (const Copy &c : copies)
-            if (c.bytes) std::memcpy(tables.data() + (c.at - tables_at), c.src, c.bytes);
-        if (!tables.empty()) {
-            if (staging) TRY(staging->upload(base + tables_at, tables.data(), tables.size(), stream));
-            else CUDA_TRY(cudaMemcpyAsync(base + tables_at, tables.data(), tables.size(), cudaMemcpyHostToDevice, stream),
-                          "upload tables");
-        }
-        set.upload_bytes += tables.size();
-    }
+    set.host_blob.assign(tables_end, 0);
+    for (const Copy &c : copies)
+        if (c.bytes) std::memcpy(set.host_blob.data() + c.at, c.src, c.bytes);
+    set.upload_bytes += tables_end - tables_at;
     // order the work list by kernel segment
     order_by_segment(set.host_items, set.bounds);
-    CUDA_TRY(cudaMemcpyAsync(set.items, set.host_items.data(), sizeof(WorkItemHost) * items, cudaMemcpyHostToDevice,
-                             stream), "upload work list");
-    CUDA_TRY(cudaMemsetAsync(set.counters, 0, kCounterWords * sizeof(uint32_t), stream), "counter reset");
-    CUDA_TRY(cudaMemsetAsync(set.status, 0, sizeof(uint32_t), stream), "status reset");
+    if (items) std::memcpy(set.host_blob.data() + items_at, set.host_items.data(), sizeof(WorkItemHost) * items);
     set.sides = sides ? sides : &set.own_sides;
     TRY(set.sides->grow(side_streams(set)));
     return JXRB_OK;
@@ -974,12 +1096,36 @@ jxrb_status upload_coefficients(DeviceSet &set, cudaStream_t stream, Staging *st
     return JXRB_OK;
 }
 
+// A resident set's blob, ahead of its first binding.
+jxrb_status upload_blob(DeviceSet &set, cudaStream_t stream) {
+    CUDA_TRY(cudaMemcpyAsync(set.mem, set.host_blob.data(), set.host_blob.size(), cudaMemcpyHostToDevice, stream),
+             "upload descriptors");
+    std::vector<uint8_t>().swap(set.host_blob);
+    return JXRB_OK;
+}
+
 // Bind the output surfaces (dense, plan order, 256-byte aligned) and upload
-// the image descriptors.
-jxrb_status bind_output(DeviceSet &set, uint8_t *dst, cudaStream_t stream) {
+// the set's blob, or, once that is on the device, the image descriptors alone:
+// through the session's pool where it takes them, through its staging ring, or
+// from pageable memory.
+jxrb_status bind_output(DeviceSet &set, uint8_t *dst, cudaStream_t stream, SubmissionPool *pool = nullptr,
+                        Staging *staging = nullptr) {
     for (size_t i = 0; i < set.host_images.size(); i++) set.host_images[i].out.base = dst + set.output_offsets[i];
-    CUDA_TRY(cudaMemcpyAsync(set.images, set.host_images.data(), sizeof(ImageDev) * set.host_images.size(),
-                             cudaMemcpyHostToDevice, stream), "upload image descriptors");
+    const size_t descriptors = sizeof(ImageDev) * set.host_images.size();
+    const void *from = set.host_images.data();
+    size_t bytes = descriptors;
+    if (!set.host_blob.empty()) {
+        std::memcpy(set.host_blob.data(), set.host_images.data(), descriptors);
+        from = set.host_blob.data();
+        bytes = set.host_blob.size();
+    }
+    uint8_t *to = static_cast<uint8_t *>(set.mem);
+    jxrb_status sent = JXRB_OK;
+    if (pool && pool->upload(to, from, bytes, stream, sent)) TRY(sent);
+    else if (staging) TRY(staging->upload(to, from, bytes, stream));
+    else CUDA_TRY(cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, stream), "upload descriptors");
+    // (a pageable source has been read when the copy returns)
+    std::vector<uint8_t>().swap(set.host_blob);
     for (size_t i = 0; i < set.host_images.size(); i++) {
         if (set.host_images[i].out.store == kStoreBits) {
             const uint64_t end = i + 1 < set.host_images.size() ? set.output_offsets[i + 1] : set.output_bytes;
@@ -1002,6 +1148,7 @@ struct jxrb_session {
     std::atomic<uint32_t> next_stream{0};
     std::mutex lock;   // serialises encoding of submissions (runtime.rs:42)
     std::atomic<uint64_t> submissions{0}, uploaded{0}, read_back{0}, held{0}, launches{0};
+    SubmissionPool pool;
     std::unique_ptr<Staging> staging;  // pinned ring for pageable sources, made at the first submission (under `lock`)
     cudaStream_t upload = nullptr;     // uploads of resident images
 };
@@ -1040,6 +1187,8 @@ struct jxrb_submission {
     bool waited = false;
     jxrb_status result = JXRB_OK;
     uint32_t status_word = 0;
+    volatile uint32_t *word = nullptr;   // the session's, which the status is copied to before `done`
+    bool timed = false;                  // plan submissions' events have timing
 };
 
 struct jxrb_resident {
@@ -1152,6 +1301,18 @@ jxrb_status status_to_error(uint32_t word) {
     return fail(JXRB_KERNEL_ARITHMETIC, buf);
 }
 
+// The end of a submission on its stream: the status word on its way to the
+// host, and the event that tells.
+jxrb_status finish_submission(jxrb_session *s, jxrb_submission *sub) {
+    sub->word = s->pool.take_word();
+    if (sub->word)
+        CUDA_TRY(cudaMemcpyAsync(const_cast<uint32_t *>(sub->word), sub->set.status, sizeof(uint32_t),
+                                 cudaMemcpyDeviceToHost, sub->stream), "status copy");
+    TRY(s->pool.take_event(sub->timed, sub->done));
+    CUDA_TRY(cudaEventRecord(sub->done, sub->stream), "cudaEventRecord");
+    return JXRB_OK;
+}
+
 jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32_t count, void *dst, uint64_t dst_len,
                           jxrb_submission **out) {
     TRY(check_session(s));
@@ -1165,11 +1326,12 @@ jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32
     const size_t lane = pick_stream(s);
     sub->stream = s->streams[lane];
     std::lock_guard<std::mutex> guard(s->lock);
-    CUDA_TRY(cudaEventCreate(&sub->begin), "cudaEventCreate");
-    CUDA_TRY(cudaEventCreate(&sub->launched), "cudaEventCreate");
+    sub->timed = true;
+    TRY(s->pool.take_event(true, sub->begin));
+    TRY(s->pool.take_event(true, sub->launched));
     CUDA_TRY(cudaEventRecord(sub->begin, sub->stream), "cudaEventRecord");
     if (!s->staging) s->staging.reset(new Staging);
-    TRY(build_device_set(plans, count, sub->stream, sub->set, s->staging.get(), &s->sides[lane]));
+    TRY(build_device_set(plans, count, sub->stream, sub->set, &s->sides[lane]));
     if (dst) {
         if (dst_len < sub->set.output_bytes) return fail(JXRB_INVALID_DESTINATION, "destination is smaller than the output");
         sub->output = static_cast<uint8_t *>(dst);
@@ -1178,12 +1340,11 @@ jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32
                  "cudaMallocAsync (output)");
         sub->output = static_cast<uint8_t *>(sub->owned_output);
     }
-    TRY(bind_output(sub->set, sub->output, sub->stream));
+    TRY(bind_output(sub->set, sub->output, sub->stream, &s->pool, s->staging.get()));
     TRY(upload_coefficients(sub->set, sub->stream, s->staging.get()));
     CUDA_TRY(cudaEventRecord(sub->launched, sub->stream), "cudaEventRecord");
     TRY(launch_set(s, sub->set, sub->stream));
-    CUDA_TRY(cudaEventCreate(&sub->done), "cudaEventCreate");
-    CUDA_TRY(cudaEventRecord(sub->done, sub->stream), "cudaEventRecord");
+    TRY(finish_submission(s, sub.get()));
     s->submissions++;
     s->uploaded += sub->set.upload_bytes;
     *out = sub.release();
@@ -1566,7 +1727,8 @@ jxrb_status jxrb_wait(jxrb_submission *sub, int64_t timeout_ns) {
     } else {
         CUDA_TRY(cudaEventSynchronize(sub->done), "cudaEventSynchronize");
     }
-    CUDA_TRY(cudaMemcpy(&sub->status_word, sub->set.status, sizeof(uint32_t), cudaMemcpyDeviceToHost), "status read");
+    if (sub->word) sub->status_word = *sub->word;
+    else CUDA_TRY(cudaMemcpy(&sub->status_word, sub->set.status, sizeof(uint32_t), cudaMemcpyDeviceToHost), "status read");
     sub->waited = true;
     sub->result = status_to_error(sub->status_word);
     return sub->result;
@@ -1621,12 +1783,12 @@ jxrb_status jxrb_readback_all(jxrb_submission *sub, void *host, uint64_t bytes) 
 void jxrb_submission_destroy(jxrb_submission *sub) {
     if (!sub) return;
     cudaSetDevice(sub->session->device);
-    if (sub->done) {
-        cudaEventSynchronize(sub->done);
-        cudaEventDestroy(sub->done);
-    }
-    if (sub->begin) cudaEventDestroy(sub->begin);
-    if (sub->launched) cudaEventDestroy(sub->launched);
+    SubmissionPool &pool = sub->session->pool;
+    if (sub->done) cudaEventSynchronize(sub->done);
+    pool.give_event(sub->timed, sub->done);
+    pool.give_event(true, sub->begin);
+    pool.give_event(true, sub->launched);
+    pool.give_word(sub->word);
     release_set(sub->set);
     if (sub->set.mem) cudaFreeAsync(sub->set.mem, sub->stream);
     if (sub->owned_output) cudaFreeAsync(sub->owned_output, sub->stream);
@@ -1636,7 +1798,25 @@ void jxrb_submission_destroy(jxrb_submission *sub) {
 jxrb_status jxrb_decode_to_host(jxrb_session *s, const jxrb_plan *plan, void *host, uint64_t bytes) {
     jxrb_submission *sub = nullptr;
     TRY(jxrb_submit(s, plan, &sub));
-    jxrb_status st = jxrb_readback(sub, 0, host, std::min<uint64_t>(bytes, plan->output_bytes));
+    const uint64_t n = std::min<uint64_t>(bytes, plan->output_bytes);
+    jxrb_status st = JXRB_OK;
+    // a small output comes back behind the kernels, with one wait for both
+    uint8_t *bounce = host && n <= SubmissionPool::kBytes ? s->pool.take_bounce() : nullptr;
+    if (bounce) {
+        const auto t0 = std::chrono::steady_clock::now();
+        cudaError_t e = cudaMemcpyAsync(bounce, sub->output, n, cudaMemcpyDeviceToHost, sub->stream);
+        const cudaError_t w = cudaStreamSynchronize(sub->stream);
+        if (e == cudaSuccess) e = w;
+        st = e == cudaSuccess ? jxrb_wait(sub, -1) : cuda_fail(e, "readback");
+        if (st == JXRB_OK) {
+            std::memcpy(host, bounce, n);
+            sub->readback_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
+            s->read_back += n;
+        }
+        s->pool.give_bounce(bounce);
+    } else {
+        st = jxrb_readback(sub, 0, host, n);
+    }
     jxrb_submission_destroy(sub);
     return st;
 }
@@ -1808,6 +1988,8 @@ jxrb_status jxrb_resident_create(jxrb_session *s, const jxrb_plan *const *plans,
     TRY(build_device_set(plans, count, st, r->set));
     r->singles.resize(count);
     for (uint32_t i = 0; i < count; i++) TRY(build_device_set(&plans[i], 1, st, r->singles[i]));
+    TRY(upload_blob(r->set, st));
+    for (DeviceSet &d : r->singles) TRY(upload_blob(d, st));
     TRY(upload_coefficients(r->set, st));
     for (DeviceSet &d : r->singles) TRY(upload_coefficients(d, st));
     CUDA_TRY(cudaStreamSynchronize(st), "resident upload");
@@ -2046,7 +2228,7 @@ jxrb_status build_request_set(jxrb_session *s, const jxrb_request *const *reqs, 
     set.counters = reinterpret_cast<uint32_t *>(base + counters_at);
     set.quarters = reinterpret_cast<QuarterImage *>(base + qimages_at);
     set.qplanes = reinterpret_cast<QuarterPlane *>(base + qplanes_at);
-    set.host_quarter.assign(q_end - q_at, 0);
+    set.host_blob.assign(q_end, 0);
     uint32_t qi = 0, qp = 0;
     set.host_items.resize(items);
     set.max_planes = 1;
@@ -2070,7 +2252,7 @@ jxrb_status build_request_set(jxrb_session *s, const jxrb_request *const *reqs, 
         im.out = r.out;
         if (r.denominator != 1) {
             const bool sixteenth = r.denominator == 16;
-            uint8_t *blob = set.host_quarter.data();
+            uint8_t *blob = set.host_blob.data() + q_at;
             QuarterImage &q = reinterpret_cast<QuarterImage *>(blob + (qimages_at - q_at))[qi++];
             q.image = i;
             q.first_plane = qp;
@@ -2150,14 +2332,7 @@ jxrb_status build_request_set(jxrb_session *s, const jxrb_request *const *reqs, 
             }
     }
     order_by_segment(set.host_items, set.bounds);
-    if (items)
-        CUDA_TRY(cudaMemcpyAsync(set.items, set.host_items.data(), sizeof(WorkItemHost) * items,
-                                 cudaMemcpyHostToDevice, stream), "upload work list");
-    if (!set.host_quarter.empty())
-        CUDA_TRY(cudaMemcpyAsync(base + q_at, set.host_quarter.data(), set.host_quarter.size(), cudaMemcpyHostToDevice,
-                                 stream), "upload quarter-resolution descriptors");
-    CUDA_TRY(cudaMemsetAsync(set.counters, 0, kCounterWords * sizeof(uint32_t), stream), "counter reset");
-    CUDA_TRY(cudaMemsetAsync(set.status, 0, sizeof(uint32_t), stream), "status reset");
+    if (items) std::memcpy(set.host_blob.data() + items_at, set.host_items.data(), sizeof(WorkItemHost) * items);
     TRY(s->sides[side_index].grow(side_streams(set)));
     set.sides = &s->sides[side_index];
     return JXRB_OK;
@@ -2464,10 +2639,9 @@ jxrb_status jxrb_submit_requests(jxrb_session *s, const jxrb_request *const *req
                  "cudaMallocAsync (output)");
         sub->output = static_cast<uint8_t *>(sub->owned_output);
     }
-    TRY(bind_output(sub->set, sub->output, sub->stream));
+    TRY(bind_output(sub->set, sub->output, sub->stream, &s->pool));
     TRY(launch_set(s, sub->set, sub->stream));
-    CUDA_TRY(cudaEventCreateWithFlags(&sub->done, cudaEventDisableTiming), "cudaEventCreate");
-    CUDA_TRY(cudaEventRecord(sub->done, sub->stream), "cudaEventRecord");
+    TRY(finish_submission(s, sub.get()));
     s->submissions++;
     *out = sub.release();
     return JXRB_OK;
