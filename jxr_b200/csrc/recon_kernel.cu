@@ -3083,27 +3083,36 @@ __device__ void interior_tile_chroma(const ImageDev &im, int tx, int ty, int32_t
             int32_t ch[2][4];
             const int ya = CV == 2 ? 8 + 2 * cy + ((r + 1) >> 1) : 2 + 4 * cy + r;
             const int row_a = (ya >> 2) * (kCB * kCPitch) + ((ya & 3) << 2);
-            const int row_b = ((ya + 1) >> 2) * (kCB * kCPitch) + (((ya + 1) & 3) << 2);
-            const int wa = (r & 1) ? 4 + cyc : cyc, wb = 8 - wa;
+            const int yb = CV == 2 ? ya + 1 : ya;
+            const int row_b = (yb >> 2) * (kCB * kCPitch) + ((yb & 3) << 2);
+            const int wa = CV == 4 ? 0 : (r & 1) ? 4 + cyc : cyc, wb = 8 - wa;
 #pragma unroll
             for (int pc = 0; pc < 2; pc++) {
                 const int32_t *t = ctile + pc * CT::kInts;
-                int32_t col[4];
-                const int2 a0 = *reinterpret_cast<const int2 *>(t + row_a + at0), a1 = *reinterpret_cast<const int2 *>(t + row_a + at1);
-                col[0] = a0.x; col[1] = a0.y; col[2] = a1.x; col[3] = a1.y;
+                const int2 b0 = *reinterpret_cast<const int2 *>(t + row_b + at0), b1 = *reinterpret_cast<const int2 *>(t + row_b + at1);
+                int32_t col[4] = {b0.x, b0.y, b1.x, b1.y};
                 if (!tile_small) m |= mag(col[0]) | mag(col[1]) | mag(col[2]) | mag(col[3]);
-                if (CV == 2) {
-                    const int2 b0 = *reinterpret_cast<const int2 *>(t + row_b + at0), b1 = *reinterpret_cast<const int2 *>(t + row_b + at1);
-                    if (!tile_small) m |= mag(b0.x) | mag(b0.y) | mag(b1.x) | mag(b1.y);
-                    col[0] = (col[0] * wa + b0.x * wb + 4) >> 3;
-                    col[1] = (col[1] * wa + b0.y * wb + 4) >> 3;
-                    col[2] = (col[2] * wa + b1.x * wb + 4) >> 3;
-                    col[3] = (col[3] * wa + b1.y * wb + 4) >> 3;
+                if (wa != 0) {   // (a weight of none leaves the other row as it is)
+                    const int2 a0 = *reinterpret_cast<const int2 *>(t + row_a + at0), a1 = *reinterpret_cast<const int2 *>(t + row_a + at1);
+                    if (!tile_small) m |= mag(a0.x) | mag(a0.y) | mag(a1.x) | mag(a1.y);
+                    col[0] = (a0.x * wa + col[0] * wb + 4) >> 3;
+                    col[1] = (a0.y * wa + col[1] * wb + 4) >> 3;
+                    col[2] = (a1.x * wa + col[2] * wb + 4) >> 3;
+                    col[3] = (a1.y * wa + col[3] * wb + 4) >> 3;
                 }
+                if (cxc == 0) {
+                    // the usual centering: a sample on each even column, the
+                    // rounded mean of two between
+                    ch[pc][0] = col[1];
+                    ch[pc][1] = (col[1] + col[2] + 1) >> 1;
+                    ch[pc][2] = col[2];
+                    ch[pc][3] = (col[2] + col[3] + 1) >> 1;
+                } else {
 #pragma unroll
-                for (int c = 0; c < 4; c++)
-                    ch[pc][c] = (c & 1) ? up_odd_small(col[1 + (c >> 1)], col[2 + (c >> 1)], cxc)
-                                        : up_even_small(col[(c >> 1)], col[1 + (c >> 1)], cxc);
+                    for (int c = 0; c < 4; c++)
+                        ch[pc][c] = (c & 1) ? up_odd_small(col[1 + (c >> 1)], col[2 + (c >> 1)], cxc)
+                                            : up_even_small(col[(c >> 1)], col[1 + (c >> 1)], cxc);
+                }
             }
             if (rgb8 && m < (1u << 28)) {
                 const ChannelScale &sc = o.ch[0];
