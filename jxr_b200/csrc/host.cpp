@@ -1148,7 +1148,9 @@ struct jxrb_session {
     std::atomic<uint32_t> next_stream{0};
     std::mutex lock;   // serialises encoding of submissions (runtime.rs:42)
     std::atomic<uint64_t> submissions{0}, uploaded{0}, read_back{0}, held{0}, launches{0};
-    SubmissionPool pool;
+    // kept by the session's submissions too: their status words and events are
+    // its, and a submission may be released after its session
+    std::shared_ptr<SubmissionPool> pool = std::make_shared<SubmissionPool>();
     std::unique_ptr<Staging> staging;  // pinned ring for pageable sources, made at the first submission (under `lock`)
     cudaStream_t upload = nullptr;     // uploads of resident images
 };
@@ -1174,6 +1176,8 @@ size_t pick_stream(jxrb_session *s) {
 
 struct jxrb_submission {
     jxrb_session *session = nullptr;
+    int device = 0;
+    std::shared_ptr<SubmissionPool> pool;   // the session's
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
     // device-timed stages of plan submissions (jxrb_submission_report):
@@ -1304,11 +1308,11 @@ jxrb_status status_to_error(uint32_t word) {
 // The end of a submission on its stream: the status word on its way to the
 // host, and the event that tells.
 jxrb_status finish_submission(jxrb_session *s, jxrb_submission *sub) {
-    sub->word = s->pool.take_word();
+    sub->word = s->pool->take_word();
     if (sub->word)
         CUDA_TRY(cudaMemcpyAsync(const_cast<uint32_t *>(sub->word), sub->set.status, sizeof(uint32_t),
                                  cudaMemcpyDeviceToHost, sub->stream), "status copy");
-    TRY(s->pool.take_event(sub->timed, sub->done));
+    TRY(s->pool->take_event(sub->timed, sub->done));
     CUDA_TRY(cudaEventRecord(sub->done, sub->stream), "cudaEventRecord");
     return JXRB_OK;
 }
@@ -1323,12 +1327,14 @@ jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32
         if (!plans[i]) return fail(JXRB_INVALID_PLAN, "null plan");
     std::unique_ptr<jxrb_submission> sub(new jxrb_submission);
     sub->session = s;
+    sub->device = s->device;
+    sub->pool = s->pool;
     const size_t lane = pick_stream(s);
     sub->stream = s->streams[lane];
     std::lock_guard<std::mutex> guard(s->lock);
     sub->timed = true;
-    TRY(s->pool.take_event(true, sub->begin));
-    TRY(s->pool.take_event(true, sub->launched));
+    TRY(s->pool->take_event(true, sub->begin));
+    TRY(s->pool->take_event(true, sub->launched));
     CUDA_TRY(cudaEventRecord(sub->begin, sub->stream), "cudaEventRecord");
     if (!s->staging) s->staging.reset(new Staging);
     TRY(build_device_set(plans, count, sub->stream, sub->set, &s->sides[lane]));
@@ -1340,7 +1346,7 @@ jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32
                  "cudaMallocAsync (output)");
         sub->output = static_cast<uint8_t *>(sub->owned_output);
     }
-    TRY(bind_output(sub->set, sub->output, sub->stream, &s->pool, s->staging.get()));
+    TRY(bind_output(sub->set, sub->output, sub->stream, s->pool.get(), s->staging.get()));
     TRY(upload_coefficients(sub->set, sub->stream, s->staging.get()));
     CUDA_TRY(cudaEventRecord(sub->launched, sub->stream), "cudaEventRecord");
     TRY(launch_set(s, sub->set, sub->stream));
@@ -1714,7 +1720,7 @@ jxrb_status jxrb_submit_batch(jxrb_session *s, const jxrb_plan *const *plans, ui
 jxrb_status jxrb_wait(jxrb_submission *sub, int64_t timeout_ns) {
     if (!sub) return fail(JXRB_INVALID_SUBMISSION_STATE, "null submission");
     if (sub->waited) return sub->result;
-    CUDA_TRY(cudaSetDevice(sub->session->device), "cudaSetDevice");
+    CUDA_TRY(cudaSetDevice(sub->device), "cudaSetDevice");
     if (timeout_ns >= 0) {
         const auto deadline = std::chrono::steady_clock::now() + std::chrono::nanoseconds(timeout_ns);
         for (;;) {
@@ -1782,8 +1788,8 @@ jxrb_status jxrb_readback_all(jxrb_submission *sub, void *host, uint64_t bytes) 
 
 void jxrb_submission_destroy(jxrb_submission *sub) {
     if (!sub) return;
-    cudaSetDevice(sub->session->device);
-    SubmissionPool &pool = sub->session->pool;
+    cudaSetDevice(sub->device);
+    SubmissionPool &pool = *sub->pool;
     if (sub->done) cudaEventSynchronize(sub->done);
     pool.give_event(sub->timed, sub->done);
     pool.give_event(true, sub->begin);
@@ -1801,7 +1807,7 @@ jxrb_status jxrb_decode_to_host(jxrb_session *s, const jxrb_plan *plan, void *ho
     const uint64_t n = std::min<uint64_t>(bytes, plan->output_bytes);
     jxrb_status st = JXRB_OK;
     // a small output comes back behind the kernels, with one wait for both
-    uint8_t *bounce = host && n <= SubmissionPool::kBytes ? s->pool.take_bounce() : nullptr;
+    uint8_t *bounce = host && n <= SubmissionPool::kBytes ? s->pool->take_bounce() : nullptr;
     if (bounce) {
         const auto t0 = std::chrono::steady_clock::now();
         cudaError_t e = cudaMemcpyAsync(bounce, sub->output, n, cudaMemcpyDeviceToHost, sub->stream);
@@ -1813,7 +1819,7 @@ jxrb_status jxrb_decode_to_host(jxrb_session *s, const jxrb_plan *plan, void *ho
             sub->readback_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
             s->read_back += n;
         }
-        s->pool.give_bounce(bounce);
+        s->pool->give_bounce(bounce);
     } else {
         st = jxrb_readback(sub, 0, host, n);
     }
@@ -2627,6 +2633,8 @@ jxrb_status jxrb_submit_requests(jxrb_session *s, const jxrb_request *const *req
     }
     std::unique_ptr<jxrb_submission> sub(new jxrb_submission);
     sub->session = s;
+    sub->device = s->device;
+    sub->pool = s->pool;
     const size_t k = pick_stream(s);
     sub->stream = s->streams[k];
     std::lock_guard<std::mutex> guard(s->lock);
@@ -2639,7 +2647,7 @@ jxrb_status jxrb_submit_requests(jxrb_session *s, const jxrb_request *const *req
                  "cudaMallocAsync (output)");
         sub->output = static_cast<uint8_t *>(sub->owned_output);
     }
-    TRY(bind_output(sub->set, sub->output, sub->stream, &s->pool));
+    TRY(bind_output(sub->set, sub->output, sub->stream, s->pool.get()));
     TRY(launch_set(s, sub->set, sub->stream));
     TRY(finish_submission(s, sub.get()));
     s->submissions++;
