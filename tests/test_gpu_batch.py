@@ -103,3 +103,71 @@ def test_autotuner_picks_a_candidate(session, batch, tmp_path, monkeypatch):
     stream.synchronize()
     check_all(dst.cpu().numpy(), plans, refs)
     res.close()
+
+
+@pytest.mark.parametrize("fmt", ["RGB", "YUV420", "YUV422", "GRAY", "RGBA"])
+@pytest.mark.parametrize("hard", [0, 1])
+def test_few_tiles_of_a_kind_and_more(session, fmt, hard):
+    """Sets with interior and edge tiles of one kind around the count at which
+    the two stop sharing a kernel (128 tiles): 32, 128, 160 and 32 tiles beside
+    another kind's."""
+    C, D, S, L = J.COLOR, J.DEPTH, J.STORE, J.LAYOUT
+    kw = dict(overlap=1, tile_width=9, tile_height=10, hard_tiles=hard)
+    w, h = 256, 512
+    if fmt == "GRAY":
+        im = J.synth(w, h, content=J.CONTENT["GRAY16"], color_format=C["LUMA"], quality=100, scaled=0, seed=3, **kw)
+        out = J.OutputFormat(C["LUMA"], D["U16"], S["U16"], L["LUMA"], w, h)
+    elif fmt == "RGBA":
+        im = J.synth(w, h, alpha_mode=J.ALPHA["INTEGRATED"], quality=80, alpha_overlap=1, seed=4, **kw)
+        out = J.OutputFormat(C["RGB"], D["U8"], S["U8"], L["RGBA"], w, h, alpha_bit_depth=D["U8"])
+    else:
+        colour = C["YUV444" if fmt == "RGB" else fmt]
+        im = J.synth(w, h, color_format=colour, quality=80, seed=5, **kw)
+        out = J.OutputFormat(C["RGB"], D["U8"], S["U8"], L["RGB"], w, h)
+    other = J.synth(w, h, content=J.CONTENT["GRAY16"] if fmt != "GRAY" else J.CONTENT["PHOTO_RGB8"],
+                    color_format=C["LUMA" if fmt != "GRAY" else "YUV444"], quality=100 if fmt != "GRAY" else 80,
+                    scaled=int(fmt == "GRAY"), seed=6, **kw)
+    other_out = (J.OutputFormat(C["LUMA"], D["U16"], S["U16"], L["LUMA"], w, h) if fmt != "GRAY" else
+                 J.OutputFormat(C["RGB"], D["U8"], S["U8"], L["RGB"], w, h))
+    rc, ref = decode_synth(im, out, threads=8)
+    rc2, ref2 = decode_synth(other, other_out, threads=8)
+    assert rc == 0 and rc2 == 0
+    plan = J.CudaDecodePlan(im.arena, im.geometry, out)
+    plan2 = J.CudaDecodePlan(other.arena, other.geometry, other_out)
+    for n, beside in ((1, 0), (4, 0), (5, 0), (1, 1)):
+        sub = session.submit_batch([plan] * n + [plan2] * beside)
+        sub.wait()
+        for i in range(n):
+            assert np.array_equal(sub.readback(i), ref), (n, i)
+        for i in range(beside):
+            assert np.array_equal(sub.readback(n + i), ref2)
+        sub.close()
+
+
+def test_submissions_in_flight_and_small_outputs(session):
+    """More submissions at once than the session keeps upload buffers for, one
+    whose descriptors fill more than a buffer, outputs around the size that
+    comes back through page-locked memory, and callers on several threads."""
+    from concurrent.futures import ThreadPoolExecutor
+    C, D, S, L = J.COLOR, J.DEPTH, J.STORE, J.LAYOUT
+    refs, plans = [], []
+    for w, h in ((256, 256), (255, 256), (257, 256), (33, 17)):
+        im = J.synth(w, h, quality=75, overlap=1, seed=50 + w)
+        out = J.OutputFormat(C["RGB"], D["U8"], S["U8"], L["RGBX"], w, h)
+        rc, ref = decode_synth(im, out, threads=8)
+        assert rc == 0
+        refs.append(ref)
+        plans.append(J.CudaDecodePlan(im.arena, im.geometry, out))
+    assert plans[0].output_bytes() == 256 << 10
+    subs = [session.submit(plans[i % 4]) for i in range(40)]
+    for i, sub in enumerate(subs):
+        sub.wait()
+        assert np.array_equal(sub.readback(), refs[i % 4])
+        sub.close()
+    many = session.submit_batch([plans[3]] * 600)
+    many.wait()
+    assert all(np.array_equal(many.readback(i), refs[3]) for i in (0, 1, 299, 598, 599))
+    many.close()
+    with ThreadPoolExecutor(8) as pool:
+        got = list(pool.map(lambda i: session.decode_to_host(plans[i % 4]), range(64)))
+    assert all(np.array_equal(g, refs[i % 4]) for i, g in enumerate(got))

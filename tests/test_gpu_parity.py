@@ -357,6 +357,41 @@ def test_yuv422_tiles(session, size, overlap, tiles):
     check(session, rnd, rgb8(w, h), expect_ok=False)
 
 
+@pytest.mark.parametrize("case", ["rgb8", "gray", "half"])
+@pytest.mark.parametrize("x", [0, 1, 2, 3])
+def test_pixel_rows_of_every_output_form(session, case, x):
+    """Rows that start and end at every byte offset, over interior and edge
+    tiles: packed RGB8; one channel of 8, 16 and 32 bits with shifts up; half
+    floats and their binary32 forms, packed and in planes, in both channel
+    orders, with alpha and without, at odd widths."""
+    w, h = 173 + x, 150
+    if case == "rgb8":
+        img = J.synth(240, 208, quality=85, overlap=2, seed=400 + x)
+        for layout in ("RGB", "BGR"):
+            check(session, img, J.OutputFormat(C_["RGB"], D["U8"], S["U8"], L[layout], w, h, crop_x=x, crop_y=3))
+    elif case == "gray":
+        img = J.synth(240, 208, content=J.CONTENT["GRAY16"], color_format=C_["LUMA"], quality=100, scaled=0,
+                      overlap=1, seed=410 + x)
+        for depth, shift in (("U8", 0), ("U16", 0), ("U16", 1), ("U16", 7), ("I32", 0), ("I32", 5), ("F16", 0)):
+            extra = {} if depth in ("U8", "F16") else dict(shift_bits=shift)
+            check(session, img, J.OutputFormat(C_["LUMA"], D[depth], S[depth], L["LUMA"], w, h, crop_x=x, **extra),
+                  expect_ok=False)
+    else:
+        img = J.synth(240, 208, content=J.CONTENT["HDR_HALF"], alpha_mode=A["SEPARATE"], scaled=0, quality=0,
+                      qp=(4, 8, 16), overlap=2, alpha_overlap=1, seed=420 + x)
+        plain = J.synth(240, 208, content=J.CONTENT["HDR_HALF"], scaled=0, quality=0, qp=(4, 8, 16), overlap=1,
+                        seed=430 + x)
+        for nchw in (0, 1):
+            for widen in (0, 1):
+                for layout in ("RGBA", "BGRA"):
+                    check(session, img, J.OutputFormat(C_["RGB"], D["F16"], S["F16"], L[layout], w, h, crop_x=x,
+                                                       alpha_bit_depth=D["F16"], nchw=nchw, widen_f16=widen),
+                          expect_ok=False)
+                for layout in ("RGB", "BGR"):
+                    check(session, plain, J.OutputFormat(C_["RGB"], D["F16"], S["F16"], L[layout], w, h, crop_x=x,
+                                                         nchw=nchw, widen_f16=widen), expect_ok=False)
+
+
 def test_edge_tiles_overflow(session):
     img = J.synth(208, 176, quality=75, overlap=2, seed=140)
     img.arena.coefficients[:64] = 2**30
