@@ -18,7 +18,7 @@ import os
 from pathlib import Path
 from typing import Dict, List, Optional, Sequence, Tuple
 
-INTERIOR_CTAS = (1, 2, 3)   # the interior kernels fit 3 CTAs an SM
+INTERIOR_CTAS = (1, 2, 3)   # what the full-resolution interior kernels fit an SM (4:2:0's fits 4)
 OTHER_CTAS = (1, 2)         # the general kernel fits 2
 
 

@@ -70,6 +70,25 @@ def test_pixel_kernels_at_tile_edges(torch, orientation, pixel_bytes, offsets):
 
 
 @pytest.mark.parametrize("orientation", range(8))
+@pytest.mark.parametrize("pixel_bytes,sizes,offsets", [
+    (1, [(1023, 1025), (1024, 1024), (65, 16191), (16231, 65), (1089, 1027)], (0, 1, 3)),
+    (2, [(1279, 1024), (1280, 1024), (65, 20223), (20233, 65), (1281, 1027)], (0, 1, 2)),
+    (3, [(767, 512), (768, 512), (63, 6301), (6303, 65), (705, 631)], (0, 1, 2, 3))])
+def test_small_and_large_surfaces_of_small_pixels(torch, orientation, pixel_bytes, sizes, offsets):
+    """Either side of the extent from which 1- to 3-byte pixels take the kernel
+    compiled for them, and beyond it rows and columns one more and one less than
+    whole tiles, on surfaces that start at every byte of a word."""
+    rng = np.random.default_rng(pixel_bytes * 8 + orientation)
+    for width, height in sizes:
+        src = rng.integers(0, 256, width * height * pixel_bytes, dtype=np.uint8)
+        rc, want = O.orient(src, width, height, pixel_bytes, orientation)
+        assert rc == 0
+        for offset in offsets:
+            got = gpu_orient(torch, src, width, height, pixel_bytes, orientation, offset)
+            assert np.array_equal(got, want), (width, height, offset)
+
+
+@pytest.mark.parametrize("orientation", range(8))
 def test_bit_packed_orientation_matches_the_oracle(torch, orientation):
     rng = np.random.default_rng(orientation)
     for width, height in [(3, 2), (9, 17), (70, 33)]:
