@@ -156,7 +156,7 @@ constexpr int kSegmentOther = kSegments - 1;
 // segment then holds their hard tiles alone.  The one-plane kernel stays small
 // enough with them (2047 x 1535 16-bit gray 13.5 us apart, 12.1 folded); in the
 // others their code costs every interior tile more fetches than the launch
-// saves (4096 x 4096 RGB8 129.7 us folded, 126.4 apart; 3999 x 2999 4:2:0 95.0
+// saves (4096 x 4096 RGB8 127.8 us folded, 120.1 apart; 3999 x 2999 4:2:0 95.0
 // and 87.5).
 constexpr bool kFoldEdges[kKinds] = {true, false, false, false, false, false};
 // Up to this many tiles of a kind in a set, its interior tiles run in the edge
