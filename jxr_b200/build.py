@@ -24,7 +24,7 @@ CSRC = PKG / "csrc"
 LIB = PKG / "libjxr_b200.so"
 SYNTH_LIB = PKG / "libjxr_synth.so"
 SOURCES = ["recon_kernel.cu", "static_scratch.cu", "orient.cu", "analysis.cu", "host.cpp", "sample_scale.cpp"]
-HEADERS = ["engine.h", "lifting.cuh", "forward.h", "sample_scale.h"]
+HEADERS = ["engine.h", "lifting.cuh", "forward.h", "sample_scale.h", "orient_tile.h"]
 SYNTH_SOURCES = ["synth.cpp"]
 SYNTH_HEADERS = ["synth.h", "forward.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]

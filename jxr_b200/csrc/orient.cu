@@ -14,6 +14,7 @@
 #include <cstdint>
 
 #include "../../include/jxr_b200.h"
+#include "orient_tile.h"
 
 namespace jxr {
 jxrb_status report_error(jxrb_status s, const char *why);
@@ -22,26 +23,11 @@ jxrb_status report_cuda(cudaError_t e, const char *what);
 
 namespace {
 
+using jxr::source_of;
+using jxr::swaps_axes;
+
 constexpr int kTile = 32;
 constexpr uint32_t kMaxPixelBytes = 48;   // a 32 x 32 tile of them fills 48 KB of shared memory
-
-__device__ __forceinline__ bool swaps_axes(int o) { return o >= JXRB_ORIENT_TRANSPOSE; }
-
-// source_coordinates (orientation.rs:193-211): the source pixel of
-// destination pixel (dx, dy) of a w x h source.
-__device__ __forceinline__ void source_of(int o, uint32_t w, uint32_t h, uint32_t dx, uint32_t dy, uint32_t &sx,
-                                          uint32_t &sy) {
-    switch (o) {
-    case JXRB_ORIENT_MIRROR_HORIZONTAL: sx = w - 1 - dx; sy = dy; break;
-    case JXRB_ORIENT_ROTATE180: sx = w - 1 - dx; sy = h - 1 - dy; break;
-    case JXRB_ORIENT_MIRROR_VERTICAL: sx = dx; sy = h - 1 - dy; break;
-    case JXRB_ORIENT_TRANSPOSE: sx = dy; sy = dx; break;
-    case JXRB_ORIENT_ROTATE90: sx = dy; sy = h - 1 - dx; break;
-    case JXRB_ORIENT_TRANSVERSE: sx = w - 1 - dy; sy = h - 1 - dx; break;
-    case JXRB_ORIENT_ROTATE270: sx = w - 1 - dy; sy = dx; break;
-    default: sx = dx; sy = dy;
-    }
-}
 
 // One destination tile of 32 x 32 pixels, `words` words of type W a pixel.
 // The source pixels of a tile form a rectangle of at most 32 x 32 (every
@@ -117,34 +103,31 @@ __global__ void __launch_bounds__(256) jxrb_orient_pixels(const uint8_t *__restr
     uint8_t *const in = reinterpret_cast<uint8_t *>(in_words);
     uint8_t *const outb = reinterpret_cast<uint8_t *>(out_words);
     const bool swap = swaps_axes(o);
-    const uint32_t ow = swap ? h : w, oh = swap ? w : h;
+    const uint32_t ow = swap ? h : w;
     const uint32_t dx0 = blockIdx.x * T, dy0 = blockIdx.y * T;
-    const int dw = (int)(min(dx0 + T, ow) - dx0), dh = (int)(min(dy0 + T, oh) - dy0);
-    // the source rectangle: the extremes of the tile's corners
-    uint32_t ax, ay, bx, by;
-    source_of(o, w, h, dx0, dy0, ax, ay);
-    source_of(o, w, h, dx0 + dw - 1, dy0 + dh - 1, bx, by);
-    const uint32_t sx0 = min(ax, bx), sy0 = min(ay, by);
-    const int sw = swap ? dh : dw, sh = swap ? dw : dh;
+    const jxr::OrientTile tile = jxr::orient_tile(o, w, h, T, dx0, dy0);
+    const int dw = tile.dw, dh = tile.dh, sw = tile.sw, sh = tile.sh;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // pass 1: a lane's words of all its rows are loaded before the first is
     // stored, so that they are in flight together (one row at a time, with the
     // rows' ends by the byte, took 88 us: a chain of load latencies).  A word
-    // may hold bytes of the neighbouring pixels too; only a tile at one of the
-    // surface's two ends, where it could reach outside, checks its words.
+    // may hold bytes of the neighbouring pixels too; a tile whose first or last
+    // word reaches outside the surface (words_inside) reads it by the byte.
     // A warp's rows are eight apart, so they all start at the same byte of a
     // word.
     constexpr int kRowWords = U == 4 ? T * PB / 4 : T * PB / 4 + 1, kLaneWords = (kRowWords + 31) / 32;
     const size_t pitch = (size_t)w * PB;
-    const uint8_t *first = src + sy0 * pitch + (size_t)sx0 * PB;
-    const bool ends = (sx0 == 0 && sy0 == 0) || (sx0 + sw == w && sy0 + sh == h);
+    const size_t offset = tile.sy0 * pitch + (size_t)tile.sx0 * PB;
+    const uint8_t *first = src + offset;
+    // (units of whole words start and end on their boundaries)
+    const bool by_word = U == 4 || jxr::words_inside(reinterpret_cast<uintptr_t>(src), h * pitch, offset, pitch, sw * PB, sh);
     const int a = (int)(reinterpret_cast<uintptr_t>(first) & 3);
     const int S = T * PB + 4 + (int)(pitch & 3);
     {
         const int mis = (a + warp * S) & 3, n = mis + sw * PB;
         const uint8_t *row = first + warp * pitch - mis;
         uint32_t held[T / 8][kLaneWords];
-        if (U == 4 || !ends) {
+        if (by_word) {
 #pragma unroll
             for (int j = 0; j < T / 8; j++, row += 8 * pitch)
 #pragma unroll
@@ -160,7 +143,7 @@ __global__ void __launch_bounds__(256) jxrb_orient_pixels(const uint8_t *__restr
                 }
             }
         }
-        if (U == 4 || !ends) {
+        if (by_word) {
             uint32_t *to = in_words + ((a + warp * S) >> 2) + lane;
 #pragma unroll
             for (int j = 0; j < T / 8; j++, to += 2 * S)

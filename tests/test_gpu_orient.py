@@ -89,6 +89,25 @@ def test_small_and_large_surfaces_of_small_pixels(torch, orientation, pixel_byte
 
 
 @pytest.mark.parametrize("orientation", range(8))
+@pytest.mark.parametrize("pixel_bytes,sizes,offsets", [
+    (1, [(1100003, 1), (1, 1100003), (2, 600001), (600001, 2), (65, 16200), (66, 16200)], (0, 1, 2, 3)),
+    (2, [(1400003, 1), (1, 1400003), (2, 700001), (65, 20300)], (0, 2)),
+    (3, [(400003, 1), (1, 400003), (2, 200001), (65, 6100)], (0, 1, 3))])
+def test_narrow_surfaces_of_small_pixels(torch, orientation, pixel_bytes, sizes, offsets):
+    """Surfaces one and two pixels wide or high, and one and two pixels wider
+    than a tile, of the extents the kernels of 1- to 3-byte pixels take: the
+    tiles whose aligned words would reach outside the surface."""
+    rng = np.random.default_rng(pixel_bytes * 8 + orientation)
+    for width, height in sizes:
+        src = rng.integers(0, 256, width * height * pixel_bytes, dtype=np.uint8)
+        rc, want = O.orient(src, width, height, pixel_bytes, orientation)
+        assert rc == 0
+        for offset in offsets:
+            got = gpu_orient(torch, src, width, height, pixel_bytes, orientation, offset)
+            assert np.array_equal(got, want), (width, height, offset)
+
+
+@pytest.mark.parametrize("orientation", range(8))
 def test_bit_packed_orientation_matches_the_oracle(torch, orientation):
     rng = np.random.default_rng(orientation)
     for width, height in [(3, 2), (9, 17), (70, 33)]:
