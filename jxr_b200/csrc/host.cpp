@@ -695,11 +695,10 @@ public:
             CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDefault, stream), "upload (page-locked source)");
             return JXRB_OK;
         }
-        if (!slots_[0].host) {
-            for (Slot &sl : slots_) {
-                CUDA_TRY(cudaHostAlloc(&sl.host, kChunk, cudaHostAllocDefault), "cudaHostAlloc (staging)");
+        for (Slot &sl : slots_) {   // each made once; one that was refused is asked for again
+            if (!sl.host) CUDA_TRY(cudaHostAlloc(&sl.host, kChunk, cudaHostAllocDefault), "cudaHostAlloc (staging)");
+            if (!sl.done)
                 CUDA_TRY(cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming), "cudaEventCreate (staging)");
-            }
         }
         const uint8_t *sp = static_cast<const uint8_t *>(src);
         for (size_t off = 0; off < bytes; off += kChunk) {

@@ -1,0 +1,89 @@
+"""The engine's host code (csrc/host.cpp) against a CUDA runtime on host memory
+(tests/_fake_cuda.cpp): what it does when a call fails, in which order it queues
+and waits, and what it leaves behind."""
+import ctypes as C
+import shutil
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+import jxr_b200 as J
+from jxr_b200 import api
+
+ROOT = Path(__file__).resolve().parents[1]
+CSRC = ROOT / "jxr_b200" / "csrc"
+CUDA = next((p for p in (Path(shutil.which("nvcc") or "/x/x").resolve().parents[1] / "include",
+                         Path("/usr/local/cuda/include")) if (p / "cuda_runtime.h").exists()), None)
+STREAMS, EVENTS, DEVICE, PINNED = range(4)
+C_, D, S, L = J.COLOR, J.DEPTH, J.STORE, J.LAYOUT
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    out = tmp_path_factory.mktemp("fake_cuda") / "libjxr_fake.so"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-I", str(CUDA), "-I", str(ROOT / "include"),
+                    "-I", str(CSRC), str(CSRC / "host.cpp"), str(CSRC / "sample_scale.cpp"),
+                    str(ROOT / "tests" / "_fake_cuda.cpp"), "-o", str(out)], check=True)
+    lib = C.CDLL(str(out))
+    for name, (res, args) in api.EXPORTS.items():
+        if hasattr(lib, name):
+            fn = getattr(lib, name)
+            fn.restype, fn.argtypes = res, args
+    lib.fake_log.restype = C.c_char_p
+    lib.fake_live.restype = C.c_long
+    lib.fake_fail.argtypes = [C.c_char_p, C.c_int]
+    return lib
+
+
+@pytest.fixture
+def fake(fake_lib, monkeypatch):
+    monkeypatch.setenv("JXRB_STAGING_THREADS", "1")
+    monkeypatch.setattr(api, "_lib", fake_lib)
+    fake_lib.fake_reset()
+    yield fake_lib
+    fake_lib.fake_reset()
+
+
+def live(lib):
+    return [lib.fake_live(k) for k in (STREAMS, EVENTS, DEVICE, PINNED)]
+
+
+def log(lib):
+    return lib.fake_log().decode().splitlines()
+
+
+def rgb_plan(w, h, **kw):
+    img = J.synth(w, h, quality=70, overlap=1, seed=9, threads=4, **kw)
+    return J.CudaDecodePlan(img.arena, img.geometry, J.OutputFormat(C_["RGB"], D["U8"], S["U8"], L["RGB"], w, h))
+
+
+def one_kernel_plan():
+    return rgb_plan(64, 64)
+
+
+@pytest.mark.parametrize("call", ["cudaHostAlloc", "cudaEventCreateWithFlags"])
+def test_uploads_survive_a_refused_buffer_or_event(fake, call):
+    """One refused page-locked buffer or event fails at most its own
+    submission: the session's next one uploads from pageable memory again."""
+    plan = one_kernel_plan()
+    refused = 0
+    for after in range(12):
+        session = J.CudaDecoderSession(0, streams=1)
+        fake.fake_reset()
+        fake.fake_fail(call.encode(), after)
+        try:
+            session.submit(plan).close()
+        except J.CudaError as e:
+            assert e.kind == "Driver"
+            refused += 1
+        fake.fake_reset()
+        for _ in range(2):
+            sub = session.submit(plan)
+            sub.wait()
+            sub.close()
+        assert not any(line.startswith("bad") for line in log(fake)), (after, log(fake))
+        session.close()
+    assert refused > 0
+    plan.close()
