@@ -869,12 +869,19 @@ struct Sides {
 
     jxrb_status grow(int n) {
         if (n > 0 && !fork) CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming), "cudaEventCreate");
+        // a stream and its event are kept together or not at all
+        streams.reserve(std::max<size_t>(streams.size(), (size_t)n));
+        joins.reserve(streams.capacity());
         while ((int)streams.size() < n) {
             cudaStream_t st = nullptr;
             cudaEvent_t e = nullptr;
             CUDA_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "cudaStreamCreate");
+            const cudaError_t made = cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+            if (made != cudaSuccess) {
+                cudaStreamDestroy(st);
+                return cuda_fail(made, "cudaEventCreate");
+            }
             streams.push_back(st);
-            CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
             joins.push_back(e);
         }
         return JXRB_OK;

@@ -87,3 +87,36 @@ def test_uploads_survive_a_refused_buffer_or_event(fake, call):
         session.close()
     assert refused > 0
     plan.close()
+
+
+# 4:2:2 keeps its interior and edge tiles in kernels of their own, so the set
+# takes a side stream
+def two_kernel_plan():
+    return rgb_plan(1024, 1024, color_format=C_["YUV422"])
+
+
+@pytest.mark.parametrize("call", ["cudaStreamCreateWithFlags", "cudaEventCreateWithFlags"])
+def test_side_streams_survive_a_refused_handle(fake, call):
+    """One refused stream or event fails its submission alone: the session's
+    next one finds each side stream with its event."""
+    plan = two_kernel_plan()
+    refused = 0
+    for after in range(8):
+        session = J.CudaDecoderSession(0, streams=1)
+        fake.fake_reset()
+        fake.fake_fail(call.encode(), after)
+        try:
+            session.submit(plan).close()
+        except J.CudaError as e:
+            assert e.kind == "Driver"
+            refused += 1
+        fake.fake_reset()
+        for _ in range(2):
+            sub = session.submit(plan)
+            sub.wait()
+            sub.close()
+        assert any(line.startswith("launch on 2") for line in log(fake))
+        assert not any(line.startswith("bad") for line in log(fake)), (after, log(fake))
+        session.close()
+    assert refused > 0
+    plan.close()
