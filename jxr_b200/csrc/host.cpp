@@ -1147,16 +1147,31 @@ jxrb_status bind_output(DeviceSet &set, uint8_t *dst, cudaStream_t stream, Submi
 // ---------------------------------------------------------------------------
 // session / submission objects
 // ---------------------------------------------------------------------------
-struct jxrb_session {
+// What a session's submissions use until they are released, which may be after
+// their session: held by the session and by each of its submissions.
+struct SessionLanes {
     int device = 0;
     std::vector<cudaStream_t> streams;
-    std::vector<Sides> sides;   // per stream: requests' kernels run on them beside it (under `lock`)
+    std::vector<Sides> sides;   // per stream: submissions' kernels run on them beside it (under the session's lock)
+    SubmissionPool pool;        // their status words and events
+    std::atomic<uint64_t> read_back{0};
+
+    ~SessionLanes() {
+        cudaSetDevice(device);
+        for (cudaStream_t st : streams) cudaStreamSynchronize(st);
+        for (Sides &sd : sides) sd.release();
+        for (cudaStream_t st : streams) cudaStreamDestroy(st);
+    }
+};
+
+struct jxrb_session {
+    int device = 0;
+    std::shared_ptr<SessionLanes> lanes = std::make_shared<SessionLanes>();
+    std::vector<cudaStream_t> &streams = lanes->streams;
+    std::vector<Sides> &sides = lanes->sides;
     std::atomic<uint32_t> next_stream{0};
     std::mutex lock;   // serialises encoding of submissions (runtime.rs:42)
-    std::atomic<uint64_t> submissions{0}, uploaded{0}, read_back{0}, held{0}, launches{0};
-    // kept by the session's submissions too: their status words and events are
-    // its, and a submission may be released after its session
-    std::shared_ptr<SubmissionPool> pool = std::make_shared<SubmissionPool>();
+    std::atomic<uint64_t> submissions{0}, uploaded{0}, held{0}, launches{0};
     std::unique_ptr<Staging> staging;  // pinned ring for pageable sources, made at the first submission (under `lock`)
     cudaStream_t upload = nullptr;     // uploads of resident images
 };
@@ -1181,9 +1196,7 @@ size_t pick_stream(jxrb_session *s) {
 }  // namespace
 
 struct jxrb_submission {
-    jxrb_session *session = nullptr;
-    int device = 0;
-    std::shared_ptr<SubmissionPool> pool;   // the session's
+    std::shared_ptr<SessionLanes> lanes;    // the session's
     cudaStream_t stream = nullptr;
     cudaEvent_t done = nullptr;
     // device-timed stages of plan submissions (jxrb_submission_report):
@@ -1199,6 +1212,23 @@ struct jxrb_submission {
     uint32_t status_word = 0;
     volatile uint32_t *word = nullptr;   // the session's, which the status is copied to before `done`
     bool timed = false;                  // plan submissions' events have timing
+    bool queued = false;                 // `done` is recorded behind all of it
+
+    jxrb_submission(jxrb_session *s, size_t lane) : lanes(s->lanes), stream(s->streams[lane]) {}
+    jxrb_submission(const jxrb_submission &) = delete;
+    // Gives back what it holds once its work is over; of a submission that
+    // failed on the way too, whose copies may still be running.
+    ~jxrb_submission() {
+        cudaSetDevice(lanes->device);
+        if (queued) cudaEventSynchronize(done);
+        else cudaStreamSynchronize(stream);
+        lanes->pool.give_event(timed, done);
+        lanes->pool.give_event(true, begin);
+        lanes->pool.give_event(true, launched);
+        lanes->pool.give_word(word);
+        if (set.mem) cudaFreeAsync(set.mem, stream);
+        if (owned_output) cudaFreeAsync(owned_output, stream);
+    }
 };
 
 struct jxrb_resident {
@@ -1313,13 +1343,15 @@ jxrb_status status_to_error(uint32_t word) {
 
 // The end of a submission on its stream: the status word on its way to the
 // host, and the event that tells.
-jxrb_status finish_submission(jxrb_session *s, jxrb_submission *sub) {
-    sub->word = s->pool->take_word();
+jxrb_status finish_submission(jxrb_submission *sub) {
+    SubmissionPool &pool = sub->lanes->pool;
+    sub->word = pool.take_word();
     if (sub->word)
         CUDA_TRY(cudaMemcpyAsync(const_cast<uint32_t *>(sub->word), sub->set.status, sizeof(uint32_t),
                                  cudaMemcpyDeviceToHost, sub->stream), "status copy");
-    TRY(s->pool->take_event(sub->timed, sub->done));
+    TRY(pool.take_event(sub->timed, sub->done));
     CUDA_TRY(cudaEventRecord(sub->done, sub->stream), "cudaEventRecord");
+    sub->queued = true;
     return JXRB_OK;
 }
 
@@ -1331,16 +1363,12 @@ jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32
     if (count > kImageMask) return fail(JXRB_RESOURCE_LIMIT, "too many images in one launch");
     for (uint32_t i = 0; i < count; i++)
         if (!plans[i]) return fail(JXRB_INVALID_PLAN, "null plan");
-    std::unique_ptr<jxrb_submission> sub(new jxrb_submission);
-    sub->session = s;
-    sub->device = s->device;
-    sub->pool = s->pool;
     const size_t lane = pick_stream(s);
-    sub->stream = s->streams[lane];
+    std::unique_ptr<jxrb_submission> sub(new jxrb_submission(s, lane));
     std::lock_guard<std::mutex> guard(s->lock);
     sub->timed = true;
-    TRY(s->pool->take_event(true, sub->begin));
-    TRY(s->pool->take_event(true, sub->launched));
+    TRY(s->lanes->pool.take_event(true, sub->begin));
+    TRY(s->lanes->pool.take_event(true, sub->launched));
     CUDA_TRY(cudaEventRecord(sub->begin, sub->stream), "cudaEventRecord");
     if (!s->staging) s->staging.reset(new Staging);
     TRY(build_device_set(plans, count, sub->stream, sub->set, &s->sides[lane]));
@@ -1352,11 +1380,11 @@ jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32
                  "cudaMallocAsync (output)");
         sub->output = static_cast<uint8_t *>(sub->owned_output);
     }
-    TRY(bind_output(sub->set, sub->output, sub->stream, s->pool.get(), s->staging.get()));
+    TRY(bind_output(sub->set, sub->output, sub->stream, &s->lanes->pool, s->staging.get()));
     TRY(upload_coefficients(sub->set, sub->stream, s->staging.get()));
     CUDA_TRY(cudaEventRecord(sub->launched, sub->stream), "cudaEventRecord");
     TRY(launch_set(s, sub->set, sub->stream));
-    TRY(finish_submission(s, sub.get()));
+    TRY(finish_submission(sub.get()));
     s->submissions++;
     s->uploaded += sub->set.upload_bytes;
     *out = sub.release();
@@ -1608,7 +1636,7 @@ jxrb_status jxrb_session_create(int ordinal, const jxrb_session_options *options
         }
     }
     std::unique_ptr<jxrb_session> s(new jxrb_session);
-    s->device = ordinal;
+    s->device = s->lanes->device = ordinal;
     const uint32_t streams = options && options->streams ? options->streams : 4;
     for (uint32_t i = 0; i < streams; i++) {
         cudaStream_t st;
@@ -1625,19 +1653,17 @@ void jxrb_session_destroy(jxrb_session *s) {
     if (!s) return;
     cudaSetDevice(s->device);
     for (cudaStream_t st : s->streams) cudaStreamSynchronize(st);
-    for (Sides &sd : s->sides) sd.release();
     if (s->upload) cudaStreamSynchronize(s->upload);
     s->staging.reset();
-    for (cudaStream_t st : s->streams) cudaStreamDestroy(st);
     if (s->upload) cudaStreamDestroy(s->upload);
-    delete s;
+    delete s;   // its streams go with the last of its submissions
 }
 
 jxrb_status jxrb_session_diagnostics(const jxrb_session *s, jxrb_diagnostics *out) {
     if (!s || !out) return fail(JXRB_INVALID_SUBMISSION_STATE, "null argument");
     out->submissions = s->submissions;
     out->bytes_uploaded = s->uploaded;
-    out->bytes_read_back = s->read_back;
+    out->bytes_read_back = s->lanes->read_back;
     out->device_bytes_held = s->held;
     out->kernel_launches = s->launches;
     out->bytes_staged = s->staging ? s->staging->staged_bytes() : 0;
@@ -1726,7 +1752,7 @@ jxrb_status jxrb_submit_batch(jxrb_session *s, const jxrb_plan *const *plans, ui
 jxrb_status jxrb_wait(jxrb_submission *sub, int64_t timeout_ns) {
     if (!sub) return fail(JXRB_INVALID_SUBMISSION_STATE, "null submission");
     if (sub->waited) return sub->result;
-    CUDA_TRY(cudaSetDevice(sub->device), "cudaSetDevice");
+    CUDA_TRY(cudaSetDevice(sub->lanes->device), "cudaSetDevice");
     if (timeout_ns >= 0) {
         const auto deadline = std::chrono::steady_clock::now() + std::chrono::nanoseconds(timeout_ns);
         for (;;) {
@@ -1777,7 +1803,7 @@ jxrb_status jxrb_readback(jxrb_submission *sub, uint32_t index, void *host, uint
     const auto t0 = std::chrono::steady_clock::now();
     CUDA_TRY(cudaMemcpy(host, sub->output + sub->set.output_offsets[index], bytes, cudaMemcpyDeviceToHost), "readback");
     sub->readback_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    sub->session->read_back += bytes;
+    sub->lanes->read_back += bytes;
     return JXRB_OK;
 }
 
@@ -1788,24 +1814,11 @@ jxrb_status jxrb_readback_all(jxrb_submission *sub, void *host, uint64_t bytes) 
     const auto t0 = std::chrono::steady_clock::now();
     CUDA_TRY(cudaMemcpy(host, sub->output, bytes, cudaMemcpyDeviceToHost), "readback");
     sub->readback_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-    sub->session->read_back += bytes;
+    sub->lanes->read_back += bytes;
     return JXRB_OK;
 }
 
-void jxrb_submission_destroy(jxrb_submission *sub) {
-    if (!sub) return;
-    cudaSetDevice(sub->device);
-    SubmissionPool &pool = *sub->pool;
-    if (sub->done) cudaEventSynchronize(sub->done);
-    pool.give_event(sub->timed, sub->done);
-    pool.give_event(true, sub->begin);
-    pool.give_event(true, sub->launched);
-    pool.give_word(sub->word);
-    release_set(sub->set);
-    if (sub->set.mem) cudaFreeAsync(sub->set.mem, sub->stream);
-    if (sub->owned_output) cudaFreeAsync(sub->owned_output, sub->stream);
-    delete sub;
-}
+void jxrb_submission_destroy(jxrb_submission *sub) { delete sub; }
 
 jxrb_status jxrb_decode_to_host(jxrb_session *s, const jxrb_plan *plan, void *host, uint64_t bytes) {
     jxrb_submission *sub = nullptr;
@@ -1813,7 +1826,7 @@ jxrb_status jxrb_decode_to_host(jxrb_session *s, const jxrb_plan *plan, void *ho
     const uint64_t n = std::min<uint64_t>(bytes, plan->output_bytes);
     jxrb_status st = JXRB_OK;
     // a small output comes back behind the kernels, with one wait for both
-    uint8_t *bounce = host && n <= SubmissionPool::kBytes ? s->pool->take_bounce() : nullptr;
+    uint8_t *bounce = host && n <= SubmissionPool::kBytes ? s->lanes->pool.take_bounce() : nullptr;
     if (bounce) {
         const auto t0 = std::chrono::steady_clock::now();
         cudaError_t e = cudaMemcpyAsync(bounce, sub->output, n, cudaMemcpyDeviceToHost, sub->stream);
@@ -1823,9 +1836,9 @@ jxrb_status jxrb_decode_to_host(jxrb_session *s, const jxrb_plan *plan, void *ho
         if (st == JXRB_OK) {
             std::memcpy(host, bounce, n);
             sub->readback_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-            s->read_back += n;
+            s->lanes->read_back += n;
         }
-        s->pool->give_bounce(bounce);
+        s->lanes->pool.give_bounce(bounce);
     } else {
         st = jxrb_readback(sub, 0, host, n);
     }
@@ -2637,12 +2650,8 @@ jxrb_status jxrb_submit_requests(jxrb_session *s, const jxrb_request *const *req
         if (!reqs[i]) return fail(JXRB_INVALID_PLAN, "null request");
         if (reqs[i]->image->session != s) return fail(JXRB_INVALID_PLAN, "request on another session's image");
     }
-    std::unique_ptr<jxrb_submission> sub(new jxrb_submission);
-    sub->session = s;
-    sub->device = s->device;
-    sub->pool = s->pool;
     const size_t k = pick_stream(s);
-    sub->stream = s->streams[k];
+    std::unique_ptr<jxrb_submission> sub(new jxrb_submission(s, k));
     std::lock_guard<std::mutex> guard(s->lock);
     TRY(build_request_set(s, reqs, count, k, sub->stream, sub->set));
     if (dst) {
@@ -2653,9 +2662,9 @@ jxrb_status jxrb_submit_requests(jxrb_session *s, const jxrb_request *const *req
                  "cudaMallocAsync (output)");
         sub->output = static_cast<uint8_t *>(sub->owned_output);
     }
-    TRY(bind_output(sub->set, sub->output, sub->stream, s->pool.get()));
+    TRY(bind_output(sub->set, sub->output, sub->stream, &s->lanes->pool));
     TRY(launch_set(s, sub->set, sub->stream));
-    TRY(finish_submission(s, sub.get()));
+    TRY(finish_submission(sub.get()));
     s->submissions++;
     *out = sub.release();
     return JXRB_OK;

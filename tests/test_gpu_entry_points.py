@@ -228,3 +228,24 @@ def test_pageable_arena_is_consumed_before_submit_returns(session, image):
     after = session.diagnostics()
     assert np.array_equal(got, want)
     assert after["bytes_staged"] - before["bytes_staged"] < coeff.nbytes   # tables only
+
+
+def test_submissions_outlive_their_session(image):
+    """A session closed before its submissions: they wait, read back and free
+    their memory all the same, and a later session finds that memory free."""
+    import torch
+    img, out, want = image
+    plan = J.CudaDecodePlan(img.arena, img.geometry, out)
+    free = []
+    for _ in range(4):
+        s = J.CudaDecoderSession(0)
+        subs = [s.submit(plan) for _ in range(6)]
+        s.close()
+        for sub in subs:
+            sub.wait()
+            assert np.array_equal(sub.readback(0), want)
+        for sub in subs:
+            sub.close()
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert min(free[1:]) >= free[0] - (2 << 20)

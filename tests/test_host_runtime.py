@@ -42,8 +42,18 @@ def fake(fake_lib, monkeypatch):
     monkeypatch.setenv("JXRB_STAGING_THREADS", "1")
     monkeypatch.setattr(api, "_lib", fake_lib)
     fake_lib.fake_reset()
+    opened = []
+
+    class Session(J.CudaDecoderSession):
+        def __init__(self, *args, **kw):
+            super().__init__(*args, **kw)
+            opened.append(self)
+
+    monkeypatch.setattr(J, "CudaDecoderSession", Session)
     yield fake_lib
     fake_lib.fake_reset()
+    for s in opened:      # while the library is still this one
+        s.close()
 
 
 def live(lib):
@@ -119,4 +129,57 @@ def test_side_streams_survive_a_refused_handle(fake, call):
         assert not any(line.startswith("bad") for line in log(fake)), (after, log(fake))
         session.close()
     assert refused > 0
+    plan.close()
+
+
+def test_submissions_outlive_their_session(fake):
+    """A submission released after its session still waits, reads back and
+    frees its memory on a live stream; then nothing is left."""
+    before = live(fake)
+    plan, small = two_kernel_plan(), one_kernel_plan()
+    session = J.CudaDecoderSession(0)
+    subs = [session.submit(plan), session.submit(small), session.submit_batch([small, plan])]
+    session.close()
+    for k, sub in enumerate(subs):
+        sub.wait()
+        assert sub.is_complete()
+        assert sub.readback(0).size == (plan, small, small)[k].output_bytes()
+        assert sub.report()["selected"] == "Cuda"
+        sub.close()
+    assert not any(line.startswith("bad") for line in log(fake)), log(fake)
+    assert live(fake) == before
+    plan.close()
+    small.close()
+
+
+@pytest.mark.parametrize("call", ["cudaMallocAsync", "cudaMemcpyAsync", "cudaEventRecord", "cudaStreamWaitEvent", "launch_tiles"])
+def test_failed_submissions_leave_nothing(fake, call):
+    """A submission that fails at any of its calls gives back its memory,
+    events and status word; so does one that is refused."""
+    before = live(fake)
+    plan = two_kernel_plan()
+    refused = 0
+    for after in range(8):
+        session = J.CudaDecoderSession(0, streams=1)
+        for _ in range(10):             # what a session makes once
+            session.submit(plan).close()
+        fake.fake_reset()
+        kept = live(fake)
+        fake.fake_fail(call.encode(), after)
+        try:
+            session.submit(plan).close()
+        except J.CudaError as e:
+            assert e.kind == "Driver"
+            refused += 1
+        fake.fake_reset()
+        assert live(fake)[DEVICE] == kept[DEVICE] and live(fake)[EVENTS] == kept[EVENTS]
+        buf = np.empty(16, np.uint8)
+        with pytest.raises(J.CudaError) as e:
+            session.submit_into(plan, buf.ctypes.data, 16)
+        assert e.value.kind == "InvalidDestination"
+        assert live(fake) == kept
+        session.close()
+        assert not any(line.startswith("bad") for line in log(fake))
+    assert refused > 0
+    assert live(fake) == before
     plan.close()
