@@ -795,6 +795,7 @@ public:
         return b;
     }
     void give_bounce(uint8_t *b) {
+        if (!b) return;
         std::lock_guard<std::mutex> guard(lock_);
         free_bounces_.push_back(b);
     }
@@ -1212,6 +1213,7 @@ struct jxrb_submission {
     uint32_t status_word = 0;
     volatile uint32_t *word = nullptr;   // the session's, which the status is copied to before `done`
     bool timed = false;                  // plan submissions' events have timing
+    uint8_t *bounce = nullptr;           // the session's, which a small output is copied to before `done`
     bool queued = false;                 // `done` is recorded behind all of it
 
     jxrb_submission(jxrb_session *s, size_t lane) : lanes(s->lanes), stream(s->streams[lane]) {}
@@ -1226,6 +1228,7 @@ struct jxrb_submission {
         lanes->pool.give_event(true, begin);
         lanes->pool.give_event(true, launched);
         lanes->pool.give_word(word);
+        lanes->pool.give_bounce(bounce);
         if (set.mem) cudaFreeAsync(set.mem, stream);
         if (owned_output) cudaFreeAsync(owned_output, stream);
     }
@@ -1341,22 +1344,28 @@ jxrb_status status_to_error(uint32_t word) {
     return fail(JXRB_KERNEL_ARITHMETIC, buf);
 }
 
-// The end of a submission on its stream: the status word on its way to the
-// host, and the event that tells.
-jxrb_status finish_submission(jxrb_submission *sub) {
+// The end of a submission on its stream: the status word and, where they fit a
+// buffer of the session's, the first `host_bytes` of the output on their way to
+// the host, and the event that tells.  The copies are queued here, under the
+// session's lock, so that no other submission's work comes between.
+jxrb_status finish_submission(jxrb_submission *sub, uint64_t host_bytes = 0) {
     SubmissionPool &pool = sub->lanes->pool;
     sub->word = pool.take_word();
     if (sub->word)
         CUDA_TRY(cudaMemcpyAsync(const_cast<uint32_t *>(sub->word), sub->set.status, sizeof(uint32_t),
                                  cudaMemcpyDeviceToHost, sub->stream), "status copy");
+    if (host_bytes > 0 && host_bytes <= SubmissionPool::kBytes && (sub->bounce = pool.take_bounce()))
+        CUDA_TRY(cudaMemcpyAsync(sub->bounce, sub->output, host_bytes, cudaMemcpyDeviceToHost, sub->stream), "readback");
     TRY(pool.take_event(sub->timed, sub->done));
     CUDA_TRY(cudaEventRecord(sub->done, sub->stream), "cudaEventRecord");
     sub->queued = true;
     return JXRB_OK;
 }
 
+// `host_bytes`: bytes of the output the caller wants on the host at once
+// (finish_submission).
 jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32_t count, void *dst, uint64_t dst_len,
-                          jxrb_submission **out) {
+                          jxrb_submission **out, uint64_t host_bytes = 0) {
     TRY(check_session(s));
     if (!out) return fail(JXRB_INVALID_SUBMISSION_STATE, "null submission out-pointer");
     if (count == 0) return fail(JXRB_INVALID_PLAN, "empty batch");
@@ -1384,7 +1393,7 @@ jxrb_status submit_common(jxrb_session *s, const jxrb_plan *const *plans, uint32
     TRY(upload_coefficients(sub->set, sub->stream, s->staging.get()));
     CUDA_TRY(cudaEventRecord(sub->launched, sub->stream), "cudaEventRecord");
     TRY(launch_set(s, sub->set, sub->stream));
-    TRY(finish_submission(sub.get()));
+    TRY(finish_submission(sub.get(), host_bytes));
     s->submissions++;
     s->uploaded += sub->set.upload_bytes;
     *out = sub.release();
@@ -1822,25 +1831,15 @@ void jxrb_submission_destroy(jxrb_submission *sub) { delete sub; }
 
 jxrb_status jxrb_decode_to_host(jxrb_session *s, const jxrb_plan *plan, void *host, uint64_t bytes) {
     jxrb_submission *sub = nullptr;
-    TRY(jxrb_submit(s, plan, &sub));
-    const uint64_t n = std::min<uint64_t>(bytes, plan->output_bytes);
-    jxrb_status st = JXRB_OK;
+    const uint64_t n = plan ? std::min<uint64_t>(bytes, plan->output_bytes) : 0;
     // a small output comes back behind the kernels, with one wait for both
-    uint8_t *bounce = host && n <= SubmissionPool::kBytes ? s->lanes->pool.take_bounce() : nullptr;
-    if (bounce) {
-        const auto t0 = std::chrono::steady_clock::now();
-        cudaError_t e = cudaMemcpyAsync(bounce, sub->output, n, cudaMemcpyDeviceToHost, sub->stream);
-        const cudaError_t w = cudaStreamSynchronize(sub->stream);
-        if (e == cudaSuccess) e = w;
-        st = e == cudaSuccess ? jxrb_wait(sub, -1) : cuda_fail(e, "readback");
-        if (st == JXRB_OK) {
-            std::memcpy(host, bounce, n);
-            sub->readback_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-            s->lanes->read_back += n;
-        }
-        s->lanes->pool.give_bounce(bounce);
-    } else {
+    TRY(submit_common(s, &plan, 1, nullptr, 0, &sub, host ? n : 0));
+    jxrb_status st;
+    if (!sub->bounce) {
         st = jxrb_readback(sub, 0, host, n);
+    } else if ((st = jxrb_wait(sub, -1)) == JXRB_OK) {
+        std::memcpy(host, sub->bounce, n);
+        sub->lanes->read_back += n;
     }
     jxrb_submission_destroy(sub);
     return st;

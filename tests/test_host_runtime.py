@@ -183,3 +183,23 @@ def test_failed_submissions_leave_nothing(fake, call):
     assert refused > 0
     assert live(fake) == before
     plan.close()
+
+
+def test_small_outputs_are_queued_with_their_submission(fake):
+    """decode_to_host of a small picture queues the copy of its pixels ahead of
+    its own event and waits for that event alone: work that other callers queue
+    on the stream afterwards is not waited for."""
+    plan = one_kernel_plan()
+    session = J.CudaDecoderSession(0, streams=1)
+    session.decode_to_host(plan)
+    fake.fake_reset()
+    session.decode_to_host(plan)
+    lines = log(fake)
+    copy = next(k for k, line in enumerate(lines) if line.startswith(f"copy device to pinned {plan.output_bytes()} on"))
+    done = next(k for k in range(len(lines) - 1, -1, -1) if lines[k].startswith("record"))
+    assert copy < done, lines
+    assert f"wait event {lines[done].split()[1]}" in lines[done:]
+    assert not any(line.startswith("wait stream") for line in lines), lines
+    assert session.diagnostics()["bytes_read_back"] == 2 * plan.output_bytes()
+    session.close()
+    plan.close()
