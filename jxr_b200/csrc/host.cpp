@@ -711,9 +711,10 @@ public:
             CUDA_TRY(cudaEventRecord(sl.done, stream), "staging slot event");
             sl.pending = true;
         }
-        staged_ += bytes;
         return JXRB_OK;
     }
+    // the diagnostics' count of uploaded bytes that came from pageable memory
+    void count(uint64_t bytes) { staged_ += bytes; }
     uint64_t staged_bytes() const { return staged_; }
 
 private:
@@ -1095,9 +1096,11 @@ jxrb_status upload_coefficients(DeviceSet &set, cudaStream_t stream, Staging *st
     uint8_t *base = static_cast<uint8_t *>(set.mem);
     for (const DeviceSet::CoefficientCopy &c : set.coefficient_copies) {
         if (c.bytes == 0) continue;
-        if (staging) TRY(staging->upload(base + c.at, c.src, c.bytes, stream));
+        bool direct = false;
+        if (staging) TRY(staging->upload(base + c.at, c.src, c.bytes, stream, &direct));
         else CUDA_TRY(cudaMemcpyAsync(base + c.at, c.src, c.bytes, cudaMemcpyHostToDevice, stream), "upload coefficients");
         set.upload_bytes += c.bytes;
+        if (staging && !direct) staging->count(c.bytes);
     }
     set.coefficient_copies.clear();
     return JXRB_OK;
@@ -1131,6 +1134,7 @@ jxrb_status bind_output(DeviceSet &set, uint8_t *dst, cudaStream_t stream, Submi
     if (pool && pool->upload(to, from, bytes, stream, sent)) TRY(sent);
     else if (staging) TRY(staging->upload(to, from, bytes, stream));
     else CUDA_TRY(cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, stream), "upload descriptors");
+    if (staging && !set.host_blob.empty()) staging->count(set.upload_bytes);   // the tables: what of the blob is the plans'
     // (a pageable source has been read when the copy returns)
     std::vector<uint8_t>().swap(set.host_blob);
     for (size_t i = 0; i < set.host_images.size(); i++) {

@@ -203,3 +203,37 @@ def test_small_outputs_are_queued_with_their_submission(fake):
     assert session.diagnostics()["bytes_read_back"] == 2 * plan.output_bytes()
     session.close()
     plan.close()
+
+
+@pytest.mark.parametrize("side", [64, 2048])
+def test_staged_bytes_are_uploaded_bytes(fake, side):
+    """bytes_staged is the part of bytes_uploaded that came from pageable
+    memory: all of it for a pageable arena, whichever page-locked buffer the
+    tables went through (2048 x 2048: more than one of the small ones holds),
+    and the tables alone for a page-locked one."""
+    img = J.synth(side, side, quality=70, overlap=1, seed=9, threads=4)
+    out = J.OutputFormat(C_["RGB"], D["U8"], S["U8"], L["RGB"], side, side)
+    session = J.CudaDecoderSession(0)
+    plan = J.CudaDecodePlan(img.arena, img.geometry, out)
+    for _ in range(2):
+        before = session.diagnostics()
+        session.decode_to_host(plan)
+        after = session.diagnostics()
+        uploaded = after["bytes_uploaded"] - before["bytes_uploaded"]
+        assert after["bytes_staged"] - before["bytes_staged"] == uploaded > img.arena.coefficients.nbytes
+    plan.close()
+    # the same arena in page-locked memory
+    a, p = img.arena, C.c_void_p()
+    fake.cudaHostAlloc(C.byref(p), C.c_size_t(a.coefficients.nbytes), 0)
+    pinned = np.ctypeslib.as_array(C.cast(p, C.POINTER(C.c_int32)), (a.coefficients.size,))
+    pinned[:] = a.coefficients
+    plan = J.CudaDecodePlan(J.Arena(pinned, a.coefficient_offsets, a.quantizers, a.bands, a.hp_predictions, a.coded_x, a.coded_y,
+                                    a.planes), img.geometry, out)
+    before = session.diagnostics()
+    session.decode_to_host(plan)
+    after = session.diagnostics()
+    assert after["bytes_uploaded"] - before["bytes_uploaded"] == uploaded
+    assert after["bytes_staged"] - before["bytes_staged"] == uploaded - pinned.nbytes
+    session.close()
+    plan.close()
+    fake.cudaFreeHost(p)
