@@ -3184,11 +3184,10 @@ __device__ __forceinline__ void hold_image(const ImageDev *__restrict__ images, 
 
 // Tiles of YUV 4:2:0 (CV 2) and 4:2:2 (CV 4) images: interior (MODE 0), edge
 // (MODE 1) or both (MODE 2).
-// Four 4:2:0 interior tiles an SM (64 registers, a few spilled), three edge
-// tiles and three of 4:2:2's larger ones: 3999 x 2999 4:2:0 87.1 us, the mixed
-// batch 127.6, against 89.0 and 129.6 with three of each.
-template <int MODE, int CV>
-__global__ void __launch_bounds__(kThreads, CV == 2 && MODE == 0 ? 4 : 3)
+// CTAS: tiles an SM, three, or four 4:2:0 interior tiles (64 registers, a few
+// spilled) in the launches that kManyTiles says.
+template <int MODE, int CV, int CTAS = 3>
+__global__ void __launch_bounds__(kThreads, CTAS)
 jxrb_interior_chroma_tiles(const ImageDev *__restrict__ images, const WorkItem *__restrict__ items, uint32_t item_count,
                        uint32_t *status, uint32_t *counters) {
     extern __shared__ __align__(16) int32_t smem_chroma[];
@@ -3293,13 +3292,33 @@ static TileKernel interior_kernel() {
     else return jxrb_interior_tiles<NP, 0>;
 }
 
-static TileKernel segment_kernel(int segment) {
-    switch (segment) {
+// From this many tiles on, 4:2:0 interior tiles run four CTAs an SM instead of
+// three.  The fourth hides more of the latency of coefficients that come from
+// HBM, at 64 registers and spills that make each tile slower: pictures whose
+// coefficients stay in L2, or few tiles, lose by it.  One picture replayed, us
+// at three and four: 1920 x 1088 30.3, 39.3; 2048 x 1536 33.3, 45.8; 3072 x 2048
+// 54.3, 61.9; 4096 x 3072 102.2, 110.9.  Read from HBM: 2048 x 1536 48.6, 50.7;
+// 3840 x 2880 112.4, 109; 3999 x 2999 120, 116; 4096 x 3072 122, 120.  Pictures in
+// turn on several streams: 2501 x 1901 40.4, 42.6; 3999 x 2999 88.4, 85.0; a mixed
+// batch 128.4, 125.6.
+constexpr uint32_t kManyTiles = 2560;
+
+// Kernels by index: one a segment, then the 4:2:0 interior kernel of many tiles.
+constexpr int kKernelMany420 = kSegments;
+constexpr int kKernels = kSegments + 1;
+
+static int kernel_of(int segment, uint32_t tiles) {
+    return segment == 4 && tiles >= kManyTiles ? kKernelMany420 : segment;
+}
+
+static TileKernel tile_kernel(int kernel) {
+    switch (kernel) {
+    case kKernelMany420: return jxrb_interior_chroma_tiles<0, 2, 4>;
     case 0: return interior_kernel<1>();
     case 1: return interior_kernel<2>();
     case 2: return interior_kernel<3>();
     case 3: return interior_kernel<4>();
-    case 4: return jxrb_interior_chroma_tiles<kFoldEdges[4] ? 2 : 0, 2>;
+    case 4: return jxrb_interior_chroma_tiles<0, 2>;
     case 5: return jxrb_interior_chroma_tiles<0, 4>;
     case 6: return jxrb_interior_tiles<1, 1>;
     case 7: return jxrb_interior_tiles<2, 1>;
@@ -3333,23 +3352,23 @@ static size_t segment_smem_bytes(int segment, int max_planes) {
     return tile_smem_bytes(max_planes);
 }
 
-// What the launcher learns about a device once: its SM count, which segment
+// What the launcher learns about a device once: its SM count, which tile
 // kernels have their dynamic shared-memory limit raised on it (a function
-// attribute holds per device), and how many CTAs of each segment kernel fit
+// attribute holds per device), and how many CTAs of each kernel fit
 // an SM at each plane count.  Guarded by a lock: sessions on several threads
 // and devices launch concurrently.
 struct DeviceLaunchState {
     int sms = 0;
-    bool configured[kSegments] = {};
-    int fit[kSegments][JXRB_MAX_PLANES + 1] = {};
+    bool configured[kKernels] = {};
+    int fit[kKernels][JXRB_MAX_PLANES + 1] = {};
 };
 constexpr int kMaxLaunchDevices = 64;
 static DeviceLaunchState g_launch_state[kMaxLaunchDevices];
 static std::mutex g_launch_lock;
 
-// SM count and CTAs per SM of segment `seg` at `planes` planes on the current
+// SM count and CTAs per SM of kernel `index` at `planes` planes on the current
 // device, raising the kernel's shared-memory limit there first.
-static cudaError_t segment_fit(int seg, int planes, size_t smem, int &sms, int &fit) {
+static cudaError_t kernel_fit(int index, int planes, size_t smem, int &sms, int &fit) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -3360,13 +3379,13 @@ static cudaError_t segment_fit(int seg, int planes, size_t smem, int &sms, int &
         e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
         if (e != cudaSuccess) return e;
     }
-    TileKernel k = segment_kernel(seg);
-    if (!d.configured[seg]) {
+    TileKernel k = tile_kernel(index);
+    if (!d.configured[index]) {
         e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem_bytes(JXRB_MAX_PLANES));
         if (e != cudaSuccess) return e;
-        d.configured[seg] = true;
+        d.configured[index] = true;
     }
-    int &f = d.fit[seg][planes];
+    int &f = d.fit[index][planes];
     if (f == 0 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, k, kThreads, smem) != cudaSuccess || f < 1)) {
         cudaGetLastError();
         f = 1;
@@ -3390,11 +3409,12 @@ cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32
                                                                                           : seg0 - (kSegmentOther - kSideSegment0) - 1;
         const uint32_t count = bounds[seg + 1] - bounds[seg];
         if (count == 0) continue;
-        TileKernel k = segment_kernel(seg);
+        const int index = kernel_of(seg, count);
+        TileKernel k = tile_kernel(index);
         const int planes = segment_planes(seg, max_planes);
         const size_t smem = segment_smem_bytes(seg, max_planes);
         int sms = 0, fit = 0;
-        cudaError_t fe = segment_fit(seg, planes, smem, sms, fit);
+        cudaError_t fe = kernel_fit(index, planes, smem, sms, fit);
         if (fe != cudaSuccess) return fe;
         int per_sm = fit;
         const int slot = seg == kSegmentOther ? 4 : planes - 1;   // entry of the launch tuning

@@ -171,3 +171,20 @@ def test_submissions_in_flight_and_small_outputs(session):
     with ThreadPoolExecutor(8) as pool:
         got = list(pool.map(lambda i: session.decode_to_host(plans[i % 4]), range(64)))
     assert all(np.array_equal(g, refs[i % 4]) for i, g in enumerate(got))
+
+
+@pytest.mark.parametrize("fmt,copies", [("YUV420", 39), ("YUV420", 40)])
+def test_many_tiles_of_a_kind(session, fmt, copies):
+    """Either side of the number of interior tiles from which the 4:2:0 kernel
+    runs more CTAs an SM (64 of them in a picture of 640 x 640)."""
+    img = J.synth(637, 640, color_format=J.COLOR[fmt], quality=80, overlap=1, tile_width=9, tile_height=7, seed=41,
+                  threads=8)
+    out = J.OutputFormat(J.COLOR["RGB"], J.DEPTH["U8"], J.STORE["U8"], J.LAYOUT["RGB"], 637, 640)
+    rc, want = decode_synth(img, out, threads=8)
+    assert rc == 0
+    plan = J.CudaDecodePlan(img.arena, img.geometry, out)
+    sub = session.submit_batch([plan] * copies)
+    sub.wait()
+    for k in range(copies):
+        assert np.array_equal(sub.readback(k), want), k
+    sub.close()
