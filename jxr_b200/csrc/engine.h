@@ -152,13 +152,23 @@ constexpr int kSideSegment0 = kKinds;          // segments run beside the interi
 constexpr int kSegments = 2 * kKinds + 1;
 constexpr int kSegmentOther = kSegments - 1;
 // Edge tiles that the interior kernel of the same images takes instead of an
-// edge kernel (one launch, edge tiles first in it), by kind; their edge
-// segment then holds their hard tiles alone.  The one-plane kernel stays small
-// enough with them (2047 x 1535 16-bit gray 13.5 us apart, 12.1 folded); in the
-// others their code costs every interior tile more fetches than the launch
-// saves (4096 x 4096 RGB8 127.8 us folded, 120.1 apart; 3999 x 2999 4:2:0 95.0
-// and 87.5).
-constexpr bool kFoldEdges[kKinds] = {true, false, false, false, false, false};
+// edge kernel ("folded": one launch, edge tiles first in it), by kind, bit
+// kind - 1.  One plane: always; its kernel stays small enough with them (2047 x
+// 1535 16-bit gray 13.5 us apart, 12.1 folded).  Three planes: in sets of fewer
+// than kApartTiles tiles of theirs, and wherever the kernels run one after
+// another on one stream, unless some of the tiles meet a hard boundary (the edge
+// kernel then runs anyway).  Folded, the edge tiles' code costs every interior
+// tile more fetches; apart, their kernel, the fork and the join cost a set that
+// runs alone more than that.  RGB8 4:4:4, two overlap levels, us folded and
+// apart: alone, from HBM, 1920 x 1088 41.9, 50.8; 2501 x 1901 66.6, 82.2; 3072 x
+// 2048 67.6, 81.7; 3840 x 2880 104, 114; 4096 x 3072 115, 122; pictures in turn
+// on one stream 37.3, 39.0; 61.8, 76.9; 63.2, 75.9; 99.3, 107.9; 110, 115; in
+// turn on several streams 2048 x 1536 27.6, 26.8; 2501 x 1901 45.3, 42.7; 3072 x
+// 2048 51.7, 49.4; 4096 x 4096 131, 124; 8192 x 8192 512, 473.  (Always folded
+// before, in a larger kernel: alone 49.2, 76.8, 74.7, 117, 129.)  The
+// others' are never folded (3999 x 2999 4:2:0 95.0 us folded, 87.5 apart).
+constexpr uint32_t kFoldAlways = 1u << 0, kFoldSome = 1u << 2;
+constexpr uint32_t kApartTiles = 2560;
 // Up to this many tiles of a kind in a set, its interior tiles run in the edge
 // kernel with the others: one launch, no fork and join.  64 tiles (512 x 512)
 // of RGB8 4:4:4, 4:2:0, RGBA: 11.3, 11.4, 11.4 us in two kernels, 10.0, 10.3,
@@ -189,6 +199,7 @@ struct StagedLayout {
     size_t status_at;
     size_t counters_at;
     uint32_t bounds[kSegments + 1];   // work-list segment boundaries
+    uint32_t folded;         // kinds whose edge tiles are folded
     int max_planes;
     uint64_t clear_bytes;    // output bytes to zero before the launch (1-bit outputs), else 0
 };

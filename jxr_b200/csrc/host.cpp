@@ -29,7 +29,7 @@
 
 namespace jxr {
 size_t tile_smem_bytes(int planes);
-cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32_t *bounds, int max_planes,
+cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32_t *bounds, uint32_t folded, int max_planes,
                          uint32_t *status, uint32_t *counters, const cudaStream_t *lanes, int lane_count,
                          const LaunchTuning *tune);
 int tile_mbs();
@@ -146,43 +146,53 @@ uint32_t tile_tag(uint32_t kind, uint32_t tx, uint32_t ty, uint32_t T, uint32_t 
     return (hard ? kTagHard : kTagEdge) + kind;
 }
 
-// Work-list segment of a tag (engine.h).  Folded edge tiles (kFoldEdges) go
-// to their interior kernel's segment -- one kernel, so that their latency
-// hides among the interior tiles -- ahead of its interior tiles.
-bool folded_edge_tag(uint32_t tag) {
-    return tag > kTagEdge && tag <= kTagHard && kFoldEdges[tag - kTagEdge - 1];
+// Where a set's tiles run, by kind (bit kind - 1): whose edge tiles the
+// interior kernel takes (engine.h), and whose interior tiles the edge kernel
+// does: kinds of no more than kMergeTiles tiles for which both would run.
+// `count`: tiles by tag; `one_stream`: the kernels run one after another.
+struct TileRoutes {
+    uint32_t folded = 0, merged = 0;
+};
+TileRoutes tile_routes(const uint32_t *count, bool one_stream) {
+    TileRoutes r;
+    for (uint32_t k = 1; k <= (uint32_t)kKinds; k++) {
+        const uint32_t bit = 1u << (k - 1), inner = count[k], hard = count[kTagHard + k];
+        uint32_t edge = count[kTagEdge + k];
+        const bool few = one_stream || inner + edge < kApartTiles;
+        if ((kFoldAlways & bit) || ((kFoldSome & bit) && edge > 0 && hard == 0 && few)) {
+            r.folded |= bit;
+            edge = 0;
+        }
+        edge += hard;
+        if (inner > 0 && edge > 0 && inner + edge <= kMergeTiles) r.merged |= bit;
+    }
+    return r;
 }
-// `merged`: the kinds (bit kind - 1) whose interior tiles run in the edge
-// kernel (merged_kinds).
-int segment_of_tag(uint32_t tag, uint32_t merged) {
+
+// Whether a tag is that of folded edge tiles: they go to their interior
+// kernel's segment -- one kernel, so that their latency hides among the
+// interior tiles -- ahead of its interior tiles.
+bool folded_edge_tag(uint32_t tag, const TileRoutes &r) {
+    return tag > kTagEdge && tag <= kTagHard && (r.folded >> (tag - kTagEdge - 1)) & 1;
+}
+// Work-list segment of a tag (engine.h).
+int segment_of_tag(uint32_t tag, const TileRoutes &r) {
     if (tag == 0) return kSegmentOther;
     if (tag > kTagHard) return kSideSegment0 + (int)(tag - kTagHard) - 1;
-    if (tag > kTagEdge) return folded_edge_tag(tag) ? (int)(tag - kTagEdge) - 1 : (int)tag - 1;
-    return (merged >> (tag - 1)) & 1 ? kSideSegment0 + (int)tag - 1 : (int)tag - 1;
+    if (tag > kTagEdge) return folded_edge_tag(tag, r) ? (int)(tag - kTagEdge) - 1 : (int)tag - 1;
+    return (r.merged >> (tag - 1)) & 1 ? kSideSegment0 + (int)tag - 1 : (int)tag - 1;
 }
-
-// The kinds whose interior and edge kernels would both run, over no more than
-// kMergeTiles tiles together.  `count`: tiles by tag.
-uint32_t merged_kinds(const uint32_t *count) {
-    uint32_t merged = 0;
-    for (uint32_t k = 1; k <= (uint32_t)kKinds; k++) {
-        const uint32_t edge = (folded_edge_tag(kTagEdge + k) ? 0 : count[kTagEdge + k]) + count[kTagHard + k];
-        if (count[k] > 0 && edge > 0 && count[k] + edge <= kMergeTiles) merged |= 1u << (k - 1);
-    }
-    return merged;
-}
-
-int rank_of_tag(uint32_t tag) { return folded_edge_tag(tag) ? 0 : 1; }
 
 // Stable order of a work list by segment (a counting sort: one pass to count,
 // one to place); `bounds` receives the kSegments + 1 segment boundaries.
-void order_by_segment(std::vector<WorkItemHost> &items, uint32_t *bounds) {
+// Returns the kinds whose edge tiles are folded.
+uint32_t order_by_segment(std::vector<WorkItemHost> &items, uint32_t *bounds) {
     uint32_t tags[kTags] = {};
     for (const WorkItemHost &w : items) tags[w.image >> kTagShift]++;
-    const uint32_t merged = merged_kinds(tags);
+    const TileRoutes routes = tile_routes(tags, false);
     auto key = [&](const WorkItemHost &w) {
         const uint32_t tag = w.image >> kTagShift;
-        return segment_of_tag(tag, merged) * 2 + rank_of_tag(tag);
+        return segment_of_tag(tag, routes) * 2 + (folded_edge_tag(tag, routes) ? 0 : 1);
     };
     uint32_t cursor[2 * kSegments] = {};
     for (const WorkItemHost &w : items) cursor[key(w)]++;
@@ -197,6 +207,7 @@ void order_by_segment(std::vector<WorkItemHost> &items, uint32_t *bounds) {
     std::vector<WorkItemHost> sorted(items.size());
     for (const WorkItemHost &w : items) sorted[cursor[key(w)]++] = w;
     items.swap(sorted);
+    return routes.folded;
 }
 
 }  // namespace
@@ -911,6 +922,7 @@ struct DeviceSet {
     uint32_t *counters = nullptr;     // two words a kernel segment (dynamic tile scheduling)
     uint32_t item_count = 0;
     uint32_t bounds[kSegments + 1] = {};   // work-list segment boundaries (engine.h)
+    uint32_t folded = 0;                   // kinds whose edge tiles are folded
     Sides own_sides;                  // this set's own side streams,
     Sides *sides = nullptr;           // or the session's for the stream it runs on
     LaunchTuning tune{{0, 0, 0, 0, 0}, 1};
@@ -1080,7 +1092,7 @@ jxrb_status build_device_set(const jxrb_plan *const *plans, uint32_t count, cuda
         if (c.bytes) std::memcpy(set.host_blob.data() + c.at, c.src, c.bytes);
     set.upload_bytes += tables_end - tables_at;
     // order the work list by kernel segment
-    order_by_segment(set.host_items, set.bounds);
+    set.folded = order_by_segment(set.host_items, set.bounds);
     if (items) std::memcpy(set.host_blob.data() + items_at, set.host_items.data(), sizeof(WorkItemHost) * items);
     set.sides = sides ? sides : &set.own_sides;
     TRY(set.sides->grow(side_streams(set)));
@@ -1323,7 +1335,7 @@ jxrb_status launch_set(jxrb_session *s, DeviceSet &set, cudaStream_t stream) {
         if (e == cudaSuccess) s->launches += 2 + (set.q_subsampled ? 3 : set.q_two_level ? 1 : 0) + (set.q_finish ? 1 : 0);
     }
     if (e == cudaSuccess) {
-        e = launch_tiles(set.images, set.items, set.bounds, set.max_planes, set.status, set.counters, lanes + first,
+        e = launch_tiles(set.images, set.items, set.bounds, set.folded, set.max_planes, set.status, set.counters, lanes + first,
                          n - first, &set.tune);
         if (e == cudaSuccess)
             for (int k = 0; k < kSegments; k++) s->launches += set.bounds[k + 1] > set.bounds[k];
@@ -1588,8 +1600,9 @@ jxrb_status stage_plan(const jxrb_plan *plan, const int32_t *coefficients, const
     uint32_t count[kSegments] = {}, tags[kTags] = {};
     for (uint32_t ty = 0; ty < tiles_y; ty++)
         for (uint32_t tx = 0; tx < tiles_x; tx++) tags[tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level)]++;
-    const uint32_t merged = merged_kinds(tags);
-    for (uint32_t tag = 0; tag < (uint32_t)kTags; tag++) count[segment_of_tag(tag, merged)] += tags[tag];
+    const TileRoutes routes = tile_routes(tags, true);
+    layout.folded = routes.folded;
+    for (uint32_t tag = 0; tag < (uint32_t)kTags; tag++) count[segment_of_tag(tag, routes)] += tags[tag];
     uint32_t cursor[kSegments];
     layout.bounds[0] = 0;
     for (int s = 0; s < kSegments; s++) {
@@ -1601,7 +1614,7 @@ jxrb_status stage_plan(const jxrb_plan *plan, const int32_t *coefficients, const
     for (uint32_t ty = 0; ty < tiles_y; ty++)
         for (uint32_t tx = 0; tx < tiles_x; tx++) {
             const uint32_t tag = tile_tag(kind, tx, ty, T, p.mbs_x, p.mbs_y, sx, sy, two_level);
-            list[cursor[segment_of_tag(tag, merged)]++] = WorkItemHost{tag << kTagShift, (uint16_t)tx, (uint16_t)ty};
+            list[cursor[segment_of_tag(tag, routes)]++] = WorkItemHost{tag << kTagShift, (uint16_t)tx, (uint16_t)ty};
         }
     return JXRB_OK;
 }
@@ -2359,7 +2372,7 @@ jxrb_status build_request_set(jxrb_session *s, const jxrb_request *const *reqs, 
                 set.host_items[it++] = WorkItemHost{i | tag << kTagShift, (uint16_t)tx, (uint16_t)ty};
             }
     }
-    order_by_segment(set.host_items, set.bounds);
+    set.folded = order_by_segment(set.host_items, set.bounds);
     if (items) std::memcpy(set.host_blob.data() + items_at, set.host_items.data(), sizeof(WorkItemHost) * items);
     TRY(s->sides[side_index].grow(side_streams(set)));
     set.sides = &s->sides[side_index];

@@ -3284,14 +3284,6 @@ static size_t interior_smem_bytes(int planes) {
 
 typedef void (*TileKernel)(const ImageDev *, const WorkItem *, uint32_t, uint32_t *, uint32_t *);
 
-// The interior segment's kernel of NP-plane images: with their edge tiles
-// folded in (kFoldEdges) or interior tiles only.
-template <int NP>
-static TileKernel interior_kernel() {
-    if constexpr (kFoldEdges[NP - 1]) return jxrb_interior_tiles<NP, 2>;
-    else return jxrb_interior_tiles<NP, 0>;
-}
-
 // From this many tiles on, 4:2:0 interior tiles run four CTAs an SM instead of
 // three.  The fourth hides more of the latency of coefficients that come from
 // HBM, at 64 registers and spills that make each tile slower: pictures whose
@@ -3303,21 +3295,26 @@ static TileKernel interior_kernel() {
 // batch 128.4, 125.6.
 constexpr uint32_t kManyTiles = 2560;
 
-// Kernels by index: one a segment, then the 4:2:0 interior kernel of many tiles.
-constexpr int kKernelMany420 = kSegments;
-constexpr int kKernels = kSegments + 1;
+// Kernels by index: one a segment, then the 4:2:0 interior kernel of many tiles
+// and the three-plane interior kernel that takes folded edge tiles too.
+constexpr int kKernelMany420 = kSegments, kKernelFolded3 = kSegments + 1;
+constexpr int kKernels = kSegments + 2;
 
-static int kernel_of(int segment, uint32_t tiles) {
-    return segment == 4 && tiles >= kManyTiles ? kKernelMany420 : segment;
+static_assert(kFoldAlways == 1u && kFoldSome == 4u, "interior kernels that take edge tiles too");
+// `folded`: the kinds whose edge tiles are folded.
+static int kernel_of(int segment, uint32_t tiles, uint32_t folded) {
+    if (segment == 4 && tiles >= kManyTiles) return kKernelMany420;
+    return segment == 2 && (folded & kFoldSome) ? kKernelFolded3 : segment;
 }
 
 static TileKernel tile_kernel(int kernel) {
     switch (kernel) {
     case kKernelMany420: return jxrb_interior_chroma_tiles<0, 2, 4>;
-    case 0: return interior_kernel<1>();
-    case 1: return interior_kernel<2>();
-    case 2: return interior_kernel<3>();
-    case 3: return interior_kernel<4>();
+    case kKernelFolded3: return jxrb_interior_tiles<3, 2>;
+    case 0: return jxrb_interior_tiles<1, 2>;
+    case 1: return jxrb_interior_tiles<2, 0>;
+    case 2: return jxrb_interior_tiles<3, 0>;
+    case 3: return jxrb_interior_tiles<4, 0>;
     case 4: return jxrb_interior_chroma_tiles<0, 2>;
     case 5: return jxrb_interior_chroma_tiles<0, 4>;
     case 6: return jxrb_interior_tiles<1, 1>;
@@ -3396,10 +3393,10 @@ static cudaError_t kernel_fit(int index, int planes, size_t smem, int &sms, int 
 }
 
 // Launch the work list's segments, each kernel on the next of `lanes` in turn.
-// `bounds` holds the kSegments + 1 segment boundaries; `counters` two words a
-// segment.  The other and edge tiles come first, so that their short,
+// `bounds` holds the kSegments + 1 segment boundaries, `folded` the kinds whose
+// edge tiles are folded; `counters` two words a segment.  The other and edge tiles come first, so that their short,
 // latency-bound launches start with the interior ones.
-cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32_t *bounds, int max_planes,
+cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32_t *bounds, uint32_t folded, int max_planes,
                          uint32_t *status, uint32_t *counters, const cudaStream_t *lanes, int lane_count,
                          const LaunchTuning *tune) {
     const WorkItem *list = static_cast<const WorkItem *>(items);
@@ -3409,7 +3406,7 @@ cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32
                                                                                           : seg0 - (kSegmentOther - kSideSegment0) - 1;
         const uint32_t count = bounds[seg + 1] - bounds[seg];
         if (count == 0) continue;
-        const int index = kernel_of(seg, count);
+        const int index = kernel_of(seg, count, folded);
         TileKernel k = tile_kernel(index);
         const int planes = segment_planes(seg, max_planes);
         const size_t smem = segment_smem_bytes(seg, max_planes);

@@ -22,7 +22,7 @@
 #include "engine.h"
 
 namespace jxr {
-cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32_t *bounds, int max_planes,
+cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32_t *bounds, uint32_t folded, int max_planes,
                          uint32_t *status, uint32_t *counters, const cudaStream_t *lanes, int lane_count,
                          const LaunchTuning *tune);
 size_t staged_bytes(const jxrb_plan &plan);
@@ -125,7 +125,7 @@ extern "C" jxrb_status jxrb_decode_static(int device, const jxrb_plan *plan, con
     }
     uint32_t *status = reinterpret_cast<uint32_t *>(scratch + layout.status_at);
     e = jxr::launch_tiles(reinterpret_cast<const jxr::ImageDev *>(scratch), scratch + layout.items_at, layout.bounds,
-                          layout.max_planes, status, reinterpret_cast<uint32_t *>(scratch + layout.counters_at),
+                          layout.folded, layout.max_planes, status, reinterpret_cast<uint32_t *>(scratch + layout.counters_at),
                           &stream, 1, nullptr);
     if (e != cudaSuccess) return drained(jxr::report_cuda(e, "kernel launch"));
     uint32_t word = 0;

@@ -127,7 +127,7 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *p) {
 namespace jxr {
 size_t tile_smem_bytes(int) { return 0; }
 int tile_mbs() { return 4; }
-cudaError_t launch_tiles(const ImageDev *, const void *, const uint32_t *, int, uint32_t *, uint32_t *,
+cudaError_t launch_tiles(const ImageDev *, const void *, const uint32_t *, uint32_t, int, uint32_t *, uint32_t *,
                          const cudaStream_t *lanes, int lane_count, const LaunchTuning *) {
     BEGIN("launch_tiles");
     note("launch on " + std::to_string(lane_count));

@@ -237,3 +237,33 @@ def test_staged_bytes_are_uploaded_bytes(fake, side):
     session.close()
     plan.close()
     fake.cudaFreeHost(p)
+
+
+@pytest.mark.parametrize("kind,size,launches", [
+    (dict(color_format=C_["YUV444"]), (640, 640), 1),                       # 100 tiles: edge tiles folded
+    (dict(color_format=C_["YUV444"]), (1600, 1200), 1),                     # 475
+    (dict(color_format=C_["YUV444"]), (3264, 3200), 2),                     # 2550, and one picture more below
+    (dict(color_format=C_["YUV444"], hard_tiles=1, tile_width=16, tile_height=16), (1600, 1200), 2),
+    (dict(color_format=C_["YUV420"]), (640, 640), 1),                       # no more than 128: one kernel
+    (dict(color_format=C_["YUV420"]), (1600, 1200), 2),
+    (dict(color_format=C_["LUMA"]), (1600, 1200), 1),
+])
+def test_launches_of_a_set(fake, kind, size, launches):
+    """Which tiles share a kernel: one-plane edge tiles always run with the
+    interior ones, three-plane ones in sets of fewer than 2560 tiles without
+    hard boundaries, others in sets of no more than 128."""
+    w, h = size
+    img = J.synth(w, h, quality=40, overlap=1, seed=9, threads=8, **kind)
+    layout, colour = ("LUMA", "LUMA") if kind["color_format"] == C_["LUMA"] else ("RGB", "RGB")
+    plan = J.CudaDecodePlan(img.arena, img.geometry, J.OutputFormat(C_[colour], D["U8"], S["U8"], L[layout], w, h))
+    few = J.synth(64, 192, quality=40, overlap=1, seed=9, **kind)           # 3 tiles more
+    more = J.CudaDecodePlan(few.arena, few.geometry, J.OutputFormat(C_[colour], D["U8"], S["U8"], L[layout], 64, 192))
+    session = J.CudaDecoderSession(0)
+    for plans in ([plan, more, more, more, more], [plan]):
+        res = session.resident(plans)
+        # 2550 tiles alone stay folded
+        assert res.launches(True) == (1 if plans == [plan] and size == (3264, 3200) else launches)
+        res.close()
+    session.close()
+    for p in (plan, more):
+        p.close()
