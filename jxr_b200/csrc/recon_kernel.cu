@@ -1767,13 +1767,14 @@ __device__ __forceinline__ bool edge_pixels(const ImageDev &im, const int32_t *t
     return bad;
 }
 
-// Samples and terms of a channel below this leave no checked scaling step
-// room to overflow: 2^28, less what the shift up after the rounding takes.
-__device__ __forceinline__ uint32_t lean_limit(const ChannelScale &s) {
-    return s.post_shift < 28 ? (1u << 28) >> max(s.post_shift, 0) : 0u;
+// Terms of a channel below 2^28 leave no checked scaling step room to overflow
+// with samples below 2^28 (or 2^30, of an inverse RCT of those).
+__device__ __forceinline__ bool lean_terms(const ChannelScale &s) {
+    return mag(s.shifted_bias) < (1u << 28) && mag(s.rounding) < (1u << 28);
 }
-__device__ __forceinline__ bool lean_channel(const ChannelScale &s) {
-    return mag(s.shifted_bias) < lean_limit(s) && mag(s.rounding) < lean_limit(s);
+// The shift up after the rounding, which saturates.
+__device__ __forceinline__ int32_t shifted_up(int32_t v, int up) {
+    return v > (INT32_MAX >> up) ? INT32_MAX : (int32_t)((uint32_t)max(v, INT32_MIN >> up) << up);
 }
 // Whether the three colour channels are R, G and B from YUV in some order,
 // each lean and without a shift up; `at`: two bits a component, its channel.
@@ -1783,7 +1784,7 @@ __device__ __forceinline__ bool lean_rgb(const OutputDev &o, int colours, uint32
     at = 0;
     for (int ch = 0; ch < 3; ch++) {
         const ChannelScale &s = o.ch[ch];
-        lean &= !s.padding && s.post_shift < 0 && lean_channel(s);
+        lean &= !s.padding && s.post_shift < 0 && lean_terms(s);
         seen |= 1u << (s.source & 31);
         at |= (uint32_t)ch << (2 * (s.source & 3));
     }
@@ -1822,10 +1823,10 @@ __device__ __forceinline__ int cell_rows(const ImageDev &im, int32_t *tiles, int
     uint32_t rgb_at = 0;
     // the specialised outputs this image's cells may take
     const bool rgb8 = NP >= 3 && inside && kind == kOutRgb8 && !o.premultiply;
-    const bool direct = NP == 1 && inside && kind == kOutDirect && lean_channel(o.ch[0]);
+    const bool direct = NP == 1 && inside && kind == kOutDirect && lean_terms(o.ch[0]);
     const bool f16 = NP >= 3 && inside && kind == kOutF16Wide && o.nchw && o.channels <= NP &&
                      lean_rgb(o, has_alpha ? o.channels - 1 : o.channels, rgb_at) &&
-                     (!has_alpha || (o.ch[o.channels - 1].post_shift < 0 && lean_channel(o.ch[o.channels - 1])));
+                     (!has_alpha || (o.ch[o.channels - 1].post_shift < 0 && lean_terms(o.ch[o.channels - 1])));
     const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
     const uint64_t chs = o.nchw ? o.plane_stride : (uint64_t)o.elem_bytes;
     uint8_t *dst = o.base + (int64_t)(y0 - (int)o.crop_y) * (int64_t)o.row_stride + (int64_t)(x0 - (int)o.crop_x) * (int64_t)pixel_bytes;
@@ -1868,13 +1869,13 @@ __device__ __forceinline__ int cell_rows(const ImageDev &im, int32_t *tiles, int
             }
             if (o.channels == 4) store16(dst, px[0], px[1], px[2], px[3]);
             else store12(dst, px);
-        } else if (direct && m < lean_limit(o.ch[0]) && (o.ch[0].post_shift <= 0 || !tile_small)) {
+        } else if (direct && m < (1u << 28)) {
             const ChannelScale &s = o.ch[0];
             const int eb = o.elem_bytes, up = max(s.post_shift, 0);
             uint32_t q[4];
 #pragma unroll
             for (int c = 0; c < 4; c++)
-                q[c] = (uint32_t)min(max(((w[0][c] + s.shifted_bias + s.rounding) >> s.shift) << up, s.lo), s.hi);
+                q[c] = (uint32_t)min(max(shifted_up((w[0][c] + s.shifted_bias + s.rounding) >> s.shift, up), s.lo), s.hi);
             if (eb == 2) store8(dst, (q[0] & 0xffffu) | (q[1] << 16), (q[2] & 0xffffu) | (q[3] << 16));
             else if (eb == 4) store16(dst, q[0], q[1], q[2], q[3]);
             else {
@@ -1931,6 +1932,76 @@ template <int NP>
 __device__ __noinline__ int cell_rows_call(const ImageDev &im, int32_t *tiles, int mx0, int my0, int gcx, int gcy,
                                            bool cut, bool tile_small) {
     return cell_rows<NP>(im, tiles, mx0, my0, gcx, gcy, cut, tile_small);
+}
+
+// A cell of a one-plane interior tile that the lean one-channel form leaves:
+// one channel in any store kind, its scaling steps checked, whole rows at once;
+// or, for other outputs and cells at the crop edge, the general store pixel by
+// pixel.  Out of line, the cell in registers: in place and row by row, as the
+// kernels of more planes have it, one plane's few instructions a pixel pay for
+// the way through shared memory (2048 x 1536, us in place and here: half floats
+// 40.3, 26.6; binary32 59.9, 47.3; RGB8 58.4, 55.9).  Returns the tile flags.
+__device__ __noinline__ int luma_cell(const ImageDev &im, const int32_t *tile, int mx0, int my0, int gcx, int gcy,
+                                      bool tile_small) {
+    const CellBlocks cell = cell_blocks(gcx, gcy);
+    const OutputDev &o = im.out;
+    int32_t y[16];
+    cell_load(tile, cell, y);
+    int bad = 0;
+    if (im.plane[0].overlap >= 1) {
+        if (tile_small) inverse_pot4x4<false>(y);
+        else if (pot16(y)) bad = kFlagOverlap;
+    }
+    const int x0 = 16 * mx0 + 2 + 4 * gcx, y0 = 16 * my0 + 2 + 4 * gcy;
+    const bool inside = x0 >= (int)o.crop_x && x0 + 4 <= (int)(o.crop_x + o.crop_w) && y0 >= (int)o.crop_y &&
+                        y0 + 4 <= (int)(o.crop_y + o.crop_h);
+    const uint64_t pixel_bytes = o.nchw ? (uint64_t)o.elem_bytes : (uint64_t)o.elem_bytes * o.channels;
+    const uint64_t chs = o.nchw ? o.plane_stride : (uint64_t)o.elem_bytes;
+    uint8_t *dst = o.base + (int64_t)(y0 - (int)o.crop_y) * (int64_t)o.row_stride + (int64_t)(x0 - (int)o.crop_x) * (int64_t)pixel_bytes;
+    bool obad = false;
+    if (inside && o.conv == kConvDirect && o.channels == 1) {
+        const ChannelScale &s = o.ch[0];
+        const int eb = o.elem_bytes;
+#pragma unroll
+        for (int k = 0; k < 16; k++) y[k] = apply_scale(s, y[k], obad);
+        if (o.store == kStoreF32) {
+#pragma unroll
+            for (int k = 0; k < 16; k++) y[k] = (int32_t)f32_bits(y[k], s.f_mantissa, s.f_bias, obad);
+        } else if (o.store == kStoreF16) {
+            const bool widen = o.widen_f16;
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                const uint32_t h = (y[k] < 0 ? 0x8000u : 0u) | min((uint32_t)(y[k] < 0 ? -(int64_t)y[k] : y[k]), 32767u);
+                y[k] = (int32_t)(widen ? widen_f16(h) : h);
+            }
+        } else {
+            const int32_t lo = s.lo, hi = s.hi;
+#pragma unroll
+            for (int k = 0; k < 16; k++) y[k] = min(max(y[k], lo), hi);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; r++, dst += o.row_stride) {
+            const uint32_t q[4] = {(uint32_t)y[4 * r], (uint32_t)y[4 * r + 1], (uint32_t)y[4 * r + 2], (uint32_t)y[4 * r + 3]};
+            if (eb == 4) {
+                store16(dst, q[0], q[1], q[2], q[3]);
+            } else if (eb == 2) {
+                store8(dst, (q[0] & 0xffffu) | (q[1] << 16), (q[2] & 0xffffu) | (q[3] << 16));
+            } else {
+                const uint32_t b[1] = {(q[0] & 0xffu) | ((q[1] & 0xffu) << 8) | ((q[2] & 0xffu) << 16) | (q[3] << 24)};
+                store_words(dst, b);
+            }
+        }
+    } else {
+        for (int r = 0; r < 4; r++, dst += o.row_stride) {
+            if (y0 + r < (int)o.crop_y || y0 + r >= (int)(o.crop_y + o.crop_h)) continue;
+            for (int c = 0; c < 4; c++) {
+                if (x0 + c < (int)o.crop_x || x0 + c >= (int)(o.crop_x + o.crop_w)) continue;
+                const int32_t comp[4] = {y[r * 4 + c], 0, 0, 0};
+                format_pixel(o, comp, 0, dst + (int64_t)c * (int64_t)pixel_bytes, chs, obad);
+            }
+        }
+    }
+    return obad ? bad | kFlagOutput : bad;
 }
 
 // A tile's status from its flags.
@@ -2224,20 +2295,26 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                     done = true;
                 }
             }
-        } else if (inside && kind == kOutDirect && NP == 1 && lean_channel(o.ch[0])) {
-            // samples and terms below the lean limit: no scaling step can
-            // overflow, so the unchecked ones give the same values
+        } else if (inside && kind == kOutDirect && NP == 1 && lean_terms(o.ch[0])) {
+            // samples and terms below 2^28: no scaling step can overflow, so
+            // the unchecked ones give the same values
             int32_t y[16];
             const bool fast = cell_samples_fast(tiles, cell, im.plane[0].overlap, y, tile_small);
-            if (fast && ((tile_small && o.ch[0].post_shift <= 0) || mag_bound<0>(y) < lean_limit(o.ch[0]))) {
+            if (fast && (tile_small || mag_bound<0>(y) < (1u << 28))) {
                 const ChannelScale &s = o.ch[0];
                 const int eb = o.elem_bytes;
-                const int32_t add = s.shifted_bias + s.rounding, shift = s.shift, up = max(s.post_shift, 0), lo = s.lo, hi = s.hi;
+                const int32_t add = s.shifted_bias + s.rounding, shift = s.shift, up = s.post_shift, lo = s.lo, hi = s.hi;
+#pragma unroll
+                for (int k = 0; k < 16; k++) y[k] = (y[k] + add) >> shift;
+                if (up > 0) {
+#pragma unroll
+                    for (int k = 0; k < 16; k++) y[k] = shifted_up(y[k], up);
+                }
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
                     uint32_t q[4];
 #pragma unroll
-                    for (int c = 0; c < 4; c++) q[c] = (uint32_t)min(max(((y[r * 4 + c] + add) >> shift) << up, lo), hi);
+                    for (int c = 0; c < 4; c++) q[c] = (uint32_t)min(max(y[r * 4 + c], lo), hi);
                     uint8_t *dst = o.base + (uint64_t)(y0 + r - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * eb;
                     if (eb == 2) store8(dst, (q[0] & 0xffffu) | (q[1] << 16), (q[2] & 0xffffu) | (q[3] << 16));
                     else if (eb == 4) store16(dst, q[0], q[1], q[2], q[3]);
@@ -2250,7 +2327,7 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
             }
         } else if (NP >= 3 && inside && kind == kOutF16Wide && o.nchw && o.channels <= NP &&
                    lean_rgb(o, has_alpha ? o.channels - 1 : o.channels, rgb_at) &&
-                   (!has_alpha || (o.ch[o.channels - 1].post_shift < 0 && lean_channel(o.ch[o.channels - 1])))) {
+                   (!has_alpha || (o.ch[o.channels - 1].post_shift < 0 && lean_terms(o.ch[o.channels - 1])))) {
             // R, G and B to their channel planes, alpha to the last.  YUV
             // below 2^28 keeps the inverse RCT below 2^30 and, with terms below
             // 2^28, every scaling step below 2^31: no checked step can
@@ -2313,7 +2390,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         }
         // any other output, cells that need the checked operator, or pixels at
         // the crop edge
-        if (!done) bad |= cell_rows_call<NP>(im, tiles, mx0, my0, gcx, gcy, false, tile_small);
+        if (!done)
+            bad |= NP == 1 ? luma_cell(im, tiles, mx0, my0, gcx, gcy, tile_small)
+                           : cell_rows_call<NP>(im, tiles, mx0, my0, gcx, gcy, false, tile_small);
     }
     if (edge && edge_pixels<NP>(im, tiles, mx0, my0, ec)) bad |= kFlagOutput;
     // One closing barrier in the interior kernels of three and four planes, two

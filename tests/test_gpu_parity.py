@@ -512,3 +512,31 @@ def test_readback_all_matches_per_image_readback(session):
     with pytest.raises(J.CudaError):
         sub.readback_all(host.ctypes.data, total + (1 << 20))
     sub.close()
+
+
+@pytest.mark.parametrize("overlap", [0, 1, 2])
+@pytest.mark.parametrize("depth,storage,extra", [
+    ("U8", "U8", {}), ("U16", "U16", {}), ("U16", "U16", dict(shift_bits=3)), ("I16", "I16", dict(shift_bits=2)),
+    ("I32", "I32", {}), ("I32", "I32", dict(shift_bits=8)), ("I32", "I32", dict(shift_bits=16)),
+    ("I32", "I32", dict(shift_bits=31)), ("F16", "F16", {}), ("F16", "F16", dict(widen_f16=1)),
+    ("F16", "F16", dict(widen_f16=1, nchw=1)), ("F32", "F32", dict(mantissa_length=13, exponent_bias=4))])
+def test_one_channel_outputs(session, overlap, depth, storage, extra):
+    """One-channel outputs of one-plane images in every store kind: shifts up
+    that saturate on both sides, rows at every alignment, cells at the crop edge,
+    and quantizer steps that take the samples past the wrapping operators'
+    bounds (and, at 2^12, some past int32: an error, as in the oracle)."""
+    for by, hard in ((1, 0), (1, 1), (1 << 9, 0), (1 << 12, 0)):
+        img = J.synth(333, 270, content=J.CONTENT["GRAY16"], color_format=C_["LUMA"], quality=100, scaled=0,
+                      overlap=overlap, tile_width=7, tile_height=6, hard_tiles=hard, seed=4)
+        img.arena.quantizers *= np.uint32(by)
+        for x, y, w, h in ((0, 0, 333, 270), (3, 5, 301, 250)):
+            out = J.OutputFormat(C_["LUMA"], D[depth], S[storage], L["LUMA"], w, h, crop_x=x, crop_y=y, **extra)
+            check(session, img, out, expect_ok=by < 1 << 12)
+
+
+@pytest.mark.parametrize("depth,layout,extra", [("U8", "RGB", {}), ("U8", "RGBX", {}), ("U8", "RGB", dict(nchw=1)),
+                                                ("U16", "BGR", {}), ("RGB565", "RGB", {})])
+def test_luma_to_rgb(session, depth, layout, extra):
+    img = J.synth(333, 270, color_format=C_["LUMA"], quality=85, overlap=2, seed=4)
+    out = J.OutputFormat(C_["RGB"], D[depth], S[depth], L[layout], 301, 250, crop_x=3, crop_y=5, **extra)
+    check(session, img, out)
