@@ -309,30 +309,16 @@ extern "C" jxrb_status jxrb_orient(const void *device_source, void *device_desti
     } else {
         // the widest word that divides the pixel and both surfaces' alignment
         const uintptr_t a = reinterpret_cast<uintptr_t>(device_source) | reinterpret_cast<uintptr_t>(device_destination);
-        // The usual pixel sizes go to the kernel compiled for them where both
-        // surfaces are aligned to its unit; other sizes, and surfaces off that
-        // alignment, keep the kernel that takes any of them.  So do small
-        // surfaces of 1 to 3 bytes a pixel: until every SM has tiles enough, a
-        // tile's latency counts, and its three passes over 64 x 64 pixels take
-        // longer than the one word a thread moves at a time over 32 x 32 (us,
-        // any size's kernel / the pixel's: 301 x 217 of 1, 2, 3 bytes 2.8 / 5.3,
-        // 2.9 / 6.1, 6.0 / 7.6; 999 x 801 5.0 / 5.6, 5.0 / 6.4, 10.5 / 7.0;
-        // 1203 x 900 of 2 bytes 6.1 / 6.4; 1600 x 1204 8.7 / 5.2, 8.8 / 5.9,
-        // 20 / 8.4; 601 x 499 of 3 bytes 7.1 / 7.9, 801 x 603 8.2 / 6.1 to 8.3).
-        const bool even = a % 2 == 0, word = a % 4 == 0;
         const uint32_t n = pixel_bytes;
-        const uint64_t pixels = (uint64_t)width * height;
-        const bool small = n <= 3 && pixels < (n == 1 ? uint64_t(1) << 20 : n == 2 ? uint64_t(5) << 18 : uint64_t(3) << 17);
-        if (small && (n != 2 || !even)) e = launch_tiles<uint8_t>(device_source, device_destination, width, height, n, orientation, stream);
-        else if (small) e = launch_tiles<uint16_t>(device_source, device_destination, width, height, 1, orientation, stream);
-        else if (n == 1) e = launch_pixels<1>(device_source, device_destination, width, height, orientation, stream);
-        else if (n == 3) e = launch_pixels<3>(device_source, device_destination, width, height, orientation, stream);
-        else if (n == 2 && even) e = launch_pixels<2>(device_source, device_destination, width, height, orientation, stream);
-        else if (n == 6 && even) e = launch_pixels<6>(device_source, device_destination, width, height, orientation, stream);
-        else if (n == 4 && word) e = launch_pixels<4>(device_source, device_destination, width, height, orientation, stream);
-        else if (n == 8 && word) e = launch_pixels<8>(device_source, device_destination, width, height, orientation, stream);
-        else if (n == 12 && word) e = launch_pixels<12>(device_source, device_destination, width, height, orientation, stream);
-        else if (n == 16 && word) e = launch_pixels<16>(device_source, device_destination, width, height, orientation, stream);
+        if (jxr::takes_pixel_kernel(n, a, width, height))
+            e = n == 1 ? launch_pixels<1>(device_source, device_destination, width, height, orientation, stream)
+              : n == 2 ? launch_pixels<2>(device_source, device_destination, width, height, orientation, stream)
+              : n == 3 ? launch_pixels<3>(device_source, device_destination, width, height, orientation, stream)
+              : n == 4 ? launch_pixels<4>(device_source, device_destination, width, height, orientation, stream)
+              : n == 6 ? launch_pixels<6>(device_source, device_destination, width, height, orientation, stream)
+              : n == 8 ? launch_pixels<8>(device_source, device_destination, width, height, orientation, stream)
+              : n == 12 ? launch_pixels<12>(device_source, device_destination, width, height, orientation, stream)
+                        : launch_pixels<16>(device_source, device_destination, width, height, orientation, stream);
         else if (pixel_bytes % 4 == 0 && a % 4 == 0)
             e = launch_tiles<uint32_t>(device_source, device_destination, width, height, pixel_bytes / 4, orientation,
                                        stream);

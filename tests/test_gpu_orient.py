@@ -90,13 +90,16 @@ def test_small_and_large_surfaces_of_small_pixels(torch, orientation, pixel_byte
 
 @pytest.mark.parametrize("orientation", range(8))
 @pytest.mark.parametrize("pixel_bytes,sizes,offsets", [
-    (1, [(1100003, 1), (1, 1100003), (2, 600001), (600001, 2), (65, 16200), (66, 16200)], (0, 1, 2, 3)),
-    (2, [(1400003, 1), (1, 1400003), (2, 700001), (65, 20300)], (0, 2)),
-    (3, [(400003, 1), (1, 400003), (2, 200001), (65, 6100)], (0, 1, 3))])
+    (1, [(1100003, 1), (1, 1100003), (2, 600001), (600001, 2), (65, 16200), (66, 16200), (11, 95400),
+         (12, 87400), (87400, 13)], (0, 1, 2, 3)),
+    (2, [(1400003, 1), (1, 1400003), (2, 700001), (65, 20300), (12, 109300)], (0, 2)),
+    (3, [(400003, 1), (1, 400003), (2, 200001), (65, 6100), (7, 56200), (8, 49200)], (0, 1, 3)),
+    (4, [(11, 700), (12, 700), (700, 13)], (0,)), (16, [(7, 700), (8, 700), (700, 9)], (0,))])
 def test_narrow_surfaces_of_small_pixels(torch, orientation, pixel_bytes, sizes, offsets):
-    """Surfaces one and two pixels wide or high, and one and two pixels wider
-    than a tile, of the extents the kernels of 1- to 3-byte pixels take: the
-    tiles whose aligned words would reach outside the surface."""
+    """Surfaces one and two pixels wide or high, one and two pixels wider than a
+    tile, and either side of the width from which the kernels compiled for a
+    pixel size take them: tiles whose aligned words would reach outside the
+    surface, and tiles with few pixels."""
     rng = np.random.default_rng(pixel_bytes * 8 + orientation)
     for width, height in sizes:
         src = rng.integers(0, 256, width * height * pixel_bytes, dtype=np.uint8)

@@ -1,4 +1,5 @@
-"""The source words an orientation tile reads, on the CPU: the kernel's own
+"""The source words an orientation tile reads and the kernel a surface takes, on
+the CPU: the kernel's own
 index arithmetic (csrc/orient_tile.h), built with the host compiler and walked
 over every tile and row.  A tile that may read whole aligned words reads none
 outside the caller's surface, at widths and heights of whole tiles and one or
@@ -64,3 +65,38 @@ def test_word_reads_stay_inside_the_surface(program, pixel_bytes):
     outside, words, by_byte = map(int, out.split())
     assert outside == 0
     assert words > 0 and by_byte > 0
+
+
+ROUTES = r"""
+#include <cstdio>
+#include <cstdlib>
+#include "orient_tile.h"
+int main(int argc, char **argv) {
+    for (int i = 1; i + 3 < argc; i += 4)
+        printf("%d\n", (int)jxr::takes_pixel_kernel(atoi(argv[i]), atoi(argv[i + 1]), atoi(argv[i + 2]), atoi(argv[i + 3])));
+    return 0;
+}
+"""
+
+
+def test_surfaces_of_each_kernel(tmp_path):
+    """Pixels of 1 to 3 bytes from an extent on, every size from a narrower side
+    on, at the alignment of their unit; other sizes never."""
+    (tmp_path / "routes.cpp").write_text(ROUTES)
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I", str(CSRC), str(tmp_path / "routes.cpp"), "-o", str(tmp_path / "routes")],
+                   check=True)
+    cases = []
+    for n, extent, side in [(1, 1 << 20, 12), (2, 5 << 18, 16), (3, 3 << 17, 8), (4, 0, 12), (6, 0, 12), (8, 0, 8), (12, 0, 8),
+                            (16, 0, 8)]:
+        big = max(extent, 1 << 12)
+        for w, h, taken in [(1 << 11, -(-big // (1 << 11)) + side, 1), (side, -(-big // side), 1), (-(-big // side), side, 1),
+                            (side - 1, 2 * big, 0), (2 * big, side - 1, 0), (1, 2 * big, 0)]:
+            cases.append((n, 0, w, h, taken))
+        if extent:
+            cases += [(n, 0, extent // 1024, 1023, 0), (n, 0, extent // 1024, 1024, 1)]
+        if n % 2 == 0:
+            cases += [(n, 1, 4096, 4096, 0), (n, 2, 4096, 4096, int(n % 4 != 0))]
+    cases += [(n, 0, 4096, 4096, 0) for n in (5, 7, 10, 20, 48)]
+    args = [str(v) for c in cases for v in c[:4]]
+    out = subprocess.run([str(tmp_path / "routes"), *args], check=True, capture_output=True, text=True).stdout.split()
+    assert [(c, int(o)) for c, o in zip(cases, out)] == [(c, c[4]) for c in cases]
