@@ -360,9 +360,9 @@ void jxrb_resident_destroy(jxrb_resident *resident);
  * fixes 128-thread CTAs per macroblock (kernels/main.rs:98-207). */
 typedef struct jxrb_launch_tuning {
     uint32_t blocks_per_sm[5];   /* resident CTAs per SM, 0 = as many as fit: entries 0..3 for interior tiles with
-                                    1..4 full-resolution planes (entry 2 also for 4:2:0 interior tiles), entry 4 for
-                                    the other tiles */
-    int32_t side_stream;         /* 1: the edge and general tile kernels run on a second stream beside the interior ones */
+                                    1..4 full-resolution planes (below 3, entry 2 also for tiles of 4:2:0 and 4:2:2
+                                    images, which else run as many as fit), entry 4 for the other tiles */
+    int32_t side_stream;         /* 1: the tile kernels run on streams beside each other */
 } jxrb_launch_tuning;
 jxrb_status jxrb_resident_set_tuning(jxrb_resident *resident, const jxrb_launch_tuning *tuning);
 /* Capture the launch sequence of one run (batched != 0: the persistent batch

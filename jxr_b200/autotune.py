@@ -6,8 +6,9 @@ pay off depends on the mix of tiles (interior tiles with 1..4 planes, edge
 tiles, subsampled chroma), and so does whether the edge-tile kernel should
 run on a second stream beside the interior kernels.  The autotuner times
 every candidate shape on the resident set itself with CUDA events, keeps the
-fastest, and caches the choice by device and by a signature of the set's
-plans (`JXRB_TUNING_CACHE`, default ~/.cache/jxr_b200/tuning.json).
+fastest, and caches the choice by device, by a signature of the set's plans and
+by the engine library it was measured with, whose kernels another build may
+have changed (`JXRB_TUNING_CACHE`, default ~/.cache/jxr_b200/tuning.json).
 """
 from __future__ import annotations
 
@@ -18,7 +19,9 @@ import os
 from pathlib import Path
 from typing import Dict, List, Optional, Sequence, Tuple
 
-INTERIOR_CTAS = (1, 2, 3)   # what the full-resolution interior kernels fit an SM (4:2:0's fits 4)
+from . import api
+
+INTERIOR_CTAS = (1, 2, 3)   # the full-resolution interior kernels fit 3; 3 leaves the subsampled ones what they fit
 OTHER_CTAS = (1, 2)         # the general kernel fits 2
 
 
@@ -37,6 +40,11 @@ def signature(plans: Sequence) -> str:
                        len(g.tile_column_widths or ()), len(g.tile_row_heights or ()), o.storage, o.layout,
                        o.nchw, o.crop_width, o.crop_height)).encode())
     return h.hexdigest()[:24]
+
+
+def cache_key(device: str, plans: Sequence, batched: bool) -> str:
+    engine = hashlib.sha256(api.LIB_PATH.read_bytes()).hexdigest()[:16]
+    return f"{device}|{signature(plans)}|{int(batched)}|{engine}"
 
 
 def _cache_path() -> Path:
@@ -81,7 +89,7 @@ def tune(res, plans: Sequence, device_ptr: int, nbytes: int, stream, batched: bo
     """Choose and apply the fastest launch shape for `res`; returns the choice
     (`blocks_per_sm`, `side_stream`, `ms`, `source`)."""
     import torch
-    key = f"{torch.cuda.get_device_name(stream.device)}|{signature(plans)}|{int(batched)}"
+    key = cache_key(torch.cuda.get_device_name(stream.device), plans, batched)
     cache = _load() if use_cache else {}
     hit: Optional[Dict] = cache.get(key)
     if hit:

@@ -3305,7 +3305,7 @@ jxrb_interior_chroma_tiles(const ImageDev *__restrict__ images, const WorkItem *
 // (about 24 KB a plane) admits two four-plane tiles, so their kernel takes the
 // registers of two (no spills); fewer planes run three (at 64 registers, for
 // four, the one- and two-plane kernels spill).
-template <int NP> constexpr int interior_ctas() { return NP == 4 ? 2 : 3; }
+template <int NP> constexpr int interior_ctas() { return NP == 4 ? 2 : (int)kThreePlaneCtas; }
 
 // Tiles of images with NP full-resolution planes: interior tiles (MODE 0),
 // edge tiles (MODE 1) or both, each by its position (MODE 2).
@@ -3485,17 +3485,17 @@ cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32
                                                                                           : seg0 - (kSegmentOther - kSideSegment0) - 1;
         const uint32_t count = bounds[seg + 1] - bounds[seg];
         if (count == 0) continue;
-        const int index = kernel_of(seg, count, folded);
-        TileKernel k = tile_kernel(index);
         const int planes = segment_planes(seg, max_planes);
+        const int slot = seg == kSegmentOther ? 4 : planes - 1;   // entry of the launch tuning
+        uint32_t cap = tune ? tune->blocks_per_sm[slot] : 0;
+        if (chroma_segment(seg) && cap >= kThreePlaneCtas) cap = 0;
+        const int index = kernel_of(seg, cap ? 0 : count, folded);   // capped, more CTAs an SM are no use
+        TileKernel k = tile_kernel(index);
         const size_t smem = segment_smem_bytes(seg, max_planes);
         int sms = 0, fit = 0;
         cudaError_t fe = kernel_fit(index, planes, smem, sms, fit);
         if (fe != cudaSuccess) return fe;
-        int per_sm = fit;
-        const int slot = seg == kSegmentOther ? 4 : planes - 1;   // entry of the launch tuning
-        if (tune && tune->blocks_per_sm[slot] > 0 && (int)tune->blocks_per_sm[slot] < fit)
-            per_sm = (int)tune->blocks_per_sm[slot];
+        const int per_sm = cap > 0 && cap < (uint32_t)fit ? (int)cap : fit;
         const long full = (long)sms * per_sm;
         const int blocks = (int)((long)count < full ? (long)count : full);
         k<<<blocks, kThreads, smem, lanes[lane]>>>(images, list + bounds[seg], count, status, counters + 2 * seg);

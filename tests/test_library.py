@@ -58,6 +58,21 @@ def test_autotune_candidates_and_signature():
     assert autotune.signature(plans) != autotune.signature(plans[:2])
 
 
+def test_autotune_choices_belong_to_a_build(tmp_path, monkeypatch):
+    """A choice measured with one build of the engine is not applied to
+    another, whose kernels it says nothing about."""
+    from jxr_b200 import api, autotune, workloads as W
+    plans = W.plans_of(W.mixed_batch(count=2, seed=1, lo=64, hi=128, threads=2))
+    keys = []
+    for text in (b"one build", b"another build", b"one build"):
+        path = tmp_path / f"engine{len(keys)}.so"
+        path.write_bytes(text)
+        monkeypatch.setattr(api, "LIB_PATH", path)
+        keys.append(autotune.cache_key("device", plans, True))
+    assert keys[0] == keys[2] != keys[1]
+    assert keys[0] != autotune.cache_key("device", plans, False)
+
+
 def test_mixed_batch_shapes():
     from jxr_b200 import workloads as W
     items = W.mixed_batch(count=12, seed=3, lo=64, hi=256, threads=2)
