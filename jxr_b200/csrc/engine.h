@@ -170,11 +170,14 @@ constexpr int kSegmentOther = kSegments - 1;
 constexpr uint32_t kFoldAlways = 1u << 0, kFoldSome = 1u << 2;
 constexpr uint32_t kApartTiles = 2560;
 // Up to this many tiles of a kind in a set, its interior tiles run in the edge
-// kernel with the others: one launch, no fork and join.  64 tiles (512 x 512)
-// of RGB8 4:4:4, 4:2:0, RGBA: 11.3, 11.4, 11.4 us in two kernels, 10.0, 10.3,
-// 10.3 in one; 256 tiles (1024 x 1024): 13.9, 14.4, 16.9 against 15.2, 16.4,
-// 16.5.
-constexpr uint32_t kMergeTiles = 128;
+// kernel with the others: one launch, no fork and join.  Sets in turn on several
+// streams: 64 tiles (512 x 512) of 4:2:0 and RGBA 11.4, 11.4 us in two kernels,
+// 10.3, 10.3 in one; 176 (1000 x 700) of 4:2:2, 4:2:0, RGBA 13.2, 12.7, 14.6
+// against 12.8, 11.9, 15.4; 256 (1024 x 1024) 14.4, 16.9 of 4:2:0 and RGBA against
+// 16.4, 16.5.  A set alone, from HBM, gains by one kernel further on (1000 x 700
+// of 4:2:2 without overlap 36.6 us in two, 30.7 in one, 32.8 when the general
+// kernel took it).
+constexpr uint32_t kMergeTiles = 128, kMergeTilesSubsampled = 192;
 constexpr int kCounterWords = 2 * kSegments;   // two scheduling words a segment
 
 // Side streams a set's kernels may run on beside its own: with the set's

@@ -148,7 +148,8 @@ uint32_t tile_tag(uint32_t kind, uint32_t tx, uint32_t ty, uint32_t T, uint32_t 
 
 // Where a set's tiles run, by kind (bit kind - 1): whose edge tiles the
 // interior kernel takes (engine.h), and whose interior tiles the edge kernel
-// does: kinds of no more than kMergeTiles tiles for which both would run.
+// does: kinds of no more than kMergeTiles tiles (subsampled ones:
+// kMergeTilesSubsampled) for which both would run.
 // `count`: tiles by tag; `one_stream`: the kernels run one after another.
 struct TileRoutes {
     uint32_t folded = 0, merged = 0;
@@ -164,7 +165,8 @@ TileRoutes tile_routes(const uint32_t *count, bool one_stream) {
             edge = 0;
         }
         edge += hard;
-        if (inner > 0 && edge > 0 && inner + edge <= kMergeTiles) r.merged |= bit;
+        const uint32_t most = k >= kTag420 ? kMergeTilesSubsampled : kMergeTiles;
+        if (inner > 0 && edge > 0 && inner + edge <= most) r.merged |= bit;
     }
     return r;
 }

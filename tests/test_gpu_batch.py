@@ -173,12 +173,13 @@ def test_submissions_in_flight_and_small_outputs(session):
     assert all(np.array_equal(g, refs[i % 4]) for i, g in enumerate(got))
 
 
-@pytest.mark.parametrize("fmt,copies", [("YUV420", 39), ("YUV420", 40), ("YUV444", 1), ("YUV444", 25), ("YUV444", 26)])
+@pytest.mark.parametrize("fmt,copies", [("YUV420", 39), ("YUV420", 40), ("YUV444", 1), ("YUV444", 25), ("YUV444", 26),
+                                        ("YUV422", 1), ("YUV422", 2)])
 def test_many_tiles_of_a_kind(session, fmt, copies):
     """Either side of the number of interior tiles from which the 4:2:0 kernel
     runs more CTAs an SM (64 of them in a picture of 640 x 640), and of the
     number of tiles from which three-plane edge tiles have a kernel of their own
-    (100 in such a picture)."""
+    (100 in such a picture), or subsampled interior tiles."""
     img = J.synth(637, 640, color_format=J.COLOR[fmt], quality=80, overlap=1, tile_width=9, tile_height=7, seed=41,
                   threads=8)
     out = J.OutputFormat(J.COLOR["RGB"], J.DEPTH["U8"], J.STORE["U8"], J.LAYOUT["RGB"], 637, 640)

@@ -244,14 +244,15 @@ def test_staged_bytes_are_uploaded_bytes(fake, side):
     (dict(color_format=C_["YUV444"]), (1600, 1200), 1),                     # 475
     (dict(color_format=C_["YUV444"]), (3264, 3200), 2),                     # 2550, and one picture more below
     (dict(color_format=C_["YUV444"], hard_tiles=1, tile_width=16, tile_height=16), (1600, 1200), 2),
-    (dict(color_format=C_["YUV420"]), (640, 640), 1),                       # no more than 128: one kernel
+    (dict(color_format=C_["YUV420"]), (640, 640), 1),                       # no more than 192: one kernel
+    (dict(color_format=C_["YUV422"]), (1024, 704), 1),                      # 176, and 188
     (dict(color_format=C_["YUV420"]), (1600, 1200), 2),
     (dict(color_format=C_["LUMA"]), (1600, 1200), 1),
 ])
 def test_launches_of_a_set(fake, kind, size, launches):
     """Which tiles share a kernel: one-plane edge tiles always run with the
     interior ones, three-plane ones in sets of fewer than 2560 tiles without
-    hard boundaries, others in sets of no more than 128."""
+    hard boundaries, subsampled ones in sets of no more than 192."""
     w, h = size
     img = J.synth(w, h, quality=40, overlap=1, seed=9, threads=8, **kind)
     layout, colour = ("LUMA", "LUMA") if kind["color_format"] == C_["LUMA"] else ("RGB", "RGB")
