@@ -2249,10 +2249,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
         const bool inside = x0 >= (int)o.crop_x && x0 + 4 <= (int)(o.crop_x + o.crop_w) && y0 >= (int)o.crop_y &&
                             y0 + 4 <= (int)(o.crop_y + o.crop_h);
         const int kind = o.kind;
-        const bool has_alpha = im.alpha >= 0;
         bool done = false;
         uint32_t rgb_at = 0;
-        if (inside && kind == kOutRgb8 && NP >= 3 && !o.premultiply) {
+        if (inside && kind == kOutRgb8 && NP == 3 && !o.premultiply) {
             int32_t y[16], u[16], v[16];
             bool fast = cell_samples_fast(tiles, cell, im.plane[0].overlap, y, tile_small);
             fast &= cell_samples_fast(tiles + kTileInts, cell, im.plane[1].overlap, u, tile_small);
@@ -2274,26 +2273,14 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                     yuv_to_rgb_fast(y[k] + add, u[k], v[k], R, G, B);
                     px[k] = pack_rgb8(clamp_u8(R >> shift), clamp_u8(G >> shift), clamp_u8(B >> shift), order);
                 }
-                bool alpha_ok = true;
-                if (NP == 4 && has_alpha) {
-                    int32_t a[16];
-                    alpha_ok = cell_samples_fast(tiles + 3 * kTileInts, cell, im.plane[3].overlap, a, tile_small);
-                    if (!tile_small) alpha_ok &= mag_bound<0>(a) < (1u << 28);
-                    const ChannelScale &sa = o.ch[3];
-                    const int32_t aadd = sa.shifted_bias + sa.rounding;
 #pragma unroll
-                    for (int k = 0; k < 16; k++) px[k] |= clamp_u8((a[k] + aadd) >> sa.shift) << 24;
+                for (int r = 0; r < 4; r++) {
+                    uint8_t *dst = o.base + (uint64_t)(y0 + r - o.crop_y) * o.row_stride +
+                                   (uint64_t)(x0 - o.crop_x) * o.channels;
+                    if (o.channels == 4) store16(dst, px[4 * r], px[4 * r + 1], px[4 * r + 2], px[4 * r + 3]);
+                    else store12(dst, &px[4 * r]);
                 }
-                if (alpha_ok) {
-#pragma unroll
-                    for (int r = 0; r < 4; r++) {
-                        uint8_t *dst = o.base + (uint64_t)(y0 + r - o.crop_y) * o.row_stride +
-                                       (uint64_t)(x0 - o.crop_x) * o.channels;
-                        if (o.channels == 4) store16(dst, px[4 * r], px[4 * r + 1], px[4 * r + 2], px[4 * r + 3]);
-                        else store12(dst, &px[4 * r]);
-                    }
-                    done = true;
-                }
+                done = true;
             }
         } else if (inside && kind == kOutDirect && NP == 1 && lean_terms(o.ch[0])) {
             // samples and terms below 2^28: no scaling step can overflow, so
@@ -2325,67 +2312,46 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
                 }
                 done = true;
             }
-        } else if (NP >= 3 && inside && kind == kOutF16Wide && o.nchw && o.channels <= NP &&
-                   lean_rgb(o, has_alpha ? o.channels - 1 : o.channels, rgb_at) &&
-                   (!has_alpha || (o.ch[o.channels - 1].post_shift < 0 && lean_terms(o.ch[o.channels - 1])))) {
-            // R, G and B to their channel planes, alpha to the last.  YUV
-            // below 2^28 keeps the inverse RCT below 2^30 and, with terms below
-            // 2^28, every scaling step below 2^31: no checked step can
-            // overflow, so the unchecked ones give the same values.  Larger
-            // samples and other conversions take the general store: unrolled
-            // beside this form, their code alone stalled instruction fetch
-            // (3072 x 3072 half with alpha: 165 -> 134 us without it, 4096 x
-            // 4096 RGB8, the same code in the three-plane kernel, 136 -> 128;
-            // with the checked operators out of line too, 125 and 130).
+        } else if (NP == 3 && inside && kind == kOutF16Wide && o.nchw && lean_rgb(o, o.channels, rgb_at)) {
+            // R, G and B to their channel planes.  YUV below 2^28 keeps the
+            // inverse RCT below 2^30 and, with terms below 2^28, every scaling
+            // step below 2^31: no checked step can overflow, so the unchecked
+            // ones give the same values.  Larger samples and other conversions
+            // take the general store: unrolled beside this form, their code
+            // alone stalled instruction fetch (4096 x 4096 RGB8, whose kernel
+            // this is too, 136 us with it, 128 without).
             uint8_t *base = o.base + (uint64_t)(y0 - o.crop_y) * o.row_stride + (uint64_t)(x0 - o.crop_x) * 4;
             const uint64_t rs = o.row_stride, ps = o.plane_stride;
-            bool lean = true;
-            if (has_alpha && NP == 4) {
-                int32_t a[16];
-                lean = cell_samples_fast(tiles + 3 * kTileInts, cell, im.plane[3].overlap, a, tile_small) &&
-                       (tile_small || mag_bound<0>(a) < (1u << 28));
-                if (lean) {
-                    const ChannelScale &s = o.ch[o.channels - 1];
-                    const int32_t add = s.shifted_bias + s.rounding, shift = s.shift;
-                    uint8_t *abase = base + (uint64_t)(o.channels - 1) * ps;
+            int32_t y[16], u[16], v[16];
+            bool fast = cell_samples_fast(tiles, cell, im.plane[0].overlap, y, tile_small);
+            fast &= cell_samples_fast(tiles + kTileInts, cell, im.plane[1].overlap, u, tile_small);
+            fast &= cell_samples_fast(tiles + 2 * kTileInts, cell, im.plane[2].overlap, v, tile_small);
+            if (fast && (tile_small || max(max(mag_bound<0>(y), mag_bound<0>(u)), mag_bound<0>(v)) < (1u << 28))) {
+                int32_t cadd[3], cshift[3];
+                uint8_t *plane[3];
 #pragma unroll
-                    for (int r = 0; r < 4; r++)
-                        store16(abase + r * rs, f16_widened((a[r * 4] + add) >> shift), f16_widened((a[r * 4 + 1] + add) >> shift),
-                                f16_widened((a[r * 4 + 2] + add) >> shift), f16_widened((a[r * 4 + 3] + add) >> shift));
+                for (int c = 0; c < 3; c++) {
+                    const int ch = (rgb_at >> (2 * c)) & 3;
+                    cadd[c] = o.ch[ch].shifted_bias + o.ch[ch].rounding;
+                    cshift[c] = o.ch[ch].shift;
+                    plane[c] = base + ch * ps;
                 }
-            }
-            if (lean) {
-                int32_t y[16], u[16], v[16];
-                bool fast = cell_samples_fast(tiles, cell, im.plane[0].overlap, y, tile_small);
-                fast &= cell_samples_fast(tiles + kTileInts, cell, im.plane[1].overlap, u, tile_small);
-                fast &= cell_samples_fast(tiles + 2 * kTileInts, cell, im.plane[2].overlap, v, tile_small);
-                if (fast && (tile_small || max(max(mag_bound<0>(y), mag_bound<0>(u)), mag_bound<0>(v)) < (1u << 28))) {
-                    int32_t cadd[3], cshift[3];
-                    uint8_t *plane[3];
 #pragma unroll
-                    for (int c = 0; c < 3; c++) {
-                        const int ch = (rgb_at >> (2 * c)) & 3;
-                        cadd[c] = o.ch[ch].shifted_bias + o.ch[ch].rounding;
-                        cshift[c] = o.ch[ch].shift;
-                        plane[c] = base + ch * ps;
+                for (int r = 0; r < 4; r++) {
+                    uint32_t q[3][4];
+#pragma unroll
+                    for (int c = 0; c < 4; c++) {
+                        const int k = r * 4 + c;
+                        int32_t R, G, B;
+                        yuv_to_rgb_fast(y[k], u[k], v[k], R, G, B);
+                        q[0][c] = f16_widened((R + cadd[0]) >> cshift[0]);
+                        q[1][c] = f16_widened((G + cadd[1]) >> cshift[1]);
+                        q[2][c] = f16_widened((B + cadd[2]) >> cshift[2]);
                     }
 #pragma unroll
-                    for (int r = 0; r < 4; r++) {
-                        uint32_t q[3][4];
-#pragma unroll
-                        for (int c = 0; c < 4; c++) {
-                            const int k = r * 4 + c;
-                            int32_t R, G, B;
-                            yuv_to_rgb_fast(y[k], u[k], v[k], R, G, B);
-                            q[0][c] = f16_widened((R + cadd[0]) >> cshift[0]);
-                            q[1][c] = f16_widened((G + cadd[1]) >> cshift[1]);
-                            q[2][c] = f16_widened((B + cadd[2]) >> cshift[2]);
-                        }
-#pragma unroll
-                        for (int c = 0; c < 3; c++) store16(plane[c] + r * rs, q[c][0], q[c][1], q[c][2], q[c][3]);
-                    }
-                    done = true;
+                    for (int c = 0; c < 3; c++) store16(plane[c] + r * rs, q[c][0], q[c][1], q[c][2], q[c][3]);
                 }
+                done = true;
             }
         }
         // any other output, cells that need the checked operator, or pixels at
