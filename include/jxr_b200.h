@@ -202,7 +202,8 @@ uint32_t jxrb_last_stage(void);
 jxrb_status jxrb_session_create(int ordinal, const jxrb_session_options *options, jxrb_session **out);
 /* CudaDecoderSession::system_default, session.rs:42-45: device 0, default options. */
 jxrb_status jxrb_session_create_default(jxrb_session **out);
-/* Drop of CudaDecoderSession: waits for pending work. */
+/* Drop of CudaDecoderSession: waits for pending work.  Submissions may be
+ * released after it; its images and resident sets go before it. */
 void jxrb_session_destroy(jxrb_session *session);
 /* CudaDecoderSession::buffer_pool_diagnostics / upload_cache_diagnostics, session.rs:250-268. */
 jxrb_status jxrb_session_diagnostics(const jxrb_session *session, jxrb_diagnostics *out);

@@ -1799,7 +1799,8 @@ __device__ __forceinline__ bool lean_rgb(const OutputDev &o, int colours, uint32
 // in registers, and no values kept across it (2500 x 1900 hard tiles 58.4 ->
 // 55.3 us, mixed batch 137.3 -> 135.5).  The interior kernels of up to three
 // planes keep that form for the usual outputs (4096 x 4096 RGB8 127.3 us, 133.5
-// this way: eight more loads and stores a plane) and come here with the rest.
+// this way: eight more loads and stores a plane); those of two and three come
+// here with the rest (one plane: luma_cell).
 // Returns the tile flags.
 template <int NP>
 __device__ __forceinline__ int cell_rows(const ImageDev &im, int32_t *tiles, int mx0, int my0, int gcx, int gcy, bool cut,

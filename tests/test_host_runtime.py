@@ -23,8 +23,9 @@ C_, D, S, L = J.COLOR, J.DEPTH, J.STORE, J.LAYOUT
 @pytest.fixture(scope="module")
 def fake_lib(tmp_path_factory):
     out = tmp_path_factory.mktemp("fake_cuda") / "libjxr_fake.so"
-    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-pthread", "-I", str(CUDA), "-I", str(ROOT / "include"),
-                    "-I", str(CSRC), str(CSRC / "host.cpp"), str(CSRC / "sample_scale.cpp"),
+    # its calls bind to the runtime built with it, not to one another library brought
+    subprocess.run(["g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-pthread", "-I", str(CUDA),
+                    "-I", str(ROOT / "include"), "-I", str(CSRC), str(CSRC / "host.cpp"), str(CSRC / "sample_scale.cpp"),
                     str(ROOT / "tests" / "_fake_cuda.cpp"), "-o", str(out)], check=True)
     lib = C.CDLL(str(out))
     for name, (res, args) in api.EXPORTS.items():
