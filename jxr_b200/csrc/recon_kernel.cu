@@ -3330,15 +3330,17 @@ static size_t interior_smem_bytes(int planes) {
 
 typedef void (*TileKernel)(const ImageDev *, const WorkItem *, uint32_t, uint32_t *, uint32_t *);
 
-// From this many tiles on, 4:2:0 interior tiles run four CTAs an SM instead of
-// three.  The fourth hides more of the latency of coefficients that come from
-// HBM, at 64 registers and spills that make each tile slower: pictures whose
-// coefficients stay in L2, or few tiles, lose by it.  One picture replayed, us
-// at three and four: 1920 x 1088 30.3, 39.3; 2048 x 1536 33.3, 45.8; 3072 x 2048
-// 54.3, 61.9; 4096 x 3072 102.2, 110.9.  Read from HBM: 2048 x 1536 48.6, 50.7;
-// 3840 x 2880 112.4, 109; 3999 x 2999 120, 116; 4096 x 3072 122, 120.  Pictures in
-// turn on several streams: 2501 x 1901 40.4, 42.6; 3999 x 2999 88.4, 85.0; a mixed
-// batch 128.4, 125.6.
+// In sets of this many tiles or more, 4:2:0 interior tiles run four CTAs an SM
+// instead of three.  The fourth hides more of the latency of coefficients that
+// come from HBM, at 64 registers and spills that make each tile slower: sets
+// whose coefficients stay in L2, or of few tiles, lose by it.  One picture
+// replayed, us at three and four: 1920 x 1088 30.3, 39.3; 2048 x 1536 33.3, 45.8;
+// 3072 x 2048 54.3, 61.9; 4096 x 3072 102.2, 110.9.  Read from HBM: 2048 x 1536
+// 48.6, 50.7; 3840 x 2880 112.4, 109; 3999 x 2999 120, 116; 4096 x 3072 122, 120.
+// Pictures in turn on several streams: 2501 x 1901 40.4, 42.6; 3999 x 2999 88.4,
+// 85.0.  The set's tiles of every kind count, since they share HBM and L2: mixed
+// batches in turn of 3491 tiles (2773 of them 4:2:0) 129.6, 126.5; 3002 (1739) 115.8,
+// 113.6; 3795 (2019) 148.8, 145.4.
 constexpr uint32_t kManyTiles = 2560;
 
 // Kernels by index: one a segment, then the 4:2:0 interior kernel of many tiles
@@ -3347,7 +3349,7 @@ constexpr int kKernelMany420 = kSegments, kKernelFolded3 = kSegments + 1;
 constexpr int kKernels = kSegments + 2;
 
 static_assert(kFoldAlways == 1u && kFoldSome == 4u, "interior kernels that take edge tiles too");
-// `folded`: the kinds whose edge tiles are folded.
+// `tiles`: the set's; `folded`: the kinds whose edge tiles are folded.
 static int kernel_of(int segment, uint32_t tiles, uint32_t folded) {
     if (segment == 4 && tiles >= kManyTiles) return kKernelMany420;
     return segment == 2 && (folded & kFoldSome) ? kKernelFolded3 : segment;
@@ -3440,12 +3442,14 @@ static cudaError_t kernel_fit(int index, int planes, size_t smem, int &sms, int 
 
 // Launch the work list's segments, each kernel on the next of `lanes` in turn.
 // `bounds` holds the kSegments + 1 segment boundaries, `folded` the kinds whose
-// edge tiles are folded; `counters` two words a segment.  The other and edge tiles come first, so that their short,
-// latency-bound launches start with the interior ones.
+// edge tiles are folded; `counters` two words a segment.  The other and edge
+// tiles come first, so that their short, latency-bound launches start with the
+// interior ones.
 cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32_t *bounds, uint32_t folded, int max_planes,
                          uint32_t *status, uint32_t *counters, const cudaStream_t *lanes, int lane_count,
                          const LaunchTuning *tune) {
     const WorkItem *list = static_cast<const WorkItem *>(items);
+    const uint32_t tiles = bounds[kSegments] - bounds[0];
     int lane = 0;
     for (int seg0 = 0; seg0 < kSegments; seg0++) {
         const int seg = seg0 == 0 ? kSegmentOther : seg0 <= kSegmentOther - kSideSegment0 ? kSideSegment0 + seg0 - 1
@@ -3456,7 +3460,7 @@ cudaError_t launch_tiles(const ImageDev *images, const void *items, const uint32
         const int slot = seg == kSegmentOther ? 4 : planes - 1;   // entry of the launch tuning
         uint32_t cap = tune ? tune->blocks_per_sm[slot] : 0;
         if (chroma_segment(seg) && cap >= kThreePlaneCtas) cap = 0;
-        const int index = kernel_of(seg, cap ? 0 : count, folded);   // capped, more CTAs an SM are no use
+        const int index = kernel_of(seg, cap ? 0 : tiles, folded);   // capped, more CTAs an SM are no use
         TileKernel k = tile_kernel(index);
         const size_t smem = segment_smem_bytes(seg, max_planes);
         int sms = 0, fit = 0;

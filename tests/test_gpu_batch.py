@@ -191,3 +191,22 @@ def test_many_tiles_of_a_kind(session, fmt, copies):
     for k in range(copies):
         assert np.array_equal(sub.readback(k), want), k
     sub.close()
+
+
+@pytest.mark.parametrize("copies", [25, 26])
+def test_many_tiles_of_a_set(session, copies):
+    """Either side of the number of tiles in a set, of any kind, from which the
+    4:2:0 kernel runs more CTAs an SM (100 of them in a picture of 640 x 640)."""
+    plans, wants = [], []
+    for kw in (dict(color_format=J.COLOR["YUV420"], quality=80, overlap=1), dict(color_format=J.COLOR["YUV422"], quality=80)):
+        img = J.synth(637, 640, tile_width=9, tile_height=7, seed=42, threads=8, **kw)
+        out = J.OutputFormat(J.COLOR["RGB"], J.DEPTH["U8"], J.STORE["U8"], J.LAYOUT["RGB"], 637, 640)
+        rc, want = decode_synth(img, out, threads=8)
+        assert rc == 0
+        plans.append(J.CudaDecodePlan(img.arena, img.geometry, out))
+        wants.append(want)
+    sub = session.submit_batch([plans[k % 2] for k in range(copies)])
+    sub.wait()
+    for k in range(copies):
+        assert np.array_equal(sub.readback(k), wants[k % 2]), k
+    sub.close()
