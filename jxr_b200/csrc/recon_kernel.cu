@@ -3612,12 +3612,16 @@ __global__ void __launch_bounds__(256) jxrb_quarter_first_level(const QuarterPla
 // The first-level overlap filter over a two-level plane's picture, one cell a
 // thread.  Full resolution: 4x4 cells at origins 2 (mod 4), disjoint, one
 // pass (phase 0); each sample lies in one cell, so a quarter's are scaled to
-// their levels as they are written.  Subsampled chroma: 2x2 cells at odd
-// origins in three ordered phases (corners lose their neighbour, squares and
-// pairs, corners regain it), the schedule of
+// their levels as they are written, unless jxrb_quarter_finish runs over all
+// the pictures anyway (`all_later`), a sample a thread: 16 divisions and their
+// terms' loads one after another in phase 0 then only add to the chain (eight
+// quarters of 256 x 256 4:2:0 submitted and waited for: 119 us, 106 this way,
+// 109 with a pass of its own for every level).  Subsampled chroma: 2x2 cells
+// at odd origins in three ordered phases (corners lose their neighbour, squares
+// and pairs, corners regain it), the schedule of
 // crates/jxr-native/src/reconstruct/subsampled_overlap.rs:244-296.
 __global__ void __launch_bounds__(256) jxrb_quarter_overlap(const QuarterPlane *__restrict__ planes, int phase,
-                                                            uint32_t *status) {
+                                                            bool all_later, uint32_t *status) {
     const QuarterPlane &p = planes[blockIdx.y];
     if (p.overlap != 2) return;
     const int W = (int)p.mbs_x * p.bc, H = (int)p.mbs_y * p.br;
@@ -3666,7 +3670,8 @@ __global__ void __launch_bounds__(256) jxrb_quarter_overlap(const QuarterPlane *
                 const int x = cx + 2 * (k & 1), y = cy + (k >> 1);
                 if (!inside(x, y)) continue;
                 int2 q = make_int2(v[2 * k], v[2 * k + 1]);
-                if (!p.sixteenth) q = make_int2(sample_level(p, q.x, x, y, lbad), sample_level(p, q.y, x + 1, y, lbad));
+                if (!p.sixteenth && !all_later)
+                    q = make_int2(sample_level(p, q.x, x, y, lbad), sample_level(p, q.y, x + 1, y, lbad));
                 *reinterpret_cast<int2 *>(&at(x, y)) = q;
             }
         }
@@ -3719,10 +3724,11 @@ __global__ void __launch_bounds__(256) jxrb_quarter_overlap(const QuarterPlane *
 // macroblock's filtered block values summed, row by row, checked, into the
 // macroblock picture (sum_macroblocks, pipeline.rs:421-457), and scaled.  A
 // subsampled quarter: its picture scaled (the overlap kernel's ordered corners
-// write some samples twice).
-__global__ void __launch_bounds__(256) jxrb_quarter_finish(const QuarterPlane *__restrict__ planes, uint32_t *status) {
+// write some samples twice); with `all_later` every other quarter's too.
+__global__ void __launch_bounds__(256) jxrb_quarter_finish(const QuarterPlane *__restrict__ planes, bool all_later,
+                                                           uint32_t *status) {
     const QuarterPlane &p = planes[blockIdx.y];
-    if (p.overlap != 2 || (!p.sixteenth && p.bc == 4)) return;
+    if (p.overlap != 2 || (!p.sixteenth && p.bc == 4 && !all_later)) return;
     const uint32_t pw = p.mbs_x * p.bc, W = p.sixteenth ? p.mbs_x : pw, n = W * (p.sixteenth ? p.mbs_y : p.mbs_y * p.br);
     bool bad = false;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -3787,10 +3793,10 @@ cudaError_t launch_quarter(const ImageDev *images, const QuarterImage *quarters,
         jxrb_quarter_first_level<<<dim3(blocks((uint64_t)max_mbs * 4), n), 256, 0, stream>>>(planes + base, status);
         for (int phase = 0; phase < (subsampled ? 3 : two_level ? 1 : 0); phase++)
             jxrb_quarter_overlap<<<dim3(blocks(max_samples / (subsampled ? 4 : 16) + 64), n), 256, 0, stream>>>(
-                planes + base, phase, status);
+                planes + base, phase, subsampled, status);
         if (finish)
-            jxrb_quarter_finish<<<dim3(blocks(subsampled ? max_samples : max_mbs), n), 256, 0, stream>>>(planes + base,
-                                                                                                    status);
+            jxrb_quarter_finish<<<dim3(blocks(subsampled ? max_samples : max_mbs), n), 256, 0, stream>>>(
+                planes + base, subsampled, status);
     }
     for (uint32_t base = 0; base < count; base += 65535) {
         const unsigned n = (unsigned)std::min<uint32_t>(count - base, 65535);

@@ -107,6 +107,20 @@ def test_reduced_and_full_requests_in_one_launch(session, images):
         assert rc == 0 and np.array_equal(g, ref)
 
 
+@pytest.mark.parametrize("beside", ["rgb420_o2_hard", "rgb422_o2", "rgb420_o1"])
+def test_two_level_quarters_beside_subsampled_ones(session, images, beside):
+    """The kernel that scales a two-level plane's samples depends on what else
+    is in the launch: beside subsampled two-level planes it is the last one."""
+    reqs, refs = [], []
+    for name, d in (("rgb444_o2_soft", 4), (beside, 4), ("rgba_o2", 4), ("rgb444_o2_hard", 16)):
+        img = images[name]
+        o = fmt(name, IMAGES[name]["width"], IMAGES[name]["height"])
+        reqs.append(session.upload(img.arena, img.geometry, img.alpha_arena).request(o, d))
+        refs.append(oracle_quarter(img, o, d))
+    for g, (rc, ref) in zip(run(session, reqs), refs):
+        assert rc == 0 and np.array_equal(g, ref)
+
+
 def test_quarter_needs_the_low_pass_band(session):
     img = J.synth(96, 80, content=J.CONTENT["RANDOM"], overlap=1, seed=5)
     assert (img.arena.bands == 0).any()
