@@ -2363,9 +2363,9 @@ __device__ void interior_tile(const ImageDev &im, int tx, int ty, int32_t *smem,
     }
     if (edge && edge_pixels<NP>(im, tiles, mx0, my0, ec)) bad |= kFlagOutput;
     // One closing barrier in the interior kernels of three and four planes, two
-    // more after a failure, which is rare (4096 x 4096 RGB8 124.1 us with three
-    // barriers, 121.1 this way; 3072 x 3072 half floats with alpha 121.2 and
-    // 120.0).  The edge and one-plane kernels keep the plain form: 2500 x 1900
+    // more after a failure, which is rare (4096 x 4096 RGB8 124.0 us with three
+    // barriers, 123.4 this way; 3072 x 3072 half floats with alpha 120.5 and
+    // 119.4).  The edge and one-plane kernels keep the plain form: 2500 x 1900
     // with hard tiles 54.7 us, 55.1 this way; 2047 x 1535 gray 12.1 and 12.5.
     constexpr bool kOneBarrier = NP >= 3 && MODE != 1;
     if constexpr (kOneBarrier) {
