@@ -178,6 +178,13 @@ constexpr uint32_t kApartTiles = 2560;
 // of 4:2:2 without overlap 36.6 us in two, 30.7 in one, 32.8 when the general
 // kernel took it).
 constexpr uint32_t kMergeTiles = 128, kMergeTilesSubsampled = 192;
+// Subsampled images with two overlap levels and hard tiles on one stream: with
+// fewer tiles than this beside those that only the general kernel takes, it
+// takes them all: their kernels would run before it, each with its own tail
+// (jxrb_decode_static, us in one kernel and in three, 256 x 256 hard tiles: 4:2:2
+// 777 x 601 93, 122; 2048 x 1536 223, 236; 2501 x 1901, 352 such tiles, 326, 339;
+// 3999 x 2999, 825 of them, 835, 815; 4:2:0 93, 122; 236, 245; 350, 351).
+constexpr uint32_t kGeneralTiles = 512;
 constexpr int kCounterWords = 2 * kSegments;   // two scheduling words a segment
 
 // Side streams a set's kernels may run on beside its own: with the set's

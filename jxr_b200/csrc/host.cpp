@@ -149,10 +149,13 @@ uint32_t tile_tag(uint32_t kind, uint32_t tx, uint32_t ty, uint32_t T, uint32_t 
 // Where a set's tiles run, by kind (bit kind - 1): whose edge tiles the
 // interior kernel takes (engine.h), and whose interior tiles the edge kernel
 // does: kinds of no more than kMergeTiles tiles (subsampled ones:
-// kMergeTilesSubsampled) for which both would run.
-// `count`: tiles by tag; `one_stream`: the kernels run one after another.
+// kMergeTilesSubsampled) for which both would run, and which kinds the general
+// kernel takes whole: subsampled ones, on one stream, of fewer than
+// kGeneralTiles tiles beside those that only it takes.
+// `count`: tiles by tag; `one_stream`: the kernels of one image run one after
+// another.
 struct TileRoutes {
-    uint32_t folded = 0, merged = 0;
+    uint32_t folded = 0, merged = 0, general = 0;
 };
 TileRoutes tile_routes(const uint32_t *count, bool one_stream) {
     TileRoutes r;
@@ -165,6 +168,7 @@ TileRoutes tile_routes(const uint32_t *count, bool one_stream) {
             edge = 0;
         }
         edge += hard;
+        if (one_stream && k >= kTag420 && count[0] > 0 && inner + edge < kGeneralTiles) r.general |= bit;
         const uint32_t most = k >= kTag420 ? kMergeTilesSubsampled : kMergeTiles;
         if (inner > 0 && edge > 0 && inner + edge <= most) r.merged |= bit;
     }
@@ -179,7 +183,7 @@ bool folded_edge_tag(uint32_t tag, const TileRoutes &r) {
 }
 // Work-list segment of a tag (engine.h).
 int segment_of_tag(uint32_t tag, const TileRoutes &r) {
-    if (tag == 0) return kSegmentOther;
+    if (tag == 0 || (r.general >> ((tag - 1) % kKinds)) & 1) return kSegmentOther;
     if (tag > kTagHard) return kSideSegment0 + (int)(tag - kTagHard) - 1;
     if (tag > kTagEdge) return folded_edge_tag(tag, r) ? (int)(tag - kTagEdge) - 1 : (int)tag - 1;
     return (r.merged >> (tag - 1)) & 1 ? kSideSegment0 + (int)tag - 1 : (int)tag - 1;
@@ -189,10 +193,11 @@ int segment_of_tag(uint32_t tag, const TileRoutes &r) {
 // one to place); `bounds` receives the kSegments + 1 segment boundaries.
 // Returns the kinds whose edge tiles are folded.  The places of the tags are
 // found once, not for each item: submitting 256 requests on pictures of 128 to
-// 4096 samples takes 560 to 630 us, 750 to 775 so.  The list is sorted into memory of its own, which the
-// set keeps: sorted straight into the blob, 12 threads' decodes of 777 x 601
-// 4:2:0 to host memory took 760 us a call instead of 560, the heap's top being
-// given back and taken again between them.
+// 4096 samples takes 560 to 630 us, 750 to 775 with two searches an item.  The
+// list is sorted into memory of its own, which the set keeps: sorted straight
+// into the blob, 12 threads' decodes of 777 x 601 4:2:0 to host memory took 760
+// us a call instead of 560, the heap's top being given back and taken again
+// between them.
 uint32_t order_by_segment(std::vector<WorkItemHost> &items, uint32_t *bounds) {
     uint32_t tags[kTags] = {};
     for (const WorkItemHost &w : items) tags[w.image >> kTagShift]++;

@@ -143,3 +143,18 @@ def test_plan_above_scratch_limit_is_refused(session):
         decode_static(plan, coeff)
     assert err.value.status == 10                       # JXRB_RESOURCE_LIMIT
     assert "4194304" in str(err.value)
+
+
+@pytest.mark.parametrize("side", [300, 1500, 1700])
+@pytest.mark.parametrize("fmt", ["YUV420", "YUV422"])
+def test_two_level_hard_tiles_of_subsampled_images(session, fmt, side):
+    """Either side of the number of other tiles (16, 484 and 625 here) up to which
+    the general kernel takes a two-level subsampled image with hard tiles whole."""
+    tile = 10 if side == 300 else 64
+    img = J.synth(side, side, color_format=C_[fmt], quality=75, overlap=2, tile_width=tile, tile_height=tile,
+                  hard_tiles=1, seed=76)
+    out = J.OutputFormat(C_["RGB"], D["U8"], S["U8"], L["RGB"], side, side)
+    rc, want = decode_synth(img, out, threads=os.cpu_count() or 1)
+    assert rc == 0
+    plan = J.CudaDecodePlan(img.arena, img.geometry, out)
+    assert np.array_equal(decode_static(plan, device_copy(img.arena.coefficients)), want)
